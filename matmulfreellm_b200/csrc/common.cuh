@@ -237,11 +237,12 @@ __device__ __forceinline__ int block_sum(int v, int* red) {
 // the exact arithmetic of the quantisation path (mirrored by the CPU oracle): every step is
 // a single IEEE round-to-nearest fp32 operation, never contracted into an fma.
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ float rstd_from_sumsq(double sumsq, int64_t K, float eps) {
-    // K a power of two (2048, 4096 ...): scaling by 2^-n is the exact quotient, without the ~100-instruction fp64 division
-    // that otherwise sits on the critical path of every row kernel of a decode step
-    const double q = (K & (K - 1)) == 0 ? sumsq * __longlong_as_double((1023ll - (long long)(__ffsll((long long)K) - 1)) << 52)
-                                        : sumsq / (double)K;
+// inv_k = 1.0 / K, which a kernel forms before it waits for its input.  The quotient is the product with it plus one correction
+// by the exact remainder (Markstein's division step): the fp64 division itself, about 100 instructions for a K that is not a
+// power of two, would sit on the critical path of every row.
+__device__ __forceinline__ float rstd_from_sumsq(double sumsq, int K, double inv_k, float eps) {
+    const double q0 = sumsq * inv_k;
+    const double q = fma(fma(-q0, (double)K, sumsq), inv_k, q0);
     const float mean = (float)q;
     return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
 }

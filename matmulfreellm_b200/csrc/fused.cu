@@ -19,6 +19,7 @@
 // shared memory BEFORE the grid-dependency wait (they do not depend on the preceding kernel), and
 // every block reduction costs a single __syncthreads.
 #include "common.cuh"
+#include "rowquant.cuh"
 
 namespace {
 
@@ -162,11 +163,15 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // BitLinear prologue on a register-resident row `v` (values already in T precision): shared sum of squares
 // `ss`, then per projection g: y = (v*rstd)*nw_g, absmax -> scale -> int8 codes, dq, rowsum.
 template <int V, int G, int P, int RT = FT>
-__device__ __forceinline__ void bitlinear_prologue(float (&v)[P], int D, double ss, float eps, const float* snw /* smem [G][D] */,
-                                                   int8_t* q, float* dq, int32_t* rowsum, int64_t M, int64_t m, RedScratch& red) {
-    double s1[1] = {ss};
-    block_sum_d<1, RT>(s1, red.d1);
-    const float rstd = rstd_from_sumsq(s1[0], D, eps);
+__device__ __forceinline__ void bitlinear_prologue(float (&v)[P], int D, double inv_d, double ss, float eps, const float* snw /* smem [G][D] */,
+                                                   int8_t* q, float* dq, int32_t* rowsum, int64_t M, int64_t m, RedScratch& red,
+                                                   bool norm = true) {
+    float rstd = 1.0f;          // without the norm: v * 1 * 1 is v itself
+    if (norm) {
+        double s1[1] = {ss};
+        block_sum_d<1, RT>(s1, red.d1);
+        rstd = rstd_from_sumsq(s1[0], D, inv_d, eps);
+    }
     float amax[G];
 #pragma unroll
     for (int g = 0; g < G; ++g) amax[g] = 0.0f;
@@ -238,23 +243,6 @@ __device__ __forceinline__ void bitlinear_prologue(float (&v)[P], int D, double 
     }
 }
 
-struct PrenormArgs {
-    const void* x; int64_t ld_x;
-    const void* res; int64_t ld_res;      // may be null
-    void* res_out;                         // [M, D] contiguous, may be null
-    void* y_out;                           // [M, D] contiguous: the normed row in T, may be null
-    const float* norm_w; float eps_norm;   // block-level RMSNorm
-    const float* nws[3]; float eps_bl;     // per-projection BitLinear norm weights
-    int8_t* q; float* dq; int32_t* rowsum; // [G][M][D], [G][M], [G][M]
-    int64_t M; int D; int G;
-    int round_sum_first;                   // 1: the reference added x+residual as a tensor op (rounded to T) before norm
-    int gsplit;                            // 1: grid.y = G CTAs per row, CTA y does projection y alone (decode-sized calls: the G
-                                           //    prologues of a row run side by side instead of one after the other)
-#ifdef MMF_EXPERIMENTS
-    long long* trace;                      // experiments build: 8 global-timer stamps of CTA 0 per launch (see mmf_row_trace)
-#endif
-};
-
 #ifdef MMF_EXPERIMENTS
 __device__ __forceinline__ long long row_now() {
     long long t;
@@ -290,6 +278,7 @@ prenorm_quant_kernel(PrenormArgs a) {
     stage_weights(sw, a.norm_w, D);
     for (int g = 0; g < Gs; ++g) stage_weights(sw + (1 + g) * D, a.nws[gy + g], D);
     ROW_TRACE(1);
+    const double inv_d = 1.0 / (double)D;
     pdl_wait();
     ROW_TRACE(2);
     __syncthreads();
@@ -350,7 +339,7 @@ prenorm_quant_kernel(PrenormArgs a) {
         ROW_TRACE(3);
         block_sum_d<1, RT>(ss, red.d0);
         ROW_TRACE(4);
-        const float rstd1 = rstd_from_sumsq(ss[0], D, a.eps_norm);
+        const float rstd1 = rstd_from_sumsq(ss[0], D, inv_d, a.eps_norm);
         T* yo = (a.y_out && gy == 0) ? reinterpret_cast<T*>(a.y_out) + m * (int64_t)D : nullptr;
         double ss2 = 0.0;
         ROW_FOREACH(V, D, it, c) {
@@ -372,10 +361,10 @@ prenorm_quant_kernel(PrenormArgs a) {
         }
         ROW_TRACE(5);
         if (a.gsplit)
-            bitlinear_prologue<V, 1, P, RT>(v, D, ss2, a.eps_bl, sw + D, a.q + (int64_t)gy * a.M * D, a.dq + (int64_t)gy * a.M,
+            bitlinear_prologue<V, 1, P, RT>(v, D, inv_d, ss2, a.eps_bl, sw + D, a.q + (int64_t)gy * a.M * D, a.dq + (int64_t)gy * a.M,
                                             a.rowsum + (int64_t)gy * a.M, a.M, m, red);
-        else if (a.G == 3) bitlinear_prologue<V, 3, P, RT>(v, D, ss2, a.eps_bl, sw + D, a.q, a.dq, a.rowsum, a.M, m, red);
-        else if (a.G == 1) bitlinear_prologue<V, 1, P, RT>(v, D, ss2, a.eps_bl, sw + D, a.q, a.dq, a.rowsum, a.M, m, red);
+        else if (a.G == 3) bitlinear_prologue<V, 3, P, RT>(v, D, inv_d, ss2, a.eps_bl, sw + D, a.q, a.dq, a.rowsum, a.M, m, red);
+        else if (a.G == 1) bitlinear_prologue<V, 1, P, RT>(v, D, inv_d, ss2, a.eps_bl, sw + D, a.q, a.dq, a.rowsum, a.M, m, red);
         ROW_TRACE(6);
     }
     ROW_TRACE(7);
@@ -383,12 +372,12 @@ prenorm_quant_kernel(PrenormArgs a) {
 
 // y = round_T( ((g*rstd)*w) * o * sigmoid(o) ), then BitLinear prologue.  `ov` holds the gate row o in registers.
 template <typename T, int V, int P, int RT = FT>
-__device__ __forceinline__ void gatenorm_tail(float (&gv)[P], const float (&ov)[P], double ssg, int D, float eps_g, float eps_bl,
+__device__ __forceinline__ void gatenorm_tail(float (&gv)[P], const float (&ov)[P], double ssg, int D, double inv_d, float eps_g, float eps_bl,
                                               const float* sw /* [2][D]: g_norm weight, BitLinear norm weight */, int8_t* q, float* dq,
                                               int32_t* rowsum, int64_t M, int64_t m, RedScratch& red) {
     double s0[1] = {ssg};
     block_sum_d<1, RT>(s0, red.d0);
-    const float rstd = rstd_from_sumsq(s0[0], D, eps_g);
+    const float rstd = rstd_from_sumsq(s0[0], D, inv_d, eps_g);
     double ss2 = 0.0;
     ROW_FOREACH(V, D, it, c) {
         float w[V], t[V];
@@ -408,7 +397,7 @@ __device__ __forceinline__ void gatenorm_tail(float (&gv)[P], const float (&ov)[
         for (int i = 0; i < V; ++i) gv[it * V + i] = t[i];
         sumsq_rounded<T, V>(t, bits, ss2);
     }
-    bitlinear_prologue<V, 1, P, RT>(gv, D, ss2, eps_bl, sw + D, q, dq, rowsum, M, m, red);
+    bitlinear_prologue<V, 1, P, RT>(gv, D, inv_d, ss2, eps_bl, sw + D, q, dq, rowsum, M, m, red);
 }
 
 template <typename T, int P, int LAT, int RT = FT>
@@ -425,6 +414,7 @@ gatenorm_quant_kernel(const T* __restrict__ gx, int64_t ld_g, const T* __restric
     pdl_trigger();
     stage_weights(sw, gw, D);
     stage_weights(sw + D, nw, D);
+    const double inv_d = 1.0 / (double)D;
     pdl_wait();
     __syncthreads();
     // Row loop (LAT = 0): next row by cp.async into thread-private slots, as in prenorm_quant_kernel
@@ -458,7 +448,54 @@ gatenorm_quant_kernel(const T* __restrict__ gx, int64_t ld_g, const T* __restric
             }
         }
         if (LAT == 0 && m + row_step < M) fetch(m + row_step);   // this thread's slots have just been read
-        gatenorm_tail<T, V, P, RT>(gv, ov, ss, D, eps_g, eps_bl, sw, q, dq, rowsum, M, m, red);
+        gatenorm_tail<T, V, P, RT>(gv, ov, ss, D, inv_d, eps_g, eps_bl, sw, q, dq, rowsum, M, m, red);
+    }
+}
+
+// BitLinear prologue alone (mmf_act_quant): RMSNorm + int8 quantisation of a given row.  Bound by memory on long batches
+// (one read of the row, one write of the codes).  The row stays in registers between its three passes and the rows of a
+// prompt go side by side through one CTA: 16384 rows of 5632 bf16 values took 211 us with the row parked in shared memory
+// as fp32 and one CTA per row (nine block-wide barriers and three shared-memory round trips per row).
+template <typename T, int P, int LAT, int RT = FT>
+__global__ void __launch_bounds__(FT, LAT)
+act_quant_regs_kernel(const T* __restrict__ x, int64_t ld, const float* __restrict__ nw, int use_norm, float eps,
+                      int8_t* __restrict__ q, float* __restrict__ dq, int32_t* __restrict__ rowsum, int64_t M, int D) {
+    extern __shared__ __align__(16) float sw[];
+    constexpr int RPC = FT / RT;                  // rows this CTA works on side by side
+    __shared__ RedScratch reds[RPC];
+    RedScratch& red = reds[threadIdx.x / RT];
+    const int rg = threadIdx.x / RT;
+    constexpr int V = 16 / sizeof(T);
+    pdl_trigger();
+    stage_weights(sw, use_norm ? nw : nullptr, D);
+    const double inv_d = 1.0 / (double)D;
+    pdl_wait();
+    __syncthreads();
+    T* sx = reinterpret_cast<T*>(sw + D) + (size_t)rg * D;   // row in flight (LAT = 0 only), as in prenorm_quant_kernel
+    auto fetch = [&](int64_t row) {
+        ROW_FOREACH(V, D, it, c) cp_async16(sx + c, x + row * ld + c);
+        cp_async_commit();
+    };
+    const int64_t row0 = (int64_t)blockIdx.x * RPC + rg, row_step = (int64_t)gridDim.x * RPC;
+    if (LAT == 0 && row0 < M) fetch(row0);
+    for (int64_t m = row0; m < M; m += row_step) {
+        const T* xr = LAT == 0 ? sx : x + m * ld;
+        if (LAT == 0) cp_async_wait_all();
+        float v[P];
+        double ss = 0.0;
+        ROW_FOREACH(V, D, it, c) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(xr + c);
+            const T* e = reinterpret_cast<const T*>(&raw);
+            float f[V];
+#pragma unroll
+            for (int i = 0; i < V; ++i) v[it * V + i] = f[i] = to_f32(e[i]);
+            uint32_t bits[V / 2];
+#pragma unroll
+            for (int i = 0; i < V / 2; ++i) bits[i] = reinterpret_cast<const uint32_t*>(&raw)[i];   // packed values (16-bit T)
+            sumsq_rounded<T, V>(f, bits, ss);
+        }
+        if (LAT == 0 && m + row_step < M) fetch(m + row_step);   // this thread's slots have just been read
+        bitlinear_prologue<V, 1, P, RT>(v, D, inv_d, ss, eps, sw, q, dq, rowsum, M, m, red, use_norm != 0);
     }
 }
 
@@ -481,6 +518,7 @@ decode_mix_kernel(const T* __restrict__ ifg, int64_t ld, const T* __restrict__ l
     // staged before the grid-dependency wait and must not be written by the kernels launched just before this one
     if (lb)
         for (int i = threadIdx.x; i < D; i += FT) sw[2 * D + i] = to_f32(lb[i]);
+    const double inv_d = 1.0 / (double)D;
     pdl_wait();
     __syncthreads();
     const int64_t m = blockIdx.x;
@@ -524,7 +562,7 @@ decode_mix_kernel(const T* __restrict__ ifg, int64_t ld, const T* __restrict__ l
             ss += (double)g8[i] * (double)g8[i];
         }
     }
-    gatenorm_tail<T, V, P>(gv, ov, ss, D, eps_g, eps_bl, sw, q, dq, rowsum, M, m, red);
+    gatenorm_tail<T, V, P>(gv, ov, ss, D, inv_d, eps_g, eps_bl, sw, q, dq, rowsum, M, m, red);
 }
 
 // z = round_T(silu(gate)*up), then BitLinear prologue.  gate/up are the two halves of a [M, 2D] tensor.
@@ -540,6 +578,7 @@ swiglu_quant_kernel(const T* __restrict__ gate, const T* __restrict__ up, int64_
     constexpr int V = 16 / sizeof(T);
     pdl_trigger();
     stage_weights(sw, nw, D);
+    const double inv_d = 1.0 / (double)D;
     pdl_wait();
     __syncthreads();
     // Row loop (LAT = 0): the next row of this CTA travels global -> shared memory by cp.async while the current one is
@@ -580,7 +619,7 @@ swiglu_quant_kernel(const T* __restrict__ gate, const T* __restrict__ up, int64_
             sumsq_rounded<T, V>(gv, bits, ss);
         }
         if (LAT == 0 && m + row_step < M) fetch(m + row_step);   // this thread's slots have just been read
-        bitlinear_prologue<V, 1, P, RT>(v, D, ss, eps_bl, sw, q, dq, rowsum, M, m, red);
+        bitlinear_prologue<V, 1, P, RT>(v, D, inv_d, ss, eps_bl, sw, q, dq, rowsum, M, m, red);
     }
 }
 
@@ -618,7 +657,8 @@ static inline unsigned row_grid(Kern kernel, size_t smem, int64_t M, int rows_pe
     const int64_t want = (M + rows_per_cta - 1) / rows_per_cta;
     return (unsigned)(want < cap ? want : cap);
 }
-// Prompt-sized calls (MMF_FOUR_ROWS_MIN_M rows and more): four rows per CTA with 64 threads each for rows of at most 2048
+// Prompt-sized calls (MMF_FOUR_ROWS_MIN_M rows and more) of fp32 rows, and of swiglu rows (16-bit rows of the other kernels take
+// rowwarp.cu): four rows per CTA with 64 threads each for rows of at most 2048
 // values, two rows with 128 threads each up to 4096 values.  A thread then holds up to 32 values of its row instead of
 // 8 - 16, so the reductions of a row (two fp64 sums, the absmax, the code sum: a fifth of all instructions at 8 values
 // per thread) cost a quarter (half) per value, and a row's threads meet at a barrier of 64 (128) instead of 256.
@@ -655,6 +695,29 @@ constexpr int64_t LAT_MAX_ROWS = MMF_LAT_MAX_ROWS;
 #define FUSED_SMEM_ATTR(kernel, smem) \
     if ((smem) + 2048 > 48 * 1024) MMF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem)))
 
+// rows per CTA by row length and count, as in mmf_prenorm_quant and mmf_swiglu_quant
+int act_quant_regs_launch(const void* x, int dtype, int64_t ld, const float* nw, int use_norm, float eps, int8_t* q, float* dq,
+                          int32_t* rowsum, int64_t M, int64_t D, cudaStream_t st) {
+#define ACT_QUANT_ROWS(P, LAT, RT)                                                                                              \
+    {                                                                                                                           \
+        constexpr int RPC = FT / (RT);                                                                                          \
+        const size_t smem = (size_t)D * sizeof(float) + (LAT ? 0 : (size_t)RPC * D * sizeof(T));   /* + row staging */           \
+        FUSED_SMEM_ATTR((act_quant_regs_kernel<T, P, LAT, RT>), smem);                                                          \
+        MMF_CUDA(mmf_launch_pdl(act_quant_regs_kernel<T, P, LAT, RT>, dim3(row_grid(act_quant_regs_kernel<T, P, LAT, RT>, smem, M, RPC)), \
+                                dim3(FT), smem, st, (const T*)x, ld, nw, use_norm, eps, q, dq, rowsum, M, (int)D));             \
+    }
+    if (row_warp_takes(M, D, dtype, ROW_WARP_MAX_D1)) return warp_act_quant_launch(x, dtype, ld, nw, use_norm, eps, q, dq, rowsum, M, D, st);
+    if (M >= MMF_FOUR_ROWS_MIN_M && D <= ROW_HALF * MAX_PER && dtype == MMF_F32) {
+        using T = float;
+        FUSED_DISPATCH_RT(D, RT, ACT_QUANT_ROWS(MAX_PER, 0, RT))
+    } else {
+        MMF_DISPATCH(dtype, T, { FUSED_DISPATCH_P(D, P, { FUSED_DISPATCH_LAT(M, LAT, ACT_QUANT_ROWS(P, LAT, FT)); }); });
+    }
+#undef ACT_QUANT_ROWS
+    MMF_LAUNCH_CHECK("act_quant_regs_kernel");
+    return MMF_OK;
+}
+
 #ifdef MMF_EXPERIMENTS
 static long long* g_row_trace = nullptr;
 // experiments build only: device buffer ([0] = launch counter, records of 8 stamps from word 8 on) or NULL to switch off
@@ -687,14 +750,16 @@ extern "C" int mmf_prenorm_quant(const void* x, int64_t ld_x, const void* residu
 #ifdef MMF_EXPERIMENTS
     a.trace = g_row_trace;
 #endif
-    if (M >= MMF_FOUR_ROWS_MIN_M && D <= ROW_HALF * MAX_PER && !a.gsplit) {
-        MMF_DISPATCH(dtype, T, { FUSED_DISPATCH_RT(D, RT, {
+    if (row_warp_takes(M, D, dtype, ROW_WARP_MAX_D)) return warp_prenorm_quant_launch(a, dtype, (cudaStream_t)stream);
+    if (M >= MMF_FOUR_ROWS_MIN_M && D <= ROW_HALF * MAX_PER && dtype == MMF_F32) {
+        using T = float;
+        { FUSED_DISPATCH_RT(D, RT, {
             constexpr int P = MAX_PER, RPC = FT / RT;
             const size_t smem = (size_t)(1 + groups) * D * sizeof(float) + (size_t)RPC * 2 * D * sizeof(T);   // + row staging
             FUSED_SMEM_ATTR((prenorm_quant_kernel<T, P, 0, RT>), smem);
             const dim3 grid(row_grid(prenorm_quant_kernel<T, P, 0, RT>, smem, M, RPC));
             MMF_CUDA(mmf_launch_pdl(prenorm_quant_kernel<T, P, 0, RT>, grid, dim3(FT), smem, (cudaStream_t)stream, a));
-        }); });
+        }); }
         MMF_LAUNCH_CHECK("prenorm_quant_kernel");
         return MMF_OK;
     }
@@ -720,15 +785,18 @@ extern "C" int mmf_gatenorm_quant(const void* g, int64_t ld_g, const void* o, in
                     mmf_aligned(gnorm_w, 16) && mmf_aligned(nw, 16),
                 MMF_ERR_ALIGN, "mmf_gatenorm_quant: rows and norm weights must be 16-byte aligned");
     if (M == 0) return MMF_OK;
-    if (M >= MMF_FOUR_ROWS_MIN_M && D <= ROW_HALF * MAX_PER) {
-        MMF_DISPATCH(dtype, T, { FUSED_DISPATCH_RT(D, RT, {
+    if (row_warp_takes(M, D, dtype, ROW_WARP_MAX_D))
+        return warp_gatenorm_quant_launch(g, ld_g, o, ld_o, dtype, gnorm_w, eps_g, nw, eps_bl, q, dq, rowsum, M, D, (cudaStream_t)stream);
+    if (M >= MMF_FOUR_ROWS_MIN_M && D <= ROW_HALF * MAX_PER && dtype == MMF_F32) {
+        using T = float;
+        { FUSED_DISPATCH_RT(D, RT, {
             constexpr int P = MAX_PER, RPC = FT / RT;
             const size_t smem = (size_t)2 * D * sizeof(float) + (size_t)RPC * 2 * D * sizeof(T);   // + row staging
             FUSED_SMEM_ATTR((gatenorm_quant_kernel<T, P, 0, RT>), smem);
             MMF_CUDA(mmf_launch_pdl(gatenorm_quant_kernel<T, P, 0, RT>, dim3(row_grid(gatenorm_quant_kernel<T, P, 0, RT>, smem, M, RPC)),
                                     dim3(FT), smem, (cudaStream_t)stream, (const T*)g, ld_g, (const T*)o, ld_o, gnorm_w, eps_g, nw, eps_bl, q, dq,
                                     rowsum, M, (int)D));
-        }); });
+        }); }
         MMF_LAUNCH_CHECK("gatenorm_quant_kernel");
         return MMF_OK;
     }

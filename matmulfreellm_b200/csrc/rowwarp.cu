@@ -1,0 +1,402 @@
+// Row-wise kernels of a prompt (many token rows, 16-bit activations): one WARP per row.
+//
+// The arithmetic is that of fused.cu (same rounding points, same operations, same bits); the layout is the one that long
+// batches want.  A warp holds its whole row in registers as packed 16-bit pairs (D / 64 registers per lane) and widens a
+// pair when it uses it, so that
+//   * a row's reductions are warp shuffles and redux instructions: no block barrier, no shared-memory round trip, and the
+//     per-row work every thread repeats (rstd, scales, the reductions themselves: about 200 instructions) is spread over
+//     64 - 176 values per lane instead of 32 - 44 (fused.cu's layouts);
+//   * the next row of the warp is on its way from memory (cp.async into slots that only this lane reads) while the current
+//     one is normalised and quantised.
+// Bound by memory on paper (one read of each input row, one write of each output row).  Measured at 32768 rows of 2048 bf16
+// values, before -> after: three-projection prenorm 162 -> 140 us (4.3 TB/s), one-projection prenorm 92 -> 84 us (5.6 TB/s), gate
+// norm 94 -> 79 us (4.2 TB/s); quantisation of 5632-value rows 386 -> 118 us (4.7 TB/s; it was the one-CTA-per-row kernel of
+// rowwise.cu), 14 instructions per value instead of 22.  What is left: shared-memory wavefronts (the norm weights are read in
+// every pass: pipe 61 - 80 % busy) and issue (2.5 per clock).
+#include "common.cuh"
+#include "rowquant.cuh"
+
+namespace {
+
+// Warps (= rows in flight) per CTA, one CTA per SM: the norm weights are staged once per SM and shared memory is left for the
+// rows.  24 warps at 80 registers were 8 % slower than 16 at 128 (2048-value rows) and leave a nearly empty last wave earlier.
+constexpr int WR_MAX_WARPS = 16;
+constexpr int V = 8;                          // values per 16-byte vector
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+template <typename T> __device__ __forceinline__ float2 widen(uint32_t u) {
+    if constexpr (cuda::std::is_same<T, __half>::value) return __half22float2(*reinterpret_cast<const __half2*>(&u));
+    else return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+}
+template <typename T> __device__ __forceinline__ uint32_t narrow(float2 v) {
+    if constexpr (cuda::std::is_same<T, __half>::value) {
+        const __half2 h = __floats2half2_rn(v.x, v.y);
+        return *reinterpret_cast<const uint32_t*>(&h);
+    } else {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
+        return *reinterpret_cast<const uint32_t*>(&h);
+    }
+}
+// s0 / s1 += squares of a packed pair (bf16: the fp64 operands are assembled from the bits, as sumsq_rounded does)
+template <typename T> __device__ __forceinline__ void sumsq_pair(uint32_t u, double& s0, double& s1) {
+    if constexpr (cuda::std::is_same<T, __half>::value) {
+        const float2 f = widen<T>(u);
+        s0 = fma((double)f.x, (double)f.x, s0);
+        s1 = fma((double)f.y, (double)f.y, s1);
+    } else {
+        const double d0 = __hiloint2double((int)(((u & 0x7fffu) << 13) + 0x38000000u), 0);
+        const double d1 = __hiloint2double((int)(((u >> 3) & 0x0fffe000u) + 0x38000000u), 0);
+        s0 = fma(d0, d0, s0);
+        s1 = fma(d1, d1, s1);
+    }
+}
+// Between two passes over a packed row: the compiler would keep the widened values of the first pass for the second, twice
+// as many registers as the packed row (at 22 vectors per lane it spilled 560 bytes), instead of widening again.
+template <int NV> __device__ __forceinline__ void forget_widened(uint32_t (&u)[NV][4]) {
+#pragma unroll
+    for (int it = 0; it < NV; ++it)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) asm volatile("" : "+r"(u[it][i]));
+}
+__device__ __forceinline__ float2 mul2(float2 a, float b) { return __fmul2_rn(a, make_float2(b, b)); }
+
+// vector `it` of a lane starts at column c = (it * 32 + lane) * 8.  NV is the even number of vectors per lane that holds a
+// row of D values, so only the last two vectors can lie (partly) past its end.
+#define WR_FOREACH(it, c) \
+    _Pragma("unroll") for (int it = 0, c = lane * V; it < NV; ++it, c += 32 * V) if (it < NV - 2 || c < D)
+
+__device__ __forceinline__ void lds8(const float* p, float2 (&w)[4]) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    w[0] = make_float2(a.x, a.y); w[1] = make_float2(a.z, a.w);
+    w[2] = make_float2(b.x, b.y); w[3] = make_float2(b.z, b.w);
+}
+__device__ __forceinline__ void stage(float* dst, const float* src, int n) {
+    for (int i = threadIdx.x * 4; i < n; i += blockDim.x * 4) {
+        float4 v = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        if (src) v = *reinterpret_cast<const float4*>(src + i);
+        *reinterpret_cast<float4*>(dst + i) = v;
+    }
+}
+
+// BitLinear prologue of the packed row u: y = (v * rstd) * w, absmax -> scale -> int8 codes, dq, code sum
+template <typename T, int NV>
+__device__ __forceinline__ void warp_quant(uint32_t (&u)[NV][4], int D, float rstd, const float* sw, int8_t* qr, float* dq,
+                                           int32_t* rowsum, int lane) {
+    float am0 = 0.0f, am1 = 0.0f;
+    forget_widened<NV>(u);
+    WR_FOREACH(it, c) {
+        float2 w[4];
+        lds8(sw + c, w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 y = __fmul2_rn(mul2(widen<T>(u[it][i]), rstd), w[i]);
+            am0 = fmaxf(am0, fabsf(y.x));
+            am1 = fmaxf(am1, fabsf(y.y));
+        }
+    }
+    // non-negative floats order like their bit patterns
+    const float a = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(am0, am1)))), 1e-5f);
+    const float s = __fdiv_rn(127.0f, a);
+    int lsum = 0;
+    forget_widened<NV>(u);
+    WR_FOREACH(it, c) {
+        float2 w[4];
+        lds8(sw + c, w);
+        uint32_t word[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            int iv[4];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float2 y = __fmul2_rn(mul2(widen<T>(u[it][2 * h + j]), rstd), w[2 * h + j]);
+                // |y * s| <= 127 (1 + 2^-23): no clamp; adding 1.5 * 2^23 leaves the code, rounded to nearest even, in the low
+                // byte.  Scalar on purpose: a packed multiply feeding a packed add can be merged into one rounding.
+                iv[2 * j] = __float_as_int(__fadd_rn(__fmul_rn(y.x, s), 12582912.0f));
+                iv[2 * j + 1] = __float_as_int(__fadd_rn(__fmul_rn(y.y, s), 12582912.0f));
+            }
+            word[h] = __byte_perm(__byte_perm(iv[0], iv[1], 0x0040), __byte_perm(iv[2], iv[3], 0x0040), 0x5410);
+            lsum = __dp4a((int)word[h], 0x01010101, lsum);
+        }
+        *reinterpret_cast<uint2*>(qr + c) = make_uint2(word[0], word[1]);
+    }
+    lsum = __reduce_add_sync(0xffffffffu, lsum);
+    if (lane == 0) {
+        *dq = __fdiv_rn(a, 127.0f);
+        *rowsum = lsum;
+    }
+}
+
+// ---- RMSNorm + quantisation of given rows (mmf_act_quant)
+template <typename T, int NV>
+__global__ void __launch_bounds__(WR_MAX_WARPS * 32, 1)
+warp_act_quant_kernel(const T* __restrict__ x, int64_t ld, const float* __restrict__ nw, int use_norm, float eps,
+                      int8_t* __restrict__ q, float* __restrict__ dq, int32_t* __restrict__ rowsum, int64_t M, int D) {
+    extern __shared__ __align__(16) float sw[];   // [D] norm weight, then per warp one row in flight
+    pdl_trigger();
+    stage(sw, use_norm ? nw : nullptr, D);
+    const double inv_d = 1.0 / (double)D;
+    pdl_wait();
+    __syncthreads();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    T* sx = reinterpret_cast<T*>(sw + D) + (size_t)wid * D;
+    auto fetch = [&](int64_t row) {
+        WR_FOREACH(it, c) cp_async16(sx + c, x + row * ld + c);
+        cp_async_commit();
+    };
+    const int64_t step = (int64_t)gridDim.x * (int)(blockDim.x >> 5);
+    int64_t m = (int64_t)blockIdx.x * (int)(blockDim.x >> 5) + wid;
+    if (m < M) fetch(m);
+    for (; m < M; m += step) {
+        cp_async_wait_all();
+        uint32_t u[NV][4] = {};
+        double s0 = 0.0, s1 = 0.0;
+        WR_FOREACH(it, c) {
+            const uint4 r = *reinterpret_cast<const uint4*>(sx + c);
+            u[it][0] = r.x; u[it][1] = r.y; u[it][2] = r.z; u[it][3] = r.w;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sumsq_pair<T>(u[it][i], s0, s1);
+        }
+        if (m + step < M) fetch(m + step);          // this lane's slots have just been read
+        const float rstd = use_norm ? rstd_from_sumsq(warp_sum(s0 + s1), D, inv_d, eps) : 1.0f;   // v * 1 * 1 is v itself
+        warp_quant<T, NV>(u, D, rstd, sw, q + m * (int64_t)D, dq + m, rowsum + m, lane);
+    }
+}
+
+// ---- [x + residual] -> residual_out; RMSNorm -> T; G BitLinear prologues
+template <typename T, int NV>
+__global__ void __launch_bounds__(WR_MAX_WARPS * 32, 1)
+warp_prenorm_quant_kernel(PrenormArgs a) {
+    extern __shared__ __align__(16) float sw[];   // [1 + G][D] norm weights, then per warp an x row and a residual row in flight
+    const int D = a.D;
+    pdl_trigger();
+    stage(sw, a.norm_w, D);
+    for (int g = 0; g < a.G; ++g) stage(sw + (1 + g) * D, a.nws[g], D);
+    const double inv_d = 1.0 / (double)D;
+    pdl_wait();
+    __syncthreads();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    T* sx = reinterpret_cast<T*>(sw + (1 + a.G) * D) + (size_t)wid * 2 * D;
+    T* sr = sx + D;
+    const T* x = reinterpret_cast<const T*>(a.x);
+    const T* res = reinterpret_cast<const T*>(a.res);
+    auto fetch = [&](int64_t row) {
+        WR_FOREACH(it, c) {
+            cp_async16(sx + c, x + row * a.ld_x + c);
+            if (res) cp_async16(sr + c, res + row * a.ld_res + c);
+        }
+        cp_async_commit();
+    };
+    const int64_t step = (int64_t)gridDim.x * (int)(blockDim.x >> 5);
+    int64_t m = (int64_t)blockIdx.x * (int)(blockDim.x >> 5) + wid;
+    if (m < a.M) fetch(m);
+    for (; m < a.M; m += step) {
+        cp_async_wait_all();
+        T* ro = a.res_out ? reinterpret_cast<T*>(a.res_out) + m * (int64_t)D : nullptr;
+        T* yo = a.y_out ? reinterpret_cast<T*>(a.y_out) + m * (int64_t)D : nullptr;
+        uint32_t u[NV][4] = {};
+        double s0 = 0.0, s1 = 0.0;
+        if (!res || a.round_sum_first) {              // what is normalised is a row of T values
+            WR_FOREACH(it, c) {
+                const uint4 r = *reinterpret_cast<const uint4*>(sx + c);
+                u[it][0] = r.x; u[it][1] = r.y; u[it][2] = r.z; u[it][3] = r.w;
+                if (res) {
+                    const uint4 q4 = *reinterpret_cast<const uint4*>(sr + c);
+                    const uint32_t b[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) u[it][i] = narrow<T>(__fadd2_rn(widen<T>(u[it][i]), widen<T>(b[i])));
+                }
+                if (ro) *reinterpret_cast<uint4*>(ro + c) = make_uint4(u[it][0], u[it][1], u[it][2], u[it][3]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sumsq_pair<T>(u[it][i], s0, s1);
+            }
+        } else {                                      // the fp32 sum is normalised: it is formed again from the two rows below
+            WR_FOREACH(it, c) {
+                const uint4 r = *reinterpret_cast<const uint4*>(sx + c);
+                const uint4 q4 = *reinterpret_cast<const uint4*>(sr + c);
+                const uint32_t xa[4] = {r.x, r.y, r.z, r.w}, xb[4] = {q4.x, q4.y, q4.z, q4.w};
+                uint32_t o[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 t = __fadd2_rn(widen<T>(xa[i]), widen<T>(xb[i]));
+                    s0 = fma((double)t.x, (double)t.x, s0);
+                    s1 = fma((double)t.y, (double)t.y, s1);
+                    o[i] = narrow<T>(t);
+                }
+                if (ro) *reinterpret_cast<uint4*>(ro + c) = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+        }
+        const float rstd1 = rstd_from_sumsq(warp_sum(s0 + s1), D, inv_d, a.eps_norm);
+        s0 = s1 = 0.0;
+        forget_widened<NV>(u);
+        if (!res || a.round_sum_first) {
+            WR_FOREACH(it, c) {
+                float2 w[4];
+                lds8(sw + c, w);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    u[it][i] = narrow<T>(__fmul2_rn(mul2(widen<T>(u[it][i]), rstd1), w[i]));
+                    sumsq_pair<T>(u[it][i], s0, s1);
+                }
+            }
+        } else {
+            WR_FOREACH(it, c) {
+                const uint4 r = *reinterpret_cast<const uint4*>(sx + c);
+                const uint4 q4 = *reinterpret_cast<const uint4*>(sr + c);
+                const uint32_t xa[4] = {r.x, r.y, r.z, r.w}, xb[4] = {q4.x, q4.y, q4.z, q4.w};
+                float2 w[4];
+                lds8(sw + c, w);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    u[it][i] = narrow<T>(__fmul2_rn(mul2(__fadd2_rn(widen<T>(xa[i]), widen<T>(xb[i])), rstd1), w[i]));
+                    sumsq_pair<T>(u[it][i], s0, s1);
+                }
+            }
+        }
+        if (m + step < a.M) fetch(m + step);          // this lane's slots have been read for the last time
+        if (yo) {
+            WR_FOREACH(it, c) *reinterpret_cast<uint4*>(yo + c) = make_uint4(u[it][0], u[it][1], u[it][2], u[it][3]);
+        }
+        if (a.G == 0) continue;
+        const float rstd2 = rstd_from_sumsq(warp_sum(s0 + s1), D, inv_d, a.eps_bl);
+        for (int g = 0; g < a.G; ++g) {
+            const int64_t gm = (int64_t)g * a.M + m;
+            warp_quant<T, NV>(u, D, rstd2, sw + (1 + g) * D, a.q + gm * D, a.dq + gm, a.rowsum + gm, lane);
+        }
+    }
+}
+
+// ---- RMSNorm(g) * w * o * sigmoid(o) -> T; BitLinear prologue
+template <typename T, int NV>
+__global__ void __launch_bounds__(WR_MAX_WARPS * 32, 1)
+warp_gatenorm_quant_kernel(const T* __restrict__ gx, int64_t ld_g, const T* __restrict__ o, int64_t ld_o,
+                           const float* __restrict__ gw, float eps_g, const float* __restrict__ nw, float eps_bl,
+                           int8_t* __restrict__ q, float* __restrict__ dq, int32_t* __restrict__ rowsum, int64_t M, int D) {
+    extern __shared__ __align__(16) float sw[];   // [2][D] norm weights, then per warp a g row and an o row in flight
+    pdl_trigger();
+    stage(sw, gw, D);
+    stage(sw + D, nw, D);
+    const double inv_d = 1.0 / (double)D;
+    pdl_wait();
+    __syncthreads();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    T* sg = reinterpret_cast<T*>(sw + 2 * D) + (size_t)wid * 2 * D;
+    T* so = sg + D;
+    auto fetch = [&](int64_t row) {
+        WR_FOREACH(it, c) {
+            cp_async16(sg + c, gx + row * ld_g + c);
+            cp_async16(so + c, o + row * ld_o + c);
+        }
+        cp_async_commit();
+    };
+    const int64_t step = (int64_t)gridDim.x * (int)(blockDim.x >> 5);
+    int64_t m = (int64_t)blockIdx.x * (int)(blockDim.x >> 5) + wid;
+    if (m < M) fetch(m);
+    for (; m < M; m += step) {
+        cp_async_wait_all();
+        uint32_t u[NV][4] = {};
+        double s0 = 0.0, s1 = 0.0;
+        WR_FOREACH(it, c) {
+            const uint4 r = *reinterpret_cast<const uint4*>(sg + c);
+            u[it][0] = r.x; u[it][1] = r.y; u[it][2] = r.z; u[it][3] = r.w;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sumsq_pair<T>(u[it][i], s0, s1);
+        }
+        const float rstd1 = rstd_from_sumsq(warp_sum(s0 + s1), D, inv_d, eps_g);
+        s0 = s1 = 0.0;
+        forget_widened<NV>(u);
+        WR_FOREACH(it, c) {
+            const uint4 r = *reinterpret_cast<const uint4*>(so + c);
+            const uint32_t ob[4] = {r.x, r.y, r.z, r.w};
+            float2 w[4];
+            lds8(sw + c, w);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 ov = widen<T>(ob[i]);
+                const float2 y = __fmul2_rn(mul2(widen<T>(u[it][i]), rstd1), w[i]);
+                u[it][i] = narrow<T>(__fmul2_rn(__fmul2_rn(y, ov), sigmoid2(ov)));
+                sumsq_pair<T>(u[it][i], s0, s1);
+            }
+        }
+        if (m + step < M) fetch(m + step);            // this lane's slots have been read for the last time
+        const float rstd2 = rstd_from_sumsq(warp_sum(s0 + s1), D, inv_d, eps_bl);
+        warp_quant<T, NV>(u, D, rstd2, sw + D, q + m * (int64_t)D, dq + m, rowsum + m, lane);
+    }
+}
+
+// One CTA per SM with up to WR_MAX_WARPS warps, as shared memory (weight_bytes once, row_bytes per warp)
+// allows, fewer when the rows are few: they are then spread over all SMs.
+template <auto kernel, typename... Args>
+int wr_launch(size_t weight_bytes, size_t row_bytes, int64_t M, cudaStream_t st, const char* name, Args... args) {
+    constexpr size_t SMEM_MAX = 227 * 1024;
+    // dynamic shared memory beyond 48 KB is switched on once per kernel, device and host thread, to the limit
+    thread_local uint64_t enabled = 0;
+    int dev = 0;
+    MMF_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !(enabled >> dev & 1)) {
+        MMF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+        if (dev < 64) enabled |= 1ull << dev;
+    }
+    const int64_t fit = (int64_t)((SMEM_MAX - weight_bytes) / row_bytes), share = (M + 147) / 148;
+    int64_t warps = fit < WR_MAX_WARPS ? fit : WR_MAX_WARPS;
+    if (share < warps) warps = share;
+    MMF_REQUIRE(warps >= 1, MMF_ERR_CUDA, "%s: a row of this length does not fit in shared memory", name);
+    const int64_t want = (M + warps - 1) / warps;
+    MMF_CUDA(mmf_launch_pdl(kernel, dim3((unsigned)(want < 148 ? want : 148)), dim3((unsigned)warps * 32), weight_bytes + (size_t)warps * row_bytes,
+                            st, args...));
+    MMF_LAUNCH_CHECK(name);
+    return MMF_OK;
+}
+
+// run `...` with NV bound to the even number of 256-value vectors per lane that holds a row of D values (D <= 256 * MAXNV)
+#define WR_CASE(N, ...) case N: { constexpr int NV = N; __VA_ARGS__; break; }
+#define WR_DISPATCH16(D, ...)                                                                                       \
+    switch ((((int)(D) + 511) / 512) * 2) {                                                                          \
+        WR_CASE(2, __VA_ARGS__) WR_CASE(4, __VA_ARGS__) WR_CASE(6, __VA_ARGS__) WR_CASE(8, __VA_ARGS__)               \
+        WR_CASE(10, __VA_ARGS__) WR_CASE(12, __VA_ARGS__) WR_CASE(14, __VA_ARGS__) default: { constexpr int NV = 16; __VA_ARGS__; } \
+    }
+#define WR_DISPATCH28(D, ...)                                                                                       \
+    switch ((((int)(D) + 511) / 512) * 2) {                                                                          \
+        WR_CASE(2, __VA_ARGS__) WR_CASE(4, __VA_ARGS__) WR_CASE(6, __VA_ARGS__) WR_CASE(8, __VA_ARGS__)               \
+        WR_CASE(10, __VA_ARGS__) WR_CASE(12, __VA_ARGS__) WR_CASE(14, __VA_ARGS__) WR_CASE(16, __VA_ARGS__)           \
+        WR_CASE(18, __VA_ARGS__) WR_CASE(20, __VA_ARGS__) WR_CASE(22, __VA_ARGS__) WR_CASE(24, __VA_ARGS__)           \
+        WR_CASE(26, __VA_ARGS__) default: { constexpr int NV = 28; __VA_ARGS__; }                                    \
+    }
+#define WR_DISPATCH_T(dtype, T, ...)                                              \
+    if ((dtype) == MMF_BF16) { using T = __nv_bfloat16; __VA_ARGS__; }            \
+    else { using T = __half; __VA_ARGS__; }
+
+}  // namespace
+
+bool row_warp_takes(int64_t M, int64_t D, int dtype, int64_t max_d) { return M >= ROW_WARP_MIN_M && D <= max_d && dtype != MMF_F32; }
+
+int warp_act_quant_launch(const void* x, int dtype, int64_t ld, const float* nw, int use_norm, float eps, int8_t* q, float* dq,
+                          int32_t* rowsum, int64_t M, int64_t D, cudaStream_t st) {
+    WR_DISPATCH_T(dtype, T, {
+        WR_DISPATCH28(D, { return wr_launch<warp_act_quant_kernel<T, NV>>((size_t)D * 4, (size_t)D * 2, M, st, "warp_act_quant_kernel",
+                                                          (const T*)x, ld, nw, use_norm, eps, q, dq, rowsum, M, (int)D); });
+    });
+    return MMF_OK;
+}
+
+int warp_prenorm_quant_launch(const PrenormArgs& a, int dtype, cudaStream_t st) {
+    WR_DISPATCH_T(dtype, T, {
+        WR_DISPATCH16(a.D, { return wr_launch<warp_prenorm_quant_kernel<T, NV>>((size_t)(1 + a.G) * a.D * 4, (size_t)a.D * 4, a.M, st,
+                                                               "warp_prenorm_quant_kernel", a); });
+    });
+    return MMF_OK;
+}
+
+int warp_gatenorm_quant_launch(const void* g, int64_t ld_g, const void* o, int64_t ld_o, int dtype, const float* gw, float eps_g,
+                               const float* nw, float eps_bl, int8_t* q, float* dq, int32_t* rowsum, int64_t M, int64_t D, cudaStream_t st) {
+    WR_DISPATCH_T(dtype, T, {
+        WR_DISPATCH16(D, { return wr_launch<warp_gatenorm_quant_kernel<T, NV>>((size_t)D * 8, (size_t)D * 4, M, st,
+                                                               "warp_gatenorm_quant_kernel", (const T*)g, ld_g, (const T*)o, ld_o,
+                                                               gw, eps_g, nw, eps_bl, q, dq, rowsum, M, (int)D); });
+    });
+    return MMF_OK;
+}

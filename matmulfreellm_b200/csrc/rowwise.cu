@@ -5,6 +5,7 @@
 // row cached in shared memory as fp32 between the statistics pass and the output pass so
 // that every input byte is read from HBM once.
 #include "common.cuh"
+#include "rowquant.cuh"
 
 namespace {
 
@@ -29,7 +30,7 @@ __device__ __forceinline__ void store_n(T* p, const float (&in)[V]) {
 }
 
 // -----------------------------------------------------------------------------------------
-// RMSNorm + activation quantisation
+// RMSNorm + activation quantisation of rows too long for the register-resident kernel (act_quant_regs_launch)
 // -----------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(ROW_THREADS)
@@ -57,7 +58,7 @@ act_quant_kernel(const T* __restrict__ x, int64_t ld_x, const float* __restrict_
         }
     }
     float rstd = 1.0f;
-    if (use_norm) rstd = rstd_from_sumsq(block_sum(ss, redd), K, eps);
+    if (use_norm) rstd = rstd_from_sumsq(block_sum(ss, redd), K, 1.0 / (double)K, eps);
 
     float amax = 0.0f;
     for (int c = threadIdx.x * V; c < K; c += ROW_THREADS * V) {
@@ -143,7 +144,7 @@ rmsnorm_kernel(const T* __restrict__ x, const R* __restrict__ res, const float* 
             ss += (double)v[i] * (double)v[i];
         }
     }
-    const float rstd = rstd_from_sumsq(block_sum(ss, redd), D, eps);
+    const float rstd = rstd_from_sumsq(block_sum(ss, redd), D, 1.0 / (double)D, eps);
     T* yr = y + m * (int64_t)D;
     for (int c = threadIdx.x * V; c < D; c += ROW_THREADS * V) {
         float o[V];
@@ -179,7 +180,7 @@ swishgate_kernel(const T* __restrict__ x, const T* __restrict__ o, const float* 
             ss += (double)v[i] * (double)v[i];
         }
     }
-    const float rstd = rstd_from_sumsq(block_sum(ss, redd), D, eps);
+    const float rstd = rstd_from_sumsq(block_sum(ss, redd), D, 1.0 / (double)D, eps);
     T* yr = y + m * (int64_t)D;
     for (int c = threadIdx.x * V; c < D; c += ROW_THREADS * V) {
         float g[V], out[V];
@@ -339,6 +340,219 @@ sample_top_p_kernel(const T* __restrict__ logits, int64_t ld, int V, float inv_t
     }
 }
 
+// The same selection for rows whose probabilities fit in shared memory (V <= SAMPLE_MAX_V).  Bound by latency: one CTA per
+// row, a chain of block-wide fp64 sums.  So logits are read and exponentiated once; a coarse threshold (2^-6, 2^-12, 2^-24, 0)
+// that keeps enough mass is looked for first, usually one or two sums over all tokens; only the tokens above it, some
+// hundreds as a rule, are then searched for tau, four ways at a time, by eight warps (all of them when the candidates are many).  At [8, 32000] bf16 the kernel above,
+// which re-reads the logits and re-evaluates expf in each of its 33 passes, takes 277 us.
+constexpr int SAMPLE_THREADS = 1024, SAMPLE_LIST = 8192, SAMPLE_MAX_V = 40960;
+template <typename T>
+__global__ void __launch_bounds__(SAMPLE_THREADS, 1)
+sample_top_p_smem_kernel(const T* __restrict__ logits, int64_t ld, int V, float inv_temp, float top_p,
+                         const float* __restrict__ uniforms, int64_t* __restrict__ out, int vec) {
+    pdl_trigger();
+    pdl_wait();
+    constexpr int W = SAMPLE_THREADS / 32, VL = 16 / sizeof(T);
+    extern __shared__ __align__(16) float p[];          // [V] probabilities (unnormalised)
+    float* list = p + ((V + 3) & ~3);                   // [SAMPLE_LIST] candidates for tau
+    __shared__ double s_sum[2][W];
+    __shared__ double s_three[2][3][W];
+    __shared__ float s_max[W];
+    __shared__ int s_cnt[W];
+    __shared__ uint32_t s_tau;
+    __shared__ int s_range, s_group, s_found;
+    __shared__ double s_before;
+    const T* r = logits + blockIdx.x * ld;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    float mx = -INFINITY;
+    if (vec) {
+        for (int c = tid * VL; c < V; c += SAMPLE_THREADS * VL) {
+            float v[VL];
+            load16<T>(r + c, v);
+#pragma unroll
+            for (int i = 0; i < VL; ++i) {
+                v[i] = __fmul_rn(v[i], inv_temp);
+                mx = fmaxf(mx, v[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < VL; i += 4) *reinterpret_cast<float4*>(p + c + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        }
+    } else {
+        for (int c = tid; c < V; c += SAMPLE_THREADS) {
+            const float v = __fmul_rn(to_f32(r[c]), inv_temp);
+            p[c] = v;
+            mx = fmaxf(mx, v);
+        }
+    }
+    mx = warp_max(mx);
+    if (lane == 0) s_max[wid] = mx;
+    if (tid == 0) s_found = 0x7fffffff;
+    __syncthreads();
+    mx = warp_max(s_max[lane]);
+    // fp64 value of a non-negative normal float from its bits (an fp32 -> fp64 conversion runs at 16 per clock and SM); zero and
+    // subnormal probabilities read as at most 2^-126, which no sum near the nucleus' mass can see
+    auto widen = [](float v) {
+        const uint32_t b = __float_as_uint(v);
+        return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+    };
+    // a block-wide sum costs one barrier: the slots alternate, and the same butterfly in every warp gives every thread the same bits
+    int flip = 0;
+    auto block_total = [&](double a) {
+        a = warp_sum(a);
+        if (lane == 0) s_sum[flip][wid] = a;
+        __syncthreads();
+        const double t = warp_sum(s_sum[flip][lane]);
+        flip ^= 1;
+        return t;
+    };
+    double sum = 0.0;
+    for (int c = tid; c < V; c += SAMPLE_THREADS) {
+        const float e = expf(__fsub_rn(p[c], mx));
+        p[c] = e;
+        sum += widen(e);
+    }
+    const double total = block_total(sum);
+    const double want = (double)top_p * total;
+    // coarse threshold: the largest of the ladder whose tokens hold the wanted mass (0 always does)
+    float floor_p = 0.0f;
+    for (int k = 0; k < 3; ++k) {
+        const float t = k == 0 ? 0.015625f : k == 1 ? 0.000244140625f : 5.9604644775390625e-8f;
+        double a = 0.0;
+        for (int c = tid; c < V; c += SAMPLE_THREADS) {
+            const float e = p[c];
+            if (e >= t) a += widen(e);
+        }
+        if (block_total(a) >= want) { floor_p = t; break; }              // uniform over the block
+    }
+    // candidates: how many per thread, where they go (scan over the block), then the list itself (its order does not matter:
+    // sums of the same values in another order differ below the 53rd bit)
+    int mine = 0;
+    for (int c = tid; c < V; c += SAMPLE_THREADS) mine += p[c] >= floor_p;
+    int at = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int n = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += n;
+    }
+    if (lane == 31) s_cnt[wid] = at;
+    __syncthreads();
+    const int wcnt = s_cnt[lane];
+    int count = __reduce_add_sync(0xffffffffu, wcnt);
+    at += __reduce_add_sync(0xffffffffu, lane < wid ? wcnt : 0) - mine;
+    const float* cand = list;
+    if (count <= SAMPLE_LIST) {
+        for (int c = tid; c < V; c += SAMPLE_THREADS)
+            if (p[c] >= floor_p) list[at++] = p[c];
+    } else {                                            // a flat distribution: search all tokens
+        cand = p;
+        count = V;
+    }
+    __syncthreads();
+    // tau on the float's bits: mass_ge(lo) >= want > mass_ge(hi), three thresholds between them per round
+    const int search_warps = count > 4096 ? W : 8;
+    if (wid < search_warps) {
+        uint32_t lo = __float_as_uint(floor_p), hi = __float_as_uint(1.0f) + 1u;   // p <= 1, and the most probable token is 1
+        int f = 0;
+        while (hi - lo > 1u) {
+            const uint32_t q = (hi - lo + 3u) / 4u;     // lo < t0 <= t1 <= t2 < hi (clipped where fewer than four steps are left)
+            const uint32_t t0 = lo + q, t1 = min(lo + 2u * q, hi - 1u), t2 = min(lo + 3u * q, hi - 1u);
+            const float f0 = __uint_as_float(t0), f1 = __uint_as_float(t1), f2 = __uint_as_float(t2);
+            double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+            for (int k = tid; k < count; k += search_warps * 32) {
+                const float e = cand[k];
+                const double d = widen(e);
+                if (e >= f0) a0 += d;
+                if (e >= f1) a1 += d;
+                if (e >= f2) a2 += d;
+            }
+            a0 = warp_sum(a0); a1 = warp_sum(a1); a2 = warp_sum(a2);
+            if (lane == 0) { s_three[f][0][wid] = a0; s_three[f][1][wid] = a1; s_three[f][2][wid] = a2; }
+            asm volatile("bar.sync 1, %0;" ::"r"(search_warps * 32) : "memory");
+            const bool in = lane < search_warps;
+            a0 = warp_sum(in ? s_three[f][0][lane] : 0.0);
+            a1 = warp_sum(in ? s_three[f][1][lane] : 0.0);
+            a2 = warp_sum(in ? s_three[f][2][lane] : 0.0);
+            f ^= 1;
+            if (a2 >= want) lo = t2;
+            else if (a1 >= want) { lo = t1; hi = t2; }
+            else if (a0 >= want) { lo = t0; hi = t1; }
+            else hi = t0;
+        }
+        if (tid == 0) s_tau = lo;
+    }
+    __syncthreads();
+    const float tau = __uint_as_float(s_tau);
+    // the draw, in token order: warp w holds the kept mass of tokens [w * R, (w + 1) * R); the range that contains the target is
+    // then cut into 32 groups, one per warp, and the group that contains it into tokens
+    const int R = ((V + W - 1) / W + 31) & ~31, GR = R / 32;
+    double a = 0.0;
+    for (int c = wid * R + lane; c < min(V, (wid + 1) * R); c += 32)
+        if (p[c] >= tau) a += widen(p[c]);
+    const double kept = block_total(a);
+    const double target = (double)uniforms[blockIdx.x] * kept;
+    // inclusive scan over the lanes and the lane whose half-open interval holds the target (-1: none, the last one was rounded shut)
+    auto locate = [&](double v, double base, double& before) {
+        double s = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double n = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += n;
+        }
+        double prev = __shfl_up_sync(0xffffffffu, s, 1);
+        if (lane == 0) prev = 0.0;
+        const unsigned hit = __ballot_sync(0xffffffffu, v > 0.0 && base + s > target);
+        if (!hit) return -1;
+        const int who = __ffs(hit) - 1;
+        before = base + __shfl_sync(0xffffffffu, prev, who);
+        return who;
+    };
+    if (wid == 0) {
+        double before = 0.0;
+        const int who = locate(s_sum[flip ^ 1][lane], 0.0, before);
+        if (lane == 0) { s_range = who; s_before = before; }
+    }
+    __syncthreads();
+    const int range = s_range;
+    const double before0 = s_before;
+    if (range >= 0) {                                   // uniform over the block
+        double g = 0.0;
+        const int g0 = range * R + wid * GR;
+        for (int c = g0 + lane; c < min(V, g0 + GR); c += 32)
+            if (p[c] >= tau) g += widen(p[c]);
+        g = warp_sum(g);
+        if (lane == 0) s_sum[flip][wid] = g;
+        __syncthreads();
+        if (wid == 0) {
+            double before = before0;
+            const int who = locate(s_sum[flip][lane], before0, before);
+            if (who >= 0)
+                for (int c0 = range * R + who * GR; c0 < min(V, range * R + (who + 1) * GR); c0 += 32) {
+                    const int c = c0 + lane;
+                    const double v = c < min(V, range * R + (who + 1) * GR) && p[c] >= tau ? widen(p[c]) : 0.0;
+                    double b2 = before;
+                    const int tok = locate(v, before, b2);
+                    if (tok >= 0) {
+                        if (lane == 0) s_found = c0 + tok;
+                        break;
+                    }
+                    before += warp_sum(v);
+                }
+        }
+    }
+    __syncthreads();
+    int found = s_found;
+    if (found == 0x7fffffff) {                          // rounding left the last interval open at its end: the last kept token
+        int last = -1;
+        for (int c = tid; c < V; c += SAMPLE_THREADS)
+            if (p[c] >= tau) last = c;
+        last = __reduce_max_sync(0xffffffffu, last);
+        if (lane == 0) s_cnt[wid] = last;
+        __syncthreads();
+        found = max(__reduce_max_sync(0xffffffffu, s_cnt[lane]), 0);
+    }
+    if (tid == 0) out[blockIdx.x] = found;
+}
+
 __global__ void __launch_bounds__(128)
 embedding_kernel(const uint8_t* __restrict__ table, int64_t V, int64_t row_bytes,
                  const int64_t* __restrict__ ids, uint8_t* __restrict__ out, int vec16) {
@@ -374,6 +588,7 @@ extern "C" int mmf_act_quant(const void* x, int dtype, int64_t ld_x, const float
                 MMF_ERR_ALIGN, "mmf_act_quant: x rows and q must be 16-byte aligned");
     if (M == 0) return MMF_OK;
     cudaStream_t st = (cudaStream_t)stream;
+    if (K <= ACT_QUANT_REGS_MAX_K && mmf_aligned(norm_w, 16)) return act_quant_regs_launch(x, dtype, ld_x, norm_w, use_norm, eps, q, dq, rowsum, M, K, st);
     const size_t smem = (size_t)K * sizeof(float);
     MMF_DISPATCH(dtype, T, {
         if (smem > 48 * 1024)
@@ -514,9 +729,19 @@ extern "C" int mmf_sample_top_p(const void* logits, int dtype, int64_t ld, float
     MMF_REQUIRE(temperature > 0.0f && top_p >= 0.0f, MMF_ERR_BAD_ARG, "mmf_sample_top_p: need temperature > 0 and top_p >= 0");
     if (M == 0) return MMF_OK;
     const float inv_temp = 1.0f / temperature;
+    const float top = top_p < 1.0f ? top_p : 1.0f;
+    // rows of more than SAMPLE_MAX_V tokens do not fit in shared memory beside the candidate list
+    const int vec = mmf_aligned(logits, 16) && (ld * mmf_dtype_size(dtype)) % 16 == 0 && V % (16 / mmf_dtype_size(dtype)) == 0;
+    const size_t smem = ((size_t)((V + 3) & ~3ll) + SAMPLE_LIST) * sizeof(float);
     MMF_DISPATCH(dtype, T, {
-        MMF_CUDA(mmf_launch_pdl(sample_top_p_kernel<T>, dim3((unsigned)M), dim3(256), 0, (cudaStream_t)stream, (const T*)logits, ld, (int)V,
-                                inv_temp, top_p < 1.0f ? top_p : 1.0f, uniforms, idx));
+        if (V <= SAMPLE_MAX_V) {
+            MMF_CUDA(cudaFuncSetAttribute(sample_top_p_smem_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (SAMPLE_MAX_V + SAMPLE_LIST) * 4));
+            MMF_CUDA(mmf_launch_pdl(sample_top_p_smem_kernel<T>, dim3((unsigned)M), dim3(SAMPLE_THREADS), smem, (cudaStream_t)stream,
+                                    (const T*)logits, ld, (int)V, inv_temp, top, uniforms, idx, vec));
+        } else {
+            MMF_CUDA(mmf_launch_pdl(sample_top_p_kernel<T>, dim3((unsigned)M), dim3(256), 0, (cudaStream_t)stream, (const T*)logits, ld,
+                                    (int)V, inv_temp, top, uniforms, idx));
+        }
     });
     MMF_LAUNCH_CHECK("sample_top_p_kernel");
     return MMF_OK;

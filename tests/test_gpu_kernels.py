@@ -77,6 +77,22 @@ def test_act_quant_bit_exact(K, dtype, M, Kdim):
         assert np.array_equal(rs.cpu().numpy(), rs_ref)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("M,Kdim,use_norm", [(3075, 2048, True), (3073, 2560, False), (3073, 5632, True), (3073, 7184, True), (600, 8192, True),
+                                             (3, 8208, True)])
+def test_act_quant_rows_side_by_side(K, dtype, M, Kdim, use_norm):
+    """Every shape of the row kernels behind act_quant (four, two or one row per CTA, rows too long for registers), with
+    ragged row counts and with and without the norm: the oracle's codes, scales and code sums bit for bit."""
+    g = torch.Generator().manual_seed(M + Kdim)
+    x = (torch.randn(M, Kdim, generator=g) * 2).to(dtype)
+    nw = 1.0 + 0.1 * torch.randn(Kdim, generator=g) if use_norm else None
+    q, dq, rs = K.act_quant(dev(x), None if nw is None else dev(nw), 1e-6, use_norm=use_norm)
+    rows = torch.unique(torch.cat([torch.arange(0, M, 97), torch.arange(max(0, M - 9), M)]))   # the oracle runs on a sample
+    q_ref, dq_ref, rs_ref = O.act_codes(x[rows], nw, 1e-6, use_norm=use_norm)
+    assert np.array_equal(q.cpu().numpy()[rows], q_ref)
+    assert np.array_equal(dq.cpu().numpy()[rows], dq_ref) and np.array_equal(rs.cpu().numpy()[rows], rs_ref)
+
+
 def test_act_quant_edge_rows(K):
     """Zero row (absmax clamps to 1e-5), a row with one huge outlier, no-norm mode, strided input, M = 0."""
     x = torch.randn(4, 256)
@@ -726,6 +742,24 @@ def test_sample_top_p_vs_oracle(K, dtype, temperature, top_p):
     # same inputs, same tokens
     again = K.sample_top_p(dev(logits), temperature, top_p, dev(u)).cpu().numpy()
     assert np.array_equal(got, again)
+
+
+@pytest.mark.parametrize("V", [1, 37, 1024, 8193, 32003, 40960, 40961])
+def test_sample_top_p_vocabulary_edges(K, V):
+    """Vocabularies that do not fill the kernel's layout (threads, warp ranges, vectors) or exceed its shared memory, rows of odd pitch,
+    a flat distribution (every token a candidate)."""
+    g = torch.Generator().manual_seed(V)
+    M = 12
+    logits = torch.randn(M, V, generator=g) * 3
+    u = torch.rand(M, generator=g)
+    u[0] = 0.0
+    u[1] = 1.0 - 2.0 ** -24
+    logits[2] = torch.rand(V, generator=g) * 1e-3
+    for top_p in (0.4, 1.0):
+        ref, margin = O.sample_top_p_ref(logits.numpy(), 0.7, top_p, u.numpy())
+        got = K.sample_top_p(dev(logits), 0.7, top_p, dev(u)).cpu().numpy()
+        safe = margin > 2e-6
+        assert np.array_equal(got[safe], ref[safe]) and (got >= 0).all() and (got < V).all()
 
 
 @pytest.mark.parametrize("gate_is_log", [True, False])
