@@ -27,6 +27,11 @@ NVCC_FLAGS = [
 ]
 
 
+# the CPython module that drives the library (host code only, compiled by the host compiler against torch's headers)
+NATIVE_PATH = PKG_DIR / "_native.so"
+NATIVE_SOURCE = CSRC / "binding.cpp"
+
+
 def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu"))
 
@@ -83,7 +88,36 @@ def build_experiments_library(force: bool = False, verbose: bool = False) -> Pat
     return _compile(EXPERIMENTS_LIB_PATH, ["-DMMF_EXPERIMENTS"], force, verbose)
 
 
+def build_native(force: bool = False) -> Path:
+    """Compile csrc/binding.cpp into the `_native` module beside the library. Idempotent."""
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    h = hashlib.sha256()
+    for p in [NATIVE_SOURCE, INCLUDE / "mmfree_b200.h"]:
+        h.update(p.read_bytes())
+    h.update((torch.__version__ + sysconfig.get_python_version()).encode())
+    digest = h.hexdigest()
+    if not force and NATIVE_PATH.exists() and _stamp(NATIVE_PATH).exists() and _stamp(NATIVE_PATH).read_text().strip() == digest:
+        return NATIVE_PATH
+    cuda = Path(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc").resolve().parent.parent
+    incs = [*include_paths(), sysconfig.get_paths()["include"], str(cuda / "include")]
+    lib_dir = Path(torch.__file__).parent / "lib"
+    tmp = NATIVE_PATH.with_suffix(".so.tmp")
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wno-deprecated-declarations",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{d}" for d in incs], str(NATIVE_SOURCE), "-o", str(tmp), f"-L{lib_dir}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-ldl"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f"g++ failed ({proc.returncode}):\n{proc.stdout}\n{proc.stderr}")
+    os.replace(tmp, NATIVE_PATH)
+    _stamp(NATIVE_PATH).write_text(digest + "\n")
+    return NATIVE_PATH
+
+
 if __name__ == "__main__":
     import sys
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
     print(build_experiments_library(force="--force" in sys.argv, verbose=False))
+    print(build_native(force="--force" in sys.argv))

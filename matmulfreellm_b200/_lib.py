@@ -133,6 +133,8 @@ class experiments_library:
             cls._handle = _open(EXPERIMENTS_LIB_PATH, {**PROTOTYPES, **_EXPERIMENT_PROTOTYPES})
         self._saved = load()
         _lib = cls._handle
+        if _native is not None:
+            _native.use_library(str(EXPERIMENTS_LIB_PATH))
         return cls._handle
 
     def __exit__(self, *exc):
@@ -140,7 +142,38 @@ class experiments_library:
         for k in range(self.KNOBS):
             experiments_library._handle.mmf_tuning(k, 0)
         _lib = self._saved
+        if _native is not None:
+            _native.use_library(str(LIB_PATH))
         return False
+
+
+NATIVE_PATH = LIB_PATH.with_name("_native.so")
+_native = None
+
+
+def native():
+    """The native host path (csrc/binding.cpp), loaded once; it calls whichever library is current (see
+    experiments_library).  Raises if it has not been built."""
+    global _native
+    if _native is None:
+        import importlib.machinery
+        import importlib.util
+
+        import torch  # noqa: F401 - its libraries must be loaded before the module that links against them
+
+        from . import kernels
+        load()
+        if not NATIVE_PATH.exists():
+            raise RuntimeError(f"{NATIVE_PATH} is missing. Build it with `python -m matmulfreellm_b200._build`; there is no "
+                               "fallback implementation.")
+        name = __package__ + "._native"
+        spec = importlib.util.spec_from_loader(name, importlib.machinery.ExtensionFileLoader(name, str(NATIVE_PATH)))
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.set_hooks(MMFreeError, kernels.stream_workspace)
+        mod.use_library(str(EXPERIMENTS_LIB_PATH if _lib is experiments_library._handle else LIB_PATH))
+        _native = mod
+    return _native
 
 
 # kernels each entry point launches per successful call (for launch accounting in benchmarks)

@@ -225,8 +225,8 @@ int bitlinear_gemv_launch(const BitLinearArgs& a, cudaStream_t st, bool force_sp
         const dim3 grid2((unsigned)(n_tiles * 4), (unsigned)mblocks);
 #define G2_LAUNCH(MBV)                                                                                              \
     {                                                                                                               \
-        auto kfn = bitlinear_gemv_rows_kernel<MBV>;                                                                 \
-        if (smem_rows > 48 * 1024) MMF_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows)); \
+        constexpr auto kfn = bitlinear_gemv_rows_kernel<MBV>;                                                       \
+        if (smem_rows > 48 * 1024) MMF_CUDA(mmf_allow_smem<kfn>(160 * 1024));                                       \
         MMF_CUDA(mmf_launch_pdl(kfn, grid2, dim3(G2_THREADS), smem_rows, st, a, KC, group_tiles));                 \
     }
         switch (MB) {

@@ -694,7 +694,7 @@ int bitlinear_mma_launch(const BitLinearArgs& a, cudaStream_t st) {
                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     MMF_REQUIRE(cr == CUDA_SUCCESS, MMF_ERR_CUDA, "mmf_bitlinear(mma): cuTensorMapEncodeTiled failed (%d)", (int)cr);
 
-    MMF_CUDA(cudaFuncSetAttribute(bitlinear_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MMF_CUDA(mmf_allow_smem<bitlinear_mma_kernel>(223 * 1024));
     const dim3 grid((unsigned)p.ksplit, (unsigned)((p.n_tiles + p.wt - 1) / p.wt), (unsigned)m_tiles);
     MMF_REQUIRE(m_tiles <= 65535 && p.n_tiles <= 65535, MMF_ERR_BAD_SHAPE, "mmf_bitlinear(mma): problem too large");
     cudaLaunchConfig_t cfg = {};

@@ -600,11 +600,9 @@ int pf_launch(const BitLinearArgs& a, cudaStream_t st) {
         p.tma_out = 1;
     }
 
-    int dev = 0, sms = 0;
-    MMF_CUDA(cudaGetDevice(&dev));
-    MMF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    auto kernel = bitlinear_mma_prefill_kernel<C>;
-    MMF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+    constexpr int sms = 148;
+    constexpr auto kernel = bitlinear_mma_prefill_kernel<C>;
+    MMF_CUDA(mmf_allow_smem<kernel>(C::SMEM));
     cudaLaunchConfig_t cfg = {};
     // one CTA per SM; in pair mode one cluster of two per work item in flight, an even number of CTAs
     const int ctas = C::PAIR ? 2 * (p.n_work < sms / 2 ? p.n_work : sms / 2) : (p.n_work < sms ? p.n_work : sms);

@@ -74,6 +74,18 @@ inline cudaError_t mmf_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Dynamic shared memory beyond 48 KB has to be switched on per kernel and device.  Done once per host thread, up to
+// `limit` (a launch that asks for less is not affected), because asking the runtime on every launch costs host time.
+template <auto kernel> inline cudaError_t mmf_allow_smem(int limit) {
+    thread_local uint64_t done = 0;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || (dev < 64 && (done >> dev & 1))) return e;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+    if (e == cudaSuccess && dev < 64) done |= 1ull << dev;
+    return e;
+}
+
 // ---------------------------------------------------------------------------------------
 // element conversion (round-to-nearest-even on store, exact on load)
 // ---------------------------------------------------------------------------------------

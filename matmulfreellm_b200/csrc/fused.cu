@@ -693,7 +693,7 @@ constexpr int64_t LAT_MAX_ROWS = MMF_LAT_MAX_ROWS;
 
 // the 48 KB that need no opt-in include the kernel's static shared memory (reduction scratch)
 #define FUSED_SMEM_ATTR(kernel, smem) \
-    if ((smem) + 2048 > 48 * 1024) MMF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem)))
+    if ((smem) + 2048 > 48 * 1024) MMF_CUDA(mmf_allow_smem<kernel>(220 * 1024))
 
 // rows per CTA by row length and count, as in mmf_prenorm_quant and mmf_swiglu_quant
 int act_quant_regs_launch(const void* x, int dtype, int64_t ld, const float* nw, int use_norm, float eps, int8_t* q, float* dq,

@@ -444,15 +444,15 @@ int hgrn_launch(const void* x, int64_t ld_x, const void* g, int64_t ld_g, const 
     if (rc != MMF_OK) return rc;
     const dim3 grid((unsigned)((D + HG_BD - 1) / HG_BD), (unsigned)NT, (unsigned)B);
     if (NT > 1) {
-        auto k1 = hgrn_scan_kernel<TX, TG, MODE, true>;
-        MMF_CUDA(cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        constexpr auto k1 = hgrn_scan_kernel<TX, TG, MODE, true>;
+        MMF_CUDA(mmf_allow_smem<k1>((int)smem));
         const dim3 grid1(grid.x, (unsigned)(NT - 1), grid.z);
         MMF_CUDA(mmf_launch_pdl(k1, grid1, dim3(HG_THREADS), smem, st, x_map, g_map, o_map, (const TX*)lb, mask, h0,
                                 (void*)nullptr, state_dt, (int)T, (int)D, NT, chunk_len, ws));
         MMF_LAUNCH_CHECK("hgrn_scan_kernel<aggregate>");
     }
-    auto k2 = hgrn_scan_kernel<TX, TG, MODE, false>;
-    MMF_CUDA(cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr auto k2 = hgrn_scan_kernel<TX, TG, MODE, false>;
+    MMF_CUDA(mmf_allow_smem<k2>((int)smem));
     MMF_CUDA(mmf_launch_pdl(k2, grid, dim3(HG_THREADS), smem, st, x_map, g_map, o_map, (const TX*)lb, mask, h0, ht, state_dt,
                             (int)T, (int)D, NT, chunk_len, ws));
     MMF_LAUNCH_CHECK("hgrn_scan_kernel<scan>");

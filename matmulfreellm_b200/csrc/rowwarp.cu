@@ -333,14 +333,7 @@ warp_gatenorm_quant_kernel(const T* __restrict__ gx, int64_t ld_g, const T* __re
 template <auto kernel, typename... Args>
 int wr_launch(size_t weight_bytes, size_t row_bytes, int64_t M, cudaStream_t st, const char* name, Args... args) {
     constexpr size_t SMEM_MAX = 227 * 1024;
-    // dynamic shared memory beyond 48 KB is switched on once per kernel, device and host thread, to the limit
-    thread_local uint64_t enabled = 0;
-    int dev = 0;
-    MMF_CUDA(cudaGetDevice(&dev));
-    if (dev >= 64 || !(enabled >> dev & 1)) {
-        MMF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
-        if (dev < 64) enabled |= 1ull << dev;
-    }
+    MMF_CUDA(mmf_allow_smem<kernel>((int)SMEM_MAX));
     const int64_t fit = (int64_t)((SMEM_MAX - weight_bytes) / row_bytes), share = (M + 147) / 148;
     int64_t warps = fit < WR_MAX_WARPS ? fit : WR_MAX_WARPS;
     if (share < warps) warps = share;

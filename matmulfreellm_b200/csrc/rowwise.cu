@@ -735,7 +735,7 @@ extern "C" int mmf_sample_top_p(const void* logits, int dtype, int64_t ld, float
     const size_t smem = ((size_t)((V + 3) & ~3ll) + SAMPLE_LIST) * sizeof(float);
     MMF_DISPATCH(dtype, T, {
         if (V <= SAMPLE_MAX_V) {
-            MMF_CUDA(cudaFuncSetAttribute(sample_top_p_smem_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (SAMPLE_MAX_V + SAMPLE_LIST) * 4));
+            MMF_CUDA(mmf_allow_smem<sample_top_p_smem_kernel<T>>((SAMPLE_MAX_V + SAMPLE_LIST) * 4));
             MMF_CUDA(mmf_launch_pdl(sample_top_p_smem_kernel<T>, dim3((unsigned)M), dim3(SAMPLE_THREADS), smem, (cudaStream_t)stream,
                                     (const T*)logits, ld, (int)V, inv_temp, top, uniforms, idx, vec));
         } else {

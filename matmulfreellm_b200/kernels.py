@@ -190,6 +190,12 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     return ws
 
 
+def stream_workspace(index: int) -> torch.Tensor:
+    """Workspace of the current stream of device `index`, for the native host path (asked for once per stream)."""
+    _lib.require_device(index)
+    return _workspace(torch.device("cuda", index), 1 << 20)
+
+
 def _rezero_workspaces() -> None:
     """After a failed launch or a device-side time-out partial sums may be left behind: clear every workspace in place
     (their addresses stay valid for captured graphs)."""
@@ -254,12 +260,24 @@ def bitlinear(q: torch.Tensor, dq: torch.Tensor, rowsum: torch.Tensor, pw: Packe
     return (out, acc) if return_acc else out
 
 
+def bitlinear_forward(x: torch.Tensor, norm_weight: Optional[torch.Tensor], pw: PackedWeight, eps: float) -> torch.Tensor:
+    """FusedBitLinear's forward: RMSNorm + int8 quantisation + contraction of x [..., K] -> [..., N] in x.dtype."""
+    out = _lib.native().bitlinear(x, norm_weight, pw.packed, pw.scale, pw.N, eps)
+    _lib.launch_count += 2
+    return out
+
+
 # ------------------------------------------------------------------------------------------
 # HGRN recurrence
 # ------------------------------------------------------------------------------------------
 def hgrn_scan(x: torch.Tensor, g: torch.Tensor, initial_state: Optional[torch.Tensor], output_final_state: bool,
               gate_is_log: bool, state_dtype: Optional[torch.dtype] = None, final_state_out: Optional[torch.Tensor] = None):
     """x, g: [..., T, D] contiguous; leading dims are independent sequences. Returns (o, final_state|None)."""
+    if final_state_out is None:
+        sdt = state_dtype or (initial_state.dtype if initial_state is not None else torch.float32)
+        out = _lib.native().hgrn_scan(x, g, initial_state, output_final_state, gate_is_log, sdt)
+        _lib.launch_count += 1
+        return out
     _need_cuda(x, g, initial_state)
     if x.shape != g.shape or x.dim() < 2:
         raise ValueError("x and g must have the same shape [..., T, D]")
@@ -484,20 +502,24 @@ def argmax_rows(logits: torch.Tensor, out: Optional[torch.Tensor] = None) -> tor
     return idx if out is not None else idx.reshape(logits.shape[:-1])
 
 
-def sample_top_p(logits: torch.Tensor, temperature: float, top_p: float, uniforms: torch.Tensor) -> torch.Tensor:
+def sample_top_p(logits: torch.Tensor, temperature: float, top_p: float, uniforms: torch.Tensor,
+                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """One token per row from softmax(logits / temperature) restricted to its top-p nucleus, using the caller's uniform
-    numbers (float32 in [0, 1), one per row): deterministic for given inputs.  Returns int64 indices."""
+    numbers (float32 in [0, 1), one per row): deterministic for given inputs.  Returns int64 indices (`out`: optional
+    contiguous int64 tensor with one element per row)."""
     _need_cuda(logits, uniforms)
     l2 = logits.reshape(-1, logits.shape[-1])
     if l2.stride(1) != 1:
         l2 = l2.contiguous()
     if uniforms.dtype != torch.float32 or uniforms.numel() != l2.shape[0] or not uniforms.is_contiguous():
         raise ValueError("uniforms must be contiguous float32 with one value per row")
-    idx = torch.empty(l2.shape[0], dtype=torch.int64, device=logits.device)
+    idx = torch.empty(l2.shape[0], dtype=torch.int64, device=logits.device) if out is None else out
+    if idx.dtype != torch.int64 or idx.numel() != l2.shape[0] or not idx.is_contiguous() or idx.device != logits.device:
+        raise ValueError("bad `out` tensor")
     if l2.shape[0]:
         _lib.call("mmf_sample_top_p", l2.data_ptr(), _code(l2.dtype), l2.stride(0), float(temperature), float(top_p),
                   uniforms.data_ptr(), idx.data_ptr(), l2.shape[0], l2.shape[1], _stream())
-    return idx.reshape(logits.shape[:-1])
+    return idx if out is not None else idx.reshape(logits.shape[:-1])
 
 
 def embedding(table: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:

@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import math
 import warnings
+import weakref
 from typing import List, Optional, Tuple, Union
 
 import torch
@@ -120,6 +121,16 @@ class HGRNBitModel(HGRNBitPreTrainedModel):
     def set_input_embeddings(self, value):
         self.embeddings = value
 
+    def init_cache(self, batch_size: int) -> RecurrentCache:
+        """Zero recurrent states of every layer (layer.attn.init_state), cut from one zero-filled allocation."""
+        cache = RecurrentCache()
+        if len(self.layers):
+            attn = self.layers[0].attn
+            states = torch.zeros(len(self.layers), batch_size, attn.num_heads, attn.head_dim, dtype=torch.float32,
+                                 device=self.embeddings.weight.device)
+            cache.states = [(s,) for s in states.unbind(0)]
+        return cache
+
     def layer_lower_bounds(self) -> Optional[torch.Tensor]:
         """[L, hidden] cumulative-softmax lower bounds of the forget gates (:231-233); row 0 is unused."""
         if not self.config.use_lower_bound:
@@ -153,7 +164,7 @@ class HGRNBitModel(HGRNBitPreTrainedModel):
 
         if use_cache:
             if past_key_values is None:
-                past_key_values = [layer.attn.init_state(batch_size) for layer in self.layers]
+                past_key_values = self.init_cache(batch_size)
             if not isinstance(past_key_values, RecurrentCache):
                 past_key_values = RecurrentCache.from_legacy_cache(past_key_values)
 
@@ -264,28 +275,24 @@ class HGRNBitForCausalLM(HGRNBitPreTrainedModel):
         through Python, several times what the GPU needs).  Same tokens as the step-by-step loop of `generate`:
         sequences are independent, so a finished sequence may keep running; its tokens after the first
         `eos_token_id` are overwritten with it, and the result is cut where the loop would have stopped.
-        `pick` (sampling) maps the step's logits [B, V] to tokens [B]; None takes the graph's own arg-max.  Sampling
+        `pick` (sampling) writes tokens [B] for the step's logits [B, V]; None takes the graph's own arg-max.  Sampling
         draws its random numbers in the same order as the step loop, so both give the same tokens."""
         from ...engine import GreedyDecoder, fused_runner
         B = input_ids.shape[0]
-        key = fused_runner(self).key
+        key = fused_runner(self)
         decs = self.__dict__.get("_greedy_decoders")
-        if decs is None or decs.get("key") != key:        # weights replaced or repacked: captured graphs are stale
+        if decs is None or decs.get("key") is not key:    # weights replaced or repacked: captured graphs are stale
             decs = {"key": key}
             object.__setattr__(self, "_greedy_decoders", decs)
         dec = decs.pop(B, None)
         if dec is None:
-            dec = GreedyDecoder(self, B)
+            dec = GreedyDecoder(weakref.proxy(self), B)     # this model keeps the decoder: no reference cycle
             while len(decs) - 1 >= self.GREEDY_DECODERS:
                 decs.pop(next(k for k in decs if k != "key"))
         decs[B] = dec                                       # most recently used last
-        if attention_mask is None and pick is None:
-            dec.prefill(input_ids)
-        else:
-            out = self(input_ids=input_ids, attention_mask=attention_mask, use_cache=True, last_token_only=True)
-            dec.seed(out.past_key_values, out.logits[:, -1])
-            if pick is not None:
-                dec.next.copy_(pick(out.logits[:, -1]))
+        dec.prefill(input_ids, attention_mask)
+        if pick is not None:
+            pick(dec.last_logits, dec.next)
         toks = torch.empty(B, max_new_tokens, dtype=torch.int64, device=input_ids.device)
         n = 0
         while n < max_new_tokens:
@@ -297,7 +304,7 @@ class HGRNBitForCausalLM(HGRNBitPreTrainedModel):
                 break                                       # every sequence has finished (checked every 16 steps)
             dec.step()
             if pick is not None:
-                dec.next.copy_(pick(dec.last_logits))
+                pick(dec.last_logits, dec.next)
         toks = toks[:, :n]
         if eos_token_id is not None:
             hit = toks == eos_token_id
@@ -330,7 +337,7 @@ class HGRNBitForCausalLM(HGRNBitPreTrainedModel):
             cache = past_key_values if isinstance(past_key_values, RecurrentCache) \
                 else RecurrentCache.from_legacy_cache(past_key_values)
         else:
-            cache = RecurrentCache.from_legacy_cache([layer.attn.init_state(B) for layer in layers])
+            cache = self.model.init_cache(B)
         # The kernels advance float32 states in place.  A cache built the reference's way holds its states in the
         # parameter dtype (init_state: param.new_zeros; fused_recurrent_hgrn returns x.dtype): such states are widened
         # for the pass and written back, rounded to their own dtype, afterwards — the reference's rounding point.
@@ -379,11 +386,11 @@ class HGRNBitForCausalLM(HGRNBitPreTrainedModel):
             raise NotImplementedError("generate(): finished sequences are padded with eos_token_id; a different pad_token_id "
                                       "is not implemented")
 
-        def pick(logits):
+        def pick(logits, out=None):
             if not do_sample:
-                return kernels.argmax_rows(logits)
+                return kernels.argmax_rows(logits, out=out)
             u = torch.rand(logits.shape[0], device=logits.device, dtype=torch.float32, generator=generator)
-            return kernels.sample_top_p(logits, temperature, top_p, u)
+            return kernels.sample_top_p(logits, temperature, top_p, u, out=out)
 
         if max_length is not None:
             max_new_tokens = max(0, max_length - input_ids.shape[1])

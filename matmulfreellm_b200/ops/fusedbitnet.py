@@ -93,16 +93,8 @@ class BitLinear(nn.Linear):
         return self._norm_w32
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        pw = self.packed()
-        shape = x.shape
-        x2 = x.reshape(-1, shape[-1])
-        if x2.stride(-1) != 1:
-            x2 = x2.contiguous()
-        q, dq, rs = kernels.act_quant(x2, self.norm_weight_f32(), self.NORM_EPS)
-        y = kernels.bitlinear(q, dq, rs, pw, x.dtype)
-        if self.bias is not None:
-            y = y + self.bias.to(y.dtype)
-        return y.reshape(*shape[:-1], self.out_features)
+        y = kernels.bitlinear_forward(x, self.norm_weight_f32(), self.packed(), self.NORM_EPS)
+        return y if self.bias is None else y + self.bias.to(y.dtype)
 
 
 class FusedBitLinear(BitLinear):
@@ -118,10 +110,5 @@ def layer_norm_linear_quant_fn(x, norm_weight, norm_bias, linear_weight, linear_
     if not is_rms_norm or norm_bias is not None or residual is not None or prenorm:
         raise NotImplementedError("only the RMSNorm, no-residual form used by FusedBitLinear is provided")
     pw = kernels.pack_weight(linear_weight)
-    shape = x.shape
-    x2 = x.reshape(-1, shape[-1]).contiguous()
-    q, dq, rs = kernels.act_quant(x2, None if norm_weight is None else norm_weight.detach().float().contiguous(), eps)
-    y = kernels.bitlinear(q, dq, rs, pw, x.dtype)
-    if linear_bias is not None:
-        y = y + linear_bias.to(y.dtype)
-    return y.reshape(*shape[:-1], linear_weight.shape[0])
+    y = kernels.bitlinear_forward(x, None if norm_weight is None else norm_weight.detach().float().contiguous(), pw, eps)
+    return y if linear_bias is None else y + linear_bias.to(y.dtype)
