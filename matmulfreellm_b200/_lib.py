@@ -61,6 +61,7 @@ PROTOTYPES = {
                                       c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p]),
     "mmf_swiglu_quant": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_void_p, c_float, c_void_p, c_void_p, c_void_p,
                                  c_int64, c_int64, c_void_p]),
+    "mmf_decode_linear": (c_int, [c_void_p, c_void_p]),
     "mmf_rmsnorm": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int64,
                             c_int64, c_void_p]),
     "mmf_rmsnorm_swishgate": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_float, c_void_p, c_int64, c_int64,

@@ -8,6 +8,7 @@
 //
 //   use_library(path)                    resolve the C ABI from this shared object
 //   set_hooks(error_class, workspace)    exception class for negative status codes, workspace(device_index) -> tensor
+//   take_launches()                      kernels launched since the last call of it
 //   bitlinear(x, norm_w, packed, scale, N, eps)       RMSNorm + int8 quantisation + contraction, [..., K] -> [..., N]
 //   hgrn_scan(x, g, h0 | None, want_state, gate_is_log, state_dtype)      -> (o, final state | None)
 //   watch(slots), unchanged(watch)       cheap "has any parameter been replaced, cast or modified" over (dict, name) slots
@@ -34,12 +35,16 @@ struct Api {
 #define MMF_FN(name) decltype(&::name) name = nullptr;
 #define MMF_FNS(F)                                                                                                      \
     F(mmf_last_error) F(mmf_act_quant) F(mmf_bitlinear) F(mmf_hgrn_workspace_bytes) F(mmf_hgrn_scan) F(mmf_hgrn_gated_masked) \
-    F(mmf_prenorm_quant) F(mmf_gatenorm_quant) F(mmf_decode_mix_masked) F(mmf_swiglu_quant) F(mmf_embedding)
+    F(mmf_prenorm_quant) F(mmf_gatenorm_quant) F(mmf_decode_mix_masked) F(mmf_swiglu_quant) F(mmf_embedding) \
+    F(mmf_decode_linear)
     MMF_FNS(MMF_FN)
 #undef MMF_FN
 };
 std::map<std::string, Api> g_apis;   // by path; the pointers stay valid because the libraries are never closed
 const Api* g_api = nullptr;
+
+int64_t g_launches = 0;    // guarded by the GIL
+int64_t g_fused_rows = MMF_DECODE_LINEAR_FUSED_MAX_M, g_codes_rows = MMF_DECODE_LINEAR_MAX_M;
 
 PyObject* g_error_class = nullptr;
 PyObject* g_workspace_fn = nullptr;
@@ -198,7 +203,23 @@ PyObject* bitlinear(PyObject*, PyObject* const* args, Py_ssize_t n) {
         std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
         shape.back() = N;
         at::Tensor out = at::empty(shape, x.options());
-        if (M > 0) {
+        if (M > 0 && M <= g_fused_rows && dt != MMF_F32 && K <= 8192) {      // a few rows: one kernel, no scratch
+            mmf_decode_linear_args a = {};
+            a.prologue = MMF_PRO_QUANT;
+            a.epilogue = MMF_EPI_STORE;
+            a.dtype = dt;
+            a.M = M; a.N = N; a.K = K;
+            a.packed = packed.data_ptr();
+            a.w_scale = scale.data_ptr<float>();
+            a.x = x2.data_ptr();
+            a.ld_x = x2.stride(0);
+            a.bl_norm_w[0] = (const float*)ptr(nw);
+            a.eps_bl = (float)eps;
+            a.out = out.data_ptr();
+            a.ld_out = N;
+            MMF_CALL(mmf_decode_linear, &a, c10::cuda::getCurrentCUDAStream(dev).stream());
+            ++g_launches;
+        } else if (M > 0) {
             void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
             const Ws ws = workspace(dev, st);
             Slab s;
@@ -209,6 +230,7 @@ PyObject* bitlinear(PyObject*, PyObject* const* args, Py_ssize_t n) {
                      (int32_t*)(b + rs), M, K, st);
             MMF_CALL(mmf_bitlinear, (const int8_t*)(b + q), (const float*)(b + dq), (const int32_t*)(b + rs), packed.data_ptr(),
                      scale.data_ptr<float>(), 1, out.data_ptr(), dt, N, nullptr, M, N, K, ws.p, ws.bytes, MMF_KERNEL_AUTO, st);
+            g_launches += 2;
         }
         return THPVariable_Wrap(std::move(out));
     });
@@ -412,9 +434,80 @@ PyObject* chain(PyObject*, PyObject* const* args, Py_ssize_t n) {
     });
 }
 
+// The blocks of a decode step.  z: last block's MLP output and the attention output; x / next: residual stream.
+template <typename ArgsOf, typename Run, typename Advance>
+void decode_blocks(const Chain& c, ArgsOf&& args_of, Run&& run, bool fuse_rows, int64_t M, uint8_t* z, uint8_t* g, uint8_t* o, uint8_t* act,
+                   const uint8_t* mask, const std::vector<float*>& states, int8_t* Q, float* DQ, int32_t* RS, void* st, const uint8_t*& x,
+                   uint8_t*& next, Advance&& advance, int64_t& launches) {
+    const int64_t h = c.h;
+    for (size_t i = 0; i < c.layers.size(); ++i) {
+        const Layer& L = c.layers[i];
+        const bool first = i == 0;
+        auto norm = [&](mmf_decode_linear_args& a, const void* row, const void* res, bool round, const float* w, void* res_out) {
+            a.x = row; a.ld_x = h;
+            a.residual = res; a.ld_residual = h;
+            a.round_sum_first = round;
+            a.norm_w = w; a.eps_norm = c.eps;
+            a.eps_bl = L.eps_bl;
+            a.residual_out = res_out;
+        };
+        // i / f / g projections, gates, state
+        mmf_decode_linear_args a = args_of(L.ifg, fuse_rows ? MMF_PRO_PRENORM : MMF_PRO_CODES, MMF_EPI_GATES, o, h);
+        a.g_out = g;
+        a.lower_bound = L.lb;
+        a.mask = mask;
+        a.state = states[i];
+        if (fuse_rows) {
+            // the reference adds residual + mlp output as a tensor op, then normalises the rounded sum
+            norm(a, first ? x : z, first ? nullptr : x, !first, L.attn_norm_w, first ? nullptr : next);
+            for (int k = 0; k < 3; ++k) a.bl_norm_w[k] = L.ifg_nw[k];
+        } else {
+            MMF_CALL(mmf_prenorm_quant, first ? x : z, h, first ? nullptr : x, h, c.dtype, first ? 0 : 1, L.attn_norm_w, c.eps, first ? nullptr : next,
+                     nullptr, 3, L.ifg_nw[0], L.ifg_nw[1], L.ifg_nw[2], L.eps_bl, Q, DQ, RS, M, h, st);
+            ++launches;
+        }
+        run(a);
+        if (!first) advance();
+        // gate norm, o_proj
+        a = args_of(L.o, fuse_rows ? MMF_PRO_GATENORM : MMF_PRO_CODES, MMF_EPI_STORE, z, h);
+        if (fuse_rows) {
+            a.x = g; a.ld_x = h;
+            a.residual = o; a.ld_residual = h;
+            a.norm_w = L.gnorm_w; a.eps_norm = L.gnorm_eps;
+            a.bl_norm_w[0] = L.o_nw; a.eps_bl = L.eps_bl;
+        } else {
+            MMF_CALL(mmf_gatenorm_quant, g, h, o, h, c.dtype, L.gnorm_w, L.gnorm_eps, L.o_nw, L.eps_bl, Q, DQ, RS, M, h, st);
+            ++launches;
+        }
+        run(a);
+        // mlp norm, gate / up projections, silu(gate) * up
+        a = args_of(L.gate, fuse_rows ? MMF_PRO_PRENORM : MMF_PRO_CODES, MMF_EPI_SWIGLU, act, L.down.K);
+        if (fuse_rows) {
+            norm(a, z, x, false, L.mlp_norm_w, next);
+            a.bl_norm_w[0] = L.gate_nw;
+        } else {
+            MMF_CALL(mmf_prenorm_quant, z, h, x, h, c.dtype, 0, L.mlp_norm_w, c.eps, next, nullptr, 1, L.gate_nw, nullptr, nullptr, L.eps_bl, Q, DQ, RS,
+                     M, h, st);
+            ++launches;
+        }
+        run(a);
+        advance();
+        // down_proj
+        a = args_of(L.down, fuse_rows ? MMF_PRO_QUANT : MMF_PRO_CODES, MMF_EPI_STORE, z, h);
+        if (fuse_rows) {
+            a.x = act; a.ld_x = L.down.K;
+            a.bl_norm_w[0] = L.down_nw; a.eps_bl = L.eps_bl;
+        } else {
+            MMF_CALL(mmf_act_quant, act, c.dtype, L.down.K, L.down_nw, 1, L.eps_bl, Q, DQ, RS, M, L.down.K, st);
+            ++launches;
+        }
+        run(a);
+    }
+}
+
 // chain_forward(chain, ids | None, embeds | None, states, mask | None, last_only, want_logits, want_hidden)
 //   ids int64 [B, T] or embeds [B, T, h]; states: list of fp32 tensors of B * h elements, advanced in place; mask uint8 [B, T]
-//   -> (logits | None, hidden | None, number of kernel launches)
+//   -> (logits | None, hidden | None)
 PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         if (n != 8) throw std::domain_error("chain_forward takes 8 arguments");
@@ -490,7 +583,29 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 next = next == b + x1 ? b + x0 : b + x1;
             };
             bool first = true;
-            for (size_t i = 0; i < c.layers.size(); ++i) {
+            // One token per sequence and few sequences: contractions with the element-wise work around them in one kernel
+            // (decode_linear.cuh); up to g_fused_rows rows the row kernels in between disappear as well.
+            const bool decode = T == 1 && M > 0 && M <= g_codes_rows && c.dtype != MMF_F32 && h % MMF_TILE_ROWS == 0 && h <= 4096 && c.inner <= 8192;
+            const bool fuse_rows = decode && M <= g_fused_rows;
+            auto args_of = [&](const Linear& l, int pro, int epi, void* out, int64_t ld_out) {
+                mmf_decode_linear_args a = {};
+                a.prologue = pro;
+                a.epilogue = epi;
+                a.dtype = c.dtype;
+                a.M = M; a.N = l.N; a.K = l.K;
+                a.packed = l.packed;
+                a.w_scale = l.scale;
+                a.q = Q; a.dq = DQ; a.rowsum = RS;
+                a.out = out;
+                a.ld_out = ld_out;
+                return a;
+            };
+            auto run = [&](const mmf_decode_linear_args& a) {
+                MMF_CALL(mmf_decode_linear, &a, st);
+                ++launches;
+            };
+            if (decode) decode_blocks(c, args_of, run, fuse_rows, M, b + z, b + ifg, b + o, b + gu, mk, states, Q, DQ, RS, st, x, next, advance, launches);
+            for (size_t i = 0; i < c.layers.size() && !decode; ++i) {
                 const Layer& L = c.layers[i];
                 if (first) {
                     MMF_CALL(mmf_prenorm_quant, x, h, nullptr, 0, c.dtype, 0, L.attn_norm_w, c.eps, nullptr, nullptr, 3, L.ifg_nw[0], L.ifg_nw[1],
@@ -524,20 +639,47 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
             }
             // final norm: only the last position of every sequence when only that feeds lm_head
             const int64_t skip = last_only ? (T - 1) * h * es : 0, ld = last_only ? T * h : h;
+            first = c.layers.empty();
             const uint8_t* rows = first ? x : b + z;
+            if (fuse_rows && want_logits && !want_hidden) {
+                mmf_decode_linear_args a = args_of(c.head, MMF_PRO_PRENORM, MMF_EPI_STORE, logits.data_ptr(), c.head.N);
+                a.x = rows; a.ld_x = h;
+                a.residual = first ? nullptr : x; a.ld_residual = h;
+                a.round_sum_first = !first;
+                a.norm_w = c.final_norm_w; a.eps_norm = c.eps;
+                a.bl_norm_w[0] = c.head_nw; a.eps_bl = c.head_eps;
+                run(a);
+            } else {
             MMF_CALL(mmf_prenorm_quant, rows + skip, ld, first ? nullptr : x + skip, ld, c.dtype, first ? 0 : 1, c.final_norm_w, c.eps, nullptr,
                      ptr(hidden), want_logits ? 1 : 0, c.head_nw, nullptr, nullptr, c.head_eps, Q, DQ, RS, Mn, h, st);
             ++launches;
-            if (want_logits) linear(c.head, logits.data_ptr(), Mn);
+            if (want_logits) {
+                if (decode) run(args_of(c.head, MMF_PRO_CODES, MMF_EPI_STORE, logits.data_ptr(), c.head.N));
+                else linear(c.head, logits.data_ptr(), Mn);
+            }
+            }
         }
+        g_launches += launches;
         PyObject* pl = logits.defined() ? THPVariable_Wrap(std::move(logits)) : Py_NewRef(Py_None);
         PyObject* ph = hidden.defined() ? THPVariable_Wrap(std::move(hidden)) : Py_NewRef(Py_None);
-        PyObject* r = Py_BuildValue("(NNL)", pl, ph, (long long)launches);
-        return r;
+        return Py_BuildValue("(NN)", pl, ph);
     });
 }
 
+PyObject* take_launches(PyObject*, PyObject*) {
+    const int64_t n = g_launches;
+    g_launches = 0;
+    return PyLong_FromLongLong(n);
+}
+PyObject* set_rows(PyObject*, PyObject* const* args, Py_ssize_t) {
+    g_fused_rows = PyLong_AsLongLong(args[0]);
+    g_codes_rows = PyLong_AsLongLong(args[1]);
+    Py_RETURN_NONE;
+}
+
 PyMethodDef methods[] = {
+    {"take_launches", take_launches, METH_NOARGS, nullptr},
+    {"set_rows", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(set_rows)), METH_FASTCALL, nullptr},
     {"use_library", use_library, METH_O, nullptr},
     {"set_hooks", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(set_hooks)), METH_FASTCALL, nullptr},
     {"bitlinear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(bitlinear)), METH_FASTCALL, nullptr},

@@ -14,6 +14,7 @@
 // rowwise.cu), 14 instructions per value instead of 22.  What is left: shared-memory wavefronts (the norm weights are read in
 // every pass: pipe 61 - 80 % busy) and issue (2.5 per clock).
 #include "common.cuh"
+#include "packed.cuh"
 #include "rowquant.cuh"
 
 namespace {
@@ -23,38 +24,6 @@ namespace {
 constexpr int WR_MAX_WARPS = 16;
 constexpr int V = 8;                          // values per 16-byte vector
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-template <typename T> __device__ __forceinline__ float2 widen(uint32_t u) {
-    if constexpr (cuda::std::is_same<T, __half>::value) return __half22float2(*reinterpret_cast<const __half2*>(&u));
-    else return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
-}
-template <typename T> __device__ __forceinline__ uint32_t narrow(float2 v) {
-    if constexpr (cuda::std::is_same<T, __half>::value) {
-        const __half2 h = __floats2half2_rn(v.x, v.y);
-        return *reinterpret_cast<const uint32_t*>(&h);
-    } else {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
-        return *reinterpret_cast<const uint32_t*>(&h);
-    }
-}
-// s0 / s1 += squares of a packed pair (bf16: the fp64 operands are assembled from the bits, as sumsq_rounded does)
-template <typename T> __device__ __forceinline__ void sumsq_pair(uint32_t u, double& s0, double& s1) {
-    if constexpr (cuda::std::is_same<T, __half>::value) {
-        const float2 f = widen<T>(u);
-        s0 = fma((double)f.x, (double)f.x, s0);
-        s1 = fma((double)f.y, (double)f.y, s1);
-    } else {
-        const double d0 = __hiloint2double((int)(((u & 0x7fffu) << 13) + 0x38000000u), 0);
-        const double d1 = __hiloint2double((int)(((u >> 3) & 0x0fffe000u) + 0x38000000u), 0);
-        s0 = fma(d0, d0, s0);
-        s1 = fma(d1, d1, s1);
-    }
-}
 // Between two passes over a packed row: the compiler would keep the widened values of the first pass for the second, twice
 // as many registers as the packed row (at 22 vectors per lane it spilled 560 bytes), instead of widening again.
 template <int NV> __device__ __forceinline__ void forget_widened(uint32_t (&u)[NV][4]) {
@@ -63,18 +32,12 @@ template <int NV> __device__ __forceinline__ void forget_widened(uint32_t (&u)[N
 #pragma unroll
         for (int i = 0; i < 4; ++i) asm volatile("" : "+r"(u[it][i]));
 }
-__device__ __forceinline__ float2 mul2(float2 a, float b) { return __fmul2_rn(a, make_float2(b, b)); }
 
 // vector `it` of a lane starts at column c = (it * 32 + lane) * 8.  NV is the even number of vectors per lane that holds a
 // row of D values, so only the last two vectors can lie (partly) past its end.
 #define WR_FOREACH(it, c) \
     _Pragma("unroll") for (int it = 0, c = lane * V; it < NV; ++it, c += 32 * V) if (it < NV - 2 || c < D)
 
-__device__ __forceinline__ void lds8(const float* p, float2 (&w)[4]) {
-    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
-    w[0] = make_float2(a.x, a.y); w[1] = make_float2(a.z, a.w);
-    w[2] = make_float2(b.x, b.y); w[3] = make_float2(b.z, b.w);
-}
 __device__ __forceinline__ void stage(float* dst, const float* src, int n) {
     for (int i = threadIdx.x * 4; i < n; i += blockDim.x * 4) {
         float4 v = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
@@ -110,16 +73,8 @@ __device__ __forceinline__ void warp_quant(uint32_t (&u)[NV][4], int D, float rs
         uint32_t word[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            int iv[4];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const float2 y = __fmul2_rn(mul2(widen<T>(u[it][2 * h + j]), rstd), w[2 * h + j]);
-                // |y * s| <= 127 (1 + 2^-23): no clamp; adding 1.5 * 2^23 leaves the code, rounded to nearest even, in the low
-                // byte.  Scalar on purpose: a packed multiply feeding a packed add can be merged into one rounding.
-                iv[2 * j] = __float_as_int(__fadd_rn(__fmul_rn(y.x, s), 12582912.0f));
-                iv[2 * j + 1] = __float_as_int(__fadd_rn(__fmul_rn(y.y, s), 12582912.0f));
-            }
-            word[h] = __byte_perm(__byte_perm(iv[0], iv[1], 0x0040), __byte_perm(iv[2], iv[3], 0x0040), 0x5410);
+            word[h] = codes4(__fmul2_rn(mul2(widen<T>(u[it][2 * h]), rstd), w[2 * h]),
+                             __fmul2_rn(mul2(widen<T>(u[it][2 * h + 1]), rstd), w[2 * h + 1]), s);
             lsum = __dp4a((int)word[h], 0x01010101, lsum);
         }
         *reinterpret_cast<uint2*>(qr + c) = make_uint2(word[0], word[1]);

@@ -258,10 +258,9 @@ class FusedRunner:
         mask = None
         if attention_mask is not None:
             mask = (attention_mask.to(self.device) != 0).to(torch.uint8).contiguous()
-        logits, hidden, launches = self._native.chain_forward(self.chain, input_ids, inputs_embeds, states, mask, last_only,
-                                                              want_logits, want_hidden)
-        _lib.launch_count += launches
-        return logits, hidden
+        out = self._native.chain_forward(self.chain, input_ids, inputs_embeds, states, mask, last_only, want_logits, want_hidden)
+        _lib.launch_count += self._native.take_launches()
+        return out
 
 
 def fused_runner(lm) -> FusedRunner:

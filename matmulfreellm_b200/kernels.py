@@ -262,8 +262,9 @@ def bitlinear(q: torch.Tensor, dq: torch.Tensor, rowsum: torch.Tensor, pw: Packe
 
 def bitlinear_forward(x: torch.Tensor, norm_weight: Optional[torch.Tensor], pw: PackedWeight, eps: float) -> torch.Tensor:
     """FusedBitLinear's forward: RMSNorm + int8 quantisation + contraction of x [..., K] -> [..., N] in x.dtype."""
-    out = _lib.native().bitlinear(x, norm_weight, pw.packed, pw.scale, pw.N, eps)
-    _lib.launch_count += 2
+    native = _lib.native()
+    out = native.bitlinear(x, norm_weight, pw.packed, pw.scale, pw.N, eps)
+    _lib.launch_count += native.take_launches()
     return out
 
 
