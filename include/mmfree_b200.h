@@ -297,8 +297,7 @@ int mmf_swiglu_quant(const void* gate, const void* up, int64_t ld, int dtype, co
  * results are bit-identical to mmf_prenorm_quant / mmf_gatenorm_quant / mmf_decode_mix /
  * mmf_swiglu_quant / mmf_act_quant around mmf_bitlinear.
  * ------------------------------------------------------------------------------------ */
-/* prologue: where the int8 codes come from */
-#define MMF_PRO_CODES 0     /* q, dq, rowsum [groups][M]... made by a row kernel; M <= MMF_DECODE_LINEAR_MAX_M */
+/* prologue: the row work that ends in int8 codes */
 #define MMF_PRO_QUANT 1     /* rows x: RMSNorm + quantisation (mmf_act_quant); K <= 8192 */
 #define MMF_PRO_PRENORM 2   /* [x + residual] -> residual_out, RMSNorm, quantisation (mmf_prenorm_quant); K <= 4096 */
 #define MMF_PRO_GATENORM 3  /* rows x = g and residual = o: mmf_gatenorm_quant; K <= 4096 */
@@ -307,8 +306,7 @@ int mmf_swiglu_quant(const void* gate, const void* up, int64_t ld, int dtype, co
 #define MMF_EPI_GATES 1     /* N = 3 K = i | f | g projections: gate math and state update (mmf_decode_mix without its
                                norm); out = o [M, K], g_out = g [M, K], state fp32 [M, K] in place */
 #define MMF_EPI_SWIGLU 2    /* N = 2 I = gate | up: out = silu(gate) * up [M, ld_out] */
-#define MMF_DECODE_LINEAR_MAX_M 32
-#define MMF_DECODE_LINEAR_FUSED_MAX_M 4
+#define MMF_DECODE_LINEAR_MAX_M 4
 
 typedef struct {
     int prologue, epilogue, dtype;          /* dtype: MMF_BF16 or MMF_F16 */
@@ -316,15 +314,14 @@ typedef struct {
     int64_t M, N, K;
     const void* packed;                     /* weights, packed; GATES: three K x K projections stacked along N */
     const float* w_scale;                   /* one per projection */
-    const void *x, *residual;               /* row inputs of the fused prologues */
+    const void *x, *residual;               /* row inputs of the prologue */
     int64_t ld_x, ld_residual;
+    const int64_t* row_ids;                 /* PRENORM without residual: row m is x[row_ids[m]] (token embedding), or NULL */
+    int64_t x_rows;                         /* rows of x when row_ids is given (ids are clamped to it) */
     const float* norm_w;                    /* block norm (PRENORM) or gate norm (GATENORM) weight, or NULL */
     float eps_norm, eps_bl;
     const float* bl_norm_w[3];              /* BitLinear norm weight per projection, or NULL */
     void* residual_out;                     /* PRENORM: [M, K], or NULL */
-    const int8_t* q;                        /* CODES */
-    const float* dq;
-    const int32_t* rowsum;
     void* out;
     int64_t ld_out;
     void* g_out;                            /* GATES */
@@ -333,7 +330,7 @@ typedef struct {
     float* state;                           /* GATES */
 } mmf_decode_linear_args;
 
-/* PRENORM goes with GATES, SWIGLU or STORE, GATENORM and QUANT with STORE, CODES with any epilogue. */
+/* PRENORM goes with GATES, SWIGLU or STORE, GATENORM and QUANT with STORE. */
 int mmf_decode_linear(const mmf_decode_linear_args* args, void* stream);
 
 /* ------------------------------------------------------------------------------------

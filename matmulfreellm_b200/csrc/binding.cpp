@@ -44,7 +44,7 @@ std::map<std::string, Api> g_apis;   // by path; the pointers stay valid because
 const Api* g_api = nullptr;
 
 int64_t g_launches = 0;    // guarded by the GIL
-int64_t g_fused_rows = MMF_DECODE_LINEAR_FUSED_MAX_M, g_codes_rows = MMF_DECODE_LINEAR_MAX_M;
+int64_t g_fused_rows = MMF_DECODE_LINEAR_MAX_M;
 
 PyObject* g_error_class = nullptr;
 PyObject* g_workspace_fn = nullptr;
@@ -434,11 +434,11 @@ PyObject* chain(PyObject*, PyObject* const* args, Py_ssize_t n) {
     });
 }
 
-// The blocks of a decode step.  z: last block's MLP output and the attention output; x / next: residual stream.
+// The blocks of a decode step for a few token rows: four kernels per block (decode_linear.cuh).  z: last block's MLP output and
+// the attention output; x / next: residual stream.
 template <typename ArgsOf, typename Run, typename Advance>
-void decode_blocks(const Chain& c, ArgsOf&& args_of, Run&& run, bool fuse_rows, int64_t M, uint8_t* z, uint8_t* g, uint8_t* o, uint8_t* act,
-                   const uint8_t* mask, const std::vector<float*>& states, int8_t* Q, float* DQ, int32_t* RS, void* st, const uint8_t*& x,
-                   uint8_t*& next, Advance&& advance, int64_t& launches) {
+void decode_blocks(const Chain& c, ArgsOf&& args_of, Run&& run, const int64_t* gather, uint8_t* z, uint8_t* g, uint8_t* o, uint8_t* act,
+                   const uint8_t* mask, const std::vector<float*>& states, const uint8_t*& x, uint8_t*& next, Advance&& advance) {
     const int64_t h = c.h;
     for (size_t i = 0; i < c.layers.size(); ++i) {
         const Layer& L = c.layers[i];
@@ -451,56 +451,37 @@ void decode_blocks(const Chain& c, ArgsOf&& args_of, Run&& run, bool fuse_rows, 
             a.eps_bl = L.eps_bl;
             a.residual_out = res_out;
         };
-        // i / f / g projections, gates, state
-        mmf_decode_linear_args a = args_of(L.ifg, fuse_rows ? MMF_PRO_PRENORM : MMF_PRO_CODES, MMF_EPI_GATES, o, h);
+        // i / f / g projections, gates, state; the reference adds residual + mlp output as a tensor op, then normalises the rounded sum
+        mmf_decode_linear_args a = args_of(L.ifg, MMF_PRO_PRENORM, MMF_EPI_GATES, o, h);
+        norm(a, first ? x : z, first ? nullptr : x, !first, L.attn_norm_w, first && !gather ? nullptr : next);
+        if (first && gather) {
+            a.row_ids = gather;
+            a.x_rows = c.table.size(0);
+        }
+        for (int k = 0; k < 3; ++k) a.bl_norm_w[k] = L.ifg_nw[k];
         a.g_out = g;
         a.lower_bound = L.lb;
         a.mask = mask;
         a.state = states[i];
-        if (fuse_rows) {
-            // the reference adds residual + mlp output as a tensor op, then normalises the rounded sum
-            norm(a, first ? x : z, first ? nullptr : x, !first, L.attn_norm_w, first ? nullptr : next);
-            for (int k = 0; k < 3; ++k) a.bl_norm_w[k] = L.ifg_nw[k];
-        } else {
-            MMF_CALL(mmf_prenorm_quant, first ? x : z, h, first ? nullptr : x, h, c.dtype, first ? 0 : 1, L.attn_norm_w, c.eps, first ? nullptr : next,
-                     nullptr, 3, L.ifg_nw[0], L.ifg_nw[1], L.ifg_nw[2], L.eps_bl, Q, DQ, RS, M, h, st);
-            ++launches;
-        }
         run(a);
-        if (!first) advance();
+        if (!first || gather) advance();
         // gate norm, o_proj
-        a = args_of(L.o, fuse_rows ? MMF_PRO_GATENORM : MMF_PRO_CODES, MMF_EPI_STORE, z, h);
-        if (fuse_rows) {
-            a.x = g; a.ld_x = h;
-            a.residual = o; a.ld_residual = h;
-            a.norm_w = L.gnorm_w; a.eps_norm = L.gnorm_eps;
-            a.bl_norm_w[0] = L.o_nw; a.eps_bl = L.eps_bl;
-        } else {
-            MMF_CALL(mmf_gatenorm_quant, g, h, o, h, c.dtype, L.gnorm_w, L.gnorm_eps, L.o_nw, L.eps_bl, Q, DQ, RS, M, h, st);
-            ++launches;
-        }
+        a = args_of(L.o, MMF_PRO_GATENORM, MMF_EPI_STORE, z, h);
+        a.x = g; a.ld_x = h;
+        a.residual = o; a.ld_residual = h;
+        a.norm_w = L.gnorm_w; a.eps_norm = L.gnorm_eps;
+        a.bl_norm_w[0] = L.o_nw; a.eps_bl = L.eps_bl;
         run(a);
         // mlp norm, gate / up projections, silu(gate) * up
-        a = args_of(L.gate, fuse_rows ? MMF_PRO_PRENORM : MMF_PRO_CODES, MMF_EPI_SWIGLU, act, L.down.K);
-        if (fuse_rows) {
-            norm(a, z, x, false, L.mlp_norm_w, next);
-            a.bl_norm_w[0] = L.gate_nw;
-        } else {
-            MMF_CALL(mmf_prenorm_quant, z, h, x, h, c.dtype, 0, L.mlp_norm_w, c.eps, next, nullptr, 1, L.gate_nw, nullptr, nullptr, L.eps_bl, Q, DQ, RS,
-                     M, h, st);
-            ++launches;
-        }
+        a = args_of(L.gate, MMF_PRO_PRENORM, MMF_EPI_SWIGLU, act, L.down.K);
+        norm(a, z, x, false, L.mlp_norm_w, next);
+        a.bl_norm_w[0] = L.gate_nw;
         run(a);
         advance();
         // down_proj
-        a = args_of(L.down, fuse_rows ? MMF_PRO_QUANT : MMF_PRO_CODES, MMF_EPI_STORE, z, h);
-        if (fuse_rows) {
-            a.x = act; a.ld_x = L.down.K;
-            a.bl_norm_w[0] = L.down_nw; a.eps_bl = L.eps_bl;
-        } else {
-            MMF_CALL(mmf_act_quant, act, c.dtype, L.down.K, L.down_nw, 1, L.eps_bl, Q, DQ, RS, M, L.down.K, st);
-            ++launches;
-        }
+        a = args_of(L.down, MMF_PRO_QUANT, MMF_EPI_STORE, z, h);
+        a.x = act; a.ld_x = L.down.K;
+        a.bl_norm_w[0] = L.down_nw; a.eps_bl = L.eps_bl;
         run(a);
     }
 }
@@ -570,8 +551,13 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                          MMF_KERNEL_AUTO, st);
                 ++launches;
             };
+            // one token per sequence and few sequences: contractions with the row work around them in one kernel
+            const bool decode = T == 1 && M > 0 && M <= g_fused_rows && c.dtype != MMF_F32 && h % MMF_TILE_ROWS == 0 && h <= 4096 && c.inner <= 8192;
+            const int64_t* gather = decode && ids.defined() && !c.layers.empty() ? ids.data_ptr<int64_t>() : nullptr;
             const uint8_t* x = b + x0;            // residual stream
-            if (ids.defined()) {
+            if (gather) {                         // the first block reads the embedding rows itself
+                x = static_cast<const uint8_t*>(c.table.data_ptr());
+            } else if (ids.defined()) {
                 MMF_CALL(mmf_embedding, c.table.data_ptr(), c.dtype, c.table.size(0), h, ids.data_ptr<int64_t>(), b + x0, M, st);
                 ++launches;
             } else {
@@ -583,10 +569,6 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 next = next == b + x1 ? b + x0 : b + x1;
             };
             bool first = true;
-            // One token per sequence and few sequences: contractions with the element-wise work around them in one kernel
-            // (decode_linear.cuh); up to g_fused_rows rows the row kernels in between disappear as well.
-            const bool decode = T == 1 && M > 0 && M <= g_codes_rows && c.dtype != MMF_F32 && h % MMF_TILE_ROWS == 0 && h <= 4096 && c.inner <= 8192;
-            const bool fuse_rows = decode && M <= g_fused_rows;
             auto args_of = [&](const Linear& l, int pro, int epi, void* out, int64_t ld_out) {
                 mmf_decode_linear_args a = {};
                 a.prologue = pro;
@@ -595,7 +577,6 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 a.M = M; a.N = l.N; a.K = l.K;
                 a.packed = l.packed;
                 a.w_scale = l.scale;
-                a.q = Q; a.dq = DQ; a.rowsum = RS;
                 a.out = out;
                 a.ld_out = ld_out;
                 return a;
@@ -604,7 +585,7 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 MMF_CALL(mmf_decode_linear, &a, st);
                 ++launches;
             };
-            if (decode) decode_blocks(c, args_of, run, fuse_rows, M, b + z, b + ifg, b + o, b + gu, mk, states, Q, DQ, RS, st, x, next, advance, launches);
+            if (decode) decode_blocks(c, args_of, run, gather, b + z, b + ifg, b + o, b + gu, mk, states, x, next, advance);
             for (size_t i = 0; i < c.layers.size() && !decode; ++i) {
                 const Layer& L = c.layers[i];
                 if (first) {
@@ -641,7 +622,7 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
             const int64_t skip = last_only ? (T - 1) * h * es : 0, ld = last_only ? T * h : h;
             first = c.layers.empty();
             const uint8_t* rows = first ? x : b + z;
-            if (fuse_rows && want_logits && !want_hidden) {
+            if (decode && want_logits && !want_hidden) {
                 mmf_decode_linear_args a = args_of(c.head, MMF_PRO_PRENORM, MMF_EPI_STORE, logits.data_ptr(), c.head.N);
                 a.x = rows; a.ld_x = h;
                 a.residual = first ? nullptr : x; a.ld_residual = h;
@@ -653,10 +634,7 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
             MMF_CALL(mmf_prenorm_quant, rows + skip, ld, first ? nullptr : x + skip, ld, c.dtype, first ? 0 : 1, c.final_norm_w, c.eps, nullptr,
                      ptr(hidden), want_logits ? 1 : 0, c.head_nw, nullptr, nullptr, c.head_eps, Q, DQ, RS, Mn, h, st);
             ++launches;
-            if (want_logits) {
-                if (decode) run(args_of(c.head, MMF_PRO_CODES, MMF_EPI_STORE, logits.data_ptr(), c.head.N));
-                else linear(c.head, logits.data_ptr(), Mn);
-            }
+            if (want_logits) linear(c.head, logits.data_ptr(), Mn);
             }
         }
         g_launches += launches;
@@ -673,7 +651,6 @@ PyObject* take_launches(PyObject*, PyObject*) {
 }
 PyObject* set_rows(PyObject*, PyObject* const* args, Py_ssize_t) {
     g_fused_rows = PyLong_AsLongLong(args[0]);
-    g_codes_rows = PyLong_AsLongLong(args[1]);
     Py_RETURN_NONE;
 }
 

@@ -19,18 +19,22 @@
 // changes nothing in an integer sum.  Weights are fetched by cp.async into slots private to a lane before the
 // grid-dependency wait.  Partial sums meet in shared memory by integer atomics (exact, so order does not matter).
 #pragma once
+#include <cstdlib>
 #include "bitlinear.cuh"
 #include "packed.cuh"
 
 namespace {
 
 constexpr int DL_TS = 20;               // accumulator words per (block, token): 16 rows, padded so that a warp's adds do not collide
-constexpr int DL_FUSED_ROWS = MMF_DECODE_LINEAR_FUSED_MAX_M;   // token rows a CTA takes through the fused prologue
+constexpr int DL_FUSED_ROWS = MMF_DECODE_LINEAR_MAX_M;   // token rows a CTA takes through the fused prologue
 
 struct DlParams {
     mmf_decode_linear_args a;
+    double inv_k;                       // 1 / K
     int KC, KG;                         // 64-column chunks, groups of four chunks
-    int units, grid;                    // unit of work: two adjacent output rows (gates, swiglu: channels)
+    int grid, base, extra;              // units (two adjacent output rows; gates, swiglu: channels) per CTA: base, the first `extra` CTAs one more
+    int kw, bw;                         // warp w takes column groups w % kw, + kw, ... of blocks w / kw, + bw, ...
+    int kgw;                            // column groups per warp
     int pf;                             // weight items per warp fetched ahead into shared memory
     int smem_codes, smem_acc, smem_w;   // byte offsets in dynamic shared memory
 };
@@ -52,24 +56,40 @@ template <int TH, int RT> __device__ __forceinline__ double dl_row_sum(double v,
     v = warp_sum(v);
     if ((threadIdx.x & 31) == 0) slot[(threadIdx.x % RT) >> 5] = v;
     dl_row_sync<TH, RT>();
-    double t[RW];
+    // every warp folds the partials by shuffles: with all lanes reading all partials the fold took 450 clocks instead of 200
+    constexpr int P = RW <= 2 ? 2 : RW <= 4 ? 4 : RW <= 8 ? 8 : 16;
+    const int l = threadIdx.x & (P - 1);
+    double t = P == RW || l < RW ? slot[l] : 0.0;
 #pragma unroll
-    for (int w = 0; w < RW; w += 2) {
-        const double2 d = *reinterpret_cast<const double2*>(slot + w);
-        t[w] = d.x;
-        t[w + 1] = d.y;
-    }
-#pragma unroll
-    for (int s = RW / 2; s > 0; s >>= 1)
-#pragma unroll
-        for (int w = 0; w < s; ++w) t[w] += t[w + s];
-    return t[0];
+    for (int o = P / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
 }
+// A kernel parameter in a register from here on: read from the constant bank where it is first used, it costs a miss of several
+// hundred clocks on the critical path.
+template <typename P> __device__ __forceinline__ void pin(P*& p) { asm volatile("" : "+l"(p)); }
+__device__ __forceinline__ void pin(int64_t& v) { asm volatile("" : "+l"(v)); }
+__device__ __forceinline__ void pin(float& v) { asm volatile("" : "+f"(v)); }
 
 template <int RT> struct __align__(16) DlScratch {      // per row; a member is written once per kernel
     double d0[RT / 32], d1[RT / 32];
     float f[3][RT / 32];
     int i[3][RT / 32];
+};
+
+// the prologue's parameters, read before the grid-dependency wait
+template <typename T> struct DlRowArgs {
+    const T *x, *r;
+    T* res_out;
+    float eps_norm, eps_bl;
+    __device__ __forceinline__ DlRowArgs(const mmf_decode_linear_args& a, int m, bool leader) {
+        x = reinterpret_cast<const T*>(a.x);
+        if (!a.row_ids) x += m * a.ld_x;
+        r = a.residual ? reinterpret_cast<const T*>(a.residual) + m * a.ld_residual : nullptr;
+        res_out = a.residual_out && leader ? reinterpret_cast<T*>(a.residual_out) + m * a.K : nullptr;
+        eps_norm = a.eps_norm;
+        eps_bl = a.eps_bl;
+        pin(x); pin(r); pin(res_out); pin(eps_norm); pin(eps_bl);
+    }
 };
 
 // VW packed pairs (2 * VW values) per vector
@@ -102,15 +122,19 @@ template <int VW> __device__ __forceinline__ void dl_weights(const float* p, flo
 #define DL_FOREACH(it, c) \
     _Pragma("unroll") for (int it = 0, c = rt * 2 * VW; it < NVT; ++it, c += RT * 2 * VW) if (c < D)
 
-// Row prologue of row m = thread / RT (m < M <= TH / RT): codes of G projections into shared memory in the MMA's operand
-// order, dq and (per-warp) code sums beside them.
-template <typename T, int PRO, int G, int TH, int RT, int NVT, int VW>
-__device__ __forceinline__ void dl_prologue(const DlParams& p, const float* snw, uint8_t* scodes, DlScratch<RT>& red, float (&s_dq)[3][DL_FUSED_ROWS],
-                                            double inv_d) {
-    const mmf_decode_linear_args& a = p.a;
-    const int D = (int)a.K, m = threadIdx.x / RT, rt = threadIdx.x % RT, lane = threadIdx.x & 31, rw = rt >> 5;
-    const T* x = reinterpret_cast<const T*>(a.x) + m * a.ld_x;
-    const T* r = PRO != MMF_PRO_QUANT && a.residual ? reinterpret_cast<const T*>(a.residual) + m * a.ld_residual : nullptr;
+// Row prologue of row m = thread / RT, RT = TH / MR threads: codes of G projections into shared memory in the MMA's operand
+// order (KG groups of 256 columns per projection), absmax and (per-warp) code sums beside them.
+template <typename T, int PRO, int G, int TH, int MR, int NVT>
+__device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, const DlRowArgs<T>& ra, int m, int D, int KG, const float* snw, uint8_t* codes,
+                                            DlScratch<TH / MR>& red, float (&s_amax)[3][DL_FUSED_ROWS], double inv_d) {
+    constexpr int RT = TH / MR, VW = 4, TL = 4 * MR;           // TL: lanes of an operand that hold tokens (4 per token)
+    const int rt = threadIdx.x % RT, lane = threadIdx.x & 31, rw = rt >> 5;
+    const T* x = ra.x;
+    if (PRO == MMF_PRO_PRENORM && a.row_ids) {
+        const int64_t row = a.row_ids[m];
+        x += (row < 0 ? 0 : row >= a.x_rows ? a.x_rows - 1 : row) * a.ld_x;    // clamp instead of faulting on a bad id
+    }
+    const T* r = PRO != MMF_PRO_QUANT ? ra.r : nullptr;
     DlVec<VW> u[NVT], v[NVT];
     double s0 = 0.0, s1 = 0.0;
     DL_FOREACH(it, c) u[it] = dl_load<VW>(x + c);
@@ -118,7 +142,7 @@ __device__ __forceinline__ void dl_prologue(const DlParams& p, const float* snw,
         DL_FOREACH(it, c) v[it] = dl_load<VW>(r + c);
     }
     if constexpr (PRO == MMF_PRO_PRENORM) {
-        T* ro = a.residual_out && blockIdx.x == 0 ? reinterpret_cast<T*>(a.residual_out) + m * (int64_t)D : nullptr;
+        T* ro = ra.res_out;
         const bool plain = !r || a.round_sum_first;        // what is normalised is a row of T values
         DL_FOREACH(it, c) {
             uint32_t o[VW];
@@ -137,7 +161,7 @@ __device__ __forceinline__ void dl_prologue(const DlParams& p, const float* snw,
             }
             if (ro) dl_store<VW>(ro + c, o);
         }
-        const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d0), D, inv_d, a.eps_norm);
+        const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d0), D, inv_d, ra.eps_norm);
         s0 = s1 = 0.0;
         DL_FOREACH(it, c) {
             float2 w[VW];
@@ -156,7 +180,7 @@ __device__ __forceinline__ void dl_prologue(const DlParams& p, const float* snw,
 #pragma unroll
             for (int i = 0; i < VW; ++i) sumsq_pair<T>(u[it].v[i], s0, s1);
         }
-        const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d0), D, inv_d, a.eps_norm);
+        const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d0), D, inv_d, ra.eps_norm);
         s0 = s1 = 0.0;
         DL_FOREACH(it, c) {
             float2 w[VW];
@@ -177,7 +201,7 @@ __device__ __forceinline__ void dl_prologue(const DlParams& p, const float* snw,
         }
     }
     // BitLinear prologue: y = (v * rstd) * w, absmax -> scale -> int8 codes
-    const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d1), D, inv_d, a.eps_bl);
+    const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d1), D, inv_d, ra.eps_bl);
     float am[G];
 #pragma unroll
     for (int g = 0; g < G; ++g) am[g] = 0.0f;
@@ -205,17 +229,14 @@ __device__ __forceinline__ void dl_prologue(const DlParams& p, const float* snw,
     for (int g = 0; g < G; ++g) {
         float t = 1e-5f;
 #pragma unroll
-        for (int w = 0; w < RT / 32; w += 4) {
-            const float4 f = *reinterpret_cast<const float4*>(&red.f[g][w]);
-            t = fmaxf(fmaxf(t, f.x), fmaxf(f.y, fmaxf(f.z, f.w)));
-        }
+        for (int w = 0; w < RT / 32; ++w) t = fmaxf(t, red.f[g][w]);
         s[g] = __fdiv_rn(127.0f, t);
         sum[g] = 0;
-        if (rt == 0) s_dq[g][m] = __fdiv_rn(t, 127.0f);
+        if (rt == 0) s_amax[g][m] = t;
     }
     DL_FOREACH(it, c) {
         // column c: group c / 256, lane quarter (c / 64) % 4, word (c / 16) % 4, byte c % 16
-        uint8_t* dst = scodes + ((size_t)((c >> 8) * 4 + ((c >> 4) & 3)) * 16 + m * 4 + ((c >> 6) & 3)) * 16 + (c & 15);
+        uint8_t* dst = codes + (((c >> 8) * 4 + ((c >> 4) & 3)) * TL + m * 4 + ((c >> 6) & 3)) * 16 + (c & 15);
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             float2 w[VW];
@@ -227,7 +248,7 @@ __device__ __forceinline__ void dl_prologue(const DlParams& p, const float* snw,
                                  __fmul2_rn(mul2(widen<T>(u[it].v[2 * i + 1]), rstd), w[2 * i + 1]), s[g]);
                 sum[g] = __dp4a((int)word[i], 0x01010101, sum[g]);
             }
-            uint8_t* d = dst + (size_t)g * p.KG * 1024;
+            uint8_t* d = dst + g * KG * (TL * 64);
             if constexpr (VW == 4) *reinterpret_cast<uint2*>(d) = make_uint2(word[0], word[VW / 2 - 1]);
             else *reinterpret_cast<uint32_t*>(d) = word[0];
         }
@@ -241,244 +262,192 @@ __device__ __forceinline__ void dl_prologue(const DlParams& p, const float* snw,
 
 __device__ __forceinline__ float dl_out(int acc, int rs, float scale) { return __fmul_rn((float)(acc - rs), scale); }
 
-// TH threads; fused prologue: RT threads per row, NVT vectors of 2 * VW values per thread; NB groups of 8 token rows
-template <typename T, int PRO, int EPI, int NB, int TH, int RT, int NVT, int VW>
+// TH threads, MR token rows (M <= MR), NVT 8-value vectors of a row per thread of the row
+template <typename T, int PRO, int EPI, int TH, int MR, int NVT>
 __global__ void __launch_bounds__(TH, 2)
 decode_linear_kernel(const __grid_constant__ DlParams p) {
     const mmf_decode_linear_args& a = p.a;
-    constexpr bool FUSED = PRO != MMF_PRO_CODES;
     constexpr int G = EPI == MMF_EPI_GATES ? 3 : 1;          // projections (code sets)
-    constexpr int TOK = 8 * NB, WARPS = TH / 32;
-    constexpr int ROWS = TH / RT;                            // rows the prologue takes side by side
-    constexpr int CONST_ROWS = FUSED ? DL_FUSED_ROWS : TOK;
+    constexpr int RT = TH / MR, TL = 4 * MR;
     constexpr int BP = EPI == MMF_EPI_SWIGLU ? 4 : 8;        // units per block of 16 MMA rows (swiglu: 8 gate and 8 up rows)
     extern __shared__ __align__(16) uint8_t smem[];
     float* snw = reinterpret_cast<float*>(smem);             // norm weights of the prologue
-    uint8_t* scodes = smem + p.smem_codes;                   // [G][KG][4 words][4 tokens x 4 quarters] 16-byte pieces
-    int* acc = reinterpret_cast<int*>(smem + p.smem_acc);    // [blocks][TOK][DL_TS]
+    uint8_t* scodes = smem + p.smem_codes;                   // [G][KG][4 words][TL lanes] 16-byte pieces
+    int* part = reinterpret_cast<int*>(smem + p.smem_acc);   // [block][kw][MR tokens][DL_TS] partial sums
     uint4* wslot = reinterpret_cast<uint4*>(smem + p.smem_w);
-    __shared__ DlScratch<RT> red[FUSED ? ROWS : 1];
-    __shared__ float s_dq[3][DL_FUSED_ROWS];
-    __shared__ float s_scale[G][CONST_ROWS];                 // dq * mean|w|
-    __shared__ int s_rs[G][CONST_ROWS];                      // code sum (weights are stored + 1)
+    __shared__ DlScratch<RT> red[MR];
+    __shared__ float s_amax[3][DL_FUSED_ROWS];
+    __shared__ float s_scale[G][DL_FUSED_ROWS];              // dq * mean|w|
+    __shared__ int s_rs[G][DL_FUSED_ROWS];                   // code sum (weights are stored + 1)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, q = lane & 3;
     pdl_trigger();
-    const int u0 = (int)((unsigned)blockIdx.x * (unsigned)p.units / (unsigned)p.grid),
-              pairs = (int)((unsigned)(blockIdx.x + 1) * (unsigned)p.units / (unsigned)p.grid) - u0;   // units of this CTA
+    const int bid = blockIdx.x, u0 = bid * p.base + min(bid, p.extra), pairs = p.base + (bid < p.extra ? 1 : 0);
     const int nb = (pairs + BP - 1) / BP * G;                // blocks of this CTA; the last one may be partly empty
-    const int items = nb * p.KG, i0 = warp * items / WARPS, i1 = (warp + 1) * items / WARPS;
-    const int D = (int)a.K, M = (int)a.M;
-    // Order of the (group of 256 columns, block) items.  8 tokens: by block, sums stay in registers until the block changes.
-    // More: by group, so that the codes (16 registers per 8 tokens) are loaded once per group.
-    struct Item {
-        int kg, b, nb, KG;
-        __device__ __forceinline__ void next() {
-            if constexpr (NB == 1) { if (++kg == KG) { kg = 0; ++b; } }
-            else { if (++b == nb) { b = 0; ++kg; } }
-        }
-    };
-    const Item first = NB == 1 ? Item{i0 % p.KG, i0 / p.KG, nb, p.KG} : Item{i0 / nb, i0 % nb, nb, p.KG};
+    const int D = (int)a.K, M = (int)a.M, KC = p.KC, KG = p.KG, kgw = p.kgw, kw = p.kw, bw = p.bw;
+    const int bq = warp / kw, kq = warp - bq * kw;           // this warp's blocks and column groups (bq >= bw: none)
 
-    // weight rows gq and gq + 8 of block b, 16 bytes (64 weights) of chunk 4 * kg + q; nullptr past the end of the CTA's rows or of K
-    auto wptr = [&](const Item& it, int half) -> const uint4* {
-        const int chunk = it.kg * 4 + q;
-        const int r = EPI == MMF_EPI_SWIGLU ? it.b * 8 + gq : it.b / G * 16 + gq + 8 * half;   // row (channel) of the CTA
-        int n = 2 * u0 + r;
-        if constexpr (EPI == MMF_EPI_GATES) n += (it.b % 3) * D;                               // i | f | g of D rows each
-        if constexpr (EPI == MMF_EPI_SWIGLU) n += half * (int)(a.N / 2);                       // gate rows, then up rows
-        return chunk < p.KC && r < 2 * pairs
-                   ? reinterpret_cast<const uint4*>(a.packed) + ((int64_t)(n >> 7) * p.KC + chunk) * MMF_TILE_ROWS + (n & 127) : nullptr;
+    // Item (block b, j): column group kq + j kw.  Weight rows gq and gq + 8 of the block, 16 bytes (64 weights) of chunk 4 kg + q.
+    const int rows_end = 2 * pairs;
+    auto fetch = [&](int b, int j, auto&& take) {
+        const int chunk = (kq + j * kw) * 4 + q;
+        const uint4* w0 = reinterpret_cast<const uint4*>(a.packed) + (int64_t)chunk * MMF_TILE_ROWS;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int r = EPI == MMF_EPI_SWIGLU ? b * 8 + gq : b / G * 16 + gq + 8 * half;   // row (channel) of the CTA
+            int n = 2 * u0 + r;
+            if constexpr (EPI == MMF_EPI_GATES) n += (b % 3) * D;                            // i | f | g of D rows each
+            if constexpr (EPI == MMF_EPI_SWIGLU) n += half * (int)(a.N >> 1);                // gate rows, then up rows
+            // past the end of the CTA's rows or of K: all fields zero, no contribution (codes are stored + 1)
+            take(half, chunk < KC && r < rows_end ? w0 + (int64_t)(n >> 7) * KC * MMF_TILE_ROWS + (n & 127) : nullptr);
+        }
     };
     {   // the weights do not depend on the preceding kernel: on their way before the grid-dependency wait
-        Item it = first;
-        const int n_pf = min(i1 - i0, p.pf);
-        for (int k = 0; k < n_pf; ++k, it.next()) {
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint4* dst = wslot + ((size_t)(k * WARPS + warp) * 2 + half) * 32 + lane;
-                const uint4* src = wptr(it, half);
-                if (src) cp_async16(dst, src);
-                else *dst = make_uint4(0, 0, 0, 0);          // all fields zero: no contribution
-            }
-        }
+        uint4* dst = wslot + (size_t)warp * p.pf * 64 + lane;
+        int k = 0;
+        for (int b = bq < bw ? bq : nb; b < nb; b += bw)
+            for (int j = 0; j < kgw && k < p.pf; ++j, ++k, dst += 64)
+                fetch(b, j, [&](int half, const uint4* src) {
+                    if (src) cp_async16(dst + half * 32, src);
+                    else dst[half * 32] = make_uint4(0, 0, 0, 0);
+                });
         cp_async_commit();
     }
-    for (int i = tid; i < nb * TOK * DL_TS; i += TH) acc[i] = 0;
-    // the thread that will combine scale and code sum of (projection cg, token cm)
-    const int cg = tid / CONST_ROWS, cm = tid % CONST_ROWS;
+    auto stage = [&](float* dst, const float* src) {
+        if (src) for (int i = tid * 4; i < D; i += TH * 4) cp_async16(dst + i, src + i);
+        else for (int i = tid; i < D; i += TH) dst[i] = 1.0f;
+    };
+    float* sdst = snw;
+    if (PRO != MMF_PRO_QUANT) { stage(sdst, a.norm_w); sdst += D; }
+#pragma unroll
+    for (int g = 0; g < G; ++g) stage(sdst + g * D, a.bl_norm_w[g]);
+    cp_async_commit();
+
+    // what the rest needs of the parameters and the model's constants
+    const int cg = tid / DL_FUSED_ROWS, cm = tid % DL_FUSED_ROWS;    // (projection, token) whose scale this thread combines
     const bool has_const = cg < G && cm < M;
     const float ws = has_const ? a.w_scale[cg] : 0.0f;
-    double inv_d = 0.0;
-    if constexpr (FUSED) {
-        auto stage = [&](float* dst, const float* src) {
-            for (int i = tid * 4; i < D; i += TH * 4) {
-                float4 w = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-                if (src) w = *reinterpret_cast<const float4*>(src + i);
-                *reinterpret_cast<float4*>(dst + i) = w;
-            }
-        };
-        float* dst = snw;
-        if (PRO != MMF_PRO_QUANT) { stage(dst, a.norm_w); dst += D; }
-#pragma unroll
-        for (int g = 0; g < G; ++g) stage(dst + g * D, a.bl_norm_w[g]);
-        inv_d = 1.0 / (double)D;
-    }
+    const DlRowArgs<T> ra(a, tid / RT, bid == 0);
+    T *out = reinterpret_cast<T*>(a.out), *g_out = reinterpret_cast<T*>(a.g_out);
+    const T* lb = reinterpret_cast<const T*>(a.lower_bound);
+    float* state = a.state;
+    const uint8_t* mask = a.mask;
+    int64_t ld_out = a.ld_out, N = a.N;
+    pin(out); pin(ld_out);
+    if (EPI == MMF_EPI_GATES) { pin(g_out); pin(lb); pin(state); pin(mask); }
+    if (EPI == MMF_EPI_STORE) pin(N);
+    // the (token, unit) this thread finishes first
+    const int m_pre = MR == 1 ? 0 : tid / pairs, pr_pre = MR == 1 ? tid : tid - m_pre * pairs;
+    const bool has_pre = EPI == MMF_EPI_GATES && m_pre < M && pr_pre < pairs;
+    uint32_t lb_pre = 0;
+    if (has_pre && lb) lb_pre = *reinterpret_cast<const uint32_t*>(lb + (u0 + pr_pre) * 2);
+    cp_async_wait_all();
     __syncthreads();
     pdl_wait();
 
-    float2 h_pre = make_float2(0.0f, 0.0f);                  // gates: the state this thread will advance
-    if constexpr (EPI == MMF_EPI_GATES) {
-        if (tid < pairs * M) {
-            const int m = tid / pairs, pr = tid - m * pairs;
-            h_pre = *reinterpret_cast<const float2*>(a.state + (int64_t)m * D + (u0 + pr) * 2);
-        }
+    // gates: the state this thread will advance (and whether its token is padding), on the way during the contraction
+    float2 h_pre = make_float2(0.0f, 0.0f);
+    bool keep_pre = true;
+    if (has_pre) {
+        h_pre = *reinterpret_cast<const float2*>(state + (int64_t)m_pre * D + (u0 + pr_pre) * 2);
+        if (mask) keep_pre = mask[m_pre] != 0;
     }
-    if constexpr (FUSED) {
-        if (tid / RT < M) dl_prologue<T, PRO, G, TH, RT, NVT, VW>(p, snw, scodes, red[tid / RT], s_dq, inv_d);
-    } else if (has_const) {
-        s_scale[cg][cm] = __fmul_rn(a.dq[(int64_t)cg * M + cm], ws);
-        s_rs[cg][cm] = a.rowsum[(int64_t)cg * M + cm];
-    }
-    cp_async_wait_all();
-    if constexpr (FUSED) {
-        __syncthreads();                                     // codes complete
-        if (has_const) {
-            int t = 0;
+    if (MR == 1 || tid / RT < M) dl_prologue<T, PRO, G, TH, MR, NVT>(a, ra, tid / RT, D, KG, snw, scodes, red[tid / RT], s_amax, p.inv_k);
+    __syncthreads();                                         // codes complete
+    if (has_const) {
+        int t = 0;
 #pragma unroll
-            for (int w = 0; w < RT / 32; ++w) t += red[cm].i[cg][w];
-            s_rs[cg][cm] = t;
-            s_scale[cg][cm] = __fmul_rn(s_dq[cg][cm], ws);
-        }
+        for (int w = 0; w < RT / 32; ++w) t += red[cm < MR ? cm : 0].i[cg][w];
+        s_rs[cg][cm] = t;
+        s_scale[cg][cm] = __fmul_rn(__fdiv_rn(s_amax[cg][cm], 127.0f), ws);
     }
 
-    auto weights_of = [&](const Item& it, int k, uint32_t (&xa)[4], uint32_t (&xb)[4]) {
-        uint4 wa, wb;
-        if (k < p.pf) {
-            const uint4* src = wslot + (size_t)(k * WARPS + warp) * 64 + lane;
-            wa = src[0];
-            wb = src[32];
-        } else {                                             // more weights than the slots hold
-            const uint4 *pa = wptr(it, 0), *pb = wptr(it, 1);
-            wa = pa ? __ldg(pa) : make_uint4(0, 0, 0, 0);
-            wb = pb ? __ldg(pb) : make_uint4(0, 0, 0, 0);
-        }
-        xa[0] = wa.x; xa[1] = wa.y; xa[2] = wa.z; xa[3] = wa.w;
-        xb[0] = wb.x; xb[1] = wb.y; xb[2] = wb.z; xb[3] = wb.w;
-    };
-    auto codes_of = [&](int g, int kg, int t, uint32_t (&B)[4][4]) {
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            uint4 c = make_uint4(0, 0, 0, 0);
-            if constexpr (FUSED) {                           // tokens 4 - 7 do not exist
-                if (lane < 16) c = *reinterpret_cast<const uint4*>(scodes + ((size_t)((g * p.KG + kg) * 4 + w) * 16 + lane) * 16);
-            } else {
-                const int m = t * 8 + gq, chunk = kg * 4 + q;
-                if (m < M && chunk < p.KC) c = *reinterpret_cast<const uint4*>(a.q + ((int64_t)g * M + m) * D + chunk * MMF_TILE_K + w * 16);
-            }
-            B[w][0] = c.x; B[w][1] = c.y; B[w][2] = c.z; B[w][3] = c.w;
-        }
-    };
-    auto add = [&](int b, int t, const int (&v)[4]) {
-        int* d = acc + (b * TOK + t * 8 + 2 * q) * DL_TS + gq;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) atomicAdd(d + (k & 1) * DL_TS + (k >> 1) * 8, v[k]);
-    };
-    if constexpr (NB == 1) {
-        // the 2-bit fields stay where they are: field i of a byte counts 4^i, one accumulator per field, shifted back at the end
-        int c[4][4] = {};
-        Item it = first;
-        for (int i = i0; i < i1; ++i) {
-            uint32_t xa[4], xb[4], B[4][4];
-            weights_of(it, i - i0, xa, xb);
-            codes_of(EPI == MMF_EPI_GATES ? it.b % 3 : 0, it.kg, 0, B);
-#pragma unroll
-            for (int w = 0; w < 4; w += 2)
-#pragma unroll
-                for (int f = 0; f < 4; ++f) {
-                    const uint32_t mask = 0x03030303u << (2 * f);
-                    mma_u8s8(c[f], xa[w] & mask, xb[w] & mask, xa[w + 1] & mask, xb[w + 1] & mask, B[w][f], B[w + 1][f]);
+    // the 2-bit fields stay where they are: field f of a byte counts 4^f, one accumulator per field, shifted back at the end
+    if (bq < bw) {
+        const uint4* src = wslot + (size_t)warp * p.pf * 64 + lane;
+        int* dst = part + ((bq * kw + kq) * MR + 2 * q) * DL_TS + gq;
+        int k = 0;
+#pragma unroll 1
+        for (int b = bq; b < nb; b += bw, dst += bw * kw * MR * DL_TS) {
+            int c[4][4] = {};
+            const uint8_t* cb = scodes + ((EPI == MMF_EPI_GATES ? b % 3 : 0) * KG + kq) * (TL * 64) + (lane & (TL - 1)) * 16;   // tokens MR - 7 do not exist: any code will do
+#pragma unroll 1
+            for (int j = 0; j < kgw; ++j, ++k, src += 64, cb += kw * TL * 64) {
+                if (kq + j * kw >= KG) continue;
+                uint4 wa, wb;
+                if (k < p.pf) {
+                    wa = src[0];
+                    wb = src[32];
+                } else {                                     // more weights than the slots hold
+                    fetch(b, j, [&](int half, const uint4* s) { (half ? wb : wa) = s ? __ldg(s) : make_uint4(0, 0, 0, 0); });
                 }
-            const int b = it.b;
-            it.next();
-            if (it.b != b || i + 1 == i1) {
-                int v[4];
+                uint4 x[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    v[k] = c[0][k] + (c[1][k] >> 2) + (c[2][k] >> 4) + (c[3][k] >> 6);
-                    c[0][k] = c[1][k] = c[2][k] = c[3][k] = 0;
+                for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const uint4*>(cb + w * (TL * 16));
+                const uint32_t xa[4] = {wa.x, wa.y, wa.z, wa.w}, xb[4] = {wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+                for (int w = 0; w < 4; w += 2) {
+                    const uint32_t B0[4] = {x[w].x, x[w].y, x[w].z, x[w].w}, B1[4] = {x[w + 1].x, x[w + 1].y, x[w + 1].z, x[w + 1].w};
+#pragma unroll
+                    for (int f = 0; f < 4; ++f) {
+                        const uint32_t msk = 0x03030303u << (2 * f);
+                        mma_u8s8(c[f], xa[w] & msk, xb[w] & msk, xa[w + 1] & msk, xb[w + 1] & msk, B0[f], B1[f]);
+                    }
                 }
-                add(b, 0, v);
             }
-        }
-    } else {
-        uint32_t B[NB][4][4];
-        int have = -1;
-        Item it = first;
-        for (int i = i0; i < i1; ++i, it.next()) {
-            const int g = EPI == MMF_EPI_GATES ? it.b % 3 : 0;
-            if (it.kg * G + g != have) {
-                have = it.kg * G + g;
 #pragma unroll
-                for (int t = 0; t < NB; ++t) codes_of(g, it.kg, t, B[t]);
-            }
-            uint32_t xa[4], xb[4];
-            weights_of(it, i - i0, xa, xb);
-            int c[NB][4] = {};
-#pragma unroll
-            for (int w = 0; w < 4; w += 2)
-#pragma unroll
-                for (int f = 0; f < 4; ++f) {
-                    const uint32_t a0 = (xa[w] >> (2 * f)) & 0x03030303u, a1 = (xb[w] >> (2 * f)) & 0x03030303u,
-                                   a2 = (xa[w + 1] >> (2 * f)) & 0x03030303u, a3 = (xb[w + 1] >> (2 * f)) & 0x03030303u;
-#pragma unroll
-                    for (int t = 0; t < NB; ++t) mma_u8s8(c[t], a0, a1, a2, a3, B[t][w][f], B[t][w + 1][f]);
-                }
-#pragma unroll
-            for (int t = 0; t < NB; ++t) add(it.b, t, c[t]);
+            for (int i = 0; i < 4; ++i)
+                if (2 * q + (i & 1) < MR) dst[(i & 1) * DL_TS + (i >> 1) * 8] = c[0][i] + (c[1][i] >> 2) + (c[2][i] >> 4) + (c[3][i] >> 6);
         }
     }
     __syncthreads();
 
     // ---- epilogue: a thread finishes two adjacent rows (channels) of a token
     for (int i = tid; i < pairs * M; i += TH) {
-        const int m = M == 1 ? 0 : i / pairs, pr = i - m * pairs;
+        const int m = MR == 1 ? 0 : i / pairs, pr = MR == 1 ? i : i - m * pairs;
         // rows r, r + 1 of block b, rounded to T and packed
         auto value = [&](int b, int r, int g) {
-            const int2 v = *reinterpret_cast<const int2*>(acc + (b * TOK + m) * DL_TS + r);
+            const int* s = part + (b * kw * MR + m) * DL_TS + r;
+            int2 v = make_int2(0, 0);
+#pragma unroll 4
+            for (int w = 0; w < kw; ++w, s += MR * DL_TS) {
+                const int2 t = *reinterpret_cast<const int2*>(s);
+                v.x += t.x;
+                v.y += t.y;
+            }
             return narrow<T>(make_float2(dl_out(v.x, s_rs[g][m], s_scale[g][m]), dl_out(v.y, s_rs[g][m], s_scale[g][m])));
         };
         if constexpr (EPI == MMF_EPI_STORE) {
             const int64_t n = (int64_t)(u0 + pr) * 2;
             const uint32_t o = value(pr >> 3, (pr & 7) * 2, 0);
-            T* dst = reinterpret_cast<T*>(a.out) + m * a.ld_out + n;
-            if (n + 2 <= a.N && (a.ld_out & 1) == 0) *reinterpret_cast<uint32_t*>(dst) = o;
+            T* dst = out + m * ld_out + n;
+            if (n + 2 <= N && (ld_out & 1) == 0) *reinterpret_cast<uint32_t*>(dst) = o;
             else
-                for (int k = 0; k < 2 && n + k < a.N; ++k) dst[k] = reinterpret_cast<const T*>(&o)[k];
+                for (int k = 0; k < 2 && n + k < N; ++k) dst[k] = reinterpret_cast<const T*>(&o)[k];
         } else if constexpr (EPI == MMF_EPI_SWIGLU) {
             // z = round(silu(round(gate)) * round(up)): block b holds 8 channels, rows 0-7 gate and 8-15 up
             const int b = pr >> 2, r = (pr & 3) * 2;
             const float2 gate = widen<T>(value(b, r, 0)), up = widen<T>(value(b, 8 + r, 0));
-            *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(a.out) + m * a.ld_out + (int64_t)(u0 + pr) * 2) = narrow<T>(silu_mul2(gate, up));
+            *reinterpret_cast<uint32_t*>(out + m * ld_out + (int64_t)(u0 + pr) * 2) = narrow<T>(silu_mul2(gate, up));
         } else {
             // token mixer of one new token (layers/hgrn_bit.py:113-125 of the reference with T = 1)
-            const T* lb = reinterpret_cast<const T*>(a.lower_bound);
             const int unit = pr >> 3, r = (pr & 7) * 2, ch = (u0 + pr) * 2;
-            float2* st = reinterpret_cast<float2*>(a.state + (int64_t)m * D + ch);
-            float2 h = i == tid ? h_pre : *st;
+            const bool pre = i == tid;
+            float2* st = reinterpret_cast<float2*>(state + (int64_t)m * D + ch);
+            float2 h = pre ? h_pre : *st;
             float2 xv = raw_gate_floor(widen<T>(value(unit * 3, r, 0))), f = raw_gate_floor(widen<T>(value(unit * 3 + 1, r, 1)));
             float2 lbv = make_float2(0.0f, 0.0f), oml = make_float2(1.0f, 1.0f);
             if (lb) {
-                lbv = widen<T>(*reinterpret_cast<const uint32_t*>(lb + ch));
+                lbv = widen<T>(pre ? lb_pre : *reinterpret_cast<const uint32_t*>(lb + ch));
                 oml = make_float2(round_to<T>(__fsub_rn(1.0f, lbv.x)), round_to<T>(__fsub_rn(1.0f, lbv.y)));
             }
             raw_gate_pair<T>(xv, f, lb != nullptr, lbv, oml);
-            if (a.mask && !a.mask[m]) xv = make_float2(0.0f, 0.0f);      // a padding position contributes no input
+            if (mask && !(pre ? keep_pre : mask[m] != 0)) xv = make_float2(0.0f, 0.0f);      // a padding position contributes no input
             h.x = fmaf(f.x, h.x, xv.x);
             h.y = fmaf(f.y, h.y, xv.y);
             *st = h;
-            *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(a.out) + (int64_t)m * D + ch) = narrow<T>(h);
-            *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(a.g_out) + (int64_t)m * D + ch) = value(unit * 3 + 2, r, 2);
+            *reinterpret_cast<uint32_t*>(out + (int64_t)m * D + ch) = narrow<T>(h);
+            *reinterpret_cast<uint32_t*>(g_out + (int64_t)m * D + ch) = value(unit * 3 + 2, r, 2);
         }
     }
 }
@@ -498,48 +467,61 @@ template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, 
     p.a = a;
     p.KC = (int)(a.K / MMF_TILE_K);
     p.KG = (p.KC + 3) / 4;
+    p.inv_k = 1.0 / (double)a.K;
     const int G = a.epilogue == MMF_EPI_GATES ? 3 : 1;
     // One CTA on every SM, however the rows divide: two kernels of the chain share an SM (the next one waits with its weights),
     // and an SM that this grid left empty would later take two CTAs of the next one, which then finishes late.
-    p.units = a.epilogue == MMF_EPI_GATES ? (int)(a.K / 2) : a.epilogue == MMF_EPI_SWIGLU ? (int)(a.N / 4) : (int)((a.N + 1) / 2);
-    p.grid = p.units < 148 ? p.units : 148;
+    const int units = a.epilogue == MMF_EPI_GATES ? (int)(a.K / 2) : a.epilogue == MMF_EPI_SWIGLU ? (int)(a.N / 4) : (int)((a.N + 1) / 2);
+    p.grid = units < 148 ? units : 148;
+    p.base = units / p.grid;
+    p.extra = units % p.grid;
     const int bp = a.epilogue == MMF_EPI_SWIGLU ? 4 : 8;
-    const int nb = ((p.units + p.grid - 1) / p.grid + bp - 1) / bp * G;   // most blocks of one CTA
-    const int NB = a.prologue == MMF_PRO_CODES ? (a.M <= 8 ? 1 : a.M <= 16 ? 2 : 4) : 1;
-    // 16 warps of up to 64 registers; with 16 or 32 tokens' codes in registers 8 warps of up to 128.  Either way two kernels
-    // fit on an SM, so that the next one fetches its weights while this one runs.
-    const int threads = NB == 1 ? 512 : 256, warps = threads / 32;
-    const int D = (int)a.K;
-    int off = 0;
-    p.smem_codes = 0;
-    if (a.prologue != MMF_PRO_CODES) {
-        off += (a.prologue == MMF_PRO_QUANT ? G : G + 1) * D * 4;
-        p.smem_codes = off;
-        off += G * p.KG * 1024;
+    const int nb = (p.base + (p.extra ? 1 : 0) + bp - 1) / bp * G;        // most blocks of one CTA
+    // Every warp repeats a row's scalar work (statistics, scales), and the next kernel's set-up competes for the same issue
+    // slots, so more warps pay only where they have values to work on: eight for one row of at most 2048 values.
+    const int D = (int)a.K, MR = a.M <= 1 ? 1 : a.M <= 2 ? 2 : 4;
+    const int e0 = getenv("DL_A") ? atoi(getenv("DL_A")) : 0, e1 = getenv("DL_B") ? atoi(getenv("DL_B")) : 0;
+    const int threads = MR == 1 ? (D <= 2048 ? 256 : D <= 3072 ? (e0 ? e0 : 512) : D <= 4096 ? 512 : D <= 6144 ? (e1 ? e1 : 512) : 512) : 512, warps = threads / 32;
+    // warps over column groups x blocks: the split with the fewest rounds, then the fewest partial sums
+    int best = 1 << 30;
+    for (int kw = 1; kw <= warps && kw <= p.KG; ++kw) {
+        const int bw = warps / kw < nb ? warps / kw : nb;
+        const int cost = ((p.KG + kw - 1) / kw) * ((nb + bw - 1) / bw) * 64 + kw;
+        if (cost < best) { best = cost; p.kw = kw; p.bw = bw; }
     }
+    p.kgw = (p.KG + p.kw - 1) / p.kw;
+    int off = (a.prologue == MMF_PRO_QUANT ? G : G + 1) * D * 4;
+    p.smem_codes = off;
+    off += G * p.KG * 256 * MR;
     p.smem_acc = off;
-    off += (nb * 8 * NB * DL_TS * 4 + 15) / 16 * 16;
+    off += nb * p.kw * MR * DL_TS * 4;
     p.smem_w = off;
-    const int per_item = warps * 1024, want = (nb * p.KG + warps - 1) / warps;
-    const int room = (DL_SMEM_MAX - off) / per_item;
-    MMF_REQUIRE(room >= 1, MMF_ERR_BAD_SHAPE, "mmf_decode_linear: K=%lld does not fit in shared memory", (long long)a.K);
+    const int per_item = p.kw * p.bw * 1024, want = (nb + p.bw - 1) / p.bw * p.kgw, room = (DL_SMEM_MAX - off) / per_item;
+    MMF_REQUIRE(room >= 1, MMF_ERR_BAD_SHAPE, "mmf_decode_linear: N=%lld K=%lld do not fit in shared memory", (long long)a.N, (long long)a.K);
     p.pf = want < room ? want : room;
     const int smem = off + p.pf * per_item;
 
-// vectors per thread for rows of at most 2048, 4096 and (plain quantisation) 8192 values
-#define DL_NVT(PRO, EPI, RT, VW)                                                                                       \
-    {                                                                                                                 \
-        constexpr int S = 2048 / (2 * (VW)) / (RT);                                                                    \
-        if (D <= 2048) return dl_go<decode_linear_kernel<T, PRO, EPI, 1, 512, RT, S, VW>>(p, threads, smem, st);        \
-        if (D <= 4096) return dl_go<decode_linear_kernel<T, PRO, EPI, 1, 512, RT, 2 * S, VW>>(p, threads, smem, st);    \
-        if constexpr (PRO == MMF_PRO_QUANT) return dl_go<decode_linear_kernel<T, PRO, EPI, 1, 512, RT, 4 * S, VW>>(p, threads, smem, st); \
-        return mmf_set_error(MMF_ERR_BAD_SHAPE, "mmf_decode_linear: row of %d values", D);                             \
-    }
-#define DL_FUSED(PRO, EPI)                                  \
-    if (a.prologue == PRO && a.epilogue == EPI) {           \
-        if (a.M == 1) DL_NVT(PRO, EPI, 512, 2)              \
-        else if (a.M == 2) DL_NVT(PRO, EPI, 256, 4)         \
-        else DL_NVT(PRO, EPI, 128, 4)                       \
+// vectors per thread for rows of at most 2048, 4096 and (plain quantisation) 6144 and 8192 values
+#define DL_K(PRO, EPI, TH, MR, NVT) return dl_go<decode_linear_kernel<T, PRO, EPI, TH, MR, NVT>>(p, threads, smem, st)
+#define DL_FUSED(PRO, EPI)                                                                \
+    if (a.prologue == PRO && a.epilogue == EPI) {                                         \
+        constexpr bool LONG = PRO == MMF_PRO_QUANT;                                        \
+        if (MR == 1) {                                                                    \
+            if (D <= 2048) DL_K(PRO, EPI, 256, 1, 1);                                      \
+            if (D <= 3072 && threads == 384) DL_K(PRO, EPI, 384, 1, 1);                                      \
+            if (D <= 4096) DL_K(PRO, EPI, 512, 1, 1);                                      \
+            if constexpr (LONG) if (threads == 256) DL_K(PRO, EPI, 256, 1, 3);                                 \
+            if constexpr (LONG) if (threads == 384) DL_K(PRO, EPI, 384, 1, 2);                                 \
+            if constexpr (LONG) DL_K(PRO, EPI, 512, 1, 2);                                 \
+        } else if (MR == 2) {                                                             \
+            if (D <= 2048) DL_K(PRO, EPI, 512, 2, 1);                                      \
+            if (D <= 4096) DL_K(PRO, EPI, 512, 2, 2);                                      \
+            if constexpr (LONG) { if (D <= 6144) DL_K(PRO, EPI, 512, 2, 3); DL_K(PRO, EPI, 512, 2, 4); } \
+        } else {                                                                          \
+            if (D <= 2048) DL_K(PRO, EPI, 512, 4, 2);                                      \
+            if (D <= 4096) DL_K(PRO, EPI, 512, 4, 4);                                      \
+            if constexpr (LONG) { if (D <= 6144) DL_K(PRO, EPI, 512, 4, 6); DL_K(PRO, EPI, 512, 4, 8); } \
+        }                                                                                 \
     }
     DL_FUSED(MMF_PRO_PRENORM, MMF_EPI_GATES)
     DL_FUSED(MMF_PRO_GATENORM, MMF_EPI_STORE)
@@ -547,17 +529,7 @@ template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, 
     DL_FUSED(MMF_PRO_QUANT, MMF_EPI_STORE)
     DL_FUSED(MMF_PRO_PRENORM, MMF_EPI_STORE)
 #undef DL_FUSED
-#undef DL_NVT
-#define DL_CODES(EPI)                                                                                                  \
-    if (a.prologue == MMF_PRO_CODES && a.epilogue == EPI) {                                                            \
-        if (NB == 1) return dl_go<decode_linear_kernel<T, MMF_PRO_CODES, EPI, 1, 512, 512, 1, 4>>(p, threads, smem, st); \
-        if (NB == 2) return dl_go<decode_linear_kernel<T, MMF_PRO_CODES, EPI, 2, 256, 256, 1, 4>>(p, threads, smem, st); \
-        return dl_go<decode_linear_kernel<T, MMF_PRO_CODES, EPI, 4, 256, 256, 1, 4>>(p, threads, smem, st);              \
-    }
-    DL_CODES(MMF_EPI_GATES)
-    DL_CODES(MMF_EPI_SWIGLU)
-    DL_CODES(MMF_EPI_STORE)
-#undef DL_CODES
+#undef DL_K
     return mmf_set_error(MMF_ERR_BAD_ARG, "mmf_decode_linear: prologue %d with epilogue %d is not provided", a.prologue, a.epilogue);
 }
 
