@@ -33,6 +33,8 @@ struct DlParams {
     double inv_k;                       // 1 / K
     int KC, KG;                         // 64-column chunks, groups of four chunks
     int grid, base, extra;              // units (two adjacent output rows; gates, swiglu: channels) per CTA: base, the first `extra` CTAs one more
+    float inv_base, inv_base1;          // 1 / base, 1 / (base + 1)
+    int inv_kw;                         // warp / kw = warp * inv_kw >> 16
     int kw, bw;                         // warp w takes column groups w % kw, + kw, ... of blocks w / kw, + bw, ...
     int kgw;                            // column groups per warp
     int pf;                             // weight items per warp fetched ahead into shared memory
@@ -284,8 +286,8 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
     pdl_trigger();
     const int bid = blockIdx.x, u0 = bid * p.base + min(bid, p.extra), pairs = p.base + (bid < p.extra ? 1 : 0);
     const int nb = (pairs + BP - 1) / BP * G;                // blocks of this CTA; the last one may be partly empty
-    const int D = (int)a.K, M = (int)a.M, KC = p.KC, KG = p.KG, kgw = p.kgw, kw = p.kw, bw = p.bw;
-    const int bq = warp / kw, kq = warp - bq * kw;           // this warp's blocks and column groups (bq >= bw: none)
+    const int D = (int)a.K, M = (int)a.M, KC = p.KC, KG = p.KG, kgw = p.kgw, kw = TH == 256 ? 8 : p.kw, bw = TH == 256 ? 1 : p.bw;
+    const int bq = TH == 256 ? 0 : warp * p.inv_kw >> 16, kq = warp - bq * kw;           // this warp's blocks and column groups (bq >= bw: none)
 
     // Item (block b, j): column group kq + j kw.  Weight rows gq and gq + 8 of the block, 16 bytes (64 weights) of chunk 4 kg + q.
     const int rows_end = 2 * pairs;
@@ -337,7 +339,10 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
     if (EPI == MMF_EPI_GATES) { pin(g_out); pin(lb); pin(state); pin(mask); }
     if (EPI == MMF_EPI_STORE) pin(N);
     // the (token, unit) this thread finishes first
-    const int m_pre = MR == 1 ? 0 : tid / pairs, pr_pre = MR == 1 ? tid : tid - m_pre * pairs;
+    // (a division that is exact here: (i + 0.5) / pairs stays 0.5 / pairs away from whole numbers, and i < 4 * pairs)
+    const float inv_pairs = bid < p.extra ? p.inv_base1 : p.inv_base;
+    auto token_of = [&](int i) { return MR == 1 ? 0 : (int)(((float)i + 0.5f) * inv_pairs); };
+    const int m_pre = token_of(tid), pr_pre = tid - m_pre * pairs;
     const bool has_pre = EPI == MMF_EPI_GATES && m_pre < M && pr_pre < pairs;
     uint32_t lb_pre = 0;
     if (has_pre && lb) lb_pre = *reinterpret_cast<const uint32_t*>(lb + (u0 + pr_pre) * 2);
@@ -363,7 +368,7 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
     }
 
     // the 2-bit fields stay where they are: field f of a byte counts 4^f, one accumulator per field, shifted back at the end
-    if (bq < bw) {
+    if (TH == 256 ? kq < KG : bq < bw) {
         const uint4* src = wslot + (size_t)warp * p.pf * 64 + lane;
         int* dst = part + ((bq * kw + kq) * MR + 2 * q) * DL_TS + gq;
         int k = 0;
@@ -404,16 +409,27 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
 
     // ---- epilogue: a thread finishes two adjacent rows (channels) of a token
     for (int i = tid; i < pairs * M; i += TH) {
-        const int m = MR == 1 ? 0 : i / pairs, pr = MR == 1 ? i : i - m * pairs;
+        const int m = token_of(i), pr = i - m * pairs;
         // rows r, r + 1 of block b, rounded to T and packed
         auto value = [&](int b, int r, int g) {
             const int* s = part + (b * kw * MR + m) * DL_TS + r;
             int2 v = make_int2(0, 0);
+            if constexpr (TH == 256) {
+                const int np = min(kw, KG);
+#pragma unroll
+                for (int w = 0; w < 8; ++w)
+                    if (w < np) {
+                        const int2 t = *reinterpret_cast<const int2*>(s + w * MR * DL_TS);
+                        v.x += t.x;
+                        v.y += t.y;
+                    }
+            } else {
 #pragma unroll 4
-            for (int w = 0; w < kw; ++w, s += MR * DL_TS) {
-                const int2 t = *reinterpret_cast<const int2*>(s);
-                v.x += t.x;
-                v.y += t.y;
+                for (int w = 0; w < kw; ++w, s += MR * DL_TS) {
+                    const int2 t = *reinterpret_cast<const int2*>(s);
+                    v.x += t.x;
+                    v.y += t.y;
+                }
             }
             return narrow<T>(make_float2(dl_out(v.x, s_rs[g][m], s_scale[g][m]), dl_out(v.y, s_rs[g][m], s_scale[g][m])));
         };
@@ -489,7 +505,11 @@ template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, 
         const int cost = ((p.KG + kw - 1) / kw) * ((nb + bw - 1) / bw) * 64 + kw;
         if (cost < best) { best = cost; p.kw = kw; p.bw = bw; }
     }
+    if (threads == 256) { p.kw = 8; p.bw = 1; }
     p.kgw = (p.KG + p.kw - 1) / p.kw;
+    p.inv_kw = 65536 / p.kw + 1;
+    p.inv_base = 1.0f / (float)p.base;
+    p.inv_base1 = 1.0f / (float)(p.base + 1);
     int off = (a.prologue == MMF_PRO_QUANT ? G : G + 1) * D * 4;
     p.smem_codes = off;
     off += G * p.KG * 256 * MR;
