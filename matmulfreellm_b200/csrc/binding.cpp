@@ -44,7 +44,7 @@ std::map<std::string, Api> g_apis;   // by path; the pointers stay valid because
 const Api* g_api = nullptr;
 
 int64_t g_launches = 0;    // guarded by the GIL
-int64_t g_fused_rows = MMF_DECODE_LINEAR_MAX_M;
+int64_t g_fused_rows = 2, g_codes_rows = 32, g_head_rows = 8;
 
 PyObject* g_error_class = nullptr;
 PyObject* g_workspace_fn = nullptr;
@@ -538,7 +538,9 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
             s.used = mix;
             const int64_t gu = s.take(2 * M * c.inner * es);
             s.used = std::max(s.used, mix_end);
-            const int64_t q = s.take(std::max({3 * M * h, M * c.inner, Mn * h})), dq = s.take(3 * M * 4), rs = s.take(3 * M * 4);
+            // codes: decode-step contractions want rows of whole 256-column groups, up to 32 of them
+            const int64_t Mc = M <= 8 ? 8 : M <= 16 ? 16 : M <= 32 ? 32 : M;
+            const int64_t q = s.take(Mc * std::max(3 * ((h + 255) & ~255ll), (c.inner + 255) & ~255ll)), dq = s.take(3 * M * 4), rs = s.take(3 * M * 4);
             const int64_t hg_bytes = T > 1 ? g_api->mmf_hgrn_workspace_bytes(B, T, h) : 0, hg = s.take(hg_bytes);
             const at::Tensor mem = at::empty({s.used}, opt.dtype(at::kByte));
             uint8_t* b = mem.data_ptr<uint8_t>();
@@ -552,7 +554,7 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 ++launches;
             };
             // one token per sequence and few sequences: contractions with the row work around them in one kernel
-            const bool decode = T == 1 && M > 0 && M <= g_fused_rows && c.dtype != MMF_F32 && h % MMF_TILE_ROWS == 0 && h <= 4096 && c.inner <= 8192;
+            const bool decode = T == 1 && M > 0 && M <= g_codes_rows && c.dtype != MMF_F32 && h % MMF_TILE_ROWS == 0 && h <= 4096 && c.inner <= 8192;
             const int64_t* gather = decode && ids.defined() && !c.layers.empty() ? ids.data_ptr<int64_t>() : nullptr;
             const uint8_t* x = b + x0;            // residual stream
             if (gather) {                         // the first block reads the embedding rows itself
@@ -579,11 +581,16 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 a.w_scale = l.scale;
                 a.out = out;
                 a.ld_out = ld_out;
+                if (M > g_fused_rows) {
+                    a.codes = Q;
+                    a.dq = DQ;
+                    a.rowsum = RS;
+                }
                 return a;
             };
             auto run = [&](const mmf_decode_linear_args& a) {
                 MMF_CALL(mmf_decode_linear, &a, st);
-                ++launches;
+                launches += a.codes ? 2 : 1;
             };
             if (decode) decode_blocks(c, args_of, run, gather, b + z, b + ifg, b + o, b + gu, mk, states, x, next, advance);
             for (size_t i = 0; i < c.layers.size() && !decode; ++i) {
@@ -622,7 +629,7 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
             const int64_t skip = last_only ? (T - 1) * h * es : 0, ld = last_only ? T * h : h;
             first = c.layers.empty();
             const uint8_t* rows = first ? x : b + z;
-            if (decode && want_logits && !want_hidden) {
+            if (decode && M <= g_head_rows && c.head.N <= 262144 && want_logits && !want_hidden) {
                 mmf_decode_linear_args a = args_of(c.head, MMF_PRO_PRENORM, MMF_EPI_STORE, logits.data_ptr(), c.head.N);
                 a.x = rows; a.ld_x = h;
                 a.residual = first ? nullptr : x; a.ld_residual = h;
@@ -631,10 +638,10 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 a.bl_norm_w[0] = c.head_nw; a.eps_bl = c.head_eps;
                 run(a);
             } else {
-            MMF_CALL(mmf_prenorm_quant, rows + skip, ld, first ? nullptr : x + skip, ld, c.dtype, first ? 0 : 1, c.final_norm_w, c.eps, nullptr,
-                     ptr(hidden), want_logits ? 1 : 0, c.head_nw, nullptr, nullptr, c.head_eps, Q, DQ, RS, Mn, h, st);
-            ++launches;
-            if (want_logits) linear(c.head, logits.data_ptr(), Mn);
+                MMF_CALL(mmf_prenorm_quant, rows + skip, ld, first ? nullptr : x + skip, ld, c.dtype, first ? 0 : 1, c.final_norm_w, c.eps, nullptr,
+                         ptr(hidden), want_logits ? 1 : 0, c.head_nw, nullptr, nullptr, c.head_eps, Q, DQ, RS, Mn, h, st);
+                ++launches;
+                if (want_logits) linear(c.head, logits.data_ptr(), Mn);
             }
         }
         g_launches += launches;
@@ -651,6 +658,8 @@ PyObject* take_launches(PyObject*, PyObject*) {
 }
 PyObject* set_rows(PyObject*, PyObject* const* args, Py_ssize_t) {
     g_fused_rows = PyLong_AsLongLong(args[0]);
+    g_codes_rows = PyLong_AsLongLong(args[1]);
+    g_head_rows = PyLong_AsLongLong(args[2]);
     Py_RETURN_NONE;
 }
 

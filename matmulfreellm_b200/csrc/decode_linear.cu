@@ -11,8 +11,9 @@ extern "C" int mmf_decode_linear(const mmf_decode_linear_args* args, void* strea
     MMF_REQUIRE(a.packed && a.w_scale && a.out, MMF_ERR_BAD_ARG, "mmf_decode_linear: null pointer");
     MMF_REQUIRE(a.M >= 0 && a.N > 0 && a.K > 0 && a.K % MMF_TILE_K == 0 && a.N < (1ll << 24), MMF_ERR_BAD_SHAPE,
                 "mmf_decode_linear: need K %% 64 == 0 (M=%lld N=%lld K=%lld)", (long long)a.M, (long long)a.N, (long long)a.K);
-    MMF_REQUIRE(a.M <= MMF_DECODE_LINEAR_MAX_M, MMF_ERR_BAD_SHAPE, "mmf_decode_linear: at most %d token rows (M=%lld)", MMF_DECODE_LINEAR_MAX_M,
-                (long long)a.M);
+    const int max_m = a.codes ? MMF_DECODE_LINEAR_MAX_M : MMF_DECODE_LINEAR_FUSED_MAX_M;
+    MMF_REQUIRE(a.M <= max_m, MMF_ERR_BAD_SHAPE, "mmf_decode_linear: at most %d token rows (M=%lld)", max_m, (long long)a.M);
+    MMF_REQUIRE(!a.codes || (a.dq && a.rowsum && mmf_aligned(a.codes, 16)), MMF_ERR_BAD_ARG, "mmf_decode_linear: incomplete workspace");
     MMF_REQUIRE(a.x && (a.prologue != MMF_PRO_GATENORM || a.residual), MMF_ERR_BAD_ARG, "mmf_decode_linear: input row missing");
     MMF_REQUIRE(mmf_aligned(a.packed, 16) && mmf_aligned(a.out, 16) && mmf_aligned(a.x, 16) && a.ld_x % 8 == 0 &&
                     (!a.residual || (mmf_aligned(a.residual, 16) && a.ld_residual % 8 == 0)) && (!a.residual_out || mmf_aligned(a.residual_out, 16)) &&
@@ -31,6 +32,8 @@ extern "C" int mmf_decode_linear(const mmf_decode_linear_args* args, void* strea
     } else {
         MMF_REQUIRE(a.epilogue == MMF_EPI_STORE && a.ld_out >= a.N, MMF_ERR_BAD_ARG, "mmf_decode_linear: unknown epilogue or ld_out < N");
     }
+    MMF_REQUIRE(a.prologue == MMF_PRO_QUANT || a.prologue == MMF_PRO_PRENORM || a.prologue == MMF_PRO_GATENORM, MMF_ERR_BAD_ARG,
+                "mmf_decode_linear: prologue %d", a.prologue);
     if (a.M == 0) return MMF_OK;
     return a.dtype == MMF_BF16 ? decode_linear_bf16(a, (cudaStream_t)stream) : decode_linear_fp16(a, (cudaStream_t)stream);
 }

@@ -26,7 +26,9 @@
 namespace {
 
 constexpr int DL_TS = 20;               // accumulator words per (block, token): 16 rows, padded so that a warp's adds do not collide
-constexpr int DL_FUSED_ROWS = MMF_DECODE_LINEAR_MAX_M;   // token rows a CTA takes through the fused prologue
+constexpr int DL_FUSED_ROWS = 4;        // most token rows a CTA takes through the fused prologue
+constexpr int DL_CODES = 0;             // prologue of the kernel whose codes were made by decode_rows_kernel
+constexpr int DL_CODES_THREADS = 384;
 
 struct DlParams {
     mmf_decode_linear_args a;
@@ -124,12 +126,13 @@ template <int VW> __device__ __forceinline__ void dl_weights(const float* p, flo
 #define DL_FOREACH(it, c) \
     _Pragma("unroll") for (int it = 0, c = rt * 2 * VW; it < NVT; ++it, c += RT * 2 * VW) if (c < D)
 
-// Row prologue of row m = thread / RT, RT = TH / MR threads: codes of G projections into shared memory in the MMA's operand
-// order (KG groups of 256 columns per projection), absmax and (per-warp) code sums beside them.
+// Row prologue of row m, RT = TH / MR threads: codes of G projections in the MMA's operand order, absmax and (per-warp) code
+// sums beside them.  Columns c .. c + 15 of a 256-column group are the 16-byte piece ((c / 16) % 4) * word + (c / 64) % 4 of
+// `codes`; a group is 4 * step pieces, a projection KG groups.
 template <typename T, int PRO, int G, int TH, int MR, int NVT>
 __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, const DlRowArgs<T>& ra, int m, int D, int KG, const float* snw, uint8_t* codes,
-                                            DlScratch<TH / MR>& red, float (&s_amax)[3][DL_FUSED_ROWS], double inv_d) {
-    constexpr int RT = TH / MR, VW = 4, TL = 4 * MR;           // TL: lanes of an operand that hold tokens (4 per token)
+                                            int word, int step, DlScratch<TH / MR>& red, float (&s_amax)[G], double inv_d) {
+    constexpr int RT = TH / MR, VW = 4;
     const int rt = threadIdx.x % RT, lane = threadIdx.x & 31, rw = rt >> 5;
     const T* x = ra.x;
     if (PRO == MMF_PRO_PRENORM && a.row_ids) {
@@ -234,11 +237,10 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
         for (int w = 0; w < RT / 32; ++w) t = fmaxf(t, red.f[g][w]);
         s[g] = __fdiv_rn(127.0f, t);
         sum[g] = 0;
-        if (rt == 0) s_amax[g][m] = t;
+        if (rt == 0) s_amax[g] = t;
     }
     DL_FOREACH(it, c) {
-        // column c: group c / 256, lane quarter (c / 64) % 4, word (c / 16) % 4, byte c % 16
-        uint8_t* dst = codes + (((c >> 8) * 4 + ((c >> 4) & 3)) * TL + m * 4 + ((c >> 6) & 3)) * 16 + (c & 15);
+        uint8_t* dst = codes + ((c >> 8) * (4 * step) + ((c >> 4) & 3) * word + ((c >> 6) & 3)) * 16 + (c & 15);
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             float2 w[VW];
@@ -250,7 +252,7 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
                                  __fmul2_rn(mul2(widen<T>(u[it].v[2 * i + 1]), rstd), w[2 * i + 1]), s[g]);
                 sum[g] = __dp4a((int)word[i], 0x01010101, sum[g]);
             }
-            uint8_t* d = dst + g * KG * (TL * 64);
+            uint8_t* d = dst + g * KG * (step * 64);
             if constexpr (VW == 4) *reinterpret_cast<uint2*>(d) = make_uint2(word[0], word[VW / 2 - 1]);
             else *reinterpret_cast<uint32_t*>(d) = word[0];
         }
@@ -264,11 +266,51 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
 
 __device__ __forceinline__ float dl_out(int acc, int rs, float scale) { return __fmul_rn((float)(acc - rs), scale); }
 
-// TH threads, MR token rows (M <= MR), NVT 8-value vectors of a row per thread of the row
+// The row work of a decode step as a kernel of its own: a CTA per token row and projection.  Codes in the operand order of the
+// contraction that follows, 8 * NB tokens side by side.
+template <typename T, int PRO, int TH, int NVT>
+__global__ void __launch_bounds__(TH)
+decode_rows_kernel(const __grid_constant__ mmf_decode_linear_args a, int KG, int NB, double inv_k) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    float* snw = reinterpret_cast<float*>(smem);
+    __shared__ DlScratch<TH> red;
+    __shared__ float s_amax[1];
+    const int m = blockIdx.x, g = blockIdx.y, D = (int)a.K, tid = threadIdx.x;
+    pdl_trigger();
+    auto stage = [&](float* dst, const float* src) {
+        if (src) for (int i = tid * 4; i < D; i += TH * 4) cp_async16(dst + i, src + i);
+        else for (int i = tid; i < D; i += TH) dst[i] = 1.0f;
+    };
+    if (PRO != MMF_PRO_QUANT) stage(snw, a.norm_w);
+    stage(snw + (PRO != MMF_PRO_QUANT ? D : 0), a.bl_norm_w[g]);
+    cp_async_commit();
+    const DlRowArgs<T> ra(a, m, g == 0);
+    uint8_t* codes = reinterpret_cast<uint8_t*>(a.codes) + ((int64_t)g * KG * NB * 128 + (m >> 3) * 128 + (m & 7) * 4) * 16;
+    float* dq = a.dq + (int64_t)g * a.M + m;
+    int32_t* rowsum = a.rowsum + (int64_t)g * a.M + m;
+    pin(codes); pin(dq); pin(rowsum);
+    cp_async_wait_all();
+    __syncthreads();
+    pdl_wait();
+    dl_prologue<T, PRO, 1, TH, 1, NVT>(a, ra, m, D, KG, snw, codes, 32, 32 * NB, red, s_amax, inv_k);
+    __syncthreads();
+    if (tid == 0) {
+        int t = 0;
+#pragma unroll
+        for (int w = 0; w < TH / 32; ++w) t += red.i[0][w];
+        *rowsum = t;
+        *dq = __fdiv_rn(s_amax[0], 127.0f);
+    }
+}
+
+// Fused: TH threads, MR token rows (M <= MR), NVT 8-value vectors of a row per thread of the row.  Codes from
+// decode_rows_kernel: MR = 8 NB token rows; at most TH threads.
 template <typename T, int PRO, int EPI, int TH, int MR, int NVT>
 __global__ void __launch_bounds__(TH, 2)
 decode_linear_kernel(const __grid_constant__ DlParams p) {
     const mmf_decode_linear_args& a = p.a;
+    constexpr bool FUSED = PRO != DL_CODES, CONST8 = FUSED && TH == 256;
+    constexpr int NB = FUSED ? 1 : MR / 8, SC = FUSED ? DL_FUSED_ROWS : MR;
     constexpr int G = EPI == MMF_EPI_GATES ? 3 : 1;          // projections (code sets)
     constexpr int RT = TH / MR, TL = 4 * MR;
     constexpr int BP = EPI == MMF_EPI_SWIGLU ? 4 : 8;        // units per block of 16 MMA rows (swiglu: 8 gate and 8 up rows)
@@ -277,17 +319,18 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
     uint8_t* scodes = smem + p.smem_codes;                   // [G][KG][4 words][TL lanes] 16-byte pieces
     int* part = reinterpret_cast<int*>(smem + p.smem_acc);   // [block][kw][MR tokens][DL_TS] partial sums
     uint4* wslot = reinterpret_cast<uint4*>(smem + p.smem_w);
-    __shared__ DlScratch<RT> red[MR];
-    __shared__ float s_amax[3][DL_FUSED_ROWS];
-    __shared__ float s_scale[G][DL_FUSED_ROWS];              // dq * mean|w|
-    __shared__ int s_rs[G][DL_FUSED_ROWS];                   // code sum (weights are stored + 1)
+    __shared__ DlScratch<FUSED ? RT : 32> red[FUSED ? MR : 1];
+    __shared__ float s_amax[DL_FUSED_ROWS][G];
+    __shared__ float s_scale[G][SC];                         // dq * mean|w|
+    __shared__ int s_rs[G][SC];                              // code sum (weights are stored + 1)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, q = lane & 3;
     pdl_trigger();
     const int bid = blockIdx.x, u0 = bid * p.base + min(bid, p.extra), pairs = p.base + (bid < p.extra ? 1 : 0);
     const int nb = (pairs + BP - 1) / BP * G;                // blocks of this CTA; the last one may be partly empty
-    const int D = (int)a.K, M = (int)a.M, KC = p.KC, KG = p.KG, kgw = p.kgw, kw = TH == 256 ? 8 : p.kw, bw = TH == 256 ? 1 : p.bw;
-    const int bq = TH == 256 ? 0 : warp * p.inv_kw >> 16, kq = warp - bq * kw;           // this warp's blocks and column groups (bq >= bw: none)
+    const int D = (int)a.K, M = (int)a.M, KC = p.KC, KG = p.KG, kgw = p.kgw, kw = CONST8 ? 8 : p.kw, bw = CONST8 ? 1 : p.bw;
+    const int nthr = FUSED ? TH : (int)blockDim.x;
+    const int bq = CONST8 ? 0 : warp * p.inv_kw >> 16, kq = warp - bq * kw;           // this warp's blocks and column groups (bq >= bw: none)
 
     // Item (block b, j): column group kq + j kw.  Weight rows gq and gq + 8 of the block, 16 bytes (64 weights) of chunk 4 kg + q.
     const int rows_end = 2 * pairs;
@@ -315,21 +358,27 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
                 });
         cp_async_commit();
     }
-    auto stage = [&](float* dst, const float* src) {
-        if (src) for (int i = tid * 4; i < D; i += TH * 4) cp_async16(dst + i, src + i);
-        else for (int i = tid; i < D; i += TH) dst[i] = 1.0f;
-    };
-    float* sdst = snw;
-    if (PRO != MMF_PRO_QUANT) { stage(sdst, a.norm_w); sdst += D; }
+    if constexpr (FUSED) {
+        auto stage = [&](float* dst, const float* src) {
+            if (src) for (int i = tid * 4; i < D; i += TH * 4) cp_async16(dst + i, src + i);
+            else for (int i = tid; i < D; i += TH) dst[i] = 1.0f;
+        };
+        float* sdst = snw;
+        if (PRO != MMF_PRO_QUANT) { stage(sdst, a.norm_w); sdst += D; }
 #pragma unroll
-    for (int g = 0; g < G; ++g) stage(sdst + g * D, a.bl_norm_w[g]);
-    cp_async_commit();
+        for (int g = 0; g < G; ++g) stage(sdst + g * D, a.bl_norm_w[g]);
+        cp_async_commit();
+    }
 
     // what the rest needs of the parameters and the model's constants
-    const int cg = tid / DL_FUSED_ROWS, cm = tid % DL_FUSED_ROWS;    // (projection, token) whose scale this thread combines
+    const int cg = tid / SC, cm = tid % SC;                  // (projection, token) whose scale this thread combines
     const bool has_const = cg < G && cm < M;
     const float ws = has_const ? a.w_scale[cg] : 0.0f;
-    const DlRowArgs<T> ra(a, tid / RT, bid == 0);
+    const DlRowArgs<T> ra(a, FUSED ? tid / RT : 0, bid == 0);
+    const uint4* codes = reinterpret_cast<const uint4*>(a.codes) + lane;
+    const float* dq = a.dq + cg * M + cm;
+    const int32_t* rowsum = a.rowsum + cg * M + cm;
+    if (!FUSED) { pin(codes); pin(dq); pin(rowsum); }
     T *out = reinterpret_cast<T*>(a.out), *g_out = reinterpret_cast<T*>(a.g_out);
     const T* lb = reinterpret_cast<const T*>(a.lower_bound);
     float* state = a.state;
@@ -339,7 +388,7 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
     if (EPI == MMF_EPI_GATES) { pin(g_out); pin(lb); pin(state); pin(mask); }
     if (EPI == MMF_EPI_STORE) pin(N);
     // the (token, unit) this thread finishes first
-    // (a division that is exact here: (i + 0.5) / pairs stays 0.5 / pairs away from whole numbers, and i < 4 * pairs)
+    // (a division that is exact here: (i + 0.5) / pairs stays 0.5 / pairs away from whole numbers, and i < 32 * pairs)
     const float inv_pairs = bid < p.extra ? p.inv_base1 : p.inv_base;
     auto token_of = [&](int i) { return MR == 1 ? 0 : (int)(((float)i + 0.5f) * inv_pairs); };
     const int m_pre = token_of(tid), pr_pre = tid - m_pre * pairs;
@@ -357,27 +406,57 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
         h_pre = *reinterpret_cast<const float2*>(state + (int64_t)m_pre * D + (u0 + pr_pre) * 2);
         if (mask) keep_pre = mask[m_pre] != 0;
     }
-    if (MR == 1 || tid / RT < M) dl_prologue<T, PRO, G, TH, MR, NVT>(a, ra, tid / RT, D, KG, snw, scodes, red[tid / RT], s_amax, p.inv_k);
-    __syncthreads();                                         // codes complete
-    if (has_const) {
-        int t = 0;
+    if constexpr (FUSED) {
+        const int m = tid / RT;
+        if (MR == 1 || m < M)
+            dl_prologue<T, PRO, G, TH, MR, NVT>(a, ra, m, D, KG, snw, scodes + m * 64, TL, TL, red[m], s_amax[m], p.inv_k);
+        __syncthreads();                                     // codes complete
+        if (has_const) {
+            int t = 0;
 #pragma unroll
-        for (int w = 0; w < RT / 32; ++w) t += red[cm < MR ? cm : 0].i[cg][w];
-        s_rs[cg][cm] = t;
-        s_scale[cg][cm] = __fmul_rn(__fdiv_rn(s_amax[cg][cm], 127.0f), ws);
+            for (int w = 0; w < RT / 32; ++w) t += red[cm < MR ? cm : 0].i[cg][w];
+            s_rs[cg][cm] = t;
+            s_scale[cg][cm] = __fmul_rn(__fdiv_rn(s_amax[cm][cg], 127.0f), ws);
+        }
+    } else {
+        if constexpr (NB == 1) {                             // all codes of this warp at once: one trip to the L2, not one per item
+            if (bq < bw) {
+                uint4* d = reinterpret_cast<uint4*>(scodes) + (size_t)warp * (G * kgw * 128) + lane;
+                for (int g = 0; g < G; ++g)
+                    for (int j = 0; j < kgw; ++j, d += 128)
+                        if (kq + j * kw < KG) {
+                            const uint4* src = codes + (g * KG + kq + j * kw) * 128;
+#pragma unroll
+                            for (int w = 0; w < 4; ++w) cp_async16(d + w * 32, src + w * 32);
+                        }
+            }
+            cp_async_commit();
+        }
+        if (has_const) {
+            s_scale[cg][cm] = __fmul_rn(*dq, ws);
+            s_rs[cg][cm] = *rowsum;
+        }
+        if (NB == 1) cp_async_wait_all();
     }
 
     // the 2-bit fields stay where they are: field f of a byte counts 4^f, one accumulator per field, shifted back at the end
-    if (TH == 256 ? kq < KG : bq < bw) {
+    if (CONST8 ? kq < KG : bq < bw) {
         const uint4* src = wslot + (size_t)warp * p.pf * 64 + lane;
         int* dst = part + ((bq * kw + kq) * MR + 2 * q) * DL_TS + gq;
         int k = 0;
 #pragma unroll 1
         for (int b = bq; b < nb; b += bw, dst += bw * kw * MR * DL_TS) {
-            int c[4][4] = {};
-            const uint8_t* cb = scodes + ((EPI == MMF_EPI_GATES ? b % 3 : 0) * KG + kq) * (TL * 64) + (lane & (TL - 1)) * 16;   // tokens MR - 7 do not exist: any code will do
+            constexpr int F = NB <= 2 ? 4 : 1;
+            int c[F][NB][4] = {};
+            const int g = EPI == MMF_EPI_GATES ? b % 3 : 0;
+            // codes of the first group.  Fused: tokens MR - 7 do not exist, any code will do
+            const uint4* cb = FUSED ? reinterpret_cast<const uint4*>(scodes) + (g * KG + kq) * (TL * 4) + (lane & (TL - 1))
+                              : NB == 1 ? reinterpret_cast<const uint4*>(scodes) + (size_t)(warp * G + g) * kgw * 128 + lane
+                                        : codes + (g * KG + kq) * (NB * 128);
+            const int cstep = FUSED ? kw * TL * 4 : NB == 1 ? 128 : kw * NB * 128;
+            constexpr int CW = FUSED ? TL : 32;              // pieces per word
 #pragma unroll 1
-            for (int j = 0; j < kgw; ++j, ++k, src += 64, cb += kw * TL * 64) {
+            for (int j = 0; j < kgw; ++j, ++k, src += 64, cb += cstep) {
                 if (kq + j * kw >= KG) continue;
                 uint4 wa, wb;
                 if (k < p.pf) {
@@ -386,35 +465,67 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
                 } else {                                     // more weights than the slots hold
                     fetch(b, j, [&](int half, const uint4* s) { (half ? wb : wa) = s ? __ldg(s) : make_uint4(0, 0, 0, 0); });
                 }
-                uint4 x[4];
-#pragma unroll
-                for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const uint4*>(cb + w * (TL * 16));
                 const uint32_t xa[4] = {wa.x, wa.y, wa.z, wa.w}, xb[4] = {wb.x, wb.y, wb.z, wb.w};
+                if constexpr (F == 4) {
+                    uint4 x[NB][4];
 #pragma unroll
-                for (int w = 0; w < 4; w += 2) {
-                    const uint32_t B0[4] = {x[w].x, x[w].y, x[w].z, x[w].w}, B1[4] = {x[w + 1].x, x[w + 1].y, x[w + 1].z, x[w + 1].w};
+                    for (int t = 0; t < NB; ++t)
 #pragma unroll
-                    for (int f = 0; f < 4; ++f) {
-                        const uint32_t msk = 0x03030303u << (2 * f);
-                        mma_u8s8(c[f], xa[w] & msk, xb[w] & msk, xa[w + 1] & msk, xb[w + 1] & msk, B0[f], B1[f]);
+                        for (int w = 0; w < 4; ++w) x[t][w] = cb[(t * 4 + w) * CW];
+#pragma unroll
+                    for (int w = 0; w < 4; w += 2)
+#pragma unroll
+                        for (int f = 0; f < 4; ++f) {
+                            const uint32_t msk = 0x03030303u << (2 * f);
+#pragma unroll
+                            for (int t = 0; t < NB; ++t) {
+                                const uint32_t B0[4] = {x[t][w].x, x[t][w].y, x[t][w].z, x[t][w].w},
+                                               B1[4] = {x[t][w + 1].x, x[t][w + 1].y, x[t][w + 1].z, x[t][w + 1].w};
+                                mma_u8s8(c[f][t], xa[w] & msk, xb[w] & msk, xa[w + 1] & msk, xb[w + 1] & msk, B0[f], B1[f]);
+                            }
+                        }
+                } else {                                     // accumulators of four fields do not fit in registers: fields shifted down
+#pragma unroll
+                    for (int w = 0; w < 4; w += 2) {
+                        uint4 x[NB][2];
+#pragma unroll
+                        for (int t = 0; t < NB; ++t) {
+                            x[t][0] = cb[(t * 4 + w) * CW];
+                            x[t][1] = cb[(t * 4 + w + 1) * CW];
+                        }
+#pragma unroll
+                        for (int f = 0; f < 4; ++f) {
+                            const uint32_t a0 = (xa[w] >> (2 * f)) & 0x03030303u, a1 = (xb[w] >> (2 * f)) & 0x03030303u,
+                                           a2 = (xa[w + 1] >> (2 * f)) & 0x03030303u, a3 = (xb[w + 1] >> (2 * f)) & 0x03030303u;
+#pragma unroll
+                            for (int t = 0; t < NB; ++t) {
+                                const uint32_t B0[4] = {x[t][0].x, x[t][0].y, x[t][0].z, x[t][0].w}, B1[4] = {x[t][1].x, x[t][1].y, x[t][1].z, x[t][1].w};
+                                mma_u8s8(c[0][t], a0, a1, a2, a3, B0[f], B1[f]);
+                            }
+                        }
                     }
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (2 * q + (i & 1) < MR) dst[(i & 1) * DL_TS + (i >> 1) * 8] = c[0][i] + (c[1][i] >> 2) + (c[2][i] >> 4) + (c[3][i] >> 6);
+            for (int t = 0; t < NB; ++t)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    int v = c[0][t][i];
+                    if constexpr (F == 4) v += (c[1][t][i] >> 2) + (c[2][t][i] >> 4) + (c[3][t][i] >> 6);
+                    if (!FUSED || 2 * q + (i & 1) < MR) dst[(t * 8 + (i & 1)) * DL_TS + (i >> 1) * 8] = v;
+                }
         }
     }
     __syncthreads();
 
     // ---- epilogue: a thread finishes two adjacent rows (channels) of a token
-    for (int i = tid; i < pairs * M; i += TH) {
+    for (int i = tid; i < pairs * M; i += nthr) {
         const int m = token_of(i), pr = i - m * pairs;
         // rows r, r + 1 of block b, rounded to T and packed
         auto value = [&](int b, int r, int g) {
             const int* s = part + (b * kw * MR + m) * DL_TS + r;
             int2 v = make_int2(0, 0);
-            if constexpr (TH == 256) {
+            if constexpr (CONST8) {
                 const int np = min(kw, KG);
 #pragma unroll
                 for (int w = 0; w < 8; ++w)
@@ -477,6 +588,25 @@ template <auto kernel> int dl_go(const DlParams& p, int threads, int smem, cudaS
     return MMF_OK;
 }
 
+template <typename T, int PRO, int TH, int NVT> int dl_rows_go(const mmf_decode_linear_args& a, int G, int KG, int NB, cudaStream_t st) {
+    MMF_CUDA(mmf_launch_pdl(decode_rows_kernel<T, PRO, TH, NVT>, dim3((unsigned)a.M, (unsigned)G), dim3(TH),
+                            (size_t)(PRO == MMF_PRO_QUANT ? 1 : 2) * a.K * 4, st, a, KG, NB, 1.0 / (double)a.K));
+    MMF_LAUNCH_CHECK("decode_rows_kernel");
+    return MMF_OK;
+}
+// the fewest threads (of 8 values each) that hold the row; a plain row of more than 4096 values takes two vectors per thread
+template <typename T, int PRO> int dl_rows(const mmf_decode_linear_args& a, int G, int KG, int NB, cudaStream_t st) {
+    if (a.K <= 1024) return dl_rows_go<T, PRO, 128, 1>(a, G, KG, NB, st);
+    if (a.K <= 2048) return dl_rows_go<T, PRO, 256, 1>(a, G, KG, NB, st);
+    if (a.K <= 3072) return dl_rows_go<T, PRO, 384, 1>(a, G, KG, NB, st);
+    if (a.K <= 4096) return dl_rows_go<T, PRO, 512, 1>(a, G, KG, NB, st);
+    if constexpr (PRO == MMF_PRO_QUANT) {
+        if (a.K <= 6144) return dl_rows_go<T, PRO, 384, 2>(a, G, KG, NB, st);
+        return dl_rows_go<T, PRO, 512, 2>(a, G, KG, NB, st);
+    }
+    return mmf_set_error(MMF_ERR_BAD_SHAPE, "mmf_decode_linear: row of %lld values", (long long)a.K);
+}
+
 // arguments are checked by mmf_decode_linear
 template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, cudaStream_t st) {
     DlParams p;
@@ -484,64 +614,97 @@ template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, 
     p.KC = (int)(a.K / MMF_TILE_K);
     p.KG = (p.KC + 3) / 4;
     p.inv_k = 1.0 / (double)a.K;
-    const int G = a.epilogue == MMF_EPI_GATES ? 3 : 1;
+    const bool fused = a.codes == nullptr;
+    const int G = a.epilogue == MMF_EPI_GATES ? 3 : 1, D = (int)a.K;
+    const int NB = fused ? 1 : a.M <= 8 ? 1 : a.M <= 16 ? 2 : 4, MR = !fused ? 8 * NB : a.M <= 1 ? 1 : a.M <= 2 ? 2 : 4;
+    if (!fused) {
+        const int rc = a.prologue == MMF_PRO_QUANT     ? dl_rows<T, MMF_PRO_QUANT>(a, G, p.KG, NB, st)
+                       : a.prologue == MMF_PRO_PRENORM ? dl_rows<T, MMF_PRO_PRENORM>(a, G, p.KG, NB, st)
+                                                       : dl_rows<T, MMF_PRO_GATENORM>(a, G, p.KG, NB, st);
+        if (rc != MMF_OK) return rc;
+    }
     // One CTA on every SM, however the rows divide: two kernels of the chain share an SM (the next one waits with its weights),
     // and an SM that this grid left empty would later take two CTAs of the next one, which then finishes late.
     const int units = a.epilogue == MMF_EPI_GATES ? (int)(a.K / 2) : a.epilogue == MMF_EPI_SWIGLU ? (int)(a.N / 4) : (int)((a.N + 1) / 2);
     p.grid = units < 148 ? units : 148;
     p.base = units / p.grid;
     p.extra = units % p.grid;
-    const int bp = a.epilogue == MMF_EPI_SWIGLU ? 4 : 8;
-    const int nb = (p.base + (p.extra ? 1 : 0) + bp - 1) / bp * G;        // most blocks of one CTA
-    // Every warp repeats a row's scalar work (statistics, scales), and the next kernel's set-up competes for the same issue
-    // slots, so more warps pay only where they have values to work on: eight for one row of at most 2048 values.
-    const int D = (int)a.K, MR = a.M <= 1 ? 1 : a.M <= 2 ? 2 : 4;
-    const int e0 = getenv("DL_A") ? atoi(getenv("DL_A")) : 0, e1 = getenv("DL_B") ? atoi(getenv("DL_B")) : 0;
-    const int threads = MR == 1 ? (D <= 2048 ? 256 : D <= 3072 ? (e0 ? e0 : 512) : D <= 4096 ? 512 : D <= 6144 ? (e1 ? e1 : 512) : 512) : 512, warps = threads / 32;
-    // warps over column groups x blocks: the split with the fewest rounds, then the fewest partial sums
-    int best = 1 << 30;
-    for (int kw = 1; kw <= warps && kw <= p.KG; ++kw) {
-        const int bw = warps / kw < nb ? warps / kw : nb;
-        const int cost = ((p.KG + kw - 1) / kw) * ((nb + bw - 1) / bw) * 64 + kw;
-        if (cost < best) { best = cost; p.kw = kw; p.bw = bw; }
-    }
-    if (threads == 256) { p.kw = 8; p.bw = 1; }
-    p.kgw = (p.KG + p.kw - 1) / p.kw;
-    p.inv_kw = 65536 / p.kw + 1;
     p.inv_base = 1.0f / (float)p.base;
     p.inv_base1 = 1.0f / (float)(p.base + 1);
-    int off = (a.prologue == MMF_PRO_QUANT ? G : G + 1) * D * 4;
+    const int bp = a.epilogue == MMF_EPI_SWIGLU ? 4 : 8;
+    const int nb = (p.base + (p.extra ? 1 : 0) + bp - 1) / bp * G;        // most blocks of one CTA
+    int threads;
+    if (fused) {
+        // Every warp repeats a row's scalar work (statistics, scales), and the next kernel's set-up competes for the same issue
+        // slots, so one row gets the fewest warps that hold it (8 values a thread).
+        threads = MR > 1 ? 512 : D <= 1024 ? 128 : D <= 2048 ? 256 : D <= 3072 ? 384 : D <= 4096 ? 512 : D <= 6144 ? 256 : 512;
+        // warps over column groups x blocks: the split with the fewest rounds, then the fewest partial sums
+        const int warps = threads / 32;
+        int best = 1 << 30;
+        for (int kw = 1; kw <= warps && kw <= p.KG; ++kw) {
+            const int bw = warps / kw < nb ? warps / kw : nb;
+            const int cost = ((p.KG + kw - 1) / kw) * ((nb + bw - 1) / bw) * 64 + kw;
+            if (cost < best) { best = cost; p.kw = kw; p.bw = bw; }
+        }
+        if (threads == 256) { p.kw = 8; p.bw = 1; }
+    } else {
+        // Column groups over as many of at most 12 warps as give the fewest rounds, so that a warp reads each code once; blocks
+        // over warps only where a short row leaves warps idle.
+        const int rounds = (p.KG + 11) / 12;
+        p.kw = (p.KG + rounds - 1) / rounds;
+        p.bw = p.kw >= 8 ? 1 : 8 / p.kw < nb ? 8 / p.kw : nb;
+        threads = p.kw * p.bw > 8 ? p.kw * p.bw * 32 : 256;
+    }
+    if (!(fused && threads == 256))                          // many blocks (lm_head): fewer partial sums per block, so that they fit
+        while (p.kw > 1 && nb * p.kw * MR * DL_TS * 4 > 80 * 1024) {
+            p.kw = (p.kw + 1) / 2;
+            p.bw = threads / 32 / p.kw < nb ? threads / 32 / p.kw : nb;
+        }
+    p.kgw = (p.KG + p.kw - 1) / p.kw;
+    p.inv_kw = 65536 / p.kw + 1;
+    int off = fused ? (a.prologue == MMF_PRO_QUANT ? G : G + 1) * D * 4 : 0;
     p.smem_codes = off;
-    off += G * p.KG * 256 * MR;
+    off += fused ? G * p.KG * 256 * MR : NB == 1 ? p.kw * p.bw * G * p.kgw * 2048 : 0;
     p.smem_acc = off;
     off += nb * p.kw * MR * DL_TS * 4;
     p.smem_w = off;
     const int per_item = p.kw * p.bw * 1024, want = (nb + p.bw - 1) / p.bw * p.kgw, room = (DL_SMEM_MAX - off) / per_item;
-    MMF_REQUIRE(room >= 1, MMF_ERR_BAD_SHAPE, "mmf_decode_linear: N=%lld K=%lld do not fit in shared memory", (long long)a.N, (long long)a.K);
+    MMF_REQUIRE(off <= DL_SMEM_MAX && room >= 0, MMF_ERR_BAD_SHAPE, "mmf_decode_linear: N=%lld K=%lld do not fit in shared memory", (long long)a.N,
+                (long long)a.K);
     p.pf = want < room ? want : room;
-    const int smem = off + p.pf * per_item;
+    int smem = off + p.pf * per_item;
+    static const int alone = getenv("DL_ALONE") ? atoi(getenv("DL_ALONE")) * 1024 : 0;
+    if (!fused && smem < alone) smem = alone;
 
-// vectors per thread for rows of at most 2048, 4096 and (plain quantisation) 6144 and 8192 values
 #define DL_K(PRO, EPI, TH, MR, NVT) return dl_go<decode_linear_kernel<T, PRO, EPI, TH, MR, NVT>>(p, threads, smem, st)
-#define DL_FUSED(PRO, EPI)                                                                \
-    if (a.prologue == PRO && a.epilogue == EPI) {                                         \
-        constexpr bool LONG = PRO == MMF_PRO_QUANT;                                        \
-        if (MR == 1) {                                                                    \
-            if (D <= 2048) DL_K(PRO, EPI, 256, 1, 1);                                      \
-            if (D <= 3072 && threads == 384) DL_K(PRO, EPI, 384, 1, 1);                                      \
-            if (D <= 4096) DL_K(PRO, EPI, 512, 1, 1);                                      \
-            if constexpr (LONG) if (threads == 256) DL_K(PRO, EPI, 256, 1, 3);                                 \
-            if constexpr (LONG) if (threads == 384) DL_K(PRO, EPI, 384, 1, 2);                                 \
-            if constexpr (LONG) DL_K(PRO, EPI, 512, 1, 2);                                 \
-        } else if (MR == 2) {                                                             \
-            if (D <= 2048) DL_K(PRO, EPI, 512, 2, 1);                                      \
-            if (D <= 4096) DL_K(PRO, EPI, 512, 2, 2);                                      \
-            if constexpr (LONG) { if (D <= 6144) DL_K(PRO, EPI, 512, 2, 3); DL_K(PRO, EPI, 512, 2, 4); } \
-        } else {                                                                          \
-            if (D <= 2048) DL_K(PRO, EPI, 512, 4, 2);                                      \
-            if (D <= 4096) DL_K(PRO, EPI, 512, 4, 4);                                      \
-            if constexpr (LONG) { if (D <= 6144) DL_K(PRO, EPI, 512, 4, 6); DL_K(PRO, EPI, 512, 4, 8); } \
-        }                                                                                 \
+#define DL_CODES_K(EPI)                                            \
+    if (!fused && a.epilogue == EPI) {                             \
+        if (NB == 1) DL_K(DL_CODES, EPI, DL_CODES_THREADS, 8, 1);  \
+        if (NB == 2) DL_K(DL_CODES, EPI, DL_CODES_THREADS, 16, 1); \
+        DL_K(DL_CODES, EPI, DL_CODES_THREADS, 32, 1);              \
+    }
+    DL_CODES_K(MMF_EPI_GATES)
+    DL_CODES_K(MMF_EPI_SWIGLU)
+    DL_CODES_K(MMF_EPI_STORE)
+#undef DL_CODES_K
+#define DL_FUSED(PRO, EPI)                                                                                            \
+    if (a.prologue == PRO && a.epilogue == EPI) {                                                                     \
+        constexpr bool LONG = PRO == MMF_PRO_QUANT;                                                                   \
+        if (MR == 1) {                                                                                                \
+            if (D <= 1024) DL_K(PRO, EPI, 128, 1, 1);                                                                 \
+            if (D <= 2048) DL_K(PRO, EPI, 256, 1, 1);                                                                 \
+            if (D <= 3072) DL_K(PRO, EPI, 384, 1, 1);                                                                 \
+            if (D <= 4096) DL_K(PRO, EPI, 512, 1, 1);                                                                 \
+            if constexpr (LONG) { if (D <= 6144) DL_K(PRO, EPI, 256, 1, 3); DL_K(PRO, EPI, 512, 1, 2); }              \
+        } else if (MR == 2) {                                                                                         \
+            if (D <= 2048) DL_K(PRO, EPI, 512, 2, 1);                                                                 \
+            if (D <= 4096) DL_K(PRO, EPI, 512, 2, 2);                                                                 \
+            if constexpr (LONG) { if (D <= 6144) DL_K(PRO, EPI, 512, 2, 3); DL_K(PRO, EPI, 512, 2, 4); }              \
+        } else {                                                                                                      \
+            if (D <= 2048) DL_K(PRO, EPI, 512, 4, 2);                                                                 \
+            if (D <= 4096) DL_K(PRO, EPI, 512, 4, 4);                                                                 \
+            if constexpr (LONG) { if (D <= 6144) DL_K(PRO, EPI, 512, 4, 6); DL_K(PRO, EPI, 512, 4, 8); }              \
+        }                                                                                                             \
     }
     DL_FUSED(MMF_PRO_PRENORM, MMF_EPI_GATES)
     DL_FUSED(MMF_PRO_GATENORM, MMF_EPI_STORE)
