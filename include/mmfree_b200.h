@@ -306,8 +306,8 @@ int mmf_swiglu_quant(const void* gate, const void* up, int64_t ld, int dtype, co
 #define MMF_EPI_GATES 1     /* N = 3 K = i | f | g projections: gate math and state update (mmf_decode_mix without its
                                norm); out = o [M, K], g_out = g [M, K], state fp32 [M, K] in place */
 #define MMF_EPI_SWIGLU 2    /* N = 2 I = gate | up: out = silu(gate) * up [M, ld_out] */
-#define MMF_DECODE_LINEAR_MAX_M 32       /* with a codes workspace */
-#define MMF_DECODE_LINEAR_FUSED_MAX_M 4  /* without */
+#define MMF_DECODE_LINEAR_MAX_M 16       /* with a codes workspace */
+#define MMF_DECODE_LINEAR_FUSED_MAX_M 2  /* without */
 
 typedef struct {
     int prologue, epilogue, dtype;          /* dtype: MMF_BF16 or MMF_F16 */
@@ -324,7 +324,7 @@ typedef struct {
     const float* bl_norm_w[3];              /* BitLinear norm weight per projection, or NULL */
     void* residual_out;                     /* PRENORM: [M, K], or NULL */
     /* Workspace for row work in a kernel of its own (two launches), 16-byte aligned: codes G * (K rounded up to 256) * (M
-     * rounded up to 8, 16 or 32) bytes, dq and rowsum G * M, with G = 3 for GATES and else 1.  codes NULL: the contraction
+     * rounded up to 8 or 16) bytes, dq and rowsum G * M, with G = 3 for GATES and else 1.  codes NULL: the contraction
      * does the row work itself (one launch). */
     int8_t* codes;
     float* dq;

@@ -203,7 +203,7 @@ PyObject* bitlinear(PyObject*, PyObject* const* args, Py_ssize_t n) {
         std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
         shape.back() = N;
         at::Tensor out = at::empty(shape, x.options());
-        if (M > 0 && M <= g_fused_rows && dt != MMF_F32 && K <= 8192) {      // a few rows: one kernel, no scratch
+        if (M > 0 && M <= g_fused_rows && dt != MMF_F32 && K <= 8192 && N <= 262144) {      // a few rows: one kernel, no scratch
             mmf_decode_linear_args a = {};
             a.prologue = MMF_PRO_QUANT;
             a.epilogue = MMF_EPI_STORE;
@@ -538,8 +538,8 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
             s.used = mix;
             const int64_t gu = s.take(2 * M * c.inner * es);
             s.used = std::max(s.used, mix_end);
-            // codes: decode-step contractions want rows of whole 256-column groups, up to 32 of them
-            const int64_t Mc = M <= 8 ? 8 : M <= 16 ? 16 : M <= 32 ? 32 : M;
+            // codes: decode-step contractions want rows of whole 256-column groups, up to 16 of them
+            const int64_t Mc = M <= 8 ? 8 : M <= 16 ? 16 : M;
             const int64_t q = s.take(Mc * std::max(3 * ((h + 255) & ~255ll), (c.inner + 255) & ~255ll)), dq = s.take(3 * M * 4), rs = s.take(3 * M * 4);
             const int64_t hg_bytes = T > 1 ? g_api->mmf_hgrn_workspace_bytes(B, T, h) : 0, hg = s.take(hg_bytes);
             const at::Tensor mem = at::empty({s.used}, opt.dtype(at::kByte));

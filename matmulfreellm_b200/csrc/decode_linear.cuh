@@ -26,9 +26,11 @@
 namespace {
 
 constexpr int DL_TS = 20;               // accumulator words per (block, token): 16 rows, padded so that a warp's adds do not collide
-constexpr int DL_FUSED_ROWS = 4;        // most token rows a CTA takes through the fused prologue
+constexpr int DL_FUSED_ROWS = MMF_DECODE_LINEAR_FUSED_MAX_M;      // most token rows a CTA takes through the fused prologue
 constexpr int DL_CODES = 0;             // prologue of the kernel whose codes were made by decode_rows_kernel
-constexpr int DL_CODES_THREADS = 384;
+// threads of the kernel with ready codes: 12 warps of up to 80 registers for 8 tokens; 16 tokens' codes and accumulators take
+// more than 80, so 8 warps of up to 128
+constexpr int dl_codes_threads(int NB) { return NB == 1 ? 384 : 256; }
 
 struct DlParams {
     mmf_decode_linear_args a;
@@ -419,24 +421,10 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
             s_scale[cg][cm] = __fmul_rn(__fdiv_rn(s_amax[cm][cg], 127.0f), ws);
         }
     } else {
-        if constexpr (NB == 1) {                             // all codes of this warp at once: one trip to the L2, not one per item
-            if (bq < bw) {
-                uint4* d = reinterpret_cast<uint4*>(scodes) + (size_t)warp * (G * kgw * 128) + lane;
-                for (int g = 0; g < G; ++g)
-                    for (int j = 0; j < kgw; ++j, d += 128)
-                        if (kq + j * kw < KG) {
-                            const uint4* src = codes + (g * KG + kq + j * kw) * 128;
-#pragma unroll
-                            for (int w = 0; w < 4; ++w) cp_async16(d + w * 32, src + w * 32);
-                        }
-            }
-            cp_async_commit();
-        }
         if (has_const) {
             s_scale[cg][cm] = __fmul_rn(*dq, ws);
             s_rs[cg][cm] = *rowsum;
         }
-        if (NB == 1) cp_async_wait_all();
     }
 
     // the 2-bit fields stay where they are: field f of a byte counts 4^f, one accumulator per field, shifted back at the end
@@ -444,16 +432,22 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
         const uint4* src = wslot + (size_t)warp * p.pf * 64 + lane;
         int* dst = part + ((bq * kw + kq) * MR + 2 * q) * DL_TS + gq;
         int k = 0;
+        constexpr bool AHEAD = !FUSED && NB == 1;            // codes of the next item on their way while this one is multiplied
+        uint4 ahead[4];
+        auto code_of = [&](int b, int kg) { return codes + ((G == 3 ? b % 3 : 0) * KG + kg) * 128; };
+        auto load_ahead = [&](const uint4* s) {
+#pragma unroll
+            for (int w = 0; w < 4; ++w) ahead[w] = s[w * 32];
+        };
+        if (AHEAD) load_ahead(code_of(bq, kq));
 #pragma unroll 1
         for (int b = bq; b < nb; b += bw, dst += bw * kw * MR * DL_TS) {
-            constexpr int F = NB <= 2 ? 4 : 1;
-            int c[F][NB][4] = {};
+            int c[4][NB][4] = {};
             const int g = EPI == MMF_EPI_GATES ? b % 3 : 0;
             // codes of the first group.  Fused: tokens MR - 7 do not exist, any code will do
             const uint4* cb = FUSED ? reinterpret_cast<const uint4*>(scodes) + (g * KG + kq) * (TL * 4) + (lane & (TL - 1))
-                              : NB == 1 ? reinterpret_cast<const uint4*>(scodes) + (size_t)(warp * G + g) * kgw * 128 + lane
-                                        : codes + (g * KG + kq) * (NB * 128);
-            const int cstep = FUSED ? kw * TL * 4 : NB == 1 ? 128 : kw * NB * 128;
+                                    : codes + (g * KG + kq) * (NB * 128);
+            const int cstep = FUSED ? kw * TL * 4 : kw * NB * 128;
             constexpr int CW = FUSED ? TL : 32;              // pieces per word
 #pragma unroll 1
             for (int j = 0; j < kgw; ++j, ++k, src += 64, cb += cstep) {
@@ -466,52 +460,33 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
                     fetch(b, j, [&](int half, const uint4* s) { (half ? wb : wa) = s ? __ldg(s) : make_uint4(0, 0, 0, 0); });
                 }
                 const uint32_t xa[4] = {wa.x, wa.y, wa.z, wa.w}, xb[4] = {wb.x, wb.y, wb.z, wb.w};
-                if constexpr (F == 4) {
-                    uint4 x[NB][4];
+                uint4 x[NB][4];
 #pragma unroll
-                    for (int t = 0; t < NB; ++t)
+                for (int t = 0; t < NB; ++t)
 #pragma unroll
-                        for (int w = 0; w < 4; ++w) x[t][w] = cb[(t * 4 + w) * CW];
+                    for (int w = 0; w < 4; ++w) x[t][w] = AHEAD ? ahead[w] : cb[(t * 4 + w) * CW];
+                if constexpr (AHEAD) {
+                    if (kq + (j + 1) * kw < KG) load_ahead(code_of(b, kq + (j + 1) * kw));
+                    else if ((G == 3 || kgw > 1) && b + bw < nb) load_ahead(code_of(b + bw, kq));
+                }
 #pragma unroll
-                    for (int w = 0; w < 4; w += 2)
+                for (int w = 0; w < 4; w += 2)
 #pragma unroll
-                        for (int f = 0; f < 4; ++f) {
-                            const uint32_t msk = 0x03030303u << (2 * f);
-#pragma unroll
-                            for (int t = 0; t < NB; ++t) {
-                                const uint32_t B0[4] = {x[t][w].x, x[t][w].y, x[t][w].z, x[t][w].w},
-                                               B1[4] = {x[t][w + 1].x, x[t][w + 1].y, x[t][w + 1].z, x[t][w + 1].w};
-                                mma_u8s8(c[f][t], xa[w] & msk, xb[w] & msk, xa[w + 1] & msk, xb[w + 1] & msk, B0[f], B1[f]);
-                            }
-                        }
-                } else {                                     // accumulators of four fields do not fit in registers: fields shifted down
-#pragma unroll
-                    for (int w = 0; w < 4; w += 2) {
-                        uint4 x[NB][2];
+                    for (int f = 0; f < 4; ++f) {
+                        const uint32_t msk = 0x03030303u << (2 * f);
 #pragma unroll
                         for (int t = 0; t < NB; ++t) {
-                            x[t][0] = cb[(t * 4 + w) * CW];
-                            x[t][1] = cb[(t * 4 + w + 1) * CW];
-                        }
-#pragma unroll
-                        for (int f = 0; f < 4; ++f) {
-                            const uint32_t a0 = (xa[w] >> (2 * f)) & 0x03030303u, a1 = (xb[w] >> (2 * f)) & 0x03030303u,
-                                           a2 = (xa[w + 1] >> (2 * f)) & 0x03030303u, a3 = (xb[w + 1] >> (2 * f)) & 0x03030303u;
-#pragma unroll
-                            for (int t = 0; t < NB; ++t) {
-                                const uint32_t B0[4] = {x[t][0].x, x[t][0].y, x[t][0].z, x[t][0].w}, B1[4] = {x[t][1].x, x[t][1].y, x[t][1].z, x[t][1].w};
-                                mma_u8s8(c[0][t], a0, a1, a2, a3, B0[f], B1[f]);
-                            }
+                            const uint32_t B0[4] = {x[t][w].x, x[t][w].y, x[t][w].z, x[t][w].w},
+                                           B1[4] = {x[t][w + 1].x, x[t][w + 1].y, x[t][w + 1].z, x[t][w + 1].w};
+                            mma_u8s8(c[f][t], xa[w] & msk, xb[w] & msk, xa[w + 1] & msk, xb[w + 1] & msk, B0[f], B1[f]);
                         }
                     }
-                }
             }
 #pragma unroll
             for (int t = 0; t < NB; ++t)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    int v = c[0][t][i];
-                    if constexpr (F == 4) v += (c[1][t][i] >> 2) + (c[2][t][i] >> 4) + (c[3][t][i] >> 6);
+                    const int v = c[0][t][i] + (c[1][t][i] >> 2) + (c[2][t][i] >> 4) + (c[3][t][i] >> 6);
                     if (!FUSED || 2 * q + (i & 1) < MR) dst[(t * 8 + (i & 1)) * DL_TS + (i >> 1) * 8] = v;
                 }
         }
@@ -616,7 +591,7 @@ template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, 
     p.inv_k = 1.0 / (double)a.K;
     const bool fused = a.codes == nullptr;
     const int G = a.epilogue == MMF_EPI_GATES ? 3 : 1, D = (int)a.K;
-    const int NB = fused ? 1 : a.M <= 8 ? 1 : a.M <= 16 ? 2 : 4, MR = !fused ? 8 * NB : a.M <= 1 ? 1 : a.M <= 2 ? 2 : 4;
+    const int NB = fused || a.M <= 8 ? 1 : 2, MR = !fused ? 8 * NB : a.M <= 1 ? 1 : 2;
     if (!fused) {
         const int rc = a.prologue == MMF_PRO_QUANT     ? dl_rows<T, MMF_PRO_QUANT>(a, G, p.KG, NB, st)
                        : a.prologue == MMF_PRO_PRENORM ? dl_rows<T, MMF_PRO_PRENORM>(a, G, p.KG, NB, st)
@@ -648,11 +623,15 @@ template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, 
         }
         if (threads == 256) { p.kw = 8; p.bw = 1; }
     } else {
-        // Column groups over as many of at most 12 warps as give the fewest rounds, so that a warp reads each code once; blocks
-        // over warps only where a short row leaves warps idle.
-        const int rounds = (p.KG + 11) / 12;
-        p.kw = (p.KG + rounds - 1) / rounds;
-        p.bw = p.kw >= 8 ? 1 : 8 / p.kw < nb ? 8 / p.kw : nb;
+        int best = 1 << 30;
+        static const int pol = getenv("DL_POL") ? atoi(getenv("DL_POL")) : 0;
+        for (int kw = 1; kw <= dl_codes_threads(NB) / 32 && kw <= p.KG; ++kw) {
+            const int bw = dl_codes_threads(NB) / 32 / kw < nb ? dl_codes_threads(NB) / 32 / kw : nb;
+            const int ra = (p.KG + kw - 1) / kw, rb = (nb + bw - 1) / bw;
+            const int cost = pol == 0 ? ra * rb * 64 + kw * bw : pol == 1 ? ra * 4096 + rb * 64 + kw * bw : pol == 2 ? ra * rb * 64 + (G == 3 ? ra * rb : ra) * 16 + kw * bw
+                             : ra * rb * 64 + (G == 3 ? ra * rb : ra) * 64 + kw * bw * 4;
+            if (cost < best) { best = cost; p.kw = kw; p.bw = bw; }
+        }
         threads = p.kw * p.bw > 8 ? p.kw * p.bw * 32 : 256;
     }
     if (!(fused && threads == 256))                          // many blocks (lm_head): fewer partial sums per block, so that they fit
@@ -664,7 +643,7 @@ template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, 
     p.inv_kw = 65536 / p.kw + 1;
     int off = fused ? (a.prologue == MMF_PRO_QUANT ? G : G + 1) * D * 4 : 0;
     p.smem_codes = off;
-    off += fused ? G * p.KG * 256 * MR : NB == 1 ? p.kw * p.bw * G * p.kgw * 2048 : 0;
+    off += fused ? G * p.KG * 256 * MR : 0;
     p.smem_acc = off;
     off += nb * p.kw * MR * DL_TS * 4;
     p.smem_w = off;
@@ -672,16 +651,13 @@ template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, 
     MMF_REQUIRE(off <= DL_SMEM_MAX && room >= 0, MMF_ERR_BAD_SHAPE, "mmf_decode_linear: N=%lld K=%lld do not fit in shared memory", (long long)a.N,
                 (long long)a.K);
     p.pf = want < room ? want : room;
-    int smem = off + p.pf * per_item;
-    static const int alone = getenv("DL_ALONE") ? atoi(getenv("DL_ALONE")) * 1024 : 0;
-    if (!fused && smem < alone) smem = alone;
+    const int smem = off + p.pf * per_item;
 
 #define DL_K(PRO, EPI, TH, MR, NVT) return dl_go<decode_linear_kernel<T, PRO, EPI, TH, MR, NVT>>(p, threads, smem, st)
 #define DL_CODES_K(EPI)                                            \
     if (!fused && a.epilogue == EPI) {                             \
-        if (NB == 1) DL_K(DL_CODES, EPI, DL_CODES_THREADS, 8, 1);  \
-        if (NB == 2) DL_K(DL_CODES, EPI, DL_CODES_THREADS, 16, 1); \
-        DL_K(DL_CODES, EPI, DL_CODES_THREADS, 32, 1);              \
+        if (NB == 1) DL_K(DL_CODES, EPI, dl_codes_threads(1), 8, 1);  \
+        DL_K(DL_CODES, EPI, dl_codes_threads(2), 16, 1);              \
     }
     DL_CODES_K(MMF_EPI_GATES)
     DL_CODES_K(MMF_EPI_SWIGLU)
@@ -696,14 +672,10 @@ template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, 
             if (D <= 3072) DL_K(PRO, EPI, 384, 1, 1);                                                                 \
             if (D <= 4096) DL_K(PRO, EPI, 512, 1, 1);                                                                 \
             if constexpr (LONG) { if (D <= 6144) DL_K(PRO, EPI, 256, 1, 3); DL_K(PRO, EPI, 512, 1, 2); }              \
-        } else if (MR == 2) {                                                                                         \
+        } else {                                                                                         \
             if (D <= 2048) DL_K(PRO, EPI, 512, 2, 1);                                                                 \
             if (D <= 4096) DL_K(PRO, EPI, 512, 2, 2);                                                                 \
             if constexpr (LONG) { if (D <= 6144) DL_K(PRO, EPI, 512, 2, 3); DL_K(PRO, EPI, 512, 2, 4); }              \
-        } else {                                                                                                      \
-            if (D <= 2048) DL_K(PRO, EPI, 512, 4, 2);                                                                 \
-            if (D <= 4096) DL_K(PRO, EPI, 512, 4, 4);                                                                 \
-            if constexpr (LONG) { if (D <= 6144) DL_K(PRO, EPI, 512, 4, 6); DL_K(PRO, EPI, 512, 4, 8); }              \
         }                                                                                                             \
     }
     DL_FUSED(MMF_PRO_PRENORM, MMF_EPI_GATES)
