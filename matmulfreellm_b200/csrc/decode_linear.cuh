@@ -19,7 +19,6 @@
 // changes nothing in an integer sum.  Weights are fetched by cp.async into slots private to a lane before the
 // grid-dependency wait.  Partial sums meet in shared memory by integer atomics (exact, so order does not matter).
 #pragma once
-#include <cstdlib>
 #include "bitlinear.cuh"
 #include "packed.cuh"
 
@@ -432,14 +431,6 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
         const uint4* src = wslot + (size_t)warp * p.pf * 64 + lane;
         int* dst = part + ((bq * kw + kq) * MR + 2 * q) * DL_TS + gq;
         int k = 0;
-        constexpr bool AHEAD = !FUSED && NB == 1;            // codes of the next item on their way while this one is multiplied
-        uint4 ahead[4];
-        auto code_of = [&](int b, int kg) { return codes + ((G == 3 ? b % 3 : 0) * KG + kg) * 128; };
-        auto load_ahead = [&](const uint4* s) {
-#pragma unroll
-            for (int w = 0; w < 4; ++w) ahead[w] = s[w * 32];
-        };
-        if (AHEAD) load_ahead(code_of(bq, kq));
 #pragma unroll 1
         for (int b = bq; b < nb; b += bw, dst += bw * kw * MR * DL_TS) {
             int c[4][NB][4] = {};
@@ -464,11 +455,7 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
 #pragma unroll
                 for (int t = 0; t < NB; ++t)
 #pragma unroll
-                    for (int w = 0; w < 4; ++w) x[t][w] = AHEAD ? ahead[w] : cb[(t * 4 + w) * CW];
-                if constexpr (AHEAD) {
-                    if (kq + (j + 1) * kw < KG) load_ahead(code_of(b, kq + (j + 1) * kw));
-                    else if ((G == 3 || kgw > 1) && b + bw < nb) load_ahead(code_of(b + bw, kq));
-                }
+                    for (int w = 0; w < 4; ++w) x[t][w] = cb[(t * 4 + w) * CW];
 #pragma unroll
                 for (int w = 0; w < 4; w += 2)
 #pragma unroll
@@ -624,12 +611,9 @@ template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, 
         if (threads == 256) { p.kw = 8; p.bw = 1; }
     } else {
         int best = 1 << 30;
-        static const int pol = getenv("DL_POL") ? atoi(getenv("DL_POL")) : 0;
         for (int kw = 1; kw <= dl_codes_threads(NB) / 32 && kw <= p.KG; ++kw) {
             const int bw = dl_codes_threads(NB) / 32 / kw < nb ? dl_codes_threads(NB) / 32 / kw : nb;
-            const int ra = (p.KG + kw - 1) / kw, rb = (nb + bw - 1) / bw;
-            const int cost = pol == 0 ? ra * rb * 64 + kw * bw : pol == 1 ? ra * 4096 + rb * 64 + kw * bw : pol == 2 ? ra * rb * 64 + (G == 3 ? ra * rb : ra) * 16 + kw * bw
-                             : ra * rb * 64 + (G == 3 ? ra * rb : ra) * 64 + kw * bw * 4;
+            const int cost = ((p.KG + kw - 1) / kw) * ((nb + bw - 1) / bw) * 64 + kw * bw;
             if (cost < best) { best = cost; p.kw = kw; p.bw = bw; }
         }
         threads = p.kw * p.bw > 8 ? p.kw * p.bw * 32 : 256;
