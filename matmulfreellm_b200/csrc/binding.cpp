@@ -44,7 +44,16 @@ std::map<std::string, Api> g_apis;   // by path; the pointers stay valid because
 const Api* g_api = nullptr;
 
 int64_t g_launches = 0;    // guarded by the GIL
-int64_t g_fused_rows = 2, g_codes_rows = 32, g_head_rows = 8;
+
+// Rows of a decode step that take the fused kernels, and from how many on the row work is a kernel of its own.  One row is
+// faster with the row work repeated in every CTA (1.3B step: 435 us against 510 with row kernels, 2.7B 688 against ~800); two
+// rows only up to 2048 columns (1.3B 498 against 519, 2.7B 952 against 806).  Above 16 rows the contraction on tcgen05 with
+// row kernels around it is faster (1.3B, 32 rows: 828 us against 1000).
+constexpr int64_t DECODE_ROWS = MMF_DECODE_LINEAR_MAX_M;
+bool rows_in_contraction(int64_t M, int64_t h) { return M == 1 || (M <= MMF_DECODE_LINEAR_FUSED_MAX_M && h <= 2048); }
+constexpr int64_t HEAD_ROWS = 8;              // lm_head alone: tcgen05 above
+bool on16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+constexpr int64_t FUSED_MAX_N = 262144;       // partial sums of more output rows would not fit in shared memory
 
 PyObject* g_error_class = nullptr;
 PyObject* g_workspace_fn = nullptr;
@@ -203,7 +212,9 @@ PyObject* bitlinear(PyObject*, PyObject* const* args, Py_ssize_t n) {
         std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
         shape.back() = N;
         at::Tensor out = at::empty(shape, x.options());
-        if (M > 0 && M <= g_fused_rows && dt != MMF_F32 && K <= 8192 && N <= 262144) {      // a few rows: one kernel, no scratch
+        // one or two rows: one kernel, no scratch
+        if (M > 0 && M <= MMF_DECODE_LINEAR_FUSED_MAX_M && dt != MMF_F32 && K <= 8192 && N <= FUSED_MAX_N && on16(x2.data_ptr()) &&
+            x2.stride(0) % 8 == 0 && on16(ptr(nw)) && on16(packed.data_ptr())) {
             mmf_decode_linear_args a = {};
             a.prologue = MMF_PRO_QUANT;
             a.epilogue = MMF_EPI_STORE;
@@ -434,7 +445,7 @@ PyObject* chain(PyObject*, PyObject* const* args, Py_ssize_t n) {
     });
 }
 
-// The blocks of a decode step for a few token rows: four kernels per block (decode_linear.cuh).  z: last block's MLP output and
+// The blocks of a decode step for a few token rows: four calls per block (decode_linear.cuh).  z: last block's MLP output and
 // the attention output; x / next: residual stream.
 template <typename ArgsOf, typename Run, typename Advance>
 void decode_blocks(const Chain& c, ArgsOf&& args_of, Run&& run, const int64_t* gather, uint8_t* z, uint8_t* g, uint8_t* o, uint8_t* act,
@@ -553,8 +564,10 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                          MMF_KERNEL_AUTO, st);
                 ++launches;
             };
-            // one token per sequence and few sequences: contractions with the row work around them in one kernel
-            const bool decode = T == 1 && M > 0 && M <= g_codes_rows && c.dtype != MMF_F32 && h % MMF_TILE_ROWS == 0 && h <= 4096 && c.inner <= 8192;
+            // one token per sequence and few sequences: contractions with the element-wise work around them in one kernel
+            bool decode = T == 1 && M > 0 && M <= DECODE_ROWS && c.dtype != MMF_F32 && h % MMF_TILE_ROWS == 0 && h <= 4096 && c.inner <= 8192 &&
+                          (ids.defined() || on16(emb.data_ptr()));
+            for (const float* s : states) decode = decode && on16(s);
             const int64_t* gather = decode && ids.defined() && !c.layers.empty() ? ids.data_ptr<int64_t>() : nullptr;
             const uint8_t* x = b + x0;            // residual stream
             if (gather) {                         // the first block reads the embedding rows itself
@@ -581,7 +594,7 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 a.w_scale = l.scale;
                 a.out = out;
                 a.ld_out = ld_out;
-                if (M > g_fused_rows) {
+                if (!rows_in_contraction(M, h)) {
                     a.codes = Q;
                     a.dq = DQ;
                     a.rowsum = RS;
@@ -629,7 +642,7 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
             const int64_t skip = last_only ? (T - 1) * h * es : 0, ld = last_only ? T * h : h;
             first = c.layers.empty();
             const uint8_t* rows = first ? x : b + z;
-            if (decode && M <= g_head_rows && c.head.N <= 262144 && want_logits && !want_hidden) {
+            if (decode && M <= HEAD_ROWS && c.head.N <= FUSED_MAX_N && want_logits && !want_hidden) {
                 mmf_decode_linear_args a = args_of(c.head, MMF_PRO_PRENORM, MMF_EPI_STORE, logits.data_ptr(), c.head.N);
                 a.x = rows; a.ld_x = h;
                 a.residual = first ? nullptr : x; a.ld_residual = h;
@@ -656,16 +669,9 @@ PyObject* take_launches(PyObject*, PyObject*) {
     g_launches = 0;
     return PyLong_FromLongLong(n);
 }
-PyObject* set_rows(PyObject*, PyObject* const* args, Py_ssize_t) {
-    g_fused_rows = PyLong_AsLongLong(args[0]);
-    g_codes_rows = PyLong_AsLongLong(args[1]);
-    g_head_rows = PyLong_AsLongLong(args[2]);
-    Py_RETURN_NONE;
-}
 
 PyMethodDef methods[] = {
     {"take_launches", take_launches, METH_NOARGS, nullptr},
-    {"set_rows", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(set_rows)), METH_FASTCALL, nullptr},
     {"use_library", use_library, METH_O, nullptr},
     {"set_hooks", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(set_hooks)), METH_FASTCALL, nullptr},
     {"bitlinear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(bitlinear)), METH_FASTCALL, nullptr},

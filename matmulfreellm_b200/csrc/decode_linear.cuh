@@ -6,18 +6,24 @@
 // A block of the model used to be eight links (row kernel, contraction, four times).  Here
 //   * the gate math and state update of the token mixer and the MLP's silu(gate) * up run in the epilogue of the contraction
 //     that produces their inputs (a CTA owns the i, f and g rows, or the gate and up rows, of the same channels), and
-//   * for a few token rows every CTA repeats the row work that precedes the contraction — norms, statistics, int8 codes —
+//   * for one or two token rows every CTA repeats the row work that precedes the contraction - norms, statistics, int8 codes -
 //     instead of waiting for a kernel that did it: the row work is latency, and the SMs would idle meanwhile.
-// That leaves four links per block.  For more rows the codes come from a row kernel (prologue MMF_PRO_CODES).
+// That leaves four links per block; up to 16 rows, where repeating the row work costs more than a link, it is a kernel of its
+// own that stores the codes in the contraction's operand order (eight links).  Step of a 24-block, 2048-wide model, before and
+// now: 1 row 595 -> 435 us, 2 rows 635 -> 500, 4 rows 735 -> 534, 8 rows 737 -> 530, 16 rows 769 -> 663; 32 blocks of 2560: 1 row
+// 980 -> 688, 8 rows 1127 -> 831.  What remains is latency: about 4.4 us per link for 1.5 us of weight traffic.
 //
 // Contraction: mma.sync m16n8k32 (8-bit, int32 accumulators) with 16 weight rows on its M axis and 8 token rows on N.
 // tcgen05 is not used: its 128-row tile needs a K split over a cluster to fill the GPU, and the exchange of the split's
 // partial sums alone (2.4 us) is longer than this kernel's whole contraction at these sizes.  A CTA (one per SM) owns
-// N / 148 output rows and all of K; the (256-column group, 16-row block) pairs of its share are dealt evenly to the warps.
-// A lane's operands are contiguous: the packed layout gives it 16 bytes (64 weights of one row) per group and block, whose
-// 2-bit fields need one mask per register; the order of K inside a group is permuted alike for weights and codes, which
-// changes nothing in an integer sum.  Weights are fetched by cp.async into slots private to a lane before the
-// grid-dependency wait.  Partial sums meet in shared memory by integer atomics (exact, so order does not matter).
+// N / 148 output rows and all of K; its 16-row blocks and 256-column groups are split over the warps, each warp keeps a block's
+// sums in registers over its groups, and the warps' partial sums meet in shared memory by plain stores (atomics there took
+// 45 clocks each and a third of the kernel).  A lane's operands are contiguous: the packed layout gives it 16 bytes (64 weights
+// of one row) per group and block, whose 2-bit fields need one mask per register; the order of K inside a group is permuted
+// alike for weights and codes, which changes nothing in an integer sum.  Weights are fetched by cp.async into slots private to
+// a lane before the grid-dependency wait; ready codes come straight from the L2 (staging them in shared memory first, or
+// loading a group ahead, was 10 % slower).  What bounds a link is the number of instructions between the wait and the last
+// store, since the next kernel's set-up shares the issue slots: few warps, constants and splits computed on the host.
 #pragma once
 #include "bitlinear.cuh"
 #include "packed.cuh"

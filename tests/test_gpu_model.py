@@ -574,3 +574,54 @@ def test_generate_graph_path_equals_step_loop(mm):
     model.pack_weights()
     assert torch.equal(model.generate(ids3, max_new_tokens=12), model.generate(ids3, max_new_tokens=12, use_graph=False))
     mm.kernels.check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("hidden,intermediate", [(384, 704), (1152, 1984), (2176, 4160), (4096, 8192)])
+def test_decode_step_rows_do_not_depend_on_the_batch(mm, dtype, hidden, intermediate):
+    """A decode step picks its kernels by the number of sequences (row work inside the contraction, in a kernel of its own,
+    or tcgen05 contractions above 16 rows).  All take the same roundings, so a sequence's logits and state are bit-identical
+    whatever the batch around it; sizes with partly filled column groups, row tiles and 16-row blocks."""
+    from mmfreelm.models import HGRNBitConfig, HGRNBitForCausalLM
+    torch.manual_seed(hidden)
+    model = HGRNBitForCausalLM(HGRNBitConfig(vocab_size=1003, hidden_size=hidden, num_hidden_layers=2, intermediate_size=intermediate,
+                                             use_lower_bound=True)).eval().cuda()
+    with torch.no_grad():
+        for n, p in model.named_parameters():
+            if "lower_bounds" in n or p.dim() == 1: p.add_(0.3 * torch.randn_like(p))
+    model.pack_weights()
+    model = model.to(dtype)
+    g = torch.Generator().manual_seed(7)
+    ids, step = torch.randint(0, 1003, (33, 5), generator=g).cuda(), torch.randint(0, 1003, (33, 1), generator=g).cuda()
+
+    def run(B, embeds):
+        past = model(ids[:B], use_cache=True).past_key_values
+        mask = torch.ones(B, 1, dtype=torch.long, device="cuda")
+        mask[B // 2] = 0
+        kw = {"inputs_embeds": model.get_input_embeddings()(step[:B])} if embeds else {"input_ids": step[:B]}
+        out = model(past_key_values=past, use_cache=True, attention_mask=mask if embeds else None, **kw)
+        return out.logits, [s[0].view(B, -1) for s in out.past_key_values]
+
+    ref, ref_states = run(33, False)
+    for B in (1, 2, 3, 8, 9, 16):
+        logits, states = run(B, False)
+        assert torch.equal(logits, ref[:B]), B
+        assert all(torch.equal(a, b[:B]) for a, b in zip(states, ref_states)), B
+        logits, _ = run(B, True)                     # embeddings given, one sequence's token is padding
+        keep = [i for i in range(B) if i != B // 2]
+        assert torch.equal(logits[keep], ref[keep]), B
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("K,N", [(64, 1), (704, 130), (2112, 37), (5632, 2048), (8192, 515)])
+def test_bitlinear_of_one_and_two_rows_equals_more_rows(mm, dtype, K, N):
+    from matmulfreellm_b200.ops.fusedbitnet import FusedBitLinear
+    torch.manual_seed(K)
+    layer = FusedBitLinear(K, N).cuda()
+    layer.pack_weights()
+    layer = layer.to(dtype)
+    x = torch.randn(40, K, device="cuda").to(dtype)
+    ref = layer(x)
+    for rows in (x[:1], x[:2], x[::7][:2]):
+        pick = ref[:rows.shape[0]] if rows.stride(0) == K or rows.shape[0] == 1 else ref[::7][:2]
+        assert torch.equal(layer(rows), pick)
