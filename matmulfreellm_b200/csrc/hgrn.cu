@@ -27,8 +27,10 @@ constexpr int HG_TS = 64;       // timesteps per stage
 constexpr int HG_SUB = 8;       // sub-chunks (warps) per stage
 constexpr int HG_SUBT = HG_TS / HG_SUB;   // timesteps per thread and stage
 constexpr int HG_THREADS = (HG_BD / 2) * HG_SUB;
-// TMA ring depth: two stages when x and g are both 16-bit (the raw projections inside the model), three when the gate is fp32
-template <typename TX, typename TG> struct HgStages { static constexpr int value = sizeof(TX) + sizeof(TG) <= 4 ? 2 : 3; };
+// TMA ring depth: three stages when x is 16-bit and the gate fp32, else two.  Three stages of two fp32 tensors take 128 KB, one
+// CTA per SM; with two (96 KB) a second CTA covers the first one's waits: 64 x 333 x 2560 130 -> 108 us, 2 x 2048 x 2048 40 -> 32,
+// 256 x 64 x 256 26 -> 20, 8 x 2048 x 2048 and larger unchanged (memory bound).
+template <typename TX, typename TG> struct HgStages { static constexpr int value = sizeof(TX) + sizeof(TG) == 6 ? 3 : 2; };
 constexpr long long HG_WAIT_LIMIT = 2000000000ll;   // clock cycles (about a second) before a wait gives up
 
 __device__ int g_hgrn_wait_failed = 0;   // set when a bounded wait on a TMA stage gave up
