@@ -31,8 +31,6 @@ constexpr int HG_THREADS = (HG_BD / 2) * HG_SUB;
 // CTA per SM; with two (96 KB) a second CTA covers the first one's waits: 64 x 333 x 2560 130 -> 108 us, 2 x 2048 x 2048 40 -> 32,
 // 256 x 64 x 256 26 -> 20, 8 x 2048 x 2048 and larger unchanged (memory bound).
 template <typename TX, typename TG> struct HgStages { static constexpr int value = sizeof(TX) + sizeof(TG) == 6 ? 3 : 2; };
-// When there are enough CTAs not to split time (NT == 1) the 16-bit / fp32 pair takes two stages too: 64 KB, three CTAs per SM
-// (64 x 333 x 2560 86 -> 82 us, 8 x 2048 x 2048 55 -> 53); with fewer CTAs the deeper ring is faster (1 x 8192 x 2048 50 us, 56 with two).
 constexpr long long HG_WAIT_LIMIT = 2000000000ll;   // clock cycles (about a second) before a wait gives up
 
 __device__ int g_hgrn_wait_failed = 0;   // set when a bounded wait on a TMA stage gave up
@@ -166,7 +164,7 @@ __device__ __forceinline__ void gate_transform2(float2& xv, float2& f, bool has_
 // AGG = false: pass 2 (or the only pass when NT == 1) -> o, ht
 // Tensor maps: x, g, o as [B][T][D] with box [1][HG_TS][64]; rows past T read as zero and are not stored, channels
 // past D likewise.  chunk_len is a multiple of HG_TS, so only the last stage of the last chunk can be partial.
-template <typename TX, typename TG, int MODE, bool AGG, int HG_STAGES>
+template <typename TX, typename TG, int MODE, bool AGG>
 __global__ void __launch_bounds__(HG_THREADS, 4)
 hgrn_scan_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap g_map,
                  const __grid_constant__ CUtensorMap o_map, const TX* __restrict__ lb, const uint8_t* __restrict__ mask,
@@ -180,6 +178,7 @@ hgrn_scan_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
     }
     extern __shared__ uint8_t smem_dyn[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 127) & ~uintptr_t(127));
+    constexpr int HG_STAGES = HgStages<TX, TG>::value;
     constexpr int XB = HG_TS * HG_BD * sizeof(TX);  // bytes of one x stage (= one output tile)
     constexpr int GB = HG_TS * HG_BD * sizeof(TG);
     TX* sx = reinterpret_cast<TX*>(smem);
@@ -407,8 +406,8 @@ int hgrn_num_chunks(int64_t B, int64_t T, int64_t D) {
 }
 
 template <typename TX, typename TG>
-size_t hgrn_smem_bytes(int stages) {
-    return (size_t)stages * HG_TS * HG_BD * (sizeof(TX) + sizeof(TG)) + (size_t)2 * HG_TS * HG_BD * sizeof(TX) + 128;
+size_t hgrn_smem_bytes() {
+    return (size_t)HgStages<TX, TG>::value * HG_TS * HG_BD * (sizeof(TX) + sizeof(TG)) + (size_t)2 * HG_TS * HG_BD * sizeof(TX) + 128;
 }
 
 // [B][T][D] view with row pitch `ld` elements (batch pitch T*ld), box = one [64 timesteps x 64 channels] tile
@@ -437,8 +436,7 @@ int hgrn_launch(const void* x, int64_t ld_x, const void* g, int64_t ld_g, const 
         MMF_LAUNCH_CHECK("hgrn_step_kernel");
         return MMF_OK;
     }
-    constexpr int STAGES = HgStages<TX, TG>::value;
-    const size_t smem = hgrn_smem_bytes<TX, TG>(NT > 1 ? STAGES : 2);
+    const size_t smem = hgrn_smem_bytes<TX, TG>();
     // chunks start on stage boundaries so that every chunk but the last consists of whole stages
     const int chunk_len = (int)(((T + NT - 1) / NT + HG_TS - 1) / HG_TS * HG_TS);
     CUtensorMap x_map, g_map, o_map;
@@ -448,24 +446,17 @@ int hgrn_launch(const void* x, int64_t ld_x, const void* g, int64_t ld_g, const 
     if (rc != MMF_OK) return rc;
     const dim3 grid((unsigned)((D + HG_BD - 1) / HG_BD), (unsigned)NT, (unsigned)B);
     if (NT > 1) {
-        constexpr auto k1 = hgrn_scan_kernel<TX, TG, MODE, true, STAGES>;
+        constexpr auto k1 = hgrn_scan_kernel<TX, TG, MODE, true>;
         MMF_CUDA(mmf_allow_smem<k1>((int)smem));
         const dim3 grid1(grid.x, (unsigned)(NT - 1), grid.z);
         MMF_CUDA(mmf_launch_pdl(k1, grid1, dim3(HG_THREADS), smem, st, x_map, g_map, o_map, (const TX*)lb, mask, h0,
                                 (void*)nullptr, state_dt, (int)T, (int)D, NT, chunk_len, ws));
         MMF_LAUNCH_CHECK("hgrn_scan_kernel<aggregate>");
     }
-    if (NT > 1) {
-        constexpr auto k2 = hgrn_scan_kernel<TX, TG, MODE, false, STAGES>;
-        MMF_CUDA(mmf_allow_smem<k2>((int)smem));
-        MMF_CUDA(mmf_launch_pdl(k2, grid, dim3(HG_THREADS), smem, st, x_map, g_map, o_map, (const TX*)lb, mask, h0, ht, state_dt,
-                                (int)T, (int)D, NT, chunk_len, ws));
-    } else {
-        constexpr auto k2 = hgrn_scan_kernel<TX, TG, MODE, false, 2>;
-        MMF_CUDA(mmf_allow_smem<k2>((int)smem));
-        MMF_CUDA(mmf_launch_pdl(k2, grid, dim3(HG_THREADS), smem, st, x_map, g_map, o_map, (const TX*)lb, mask, h0, ht, state_dt,
-                                (int)T, (int)D, NT, chunk_len, ws));
-    }
+    constexpr auto k2 = hgrn_scan_kernel<TX, TG, MODE, false>;
+    MMF_CUDA(mmf_allow_smem<k2>((int)smem));
+    MMF_CUDA(mmf_launch_pdl(k2, grid, dim3(HG_THREADS), smem, st, x_map, g_map, o_map, (const TX*)lb, mask, h0, ht, state_dt,
+                            (int)T, (int)D, NT, chunk_len, ws));
     MMF_LAUNCH_CHECK("hgrn_scan_kernel<scan>");
     return MMF_OK;
 }
