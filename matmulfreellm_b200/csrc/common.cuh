@@ -251,10 +251,11 @@ __device__ __forceinline__ int block_sum(int v, int* red) {
 // ---------------------------------------------------------------------------------------
 // inv_k = 1.0 / K, which a kernel forms before it waits for its input.  The quotient is the product with it plus one correction
 // by the exact remainder (Markstein's division step): the fp64 division itself, about 100 instructions for a K that is not a
-// power of two, would sit on the critical path of every row.
+// power of two, would sit on the critical path of every row.  An infinite sum (a row with an infinite entry) has no remainder
+// (inf - inf) and is its own quotient: rstd 0, as the division gives.  The test is on the high word, beside the fp64 chain.
 __device__ __forceinline__ float rstd_from_sumsq(double sumsq, int K, double inv_k, float eps) {
     const double q0 = sumsq * inv_k;
-    const double q = fma(fma(-q0, (double)K, sumsq), inv_k, q0);
+    const double q = __double2hiint(sumsq) == 0x7ff00000 ? q0 : fma(fma(-q0, (double)K, sumsq), inv_k, q0);
     const float mean = (float)q;
     return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
 }

@@ -409,6 +409,31 @@ def test_rowwise_ops_vs_oracle(K, dtype, D):
     assert close(K.swiglu(dev(x), dev(o)), O.swiglu_ref(x, o))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("M,D", [(3, 256), (3, 100), (1500, 2048), (2, 8208)])
+def test_row_with_an_infinite_entry(K, dtype, M, D):
+    """The statistic of a row with an infinite entry is infinite and its rstd 0, as in PyTorch: finite entries come out 0, the
+    infinite one NaN, other rows unchanged.  The int8 codes of its finite entries are 0."""
+    g = torch.Generator().manual_seed(D)
+    x, o, w = torch.randn(M, D, generator=g).to(dtype), torch.randn(M, D, generator=g).to(dtype), torch.rand(D, generator=g) + 0.5
+    clean = x.clone()
+    x[1, 5] = float("inf")
+    xf = x.float()
+    y = xf * torch.rsqrt(xf.square().mean(-1, keepdim=True) + 1e-6) * w
+    got = K.rmsnorm(dev(x), dev(w), 1e-6).float().cpu()
+    gated = K.rmsnorm_swishgate(dev(x), dev(o), dev(w), 1e-6).float().cpu()
+    for t in (got, gated):
+        assert torch.isnan(t[1, 5]) and torch.equal(torch.isnan(t), torch.isnan(y))
+        assert int((t[1] != 0).sum()) == 1                       # the NaN alone
+    keep = [r for r in range(M) if r != 1]
+    assert torch.equal(got[keep], K.rmsnorm(dev(clean), dev(w), 1e-6).float().cpu()[keep])
+    if D % 16 == 0:
+        q, dq, rs = K.act_quant(dev(x), dev(w), 1e-6)
+        q0, dq0, rs0 = K.act_quant(dev(clean), dev(w), 1e-6)
+        assert int((q[1] != 0).sum()) <= 1
+        assert torch.equal(q[keep], q0[keep]) and torch.equal(dq[keep], dq0[keep]) and torch.equal(rs[keep], rs0[keep])
+
+
 def test_swiglu_on_chunk_views(K):
     y = torch.randn(2, 5, 512, generator=torch.Generator().manual_seed(0)).bfloat16()
     gate, up = dev(y).chunk(2, -1)
