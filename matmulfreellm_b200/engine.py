@@ -29,6 +29,7 @@ class GreedyDecoder:
         self.ids = self.next.view(batch_size, 1)
         self.cache = model.model.init_cache(batch_size)
         self.graph: Optional[torch.cuda.CUDAGraph] = None
+        self._graph_logits: Optional[torch.Tensor] = None     # [B, V] buffer that a replay of self.graph writes
         self.kernels_per_step = 0
         self.last_logits: Optional[torch.Tensor] = None
         self._use_graph = use_graph
@@ -36,19 +37,20 @@ class GreedyDecoder:
         # through Python (about 19 us of host time each), which is more than the GPU needs for a short prompt
         self._prompt_seen: dict = {}       # prompt length -> times seen
         self._prompt_graphs: dict = {}     # prompt length -> (graph, static ids and logits buffers), at most PROMPT_GRAPHS entries
-        self._host_graphs: dict = {}       # (ids_host ptr, out_host ptr) -> (graph with the two copies, the buffers)
+        self._host_graphs: dict = {}       # (ids_host ptr, out_host ptr) -> (graph with the two copies, its logits buffer, the host buffers)
 
-    def _step_eager(self):
+    def _step_eager(self) -> torch.Tensor:
+        """One step; returns its logits [B, V].  Inside a captured graph they are a fixed buffer that every replay of that
+        graph rewrites: a caller that samples instead of taking the arg-max reads self.last_logits after step() and
+        overwrites self.next."""
         out = self.model(input_ids=self.ids, past_key_values=self.cache, use_cache=True)
-        # [B, V] logits of the step; inside the captured graph this is a fixed buffer that every replay rewrites, so a
-        # caller that samples instead of taking the arg-max reads it after step() and overwrites self.next
-        self.last_logits = out.logits[:, -1]
-        kernels.argmax_rows(self.last_logits, out=self.next)
-        self._step_logits = self.last_logits
+        logits = out.logits[:, -1]
+        kernels.argmax_rows(logits, out=self.next)
+        return logits
 
     def _capture(self, ids_host: Optional[torch.Tensor] = None, out_host: Optional[torch.Tensor] = None):
-        """Capture one decode step.  With pinned host buffers the copy of the input ids to the device and of the new
-        tokens back are nodes of the same graph (returned, not stored in self.graph)."""
+        """Capture one decode step; returns (graph, its logits buffer).  With pinned host buffers the copy of the input ids
+        to the device and of the new tokens back are nodes of the same graph."""
         saved = [tuple(s.clone() for s in layer) for layer in self.cache.states]
         saved_ids = self.ids.clone()
         side = torch.cuda.Stream(device=self.device)
@@ -64,17 +66,15 @@ class GreedyDecoder:
         with torch.cuda.graph(graph, stream=side):
             if ids_host is not None:
                 self.ids.copy_(ids_host, non_blocking=True)
-            self._step_eager()
+            logits = self._step_eager()
             if out_host is not None:
                 out_host.copy_(self.next, non_blocking=True)
         self.kernels_per_step = _lib.launch_count - before
-        if ids_host is None and out_host is None:
-            self.graph = graph
         for layer, keep in zip(self.cache.states, saved):   # undo the warm-up steps' effect on the state
             for dst, src in zip(layer, keep):
                 dst.copy_(src)
         self.ids.copy_(saved_ids)
-        return graph
+        return graph, logits
 
     PROMPT_GRAPH_MAX_TOKENS = 8192   # larger prompts are bound by the GPU, and their graphs would pin gigabytes
     PROMPT_GRAPHS = 4
@@ -128,9 +128,11 @@ class GreedyDecoder:
     @torch.no_grad()
     def seed(self, past_key_values, last_logits: torch.Tensor) -> torch.Tensor:
         """Take over after a prompt pass made elsewhere (e.g. one with a padding mask): copy its recurrent states
-        into the static cache and pick the first token from its last-position logits [B, V]."""
+        into the static cache and pick the first token from its last-position logits [B, V], which become
+        self.last_logits."""
         torch._foreach_copy_([s for layer in self.cache.states for s in layer], [s for layer in past_key_values for s in layer])
         kernels.argmax_rows(last_logits, out=self.next)
+        self.last_logits = last_logits
         return self.next
 
     @torch.no_grad()
@@ -138,20 +140,21 @@ class GreedyDecoder:
         """Consume self.ids, produce the next token in self.next (and feed it back). Returns self.next."""
         if not self._use_graph:
             before = _lib.launch_count
-            self._step_eager()
+            self.last_logits = self._step_eager()
             self.kernels_per_step = _lib.launch_count - before
         else:
             if self.graph is None:
-                self._capture()
+                self.graph, self._graph_logits = self._capture()
             self.graph.replay()
-            self.last_logits = self._step_logits
+            self.last_logits = self._graph_logits
         return self.next
 
     @torch.no_grad()
     def step_host(self, ids_host: torch.Tensor, out_host: torch.Tensor) -> None:
         """One decode step driven from the host: the token ids [B, 1] are read from `ids_host`, the new tokens [B] are
-        written to `out_host` (both int64 in pinned memory).  The two copies and the step's kernels are one CUDA graph
-        launch; the call returns once it is enqueued — synchronise the stream before reading `out_host`."""
+        written to `out_host` (both int64 in pinned memory); the step's logits are left in self.last_logits.  The two
+        copies and the step's kernels are one CUDA graph launch; the call returns once it is enqueued — synchronise the
+        stream before reading `out_host`."""
         if not (ids_host.is_pinned() and out_host.is_pinned()):
             raise ValueError("step_host needs pinned host buffers")
         if ids_host.shape != self.ids.shape or out_host.shape != self.next.shape or ids_host.dtype != torch.int64 \
@@ -165,9 +168,10 @@ class GreedyDecoder:
         key = (ids_host.data_ptr(), out_host.data_ptr())
         entry = self._host_graphs.get(key)
         if entry is None:
-            entry = (self._capture(ids_host, out_host), ids_host, out_host)   # the graph keeps pointing at these buffers
+            entry = (*self._capture(ids_host, out_host), ids_host, out_host)   # the graph keeps pointing at these buffers
             self._host_graphs = {key: entry}
         entry[0].replay()
+        self.last_logits = entry[1]
 
     @torch.no_grad()
     def generate(self, prompt_ids: torch.Tensor, max_new_tokens: int) -> torch.Tensor:

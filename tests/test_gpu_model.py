@@ -532,6 +532,40 @@ def test_decoder_step_driven_from_pinned_host_buffers(mm):
         dec.step_host(ids_host, torch.empty(4, dtype=torch.int64).pin_memory())
 
 
+def test_last_logits_follow_the_graph_that_ran(mm):
+    """`GreedyDecoder.last_logits` after every kind of step is the logits of that step, whichever graphs were captured before:
+    the token of the step is their arg-max, and they equal those of a decoder without graphs bit for bit."""
+    from matmulfreellm_b200.engine import GreedyDecoder
+    cfg = tiny_cfg()
+    model = build_gpu_model(O.random_weights(cfg, seed=27), cfg, torch.bfloat16)
+    g = torch.Generator().manual_seed(5)
+    B = 3
+    prompts = [torch.randint(0, cfg.vocab_size, (B, 7), generator=g).cuda() for _ in range(4)]
+    dec, eager = GreedyDecoder(model, B), GreedyDecoder(model, B, use_graph=False)
+    ids_host = torch.zeros(B, 1, dtype=torch.int64).pin_memory()
+    out_host = torch.zeros(B, dtype=torch.int64).pin_memory()
+
+    def advance(kind):
+        for d in (dec, eager):
+            if kind == "host":
+                ids_host.copy_(d.ids)
+                torch.cuda.synchronize()
+                d.step_host(ids_host, out_host)
+                torch.cuda.synchronize()
+            elif kind == "step":
+                d.step()
+            else:
+                d.prefill(prompts[kind])
+        assert torch.equal(dec.last_logits, eager.last_logits), kind
+        assert torch.equal(dec.last_logits.gather(1, dec.ids)[:, 0], dec.last_logits.amax(1)), kind
+
+    for kind in (0, "host", 1, "host", "step", "host", "step", 2, "step", "step", 3, "host"):
+        advance(kind)
+    out = model(input_ids=prompts[0], use_cache=True, last_token_only=True)
+    dec.seed(out.past_key_values, out.logits[:, -1])
+    assert torch.equal(dec.last_logits, out.logits[:, -1])
+
+
 def test_generate_graph_path_equals_step_loop(mm):
     """`generate` replays greedy decode steps from a CUDA graph; tokens, the handling of eos (finished sequences
     keep emitting it, the result ends where the last sequence finishes) and left-padded prompts must equal the
