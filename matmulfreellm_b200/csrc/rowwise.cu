@@ -265,6 +265,8 @@ argmax_kernel(const T* __restrict__ logits, int64_t ld, int V, int64_t* __restri
 //   p_i = softmax(logits_i / temperature); keep the smallest set of most probable tokens whose mass reaches top_p
 //   (all tokens with p_i >= tau, tau found by bisection on the float bit pattern; tokens tied at tau are all kept);
 //   the sample is the first kept token, in index order, at which the running kept mass exceeds u * (kept mass).
+// tau is at least the smallest positive float: with top_p = 1 the search can end at 0 (its sums and the total are formed in
+// different orders), and a token of probability zero is never kept.
 // Sums are accumulated in fp64 in a fixed order, so the result does not depend on scheduling.
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -302,7 +304,7 @@ sample_top_p_kernel(const T* __restrict__ logits, int64_t ld, int V, float inv_t
         const uint32_t mid = lo + (hi - lo) / 2u;
         if (mass_ge(__uint_as_float(mid)) >= want) lo = mid; else hi = mid;
     }
-    const float tau = __uint_as_float(lo);
+    const float tau = __uint_as_float(max(lo, 1u));
     // kept mass per thread, then an exclusive prefix in thread order (= token order)
     double part = 0.0;
     for (int c = c0; c < c1; ++c) {
@@ -481,7 +483,7 @@ sample_top_p_smem_kernel(const T* __restrict__ logits, int64_t ld, int V, float 
         if (tid == 0) s_tau = lo;
     }
     __syncthreads();
-    const float tau = __uint_as_float(s_tau);
+    const float tau = __uint_as_float(max(s_tau, 1u));
     // the draw, in token order: warp w holds the kept mass of tokens [w * R, (w + 1) * R); the range that contains the target is
     // then cut into 32 groups, one per warp, and the group that contains it into tokens
     const int R = ((V + W - 1) / W + 31) & ~31, GR = R / 32;

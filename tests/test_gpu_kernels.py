@@ -787,6 +787,28 @@ def test_sample_top_p_vocabulary_edges(K, V):
         assert np.array_equal(got[safe], ref[safe]) and (got >= 0).all() and (got < V).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("V", [1000, 9001, 40960])
+def test_sample_top_p_zero_probabilities(K, dtype, V):
+    """A token whose probability is zero (logit -inf, or so low that exp underflows) is never drawn, not even with u = 0 and
+    top_p = 1.  The kernel of short rows and the one of long rows (the same logits followed by
+    -inf up to 41000) draw the same token."""
+    g = torch.Generator().manual_seed(V)
+    M = 32
+    logits = torch.randn(M, V, generator=g) * 3
+    logits[:, :5] = -float("inf")
+    logits[:, 5:9] = -1e4
+    logits = logits.to(dtype)
+    pad = torch.cat([logits, torch.full((M, 41000 - V), -float("inf"), dtype=dtype)], 1)
+    for top_p in (1.0, 0.9, 0.3):
+        for u in (torch.zeros(M), torch.full((M,), 1.0 - 2.0 ** -24), torch.rand(M, generator=g)):
+            got = K.sample_top_p(dev(logits), 1.0, top_p, dev(u)).cpu()
+            assert int(got.min()) >= 9, (top_p, u[0])
+            assert torch.equal(K.sample_top_p(dev(pad), 1.0, top_p, dev(u)).cpu(), got)
+        if top_p == 1.0:
+            assert torch.equal(K.sample_top_p(dev(logits), 1.0, top_p, dev(torch.zeros(M))).cpu(), torch.full((M,), 9))
+
+
 @pytest.mark.parametrize("gate_is_log", [True, False])
 def test_time_sliced_scan_stitches_to_whole_scan(K, gate_is_log):
     """The exchange of the sequence-sharded scan, with the ranks emulated one after the other on one GPU: every
