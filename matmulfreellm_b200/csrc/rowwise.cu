@@ -266,7 +266,7 @@ argmax_kernel(const T* __restrict__ logits, int64_t ld, int V, int64_t* __restri
 //   (all tokens with p_i >= tau, tau found by bisection on the float bit pattern; tokens tied at tau are all kept);
 //   the sample is the first kept token, in index order, at which the running kept mass exceeds u * (kept mass).
 // tau is at least the smallest positive float: with top_p = 1 the search can end at 0 (its sums and the total are formed in
-// different orders), and a token of probability zero is never kept.
+// different orders), and a token of probability zero is never kept.  A NaN logit is in no sum and never kept.
 // Sums are accumulated in fp64 in a fixed order, so the result does not depend on scheduling.
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -411,7 +411,7 @@ sample_top_p_smem_kernel(const T* __restrict__ logits, int64_t ld, int V, float 
     for (int c = tid; c < V; c += SAMPLE_THREADS) {
         const float e = expf(__fsub_rn(p[c], mx));
         p[c] = e;
-        sum += widen(e);
+        if (e >= 0.0f) sum += widen(e);
     }
     const double total = block_total(sum);
     const double want = (double)top_p * total;

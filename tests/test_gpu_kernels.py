@@ -789,9 +789,9 @@ def test_sample_top_p_vocabulary_edges(K, V):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("V", [1000, 9001, 40960])
-def test_sample_top_p_zero_probabilities(K, dtype, V):
+def test_sample_top_p_zero_probabilities_and_nan(K, dtype, V):
     """A token whose probability is zero (logit -inf, or so low that exp underflows) is never drawn, not even with u = 0 and
-    top_p = 1.  The kernel of short rows and the one of long rows (the same logits followed by
+    top_p = 1; a NaN logit counts as -inf.  The kernel of short rows and the one of long rows (the same logits followed by
     -inf up to 41000) draw the same token."""
     g = torch.Generator().manual_seed(V)
     M = 32
@@ -800,11 +800,14 @@ def test_sample_top_p_zero_probabilities(K, dtype, V):
     logits[:, 5:9] = -1e4
     logits = logits.to(dtype)
     pad = torch.cat([logits, torch.full((M, 41000 - V), -float("inf"), dtype=dtype)], 1)
+    nan = logits.clone()
+    nan[:, :9] = float("nan")
     for top_p in (1.0, 0.9, 0.3):
         for u in (torch.zeros(M), torch.full((M,), 1.0 - 2.0 ** -24), torch.rand(M, generator=g)):
             got = K.sample_top_p(dev(logits), 1.0, top_p, dev(u)).cpu()
             assert int(got.min()) >= 9, (top_p, u[0])
             assert torch.equal(K.sample_top_p(dev(pad), 1.0, top_p, dev(u)).cpu(), got)
+            assert torch.equal(K.sample_top_p(dev(nan), 1.0, top_p, dev(u)).cpu(), got)
         if top_p == 1.0:
             assert torch.equal(K.sample_top_p(dev(logits), 1.0, top_p, dev(torch.zeros(M))).cpu(), torch.full((M,), 9))
 
