@@ -788,7 +788,7 @@ def test_sample_top_p_vocabulary_edges(K, V):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("V", [1000, 9001, 40960])
+@pytest.mark.parametrize("V", [1000, 5000, 9001, 40960])      # at 5000 the search ends at threshold 0 in one row of seven
 def test_sample_top_p_zero_probabilities_and_nan(K, dtype, V):
     """A token whose probability is zero (logit -inf, or so low that exp underflows) is never drawn, not even with u = 0 and
     top_p = 1; a NaN logit counts as -inf.  The kernel of short rows and the one of long rows (the same logits followed by
