@@ -600,7 +600,8 @@ int pf_launch(const BitLinearArgs& a, cudaStream_t st) {
         p.tma_out = 1;
     }
 
-    constexpr int sms = 148;
+    int sms = 0;
+    MMF_CUDA(mmf_sm_count(&sms));
     constexpr auto kernel = bitlinear_mma_prefill_kernel<C>;
     MMF_CUDA(mmf_allow_smem<kernel>(C::SMEM));
     cudaLaunchConfig_t cfg = {};

@@ -86,6 +86,18 @@ template <auto kernel> inline cudaError_t mmf_allow_smem(int limit) {
     return e;
 }
 
+// SMs of the current device (148 on a whole B200, fewer on a partition of one), asked of the runtime once per host thread.
+inline cudaError_t mmf_sm_count(int* sms) {
+    thread_local int known[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 64 && known[dev]) { *sms = known[dev]; return cudaSuccess; }
+    e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess && dev < 64) known[dev] = *sms;
+    return e;
+}
+
 // ---------------------------------------------------------------------------------------
 // element conversion (round-to-nearest-even on store, exact on load)
 // ---------------------------------------------------------------------------------------
