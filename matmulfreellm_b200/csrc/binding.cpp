@@ -276,6 +276,7 @@ PyObject* hgrn_scan(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (bytes) ws = at::empty({bytes}, x.options().dtype(at::kByte));
         MMF_CALL(mmf_hgrn_scan, x.data_ptr(), dtype_code(x), g.data_ptr(), dtype_code(g), ptr(h0), ptr(ht), state_code, o.data_ptr(), B, T, D,
                  (int)is_log, ptr(ws), bytes, c10::cuda::getCurrentCUDAStream(dev).stream());
+        if (x.numel()) g_launches += bytes ? 2 : 1;          // a scan whose time is split makes two passes
         PyObject* po = THPVariable_Wrap(std::move(o));
         PyObject* ph = want ? THPVariable_Wrap(std::move(ht)) : Py_NewRef(Py_None);
         PyObject* t = PyTuple_Pack(2, po, ph);
@@ -626,7 +627,7 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                              hg_bytes ? b + hg : nullptr, hg_bytes, st);
                     MMF_CALL(mmf_gatenorm_quant, b + ifg + 2 * h * es, 3 * h, b + o, h, c.dtype, L.gnorm_w, L.gnorm_eps, L.o_nw, L.eps_bl, Q, DQ, RS,
                              M, h, st);
-                    ++launches;
+                    launches += hg_bytes ? 2 : 1;
                 }
                 linear(L.o, b + z, M);
                 MMF_CALL(mmf_prenorm_quant, b + z, h, x, h, c.dtype, 0, L.mlp_norm_w, c.eps, next, nullptr, 1, L.gate_nw, nullptr, nullptr, L.eps_bl,

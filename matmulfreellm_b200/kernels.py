@@ -276,8 +276,9 @@ def hgrn_scan(x: torch.Tensor, g: torch.Tensor, initial_state: Optional[torch.Te
     """x, g: [..., T, D] contiguous; leading dims are independent sequences. Returns (o, final_state|None)."""
     if final_state_out is None:
         sdt = state_dtype or (initial_state.dtype if initial_state is not None else torch.float32)
-        out = _lib.native().hgrn_scan(x, g, initial_state, output_final_state, gate_is_log, sdt)
-        _lib.launch_count += 1
+        native = _lib.native()
+        out = native.hgrn_scan(x, g, initial_state, output_final_state, gate_is_log, sdt)
+        _lib.launch_count += native.take_launches()
         return out
     _need_cuda(x, g, initial_state)
     if x.shape != g.shape or x.dim() < 2:
@@ -302,6 +303,7 @@ def hgrn_scan(x: torch.Tensor, g: torch.Tensor, initial_state: Optional[torch.Te
     ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device) if nbytes else None
     _lib.call("mmf_hgrn_scan", x.data_ptr(), _code(x.dtype), g.data_ptr(), _code(g.dtype), _ptr(h0), _ptr(ht),
               _code(sdt), o.data_ptr(), B, T, D, int(gate_is_log), _ptr(ws), nbytes, _stream())
+    _lib.launch_count += nbytes > 0         # a scan whose time is split makes two passes
     return o, ht
 
 
@@ -328,6 +330,7 @@ def hgrn_gated(i_raw: torch.Tensor, f_raw: torch.Tensor, lower_bound: Optional[t
         raise ValueError("mask must be a contiguous uint8 CUDA tensor [B, T]")
     _lib.call("mmf_hgrn_gated_masked", i_raw.data_ptr(), f_raw.data_ptr(), ld, _code(i_raw.dtype), _ptr(lower_bound),
               _ptr(mask), state.data_ptr(), o.data_ptr(), B, T, D, _ptr(ws), nbytes, _stream())
+    _lib.launch_count += nbytes > 0
     return o
 
 

@@ -566,6 +566,56 @@ def test_last_logits_follow_the_graph_that_ran(mm):
     assert torch.equal(dec.last_logits, out.logits[:, -1])
 
 
+def test_launch_count_is_the_number_of_kernels(mm):
+    """`_lib.launch_count`, which the benchmark reports, advances by the kernels that a call really launches: the kernel nodes
+    of a graph captured from it (time-split scans make two passes; a forward of one, four or 32 rows takes different chains)."""
+    from cuda.bindings import runtime as rt
+    from matmulfreellm_b200 import _lib, kernels
+    cfg = tiny_cfg()
+    model = build_gpu_model(O.random_weights(cfg, seed=4), cfg, torch.bfloat16)
+    layer = model.model.layers[0].mlp.down_proj
+    g = torch.Generator(device="cuda").manual_seed(1)
+
+    def scan(B, T, D, into=None):
+        x = torch.randn(B, T, D, generator=g, device="cuda").bfloat16()
+        gate = torch.rand(B, T, D, generator=g, device="cuda").bfloat16()
+        return lambda: kernels.hgrn_scan(x, gate, None, True, False, torch.float32, into)
+
+    def gated(B, T, D):
+        x, s = torch.randn(B, T, 2 * D, generator=g, device="cuda").bfloat16(), torch.zeros(B, D, device="cuda")
+        return lambda: kernels.hgrn_gated(x[:, :, :D], x[:, :, D:], None, s)
+
+    def forward(B, T):
+        ids = torch.randint(0, cfg.vocab_size, (B, T), device="cuda")
+        cache = model.model.init_cache(B)
+        return lambda: model(input_ids=ids, past_key_values=cache, use_cache=True)
+
+    def linear(M):
+        x = torch.randn(M, cfg.intermediate_size, generator=g, device="cuda").bfloat16()
+        return lambda: layer(x)
+
+    calls = {"scan, split": scan(1, 2048, 128), "scan": scan(8, 64, 128), "scan of one step": scan(3, 1, 128),
+             "scan into a given state": scan(1, 2048, 128, torch.empty(1, 128, device="cuda")), "gated, split": gated(1, 1024, 64),
+             "prompt, split": forward(1, 1024), "prompt": forward(2, 40), "step of 1": forward(1, 1), "step of 4": forward(4, 1),
+             "step of 12": forward(12, 1), "step of 32": forward(32, 1), "linear 1": linear(1), "linear 5": linear(5)}
+    side = torch.cuda.Stream()
+    with torch.no_grad():
+        for name, call in calls.items():
+            with torch.cuda.stream(side):
+                call()
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph(keep_graph=True)
+            with torch.cuda.graph(graph, stream=side):
+                before = _lib.launch_count
+                call()
+                counted = _lib.launch_count - before
+            raw = rt.cudaGraph_t(init_value=graph.raw_cuda_graph())
+            err, _, n = rt.cudaGraphGetNodes(raw, 0)
+            err, nodes, n = rt.cudaGraphGetNodes(raw, n)
+            kinds = [rt.cudaGraphNodeGetType(node)[1] for node in nodes[:n]]
+            assert counted == sum(k == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel for k in kinds), name
+
+
 def test_generate_graph_path_equals_step_loop(mm):
     """`generate` replays greedy decode steps from a CUDA graph; tokens, the handling of eos (finished sequences
     keep emitting it, the result ends where the last sequence finishes) and left-padded prompts must equal the
