@@ -110,5 +110,6 @@ def layer_norm_linear_quant_fn(x, norm_weight, norm_bias, linear_weight, linear_
     if not is_rms_norm or norm_bias is not None or residual is not None or prenorm:
         raise NotImplementedError("only the RMSNorm, no-residual form used by FusedBitLinear is provided")
     pw = kernels.pack_weight(linear_weight)
+    x = x.contiguous()          # any strides and row alignment are taken
     y = kernels.bitlinear_forward(x, None if norm_weight is None else norm_weight.detach().float().contiguous(), pw, eps)
     return y if linear_bias is None else y + linear_bias.to(y.dtype)

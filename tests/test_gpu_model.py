@@ -83,6 +83,20 @@ def test_fused_bitlinear_module(mm):
     assert torch.allclose(weight_quant(wf.cuda()).cpu(), O.weight_quant(wf), rtol=1e-6, atol=1e-9)
 
 
+@pytest.mark.parametrize("M", [2, 5])
+def test_linear_quant_fn_takes_any_strides(mm, M):
+    """layer_norm_linear_quant_fn on a slice with an odd row pitch and start, on a transposed and on an expanded input: the result
+    of a contiguous copy."""
+    from mmfreelm.ops.fusedbitnet import layer_norm_linear_quant_fn
+    K, N = 256, 384
+    g = torch.Generator().manual_seed(M)
+    w, nw = (torch.randn(N, K, generator=g) * 0.02).cuda(), torch.rand(K, generator=g).cuda()
+    wide = torch.randn(M, K + 3, generator=g).bfloat16().cuda()
+    for x in (wide[:, 1:K + 1], torch.randn(K, M, generator=g).bfloat16().cuda().t(), wide[:1, :K].expand(M, K), wide[:, :K].view(1, M, K)):
+        want = layer_norm_linear_quant_fn(x.clone(memory_format=torch.contiguous_format), nw, None, w, None, is_rms_norm=True)
+        assert torch.equal(layer_norm_linear_quant_fn(x, nw, None, w, None, is_rms_norm=True), want)
+
+
 def test_hgrn_ops_reference_selfcheck_shapes(mm):
     """The reference's own self-check (recurrent_fuse.py:188-217): B,H,T,D = 8,4,512,128, bf16, seed 42,
     g = sigmoid(randn), x = (1-g)*randn, random h0 — fused op against the naive loop."""
