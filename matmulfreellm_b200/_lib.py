@@ -24,6 +24,19 @@ _ERR_NAMES = {
     -5: "MMF_ERR_ARCH", -6: "MMF_ERR_WORKSPACE", -7: "MMF_ERR_TIMEOUT",
 }
 
+class DecodeLinearArgs(ctypes.Structure):
+    """mmf_decode_linear_args of the header, field by field."""
+    _fields_ = [("prologue", c_int), ("epilogue", c_int), ("dtype", c_int), ("round_sum_first", c_int), ("M", c_int64),
+                ("N", c_int64), ("K", c_int64), ("packed", c_void_p), ("w_scale", c_void_p), ("x", c_void_p),
+                ("residual", c_void_p), ("ld_x", c_int64), ("ld_residual", c_int64), ("row_ids", c_void_p), ("x_rows", c_int64),
+                ("norm_w", c_void_p), ("eps_norm", c_float), ("eps_bl", c_float), ("bl_norm_w", c_void_p * 3),
+                ("residual_out", c_void_p), ("codes", c_void_p), ("dq", c_void_p), ("rowsum", c_void_p), ("out", c_void_p),
+                ("ld_out", c_int64), ("g_out", c_void_p), ("lower_bound", c_void_p), ("mask", c_void_p), ("state", c_void_p)]
+
+
+PRO_QUANT, PRO_PRENORM, PRO_GATENORM = 1, 2, 3
+EPI_STORE, EPI_GATES, EPI_SWIGLU = 0, 1, 2
+
 # name -> (restype, argtypes); must list every symbol include/mmfree_b200.h declares
 PROTOTYPES = {
     "mmf_last_error": (c_char_p, []),

@@ -14,6 +14,8 @@ extern "C" int mmf_decode_linear(const mmf_decode_linear_args* args, void* strea
     const int max_m = a.codes ? MMF_DECODE_LINEAR_MAX_M : MMF_DECODE_LINEAR_FUSED_MAX_M;
     MMF_REQUIRE(a.M <= max_m, MMF_ERR_BAD_SHAPE, "mmf_decode_linear: at most %d token rows (M=%lld)", max_m, (long long)a.M);
     MMF_REQUIRE(!a.codes || (a.dq && a.rowsum && mmf_aligned(a.codes, 16)), MMF_ERR_BAD_ARG, "mmf_decode_linear: incomplete workspace");
+    MMF_REQUIRE(((a.M <= 1 && !a.row_ids) || a.ld_x >= a.K) && (!a.residual || a.M <= 1 || a.ld_residual >= a.K), MMF_ERR_BAD_SHAPE,
+                "mmf_decode_linear: row pitch below K");
     MMF_REQUIRE(a.x && (a.prologue != MMF_PRO_GATENORM || a.residual), MMF_ERR_BAD_ARG, "mmf_decode_linear: input row missing");
     MMF_REQUIRE(mmf_aligned(a.packed, 16) && mmf_aligned(a.out, 16) && mmf_aligned(a.x, 16) && a.ld_x % 8 == 0 &&
                     (!a.residual || (mmf_aligned(a.residual, 16) && a.ld_residual % 8 == 0)) && (!a.residual_out || mmf_aligned(a.residual_out, 16)) &&

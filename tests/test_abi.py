@@ -74,6 +74,45 @@ def test_argument_validation_needs_no_device(lib):
     _lib.call("mmf_hgrn_scan", p, 1, p, 1, None, None, 0, p, 0, 4, 16, 0, None, 0, None)
 
 
+def test_decode_linear_refuses_bad_arguments(lib):
+    """Every refusal of mmf_decode_linear comes from the host, before any CUDA call."""
+    buf = (ctypes.c_char * 4096)()
+    p = (ctypes.addressof(buf) + 15) & ~15
+    L = _lib
+
+    def rc(**change):
+        args = dict(prologue=L.PRO_PRENORM, epilogue=L.EPI_STORE, dtype=L.BF16, M=2, N=64, K=128, packed=p, w_scale=p, x=p, ld_x=128,
+                    out=p, ld_out=64)
+        args.update(change)
+        bl = args.pop("bl_norm_w", (None, None, None))
+        return lib.mmf_decode_linear(ctypes.byref(L.DecodeLinearArgs(bl_norm_w=(ctypes.c_void_p * 3)(*bl), **args)), None)
+
+    BAD_ARG, BAD_SHAPE, ALIGN = -1, -2, -3
+    assert lib.mmf_decode_linear(None, None) == BAD_ARG
+    ws = dict(codes=p, dq=p, rowsum=p)
+    gates = dict(epilogue=L.EPI_GATES, N=384, state=p, g_out=p)
+    gatenorm = dict(prologue=L.PRO_GATENORM, residual=p, ld_residual=128)
+    for want, cases in {
+        BAD_ARG: [dict(dtype=L.F32), dict(dtype=7), dict(packed=None), dict(w_scale=None), dict(out=None), dict(x=None), dict(prologue=0),
+                  dict(prologue=9), dict(epilogue=9), dict(gatenorm, residual=None), dict(ws, dq=None), dict(ws, rowsum=None),
+                  dict(ws, codes=p + 8), dict(gates, state=None), dict(gates, g_out=None), dict(gates, state=p + 4),
+                  dict(gates, g_out=p + 2), dict(gates, lower_bound=p + 2), dict(ld_out=63), dict(row_ids=p, x_rows=0),
+                  dict(row_ids=p, x_rows=5, residual=p, ld_residual=128), dict(row_ids=p, x_rows=5, prologue=L.PRO_QUANT)],
+        BAD_SHAPE: [dict(M=-1), dict(M=3), dict(ws, M=17), dict(N=0), dict(N=1 << 24), dict(K=0), dict(K=96), dict(K=4160, ld_x=4160),
+                    dict(K=8256, ld_x=8256, prologue=L.PRO_QUANT), dict(gatenorm, K=4160, ld_x=4160, ld_residual=4160),
+                    dict(gates, N=256), dict(gates, K=192, N=576, ld_x=192), dict(epilogue=L.EPI_SWIGLU, N=66, ld_out=34),
+                    dict(epilogue=L.EPI_SWIGLU, ld_out=33), dict(epilogue=L.EPI_SWIGLU, ld_out=30), dict(ld_x=120), dict(ld_x=0),
+                    dict(gatenorm, ld_residual=120), dict(row_ids=p, x_rows=5, M=1, ld_x=64)],
+        ALIGN: [dict(packed=p + 8), dict(x=p + 2), dict(out=p + 8), dict(ld_x=129), dict(residual=p + 8, ld_residual=128),
+                dict(residual=p, ld_residual=132), dict(residual_out=p + 8), dict(norm_w=p + 4), dict(bl_norm_w=(p + 4, None, None)),
+                dict(gates, bl_norm_w=(p, p, p + 8))],
+    }.items():
+        for change in cases:
+            assert rc(**change) == want, (change, lib.mmf_last_error())
+    for change in (dict(), ws, gates, gatenorm, dict(epilogue=L.EPI_SWIGLU, ld_out=32)):
+        assert rc(**change, M=0) == 0           # an empty problem is accepted without a launch
+
+
 def test_cpu_tensors_are_refused():
     import torch
     from matmulfreellm_b200 import kernels
