@@ -263,6 +263,8 @@ def bitlinear(q: torch.Tensor, dq: torch.Tensor, rowsum: torch.Tensor, pw: Packe
 def bitlinear_forward(x: torch.Tensor, norm_weight: Optional[torch.Tensor], pw: PackedWeight, eps: float) -> torch.Tensor:
     """FusedBitLinear's forward: RMSNorm + int8 quantisation + contraction of x [..., K] -> [..., N] in x.dtype."""
     native = _lib.native()
+    if x.is_cuda:
+        _lib.require_device(x.get_device())
     out = native.bitlinear(x, norm_weight, pw.packed, pw.scale, pw.N, eps)
     _lib.launch_count += native.take_launches()
     return out
@@ -277,6 +279,8 @@ def hgrn_scan(x: torch.Tensor, g: torch.Tensor, initial_state: Optional[torch.Te
     if final_state_out is None:
         sdt = state_dtype or (initial_state.dtype if initial_state is not None else torch.float32)
         native = _lib.native()
+        if x.is_cuda:
+            _lib.require_device(x.get_device())
         out = native.hgrn_scan(x, g, initial_state, output_final_state, gate_is_log, sdt)
         _lib.launch_count += native.take_launches()
         return out

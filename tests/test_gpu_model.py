@@ -580,6 +580,28 @@ def test_last_logits_follow_the_graph_that_ran(mm):
     assert torch.equal(dec.last_logits, out.logits[:, -1])
 
 
+def test_native_calls_check_the_device(mm, monkeypatch):
+    """On a GPU that the library was not built for, the calls that go through the native host path raise the device check's
+    error, as the others do (the check is made to fail here: it runs once per device)."""
+    from matmulfreellm_b200 import _lib, kernels
+    cfg = tiny_cfg()
+    model = build_gpu_model(O.random_weights(cfg, seed=4), cfg, torch.bfloat16)
+    ids = torch.zeros(1, 3, dtype=torch.int64, device="cuda")
+    model(input_ids=ids)
+    layer = model.model.layers[0].mlp.down_proj
+    x = torch.randn(2, 8, cfg.intermediate_size, device="cuda").bfloat16()
+
+    def call(name, *args):
+        raise _lib.MMFreeError(name, -5, "built for sm_100a only")
+
+    monkeypatch.setattr(_lib, "_device_checked", set())
+    monkeypatch.setattr(_lib, "call", call)
+    object.__setattr__(model, "_fused_runner", None)
+    for fn in (lambda: layer(x), lambda: kernels.hgrn_scan(x, x, None, True, False), lambda: model(input_ids=ids)):
+        with pytest.raises(_lib.MMFreeError, match="mmf_check_device failed with MMF_ERR_ARCH"):
+            fn()
+
+
 def test_launch_count_is_the_number_of_kernels(mm):
     """`_lib.launch_count`, which the benchmark reports, advances by the kernels that a call really launches: the kernel nodes
     of a graph captured from it (time-split scans make two passes; a forward of one, four or 32 rows takes different chains)."""
