@@ -19,6 +19,7 @@ TILE_ROWS, TILE_K = 128, 64
 ABSMEAN_PARTIALS = 1024
 ABI_VERSION = 2
 
+ERR_CUDA = -4
 _ERR_NAMES = {
     -1: "MMF_ERR_BAD_ARG", -2: "MMF_ERR_BAD_SHAPE", -3: "MMF_ERR_ALIGN", -4: "MMF_ERR_CUDA",
     -5: "MMF_ERR_ARCH", -6: "MMF_ERR_WORKSPACE", -7: "MMF_ERR_TIMEOUT",

@@ -264,7 +264,11 @@ class FusedRunner:
         mask = None
         if attention_mask is not None:
             mask = (attention_mask.to(self.device) != 0).to(torch.uint8).contiguous()
-        out = self._native.chain_forward(self.chain, input_ids, inputs_embeds, states, mask, last_only, want_logits, want_hidden)
+        try:
+            out = self._native.chain_forward(self.chain, input_ids, inputs_embeds, states, mask, last_only, want_logits, want_hidden)
+        except _lib.MMFreeError as e:
+            kernels._after_failure(e)
+            raise
         _lib.launch_count += self._native.take_launches()
         return out
 

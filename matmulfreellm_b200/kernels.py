@@ -204,6 +204,12 @@ def _rezero_workspaces() -> None:
             ws.zero_()
 
 
+def _after_failure(e: _lib.MMFreeError) -> None:
+    """After a native call failed: clear the workspaces unless its arguments were refused, when nothing was launched."""
+    if e.code == _lib.ERR_CUDA:
+        _rezero_workspaces()
+
+
 def check_status() -> None:
     """Synchronise and raise if any BitLinear kernel reported a device-side wait that gave up (status word
     at the start of the split-K workspace).  Costs a device sync; meant for tests and debugging."""
@@ -265,7 +271,11 @@ def bitlinear_forward(x: torch.Tensor, norm_weight: Optional[torch.Tensor], pw: 
     native = _lib.native()
     if x.is_cuda:
         _lib.require_device(x.get_device())
-    out = native.bitlinear(x, norm_weight, pw.packed, pw.scale, pw.N, eps)
+    try:
+        out = native.bitlinear(x, norm_weight, pw.packed, pw.scale, pw.N, eps)
+    except _lib.MMFreeError as e:
+        _after_failure(e)
+        raise
     _lib.launch_count += native.take_launches()
     return out
 

@@ -1,0 +1,44 @@
+"""The host path around the kernels, without a GPU: what happens after a failed native call, and how a replaced parameter is noticed."""
+import pytest
+import torch
+
+from matmulfreellm_b200 import _build, _lib, kernels
+
+
+@pytest.fixture(scope="module", autouse=True)
+def built():
+    _build.build_library()
+    _build.build_native()
+
+
+def test_failed_native_call_clears_the_workspaces(monkeypatch):
+    """A failed launch may leave partial sums in the split-K workspaces, which the kernels expect zeroed: they are cleared before
+    the error is raised, on the native path as on the ctypes one; refused arguments (nothing was launched) clear nothing."""
+    from matmulfreellm_b200.engine import FusedRunner
+
+    class Failing:
+        code = -4
+
+        def bitlinear(self, *args):
+            raise _lib.MMFreeError("mmf_bitlinear", self.code, "launch failed")
+
+        chain_forward = bitlinear
+
+    cleared = []
+    monkeypatch.setattr(kernels, "_rezero_workspaces", lambda: cleared.append(1))
+    monkeypatch.setattr(_lib, "native", Failing)
+    pw = kernels.PackedWeight(torch.zeros(1), torch.zeros(1), 1, 64)
+    with pytest.raises(_lib.MMFreeError, match="launch failed"):
+        kernels.bitlinear_forward(torch.zeros(1, 64), None, pw, 1e-6)
+    assert len(cleared) == 1
+    runner = object.__new__(FusedRunner)
+    runner._native, runner.chain, runner.device = Failing(), None, torch.device("cpu")
+    with pytest.raises(_lib.MMFreeError, match="launch failed"):
+        runner.forward(None, None, [], False)
+    assert len(cleared) == 2
+    monkeypatch.setattr(Failing, "code", -3)
+    with pytest.raises(_lib.MMFreeError):
+        kernels.bitlinear_forward(torch.zeros(1, 64), None, pw, 1e-6)
+    with pytest.raises(_lib.MMFreeError):
+        runner.forward(None, None, [], False)
+    assert len(cleared) == 2
