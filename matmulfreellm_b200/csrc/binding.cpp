@@ -289,11 +289,22 @@ PyObject* hgrn_scan(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // ---------------------------------------------------------------------------------------------------------------
 // parameter watch
 // ---------------------------------------------------------------------------------------------------------------
+// What a slot holds is told by addresses and a version number.  The weak references keep the addresses of the tensor and of its
+// storage from being used again for others (they do not keep the memory of the values): without them a parameter that was dropped
+// and replaced could leave every address as it was.
+struct Held {
+    const void *impl = nullptr, *storage = nullptr, *data = nullptr;
+    int64_t version = 0;
+    at::ScalarType dtype = at::kByte;
+    bool operator==(const Held& o) const {
+        return impl == o.impl && storage == o.storage && data == o.data && version == o.version && dtype == o.dtype;
+    }
+};
 struct Slot {
     PyObject *dict, *name;        // owned references
-    const void *impl, *data;      // what the slot held when the watch was made
-    int64_t version;
-    at::ScalarType dtype;
+    Held held;                    // what the slot held when the watch was made
+    c10::weak_intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl> impl{c10::intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl>()};
+    c10::weak_intrusive_ptr<c10::StorageImpl> storage{c10::intrusive_ptr<c10::StorageImpl>()};
 };
 struct Watch {
     std::vector<Slot> slots;
@@ -301,18 +312,22 @@ struct Watch {
         for (Slot& s : slots) { Py_DECREF(s.dict); Py_DECREF(s.name); }
     }
 };
-void look(PyObject* dict, PyObject* name, Slot& s) {
+const at::Tensor* in_slot(PyObject* dict, PyObject* name) {
     PyObject* v = PyDict_GetItem(dict, name);     // borrowed
-    s.impl = s.data = nullptr;
-    s.version = 0;
-    s.dtype = at::kByte;
-    if (v && THPVariable_Check(v)) {
-        const at::Tensor& t = THPVariable_Unpack(v);
-        s.impl = t.unsafeGetTensorImpl();
-        s.data = t.has_storage() ? t.const_data_ptr() : nullptr;
-        s.version = t.is_inference() ? 0 : (int64_t)t._version();
-        s.dtype = t.scalar_type();
+    return v && THPVariable_Check(v) ? &THPVariable_Unpack(v) : nullptr;
+}
+Held look(const at::Tensor* t) {
+    Held h;
+    if (t) {
+        h.impl = t->unsafeGetTensorImpl();
+        if (t->has_storage()) {
+            h.storage = t->storage().unsafeGetStorageImpl();
+            h.data = t->const_data_ptr();
+        }
+        h.version = t->is_inference() ? 0 : (int64_t)t->_version();
+        h.dtype = t->scalar_type();
     }
+    return h;
 }
 PyObject* watch(PyObject*, PyObject* slots) {
     return guarded([&]() -> PyObject* {
@@ -325,11 +340,15 @@ PyObject* watch(PyObject*, PyObject* slots) {
                 Py_DECREF(seq);
                 throw std::domain_error("slots must be a sequence of (dict, name)");
             }
-            Slot s;
+            w->slots.emplace_back();
+            Slot& s = w->slots.back();
             s.dict = Py_NewRef(PyTuple_GET_ITEM(item, 0));
             s.name = Py_NewRef(PyTuple_GET_ITEM(item, 1));
-            look(s.dict, s.name, s);
-            w->slots.push_back(s);
+            if (const at::Tensor* t = in_slot(s.dict, s.name)) {
+                s.held = look(t);
+                s.impl = decltype(s.impl)(t->getIntrusivePtr());
+                if (t->has_storage()) s.storage = t->storage().getWeakStorageImpl();
+            }
         }
         Py_DECREF(seq);
         return PyCapsule_New(w.release(), "mmf.watch", [](PyObject* c) { delete static_cast<Watch*>(PyCapsule_GetPointer(c, "mmf.watch")); });
@@ -340,9 +359,7 @@ PyObject* unchanged(PyObject*, PyObject* cap) {
         auto* w = static_cast<Watch*>(PyCapsule_GetPointer(cap, "mmf.watch"));
         if (!w) return nullptr;
         for (const Slot& s : w->slots) {
-            Slot now;
-            look(s.dict, s.name, now);
-            if (now.impl != s.impl || now.data != s.data || now.version != s.version || now.dtype != s.dtype) Py_RETURN_FALSE;
+            if (!(look(in_slot(s.dict, s.name)) == s.held)) Py_RETURN_FALSE;
         }
         Py_RETURN_TRUE;
     });

@@ -42,3 +42,34 @@ def test_failed_native_call_clears_the_workspaces(monkeypatch):
     with pytest.raises(_lib.MMFreeError):
         runner.forward(None, None, [], False)
     assert len(cleared) == 2
+
+
+@pytest.mark.parametrize("n", [16, 300, 5000])
+def test_replaced_parameter_is_noticed_where_memory_is_reused(n):
+    """A parameter that is dropped and replaced changes the watch even where the allocator hands out the same addresses again, by
+    assignment of the parameter and of its .data; what is not touched does not."""
+    native = _lib.native()
+    for _ in range(200):
+        slots = {"w": torch.nn.Parameter(torch.zeros(n))}
+        watch = native.watch([(slots, "w")])
+        assert native.unchanged(watch)
+        del slots["w"]
+        slots["w"] = torch.nn.Parameter(torch.ones(n))
+        assert not native.unchanged(watch)
+        watch = native.watch([(slots, "w")])
+        slots["w"].data = torch.empty(0)
+        slots["w"].data = torch.full((n,), 2.0)
+        assert not native.unchanged(watch)
+        watch = native.watch([(slots, "w"), (slots, "absent")])
+        assert native.unchanged(watch)
+        with torch.no_grad():
+            slots["w"].add_(1)
+        assert not native.unchanged(watch)
+
+
+def test_watch_does_not_keep_a_dropped_parameter():
+    import weakref
+    slots = {"w": torch.nn.Parameter(torch.zeros(8))}
+    watch = _lib.native().watch([(slots, "w")])
+    gone = weakref.ref(slots.pop("w"))
+    assert gone() is None and not _lib.native().unchanged(watch)
