@@ -45,6 +45,7 @@ class BitLinear(nn.Linear):
         self._packed_from = None    # (parameter object, its _version, its dtype, packed by an explicit call) at pack time
         self._norm_w32: Optional[torch.Tensor] = None
         self._norm_version = None
+        self._norm_seen: Optional[torch.Tensor] = None   # alias of the norm weight that _norm_w32 was made from
 
     # -- offline packing -------------------------------------------------------------------------
     def _pack(self, explicit: bool) -> kernels.PackedWeight:
@@ -88,7 +89,8 @@ class BitLinear(nn.Linear):
         w = self.norm.weight
         key = (w._version, w.data_ptr())
         if self._norm_w32 is None or self._norm_version != key:
-            self._norm_w32 = w.detach().float().contiguous()
+            self._norm_seen = w.detach()      # keeps the memory, so that no other weight can come to lie at this address
+            self._norm_w32 = self._norm_seen.float().contiguous()
             self._norm_version = key
         return self._norm_w32
 

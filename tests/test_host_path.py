@@ -73,3 +73,16 @@ def test_watch_does_not_keep_a_dropped_parameter():
     watch = _lib.native().watch([(slots, "w")])
     gone = weakref.ref(slots.pop("w"))
     assert gone() is None and not _lib.native().unchanged(watch)
+
+
+def test_replaced_norm_weight_is_noticed_where_memory_is_reused():
+    from matmulfreellm_b200.ops.fusedbitnet import BitLinear
+    lin = BitLinear(64, 128).bfloat16()
+    for i in range(200):
+        lin.norm.weight = None
+        lin.norm.weight = torch.nn.Parameter(torch.full((64,), float(i % 7), dtype=torch.bfloat16))
+        assert torch.equal(lin.norm_weight_f32(), torch.full((64,), float(i % 7)))
+    with torch.no_grad():
+        lin.norm.weight.add_(1)
+    assert torch.equal(lin.norm_weight_f32(), lin.norm.weight.float())
+    assert lin.norm_weight_f32() is lin.norm_weight_f32()
