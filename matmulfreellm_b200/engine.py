@@ -30,14 +30,15 @@ class GreedyDecoder:
         self.cache = model.model.init_cache(batch_size)
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self._graph_logits: Optional[torch.Tensor] = None     # [B, V] buffer that a replay of self.graph writes
+        self._graph_reads: list = []
         self.kernels_per_step = 0
         self.last_logits: Optional[torch.Tensor] = None
         self._use_graph = use_graph
         # prompt passes of a repeated length are replayed from a graph as well: an eager pass is about 200 launches
         # through Python (about 19 us of host time each), which is more than the GPU needs for a short prompt
         self._prompt_seen: dict = {}       # prompt length -> times seen
-        self._prompt_graphs: dict = {}     # prompt length -> (graph, static ids and logits buffers), at most PROMPT_GRAPHS entries
-        self._host_graphs: dict = {}       # (ids_host ptr, out_host ptr) -> (graph with the two copies, its logits buffer, the host buffers)
+        self._prompt_graphs: dict = {}     # prompt length -> (graph, static ids and logits buffers, what it reads), at most PROMPT_GRAPHS entries
+        self._host_graphs: dict = {}       # (ids_host ptr, out_host ptr) -> (graph with the two copies, its logits buffer, what it reads, the host buffers)
 
     def _step_eager(self) -> torch.Tensor:
         """One step; returns its logits [B, V].  Inside a captured graph they are a fixed buffer that every replay of that
@@ -48,8 +49,19 @@ class GreedyDecoder:
         kernels.argmax_rows(logits, out=self.next)
         return logits
 
+    def _read_by_graphs(self) -> list:
+        """What a captured pass reads through raw addresses and the model may drop later (weights replaced or repacked): kept with
+        the graph, whose replays then still compute what was captured instead of reading freed memory."""
+        model = self.model
+        runner = getattr(model, "_fused_runner", None)
+        if runner is not None and model.fuse:
+            return [runner]
+        layers = bitlinear_modules(model)
+        latent = {id(m.weight) for m in layers}
+        return [(m._packed, m._norm_w32, m._norm_seen) for m in layers] + [p.detach() for p in model.parameters() if id(p) not in latent]
+
     def _capture(self, ids_host: Optional[torch.Tensor] = None, out_host: Optional[torch.Tensor] = None):
-        """Capture one decode step; returns (graph, its logits buffer).  With pinned host buffers the copy of the input ids
+        """Capture one decode step; returns (graph, its logits buffer, what it reads).  With pinned host buffers the copy of the input ids
         to the device and of the new tokens back are nodes of the same graph."""
         saved = [tuple(s.clone() for s in layer) for layer in self.cache.states]
         saved_ids = self.ids.clone()
@@ -74,7 +86,7 @@ class GreedyDecoder:
             for dst, src in zip(layer, keep):
                 dst.copy_(src)
         self.ids.copy_(saved_ids)
-        return graph, logits
+        return graph, logits, self._read_by_graphs()
 
     PROMPT_GRAPH_MAX_TOKENS = 8192   # larger prompts are bound by the GPU, and their graphs would pin gigabytes
     PROMPT_GRAPHS = 4
@@ -99,7 +111,7 @@ class GreedyDecoder:
             logits = self._prefill_eager(ids)
         if len(self._prompt_graphs) >= self.PROMPT_GRAPHS:
             self._prompt_graphs.pop(next(iter(self._prompt_graphs)))
-        self._prompt_graphs[T] = (graph, ids, logits)
+        self._prompt_graphs[T] = (graph, ids, logits, self._read_by_graphs())
         return self._prompt_graphs[T]
 
     @torch.no_grad()
@@ -118,7 +130,7 @@ class GreedyDecoder:
             if entry is None and seen >= 1:
                 entry = self._capture_prompt(T)
             if entry is not None:
-                graph, ids, self.last_logits = entry
+                graph, ids, self.last_logits, _ = entry
                 ids.copy_(prompt_ids)
                 graph.replay()
                 return self.next
@@ -144,7 +156,7 @@ class GreedyDecoder:
             self.kernels_per_step = _lib.launch_count - before
         else:
             if self.graph is None:
-                self.graph, self._graph_logits = self._capture()
+                self.graph, self._graph_logits, self._graph_reads = self._capture()
             self.graph.replay()
             self.last_logits = self._graph_logits
         return self.next

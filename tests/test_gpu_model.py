@@ -580,6 +580,46 @@ def test_last_logits_follow_the_graph_that_ran(mm):
     assert torch.equal(dec.last_logits, out.logits[:, -1])
 
 
+@pytest.mark.parametrize("fuse", [True, False])
+def test_captured_graphs_keep_the_weights_they_read(mm, fuse):
+    """Packed weights that were replaced stay alive while a decoder holds a graph that reads them (only their lifetime is looked
+    at), and no longer."""
+    import gc
+    import weakref
+    from matmulfreellm_b200.engine import GreedyDecoder
+    cfg = tiny_cfg()
+    model = build_gpu_model(O.random_weights(cfg, seed=4), cfg, torch.bfloat16)
+    model.fuse = fuse
+    ids = torch.randint(0, cfg.vocab_size, (2, 6), device="cuda")
+    out_host = torch.zeros(2, dtype=torch.int64).pin_memory()
+
+    def step(dec):
+        dec.step()
+
+    def host(dec):
+        dec.step_host(torch.zeros(2, 1, dtype=torch.int64).pin_memory(), out_host)
+
+    def prompt(dec):
+        dec.prefill(ids)
+        dec.prefill(ids)
+
+    with torch.no_grad():
+        for capture in (step, host, prompt):
+            dec = GreedyDecoder(model, 2)
+            capture(dec)
+            torch.cuda.synchronize()
+            read = [weakref.ref(model._fused_runner)] if fuse else \
+                [weakref.ref(m._packed) for m in model.modules() if getattr(m, "_packed", None) is not None]
+            for p in model.parameters():
+                p.mul_(0.5)
+            model(input_ids=ids)                      # repacks
+            gc.collect()
+            assert all(r() is not None for r in read), capture
+            del dec
+            gc.collect()
+            assert all(r() is None for r in read), capture
+
+
 def test_native_calls_check_the_device(mm, monkeypatch):
     """On a GPU that the library was not built for, the calls that go through the native host path raise the device check's
     error, as the others do (the check is made to fail here: it runs once per device)."""
