@@ -208,13 +208,13 @@ PyObject* bitlinear(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (packed.numel() != (N + MMF_TILE_ROWS - 1) / MMF_TILE_ROWS * MMF_TILE_ROWS * K / 4)
             throw std::invalid_argument("x does not have the layer's in_features columns");
         const at::Tensor x2 = rows_of(x);
-        const int64_t M = x2.size(0);
+        const int64_t M = x2.size(0), ld = M == 1 ? K : x2.stride(0);      // the pitch of a single row means nothing
         std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
         shape.back() = N;
         at::Tensor out = at::empty(shape, x.options());
         // one or two rows: one kernel, no scratch
         if (M > 0 && M <= MMF_DECODE_LINEAR_FUSED_MAX_M && dt != MMF_F32 && K <= 8192 && N <= FUSED_MAX_N && on16(x2.data_ptr()) &&
-            x2.stride(0) % 8 == 0 && on16(ptr(nw)) && on16(packed.data_ptr())) {
+            ld % 8 == 0 && on16(ptr(nw)) && on16(packed.data_ptr())) {
             mmf_decode_linear_args a = {};
             a.prologue = MMF_PRO_QUANT;
             a.epilogue = MMF_EPI_STORE;
@@ -223,7 +223,7 @@ PyObject* bitlinear(PyObject*, PyObject* const* args, Py_ssize_t n) {
             a.packed = packed.data_ptr();
             a.w_scale = scale.data_ptr<float>();
             a.x = x2.data_ptr();
-            a.ld_x = x2.stride(0);
+            a.ld_x = ld;
             a.bl_norm_w[0] = (const float*)ptr(nw);
             a.eps_bl = (float)eps;
             a.out = out.data_ptr();
@@ -237,7 +237,7 @@ PyObject* bitlinear(PyObject*, PyObject* const* args, Py_ssize_t n) {
             const int64_t q = s.take(M * K), dq = s.take(M * 4), rs = s.take(M * 4);
             const at::Tensor mem = at::empty({s.used}, x.options().dtype(at::kByte));
             uint8_t* b = mem.data_ptr<uint8_t>();
-            MMF_CALL(mmf_act_quant, x2.data_ptr(), dt, x2.stride(0), (const float*)ptr(nw), 1, (float)eps, (int8_t*)(b + q), (float*)(b + dq),
+            MMF_CALL(mmf_act_quant, x2.data_ptr(), dt, ld, (const float*)ptr(nw), 1, (float)eps, (int8_t*)(b + q), (float*)(b + dq),
                      (int32_t*)(b + rs), M, K, st);
             MMF_CALL(mmf_bitlinear, (const int8_t*)(b + q), (const float*)(b + dq), (const int32_t*)(b + rs), packed.data_ptr(),
                      scale.data_ptr<float>(), 1, out.data_ptr(), dt, N, nullptr, M, N, K, ws.p, ws.bytes, MMF_KERNEL_AUTO, st);

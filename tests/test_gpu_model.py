@@ -97,6 +97,28 @@ def test_linear_quant_fn_takes_any_strides(mm, M):
         assert torch.equal(layer_norm_linear_quant_fn(x, nw, None, w, None, is_rms_norm=True), want)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_bitlinear_row_pitches(mm, dtype):
+    """A BitLinear takes a single row whatever its pitch says (a slice of a wider tensor, an expanded row); rows at a pitch that is
+    not a multiple of 16 bytes, or below their length, are refused, and so is a row that does not start on 16 bytes."""
+    from matmulfreellm_b200._lib import MMFreeError
+    from mmfreelm.ops.fusedbitnet import FusedBitLinear
+    K, N = 256, 130
+    layer = FusedBitLinear(K, N).cuda()
+    layer.pack_weights()
+    layer = layer.to(dtype)
+    wide = torch.randn(4, K + 9, generator=torch.Generator().manual_seed(1)).cuda().to(dtype)
+    want = layer(wide[:, :K].contiguous())
+    assert torch.equal(layer(wide[:1, :K]), want[:1]) and torch.equal(layer(wide[0, :K].expand(1, K)), want[:1])
+    assert torch.equal(layer(wide[:1, None, :K]), want[:1, None])
+    padded = torch.nn.functional.pad(wide, (0, 7))
+    for M in (1, 2, 3, 4):
+        assert torch.equal(layer(padded[:M, :K]), want[:M])
+        for bad in (wide[:M, 1:K + 1], *([wide[:M, :K], wide[0, :K].expand(M, K)] if M > 1 else [])):
+            with pytest.raises(MMFreeError):
+                layer(bad)
+
+
 def test_hgrn_ops_reference_selfcheck_shapes(mm):
     """The reference's own self-check (recurrent_fuse.py:188-217): B,H,T,D = 8,4,512,128, bf16, seed 42,
     g = sigmoid(randn), x = (1-g)*randn, random h0 — fused op against the naive loop."""
