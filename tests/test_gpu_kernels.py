@@ -836,3 +836,110 @@ def test_time_sliced_scan_stitches_to_whole_scan(K, gate_is_log):
     o = torch.cat(outs, dim=1)
     assert (o.float() - o_ref.float()).abs().max().item() <= 1e-2 * o_ref.float().abs().max().item()
     assert (last - h_ref).abs().max().item() <= 1e-4 * h_ref.abs().max().item()
+
+
+# ----------------------------------------------------------------------------------------------------------
+# the decode step's BitLinear, called through the C ABI
+# ----------------------------------------------------------------------------------------------------------
+class _Guarded:
+    """Device buffers with a margin on both sides that nothing may write."""
+    MARGIN, FILL = 128, 0x5A
+
+    def __init__(self):
+        self.whole = []
+
+    def __call__(self, *shape, dtype):
+        n = int(np.prod(shape)) * torch.empty(0, dtype=dtype).element_size()
+        buf = torch.full((n + 2 * self.MARGIN,), self.FILL, dtype=torch.uint8, device="cuda")
+        self.whole.append((buf, n))
+        return buf[self.MARGIN:self.MARGIN + n].view(dtype).view(*shape)
+
+    def untouched(self):
+        return all(bool((b[:self.MARGIN] == self.FILL).all()) and bool((b[self.MARGIN + n:] == self.FILL).all()) for b, n in self.whole)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M", [1, 2, 3, 8, 9, 16])
+@pytest.mark.parametrize("D,N,inner", [(128, 1, 4), (320, 37, 68), (1088, 515, 130), (2176, 128, 2050)])
+def test_decode_linear_equals_the_separate_kernels(K, dtype, M, D, N, inner):
+    """mmf_decode_linear with and without a codes workspace, every prologue and epilogue, against the row kernels and contractions
+    it stands for, bit for bit; nothing is written outside its outputs, its workspace and their row gaps."""
+    import ctypes
+    from matmulfreellm_b200 import _lib as L
+    g = torch.Generator().manual_seed(M * 1000 + D)
+    rand = lambda *shape: torch.randn(*shape, generator=g)                                       # noqa: E731
+    nw = lambda n: (1 + 0.1 * rand(n)).cuda()                                                    # noqa: E731
+    x, res, table = rand(M, D).to(dtype).cuda(), rand(M, D).to(dtype).cuda(), rand(11, D).to(dtype).cuda()
+    ids = torch.randint(0, 11, (M,), generator=g).cuda()
+    norm_w, eps_norm, eps_bl = nw(D), 1e-5, 1e-6
+    single = {n: K.pack_weight((0.05 * rand(n, D)).cuda()) for n in {N, 2 * inner}}
+    down = nw(inner) if inner % 16 == 0 else None
+
+    for codes in ([False, True] if M <= 2 else [True]):
+        guard = _Guarded()
+
+        def run(pro, epi, pw, bl, **fields):
+            G, c = (3, len(bl)) if epi == L.EPI_GATES else (1, 1)
+            assert c == G
+            a = L.DecodeLinearArgs(prologue=pro, epilogue=epi, dtype=L.BF16 if dtype == torch.bfloat16 else L.F16, M=M, N=pw.N, K=D,
+                                   packed=pw.packed.data_ptr(), w_scale=pw.scale.data_ptr(), eps_norm=eps_norm, eps_bl=eps_bl,
+                                   bl_norm_w=(ctypes.c_void_p * 3)(*[w.data_ptr() for w in bl]), ld_x=D, ld_residual=D)
+            for k, v in fields.items():
+                setattr(a, k, v.data_ptr() if isinstance(v, torch.Tensor) else v)
+            if codes:
+                a.codes = guard(G, (D + 255) // 256 * 256 * (8 if M <= 8 else 16), dtype=torch.int8).data_ptr()
+                a.dq, a.rowsum = guard(G, M, dtype=torch.float32).data_ptr(), guard(G, M, dtype=torch.int32).data_ptr()
+            L.call("mmf_decode_linear", ctypes.addressof(a), torch.cuda.current_stream().cuda_stream)
+
+        def contraction(q, dq, rs, pw):
+            return K.bitlinear(q, dq, rs, pw, dtype, kernel=K.KERNEL_MMA)
+
+        bl = nw(D)
+        # STORE after each prologue; the gap between rows of `out` stays as it was
+        q, dq, rs = K.act_quant(x, bl, eps_bl)
+        pq, pdq, prs, psum, _ = K.prenorm_quant(x, res, norm_w, eps_norm, [bl], eps_bl, True, want_residual_out=True)
+        uq, udq, urs, usum, _ = K.prenorm_quant(x, res, norm_w, eps_norm, [bl], eps_bl, False, want_residual_out=True)
+        eq, edq, ers, esum, _ = K.prenorm_quant(table[ids].contiguous(), None, norm_w, eps_norm, [bl], eps_bl, False)
+        forms = [(L.PRO_QUANT, dict(x=x), (q, dq, rs), None),
+                 (L.PRO_PRENORM, dict(x=x, residual=res, norm_w=norm_w, round_sum_first=1), (pq, pdq, prs), psum),
+                 (L.PRO_PRENORM, dict(x=x, residual=res, norm_w=norm_w, round_sum_first=0), (uq, udq, urs), usum),
+                 (L.PRO_PRENORM, dict(x=table, row_ids=ids, x_rows=11, norm_w=norm_w), (eq, edq, ers), table[ids]),
+                 (L.PRO_GATENORM, dict(x=x, residual=res, norm_w=norm_w), K.gatenorm_quant(x, res, norm_w, eps_norm, bl, eps_bl), None)]
+        for pro, fields, quantised, row in forms:
+            out = guard(M, N + 3, dtype=dtype)
+            before = out.clone()
+            extra = {} if row is None else {"residual_out": guard(M, D, dtype=dtype)}
+            kept = extra.get("residual_out")
+            run(pro, L.EPI_STORE, single[N], [bl], out=out, ld_out=N + 3, **fields, **extra)
+            assert torch.equal(out[:, :N], contraction(*quantised, single[N])), (pro, codes)
+            assert torch.equal(out[:, N:].view(torch.int16), before[:, N:].view(torch.int16))
+            assert row is None or torch.equal(kept, row), (pro, codes)
+        # SWIGLU
+        out = guard(M, inner + inner % 2 + 2, dtype=dtype)
+        run(L.PRO_PRENORM, L.EPI_SWIGLU, single[2 * inner], [bl], x=x, residual=res, norm_w=norm_w, out=out, ld_out=out.shape[1])
+        gu = contraction(uq, udq, urs, single[2 * inner])
+        want = K.swiglu(gu[:, :inner], gu[:, inner:])
+        # (the two sigmoids share a reciprocal in one and not in the other: results one rounding apart, 2^-8 of the value in bf16)
+        assert (out[:, :inner].float() - want.float()).abs().max() <= 2.0 ** -7 * want.float().abs().max()
+        if down is not None:                       # the fused row kernel's own rounding, through its codes
+            z = [K.act_quant(out[:, :inner].contiguous(), down, eps_bl), K.swiglu_quant(gu, down, eps_bl)]
+            assert all(torch.equal(a, b) for a, b in zip(*z))
+        # GATES
+        if D % 128 == 0:
+            three, bls = K.stack_packed([K.pack_weight((0.05 * rand(D, D)).cuda()) for _ in range(3)]), [nw(D) for _ in range(3)]
+            lb, mask = torch.rand(D, generator=g).to(dtype).cuda(), (torch.arange(M) % 3 != 1).to(torch.uint8).cuda()
+            h0 = rand(M, D).cuda()
+            q3, dq3, rs3, _, _ = K.prenorm_quant(x, None, norm_w, eps_norm, bls, eps_bl, False)
+            ifg = contraction(q3, dq3, rs3, three)
+            for lower, padding in ((lb, None), (None, mask), (lb, mask)):
+                state, o, go = guard(M, D, dtype=torch.float32), guard(M, D, dtype=dtype), guard(M, D, dtype=dtype)
+                state.copy_(h0)
+                run(L.PRO_PRENORM, L.EPI_GATES, three, bls, x=x, norm_w=norm_w, out=o, g_out=go, state=state,
+                    **({} if lower is None else {"lower_bound": lower}), **({} if padding is None else {"mask": padding}))
+                ref = h0.clone()
+                codes_ref = K.decode_mix(ifg, lower, ref, norm_w, eps_norm, bl, eps_bl, mask=padding)
+                assert torch.equal(state, ref) and torch.equal(go, ifg[:, 2 * D:])
+                got = K.gatenorm_quant(go, o, norm_w, eps_norm, bl, eps_bl)
+                assert all(torch.equal(a, b) for a, b in zip(got, codes_ref))
+        torch.cuda.synchronize()
+        assert guard.untouched()
