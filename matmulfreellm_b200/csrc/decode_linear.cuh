@@ -103,35 +103,15 @@ template <typename T> struct DlRowArgs {
     }
 };
 
-// VW packed pairs (2 * VW values) per vector
-template <int VW> struct DlVec { uint32_t v[VW]; };
-template <int VW, typename T> __device__ __forceinline__ DlVec<VW> dl_load(const T* p) {
-    DlVec<VW> r;
-    if constexpr (VW == 4) {
-        const uint4 t = *reinterpret_cast<const uint4*>(p);
-        r.v[0] = t.x; r.v[1] = t.y; r.v[2] = t.z; r.v[3] = t.w;
-    } else {
-        const uint2 t = *reinterpret_cast<const uint2*>(p);
-        r.v[0] = t.x; r.v[1] = t.y;
-    }
-    return r;
-}
-template <int VW, typename T> __device__ __forceinline__ void dl_store(T* p, const uint32_t (&o)[VW]) {
-    if constexpr (VW == 4) *reinterpret_cast<uint4*>(p) = make_uint4(o[0], o[1], o[2], o[3]);
-    else *reinterpret_cast<uint2*>(p) = make_uint2(o[0], o[1]);
-}
-template <int VW> __device__ __forceinline__ void dl_weights(const float* p, float2 (&w)[VW]) {
-#pragma unroll
-    for (int i = 0; i < VW; i += 2) {
-        const float4 t = *reinterpret_cast<const float4*>(p + 2 * i);
-        w[i] = make_float2(t.x, t.y);
-        w[i + 1] = make_float2(t.z, t.w);
-    }
+// eight values of a row, as packed pairs
+struct DlVec { uint32_t v[4]; };
+template <typename T> __device__ __forceinline__ DlVec dl_load(const T* p) {
+    const uint4 t = *reinterpret_cast<const uint4*>(p);
+    return DlVec{{t.x, t.y, t.z, t.w}};
 }
 
-// vector `it` of a thread starts at column c; NVT vectors of 2 * VW values cover a row of D values
-#define DL_FOREACH(it, c) \
-    _Pragma("unroll") for (int it = 0, c = rt * 2 * VW; it < NVT; ++it, c += RT * 2 * VW) if (c < D)
+// vector `it` of a thread starts at column c; NVT vectors of eight values cover a row of D values
+#define DL_FOREACH(it, c) _Pragma("unroll") for (int it = 0, c = rt * 8; it < NVT; ++it, c += RT * 8) if (c < D)
 
 // Row prologue of row m, RT = TH / MR threads: codes of G projections in the MMA's operand order, absmax and (per-warp) code
 // sums beside them.  Columns c .. c + 15 of a 256-column group are the 16-byte piece ((c / 16) % 4) * word + (c / 64) % 4 of
@@ -139,7 +119,7 @@ template <int VW> __device__ __forceinline__ void dl_weights(const float* p, flo
 template <typename T, int PRO, int G, int TH, int MR, int NVT>
 __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, const DlRowArgs<T>& ra, int m, int D, int KG, const float* snw, uint8_t* codes,
                                             int word, int step, DlScratch<TH / MR>& red, float (&s_amax)[G], double inv_d) {
-    constexpr int RT = TH / MR, VW = 4;
+    constexpr int RT = TH / MR;
     const int rt = threadIdx.x % RT, lane = threadIdx.x & 31, rw = rt >> 5;
     const T* x = ra.x;
     if (PRO == MMF_PRO_PRENORM && a.row_ids) {
@@ -147,19 +127,19 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
         x += (row < 0 ? 0 : row >= a.x_rows ? a.x_rows - 1 : row) * a.ld_x;    // clamp instead of faulting on a bad id
     }
     const T* r = PRO != MMF_PRO_QUANT ? ra.r : nullptr;
-    DlVec<VW> u[NVT], v[NVT];
+    DlVec u[NVT], v[NVT];
     double s0 = 0.0, s1 = 0.0;
-    DL_FOREACH(it, c) u[it] = dl_load<VW>(x + c);
+    DL_FOREACH(it, c) u[it] = dl_load(x + c);
     if (r) {
-        DL_FOREACH(it, c) v[it] = dl_load<VW>(r + c);
+        DL_FOREACH(it, c) v[it] = dl_load(r + c);
     }
     if constexpr (PRO == MMF_PRO_PRENORM) {
         T* ro = ra.res_out;
         const bool plain = !r || a.round_sum_first;        // what is normalised is a row of T values
         DL_FOREACH(it, c) {
-            uint32_t o[VW];
+            uint32_t o[4];
 #pragma unroll
-            for (int i = 0; i < VW; ++i) {
+            for (int i = 0; i < 4; ++i) {
                 if (plain) {
                     if (r) u[it].v[i] = narrow<T>(__fadd2_rn(widen<T>(u[it].v[i]), widen<T>(v[it].v[i])));
                     o[i] = u[it].v[i];
@@ -171,15 +151,15 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
                     o[i] = narrow<T>(t);
                 }
             }
-            if (ro) dl_store<VW>(ro + c, o);
+            if (ro) *reinterpret_cast<uint4*>(ro + c) = make_uint4(o[0], o[1], o[2], o[3]);
         }
         const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d0), D, inv_d, ra.eps_norm);
         s0 = s1 = 0.0;
         DL_FOREACH(it, c) {
-            float2 w[VW];
-            dl_weights<VW>(snw + c, w);
+            float2 w[4];
+            lds8(snw + c, w);
 #pragma unroll
-            for (int i = 0; i < VW; ++i) {
+            for (int i = 0; i < 4; ++i) {
                 float2 t = widen<T>(u[it].v[i]);
                 if (!plain) t = __fadd2_rn(t, widen<T>(v[it].v[i]));
                 u[it].v[i] = narrow<T>(__fmul2_rn(mul2(t, rstd), w[i]));
@@ -190,15 +170,15 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
     } else if constexpr (PRO == MMF_PRO_GATENORM) {
         DL_FOREACH(it, c) {
 #pragma unroll
-            for (int i = 0; i < VW; ++i) sumsq_pair<T>(u[it].v[i], s0, s1);
+            for (int i = 0; i < 4; ++i) sumsq_pair<T>(u[it].v[i], s0, s1);
         }
         const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d0), D, inv_d, ra.eps_norm);
         s0 = s1 = 0.0;
         DL_FOREACH(it, c) {
-            float2 w[VW];
-            dl_weights<VW>(snw + c, w);
+            float2 w[4];
+            lds8(snw + c, w);
 #pragma unroll
-            for (int i = 0; i < VW; ++i) {
+            for (int i = 0; i < 4; ++i) {
                 const float2 o = widen<T>(v[it].v[i]);
                 const float2 y = __fmul2_rn(mul2(widen<T>(u[it].v[i]), rstd), w[i]);
                 u[it].v[i] = narrow<T>(__fmul2_rn(__fmul2_rn(y, o), sigmoid2(o)));
@@ -209,7 +189,7 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
     } else {
         DL_FOREACH(it, c) {
 #pragma unroll
-            for (int i = 0; i < VW; ++i) sumsq_pair<T>(u[it].v[i], s0, s1);
+            for (int i = 0; i < 4; ++i) sumsq_pair<T>(u[it].v[i], s0, s1);
         }
     }
     // BitLinear prologue: y = (v * rstd) * w, absmax -> scale -> int8 codes
@@ -220,10 +200,10 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
     DL_FOREACH(it, c) {
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-            float2 w[VW];
-            dl_weights<VW>(snw + g * D + c, w);
+            float2 w[4];
+            lds8(snw + g * D + c, w);
 #pragma unroll
-            for (int i = 0; i < VW; ++i) {
+            for (int i = 0; i < 4; ++i) {
                 const float2 y = __fmul2_rn(mul2(widen<T>(u[it].v[i]), rstd), w[i]);
                 am[g] = fmaxf(am[g], fmaxf(fabsf(y.x), fabsf(y.y)));
             }
@@ -250,18 +230,17 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
         uint8_t* dst = codes + ((c >> 8) * (4 * step) + ((c >> 4) & 3) * word + ((c >> 6) & 3)) * 16 + (c & 15);
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-            float2 w[VW];
-            dl_weights<VW>(snw + g * D + c, w);
-            uint32_t word[VW / 2];
+            float2 w[4];
+            lds8(snw + g * D + c, w);
+            uint32_t word[2];
 #pragma unroll
-            for (int i = 0; i < VW / 2; ++i) {
+            for (int i = 0; i < 2; ++i) {
                 word[i] = codes4(__fmul2_rn(mul2(widen<T>(u[it].v[2 * i]), rstd), w[2 * i]),
                                  __fmul2_rn(mul2(widen<T>(u[it].v[2 * i + 1]), rstd), w[2 * i + 1]), s[g]);
                 sum[g] = __dp4a((int)word[i], 0x01010101, sum[g]);
             }
             uint8_t* d = dst + g * KG * (step * 64);
-            if constexpr (VW == 4) *reinterpret_cast<uint2*>(d) = make_uint2(word[0], word[VW / 2 - 1]);
-            else *reinterpret_cast<uint32_t*>(d) = word[0];
+            *reinterpret_cast<uint2*>(d) = make_uint2(word[0], word[1]);
         }
     }
 #pragma unroll

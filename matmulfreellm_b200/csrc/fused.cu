@@ -19,6 +19,7 @@
 // shared memory BEFORE the grid-dependency wait (they do not depend on the preceding kernel), and
 // every block reduction costs a single __syncthreads.
 #include "common.cuh"
+#include "packed.cuh"
 #include "rowquant.cuh"
 
 namespace {
@@ -147,13 +148,6 @@ __device__ __forceinline__ void lds_weights(const float* p, float (&w)[V]) {
         w[i] = t.x; w[i + 1] = t.y; w[i + 2] = t.z; w[i + 3] = t.w;
     }
 }
-
-// asynchronous 16-byte copy global -> shared memory (no register staging) and its group bookkeeping
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // iterate over the 16-byte vectors of a row held as v[P] (P: the enclosing template parameter): vector `it` of this thread starts at column c
 // (RT, the threads per row, is a template parameter or constant of the enclosing function)

@@ -4,6 +4,7 @@
 
 namespace {
 
+// asynchronous 16-byte copy global -> shared memory (no register staging) and its group bookkeeping
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
 }
