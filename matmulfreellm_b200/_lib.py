@@ -185,7 +185,7 @@ def native():
         spec = importlib.util.spec_from_loader(name, importlib.machinery.ExtensionFileLoader(name, str(NATIVE_PATH)))
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
-        mod.set_hooks(MMFreeError, kernels.stream_workspace)
+        mod.set_hooks(MMFreeError, kernels.stream_workspace, require_device)
         mod.use_library(str(EXPERIMENTS_LIB_PATH if _lib is experiments_library._handle else LIB_PATH))
         _native = mod
     return _native

@@ -7,7 +7,8 @@
 // experiments build of the same library (use_library).
 //
 //   use_library(path)                    resolve the C ABI from this shared object
-//   set_hooks(error_class, workspace)    exception class for negative status codes, workspace(device_index) -> tensor
+//   set_hooks(error_class, workspace, require_device)     exception class for negative status codes, workspace(device_index) ->
+//                                        tensor, require_device(device_index) raises if the GPU is not one the library runs on
 //   take_launches()                      kernels launched since the last call of it
 //   bitlinear(x, norm_w, packed, scale, N, eps)       RMSNorm + int8 quantisation + contraction, [..., K] -> [..., N]
 //   hgrn_scan(x, g, h0 | None, want_state, gate_is_log, state_dtype)      -> (o, final state | None)
@@ -57,6 +58,8 @@ constexpr int64_t FUSED_MAX_N = 262144;       // partial sums of more output row
 
 PyObject* g_error_class = nullptr;
 PyObject* g_workspace_fn = nullptr;
+PyObject* g_require_device_fn = nullptr;
+uint64_t g_device_ok = 0;         // devices that require_device has accepted (guarded by the GIL)
 
 // a C-ABI call returned a negative status: carried as a C++ exception so that it can cross code that runs without the GIL
 struct MmfStatus {
@@ -70,10 +73,13 @@ struct MmfStatus {
         if (rc__ != MMF_OK) throw MmfStatus{#fn, rc__, g_api->mmf_last_error()}; \
     } while (0)
 
+struct PythonError {};            // a Python call failed and its exception is set
+
 // run `body` and turn C++ exceptions into Python ones
 template <typename F> PyObject* guarded(F&& body) {
     try {
         return body();
+    } catch (const PythonError&) {
     } catch (const MmfStatus& s) {
         PyObject* e = PyObject_CallFunction(g_error_class, "sis", s.fn, s.code, s.text.c_str());
         if (e) {
@@ -113,7 +119,7 @@ int dtype_code(const at::Tensor& t) {
 }
 void* ptr(const at::Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 
-// The C entry points launch on the current device: every tensor has to live there.
+// The C entry points launch on the current device: every tensor has to live there, and the device is checked before its first launch.
 int need_cuda(std::initializer_list<const at::Tensor*> ts) {
     int dev = -1;
     for (const at::Tensor* t : ts) {
@@ -126,6 +132,12 @@ int need_cuda(std::initializer_list<const at::Tensor*> ts) {
     if (dev >= 0 && dev != cur)
         throw std::runtime_error("tensors live on cuda:" + std::to_string(dev) + " but the current device is cuda:" + std::to_string(cur) +
                                  "; wrap the call in `with torch.cuda.device(" + std::to_string(dev) + "):`");
+    if (cur >= 64 || !(g_device_ok >> cur & 1)) {
+        PyObject* o = PyObject_CallFunction(g_require_device_fn, "i", cur);
+        if (!o) throw PythonError{};
+        Py_DECREF(o);
+        if (cur < 64) g_device_ok |= 1ull << cur;
+    }
     return cur;
 }
 
@@ -136,10 +148,7 @@ Ws workspace(int dev, void* stream) {
     for (const Ws& w : g_ws)
         if (w.dev == dev && w.stream == stream) return w;
     PyObject* o = PyObject_CallFunction(g_workspace_fn, "i", dev);
-    if (!o) {
-        PyErr_Clear();
-        throw std::runtime_error("no workspace for this stream");
-    }
+    if (!o) throw PythonError{};
     const at::Tensor t = THPVariable_Unpack(o);
     Py_DECREF(o);
     g_ws.push_back(Ws{dev, stream, t.data_ptr(), t.numel()});
@@ -184,9 +193,11 @@ PyObject* use_library(PyObject*, PyObject* path) {
 }
 
 PyObject* set_hooks(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    if (n != 2) { PyErr_SetString(PyExc_TypeError, "set_hooks(error_class, workspace)"); return nullptr; }
+    if (n != 3) { PyErr_SetString(PyExc_TypeError, "set_hooks(error_class, workspace, require_device)"); return nullptr; }
     Py_INCREF(args[0]); Py_XSETREF(g_error_class, args[0]);
     Py_INCREF(args[1]); Py_XSETREF(g_workspace_fn, args[1]);
+    Py_INCREF(args[2]); Py_XSETREF(g_require_device_fn, args[2]);
+    g_device_ok = 0;
     Py_RETURN_NONE;
 }
 

@@ -210,8 +210,6 @@ class FusedRunner:
         model = lm.model
         cfg = lm.config
         self.device = model.embeddings.weight.device
-        if self.device.type == "cuda":
-            _lib.require_device(self.device.index)
         self.h = cfg.hidden_size
         self.dtype = model.embeddings.weight.dtype
         # per-layer lower bounds of the forget gates depend on parameters only: evaluated once (in the parameter

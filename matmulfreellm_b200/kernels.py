@@ -192,7 +192,6 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
 
 def stream_workspace(index: int) -> torch.Tensor:
     """Workspace of the current stream of device `index`, for the native host path (asked for once per stream)."""
-    _lib.require_device(index)
     return _workspace(torch.device("cuda", index), 1 << 20)
 
 
@@ -269,8 +268,6 @@ def bitlinear(q: torch.Tensor, dq: torch.Tensor, rowsum: torch.Tensor, pw: Packe
 def bitlinear_forward(x: torch.Tensor, norm_weight: Optional[torch.Tensor], pw: PackedWeight, eps: float) -> torch.Tensor:
     """FusedBitLinear's forward: RMSNorm + int8 quantisation + contraction of x [..., K] -> [..., N] in x.dtype."""
     native = _lib.native()
-    if x.is_cuda:
-        _lib.require_device(x.get_device())
     try:
         out = native.bitlinear(x, norm_weight, pw.packed, pw.scale, pw.N, eps)
     except _lib.MMFreeError as e:
@@ -289,8 +286,6 @@ def hgrn_scan(x: torch.Tensor, g: torch.Tensor, initial_state: Optional[torch.Te
     if final_state_out is None:
         sdt = state_dtype or (initial_state.dtype if initial_state is not None else torch.float32)
         native = _lib.native()
-        if x.is_cuda:
-            _lib.require_device(x.get_device())
         out = native.hgrn_scan(x, g, initial_state, output_final_state, gate_is_log, sdt)
         _lib.launch_count += native.take_launches()
         return out

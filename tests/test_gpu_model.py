@@ -642,7 +642,7 @@ def test_captured_graphs_keep_the_weights_they_read(mm, fuse):
             assert all(r() is None for r in read), capture
 
 
-def test_native_calls_check_the_device(mm, monkeypatch):
+def test_native_calls_check_the_device(mm):
     """On a GPU that the library was not built for, the calls that go through the native host path raise the device check's
     error, as the others do (the check is made to fail here: it runs once per device)."""
     from matmulfreellm_b200 import _lib, kernels
@@ -653,15 +653,21 @@ def test_native_calls_check_the_device(mm, monkeypatch):
     layer = model.model.layers[0].mlp.down_proj
     x = torch.randn(2, 8, cfg.intermediate_size, device="cuda").bfloat16()
 
-    def call(name, *args):
-        raise _lib.MMFreeError(name, -5, "built for sm_100a only")
+    def refuse(index):
+        assert index == torch.cuda.current_device()
+        raise _lib.MMFreeError("mmf_check_device", -5, "built for sm_100a only")
 
-    monkeypatch.setattr(_lib, "_device_checked", set())
-    monkeypatch.setattr(_lib, "call", call)
-    object.__setattr__(model, "_fused_runner", None)
-    for fn in (lambda: layer(x), lambda: kernels.hgrn_scan(x, x, None, True, False), lambda: model(input_ids=ids)):
-        with pytest.raises(_lib.MMFreeError, match="mmf_check_device failed with MMF_ERR_ARCH"):
-            fn()
+    native = _lib.native()
+    calls = (lambda: layer(x), lambda: layer(x[0, :1]), lambda: kernels.hgrn_scan(x, x, None, True, False), lambda: model(input_ids=ids))
+    native.set_hooks(_lib.MMFreeError, kernels.stream_workspace, refuse)
+    try:
+        for fn in calls:
+            with pytest.raises(_lib.MMFreeError, match="mmf_check_device failed with MMF_ERR_ARCH"):
+                fn()
+    finally:
+        native.set_hooks(_lib.MMFreeError, kernels.stream_workspace, _lib.require_device)
+    for fn in calls:
+        fn()
 
 
 def test_launch_count_is_the_number_of_kernels(mm):
