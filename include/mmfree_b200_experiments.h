@@ -32,9 +32,12 @@ extern "C" {
 #define MMF_TUNE_ASYNC_REDUCE 10 /* split-K partial sums by st.async + the owner's mbarrier: 1 = on, 2 = off, 0 = library default */
 int mmf_tuning(int knob, int value);
 
-/* Timeline trace of mmf_prenorm_quant launches: buffer_dev is a device buffer of at least 8 + 8 * 1000 int64 ([0] = launch
- * counter, then one record of 8 global-timer stamps per launch, taken by thread 0 of CTA 0: start, weights staged, grid
- * dependency resolved, row loaded, first row sum done, second norm done, codes written, end); NULL switches it off. */
+/* Timeline trace: buffer_dev is a device buffer of at least 8 + 8 * 1000 int64 ([0] = launch counter, then one record of 8
+ * global-timer stamps per launch, taken by thread 0 of CTA 0); NULL switches it off.
+ * mmf_prenorm_quant: start, weights staged, grid dependency resolved, row loaded, first row sum done, second norm done, codes
+ * written, end.
+ * mmf_decode_linear (row kernel and contraction): start, set up, grid dependency resolved, row loaded, last norm's statistic known
+ * (these two stay 0 in a contraction with ready codes), codes complete, products done (row kernel: as before), end. */
 int mmf_row_trace(long long* buffer_dev);
 
 /* Slab-major copy of a packed weight for mmf_bitlinear_decode (experiment; no counterpart in the reference).  The tile-major layout of mmf_pack_ternary keeps a 16-row slab as K/64 pieces of 256 bytes that lie

@@ -6,12 +6,15 @@
 // A block of the model used to be eight links (row kernel, contraction, four times).  Here
 //   * the gate math and state update of the token mixer and the MLP's silu(gate) * up run in the epilogue of the contraction
 //     that produces their inputs (a CTA owns the i, f and g rows, or the gate and up rows, of the same channels), and
-//   * for one or two token rows every CTA repeats the row work that precedes the contraction - norms, statistics, int8 codes -
-//     instead of waiting for a kernel that did it: the row work is latency, and the SMs would idle meanwhile.
+//   * for one token row, and for two of at most 2048 values, every CTA repeats the row work that precedes the contraction - norms,
+//     statistics, int8 codes - instead of waiting for a kernel that did it: the row work is latency, and the SMs would idle meanwhile.
 // That leaves four links per block; up to 16 rows, where repeating the row work costs more than a link, it is a kernel of its
 // own that stores the codes in the contraction's operand order (eight links).  Step of a 24-block, 2048-wide model, before and
 // now: 1 row 595 -> 435 us, 2 rows 635 -> 500, 4 rows 735 -> 534, 8 rows 737 -> 530, 16 rows 769 -> 663; 32 blocks of 2560: 1 row
-// 980 -> 688, 8 rows 1127 -> 831.  What remains is latency: about 4.4 us per link for 1.5 us of weight traffic.
+// 980 -> 688, 8 rows 1127 -> 831.  What remains is latency.  One row, 2048 wide, a link of 4.3 us on average: 0.85 us from the end
+// of the link before it to its release, 0.8 until the row is there, 0.8 - 1.1 until the last norm's statistic is known (down_proj,
+// which has one norm: 0.35), 0.45 - 0.95 codes, 0.35 - 1.5 products, 0.2 - 0.4 epilogue.  Four rows: row kernel 1.8 us, of which 0.55 is the row's load;
+// contraction 1.2 - 2.4; 0.65 - 1.1 between two of them.
 //
 // Contraction: mma.sync m16n8k32 (8-bit, int32 accumulators) with 16 weight rows on its M axis and 8 token rows on N.
 // tcgen05 is not used: its 128-row tile needs a K split over a cluster to fill the GPU, and the exchange of the split's
@@ -27,6 +30,7 @@
 #pragma once
 #include "bitlinear.cuh"
 #include "packed.cuh"
+#include "rowquant.cuh"
 
 namespace {
 
@@ -48,6 +52,9 @@ struct DlParams {
     int kgw;                            // column groups per warp
     int pf;                             // weight items per warp fetched ahead into shared memory
     int smem_codes, smem_acc, smem_w;   // byte offsets in dynamic shared memory
+#ifdef MMF_EXPERIMENTS
+    long long* trace;
+#endif
 };
 
 // weights unsigned (2-bit fields in place, up to 2 << 6), codes signed
@@ -67,7 +74,8 @@ template <int TH, int RT> __device__ __forceinline__ double dl_row_sum(double v,
     v = warp_sum(v);
     if ((threadIdx.x & 31) == 0) slot[(threadIdx.x % RT) >> 5] = v;
     dl_row_sync<TH, RT>();
-    // every warp folds the partials by shuffles: with all lanes reading all partials the fold took 450 clocks instead of 200
+    // Every warp folds the partials by shuffles.  Alone on an SM, a whole sum takes 306 / 356 / 438 clocks with 4 / 8 / 16 warps
+    // (271 / 319 / 531 with every lane reading all partials).
     constexpr int P = RW <= 2 ? 2 : RW <= 4 ? 4 : RW <= 8 ? 8 : 16;
     const int l = threadIdx.x & (P - 1);
     double t = P == RW || l < RW ? slot[l] : 0.0;
@@ -75,8 +83,8 @@ template <int TH, int RT> __device__ __forceinline__ double dl_row_sum(double v,
     for (int o = P / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     return t;
 }
-// A kernel parameter in a register from here on: read from the constant bank where it is first used, it costs a miss of several
-// hundred clocks on the critical path.
+// A kernel parameter in a register from here on: read from the constant bank only where it is first used, it would miss there, on
+// the critical path.
 template <typename P> __device__ __forceinline__ void pin(P*& p) { asm volatile("" : "+l"(p)); }
 __device__ __forceinline__ void pin(int64_t& v) { asm volatile("" : "+l"(v)); }
 __device__ __forceinline__ void pin(float& v) { asm volatile("" : "+f"(v)); }
@@ -118,7 +126,7 @@ template <typename T> __device__ __forceinline__ DlVec dl_load(const T* p) {
 // `codes`; a group is 4 * step pieces, a projection KG groups.
 template <typename T, int PRO, int G, int TH, int MR, int NVT>
 __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, const DlRowArgs<T>& ra, int m, int D, int KG, const float* snw, uint8_t* codes,
-                                            int word, int step, DlScratch<TH / MR>& red, float (&s_amax)[G], double inv_d) {
+                                            int word, int step, DlScratch<TH / MR>& red, float (&s_amax)[G], double inv_d ROW_TRACE_PARAM) {
     constexpr int RT = TH / MR;
     const int rt = threadIdx.x % RT, lane = threadIdx.x & 31, rw = rt >> 5;
     const T* x = ra.x;
@@ -153,6 +161,7 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
             }
             if (ro) *reinterpret_cast<uint4*>(ro + c) = make_uint4(o[0], o[1], o[2], o[3]);
         }
+        ROW_TRACE_AFTER(3, s0 + s1);
         const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d0), D, inv_d, ra.eps_norm);
         s0 = s1 = 0.0;
         DL_FOREACH(it, c) {
@@ -172,6 +181,7 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
 #pragma unroll
             for (int i = 0; i < 4; ++i) sumsq_pair<T>(u[it].v[i], s0, s1);
         }
+        ROW_TRACE_AFTER(3, s0 + s1);
         const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d0), D, inv_d, ra.eps_norm);
         s0 = s1 = 0.0;
         DL_FOREACH(it, c) {
@@ -191,9 +201,11 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
 #pragma unroll
             for (int i = 0; i < 4; ++i) sumsq_pair<T>(u[it].v[i], s0, s1);
         }
+        ROW_TRACE_AFTER(3, s0 + s1);
     }
     // BitLinear prologue: y = (v * rstd) * w, absmax -> scale -> int8 codes
     const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d1), D, inv_d, ra.eps_bl);
+    ROW_TRACE_AFTER(4, (double)rstd);
     float am[G];
 #pragma unroll
     for (int g = 0; g < G; ++g) am[g] = 0.0f;
@@ -256,12 +268,16 @@ __device__ __forceinline__ float dl_out(int acc, int rs, float scale) { return _
 // contraction that follows, 8 * NB tokens side by side.
 template <typename T, int PRO, int TH, int NVT>
 __global__ void __launch_bounds__(TH)
-decode_rows_kernel(const __grid_constant__ mmf_decode_linear_args a, int KG, int NB, double inv_k) {
+decode_rows_kernel(const __grid_constant__ mmf_decode_linear_args a, int KG, int NB, double inv_k ROW_TRACE_PARAM) {
     extern __shared__ __align__(16) uint8_t smem[];
     float* snw = reinterpret_cast<float*>(smem);
     __shared__ DlScratch<TH> red;
     __shared__ float s_amax[1];
     const int m = blockIdx.x, g = blockIdx.y, D = (int)a.K, tid = threadIdx.x;
+#ifdef MMF_EXPERIMENTS
+    trace = row_trace_record(trace);
+#endif
+    ROW_TRACE(0);
     pdl_trigger();
     auto stage = [&](float* dst, const float* src) {
         if (src) for (int i = tid * 4; i < D; i += TH * 4) cp_async16(dst + i, src + i);
@@ -277,9 +293,13 @@ decode_rows_kernel(const __grid_constant__ mmf_decode_linear_args a, int KG, int
     pin(codes); pin(dq); pin(rowsum);
     cp_async_wait_all();
     __syncthreads();
+    ROW_TRACE(1);
     pdl_wait();
-    dl_prologue<T, PRO, 1, TH, 1, NVT>(a, ra, m, D, KG, snw, codes, 32, 32 * NB, red, s_amax, inv_k);
+    ROW_TRACE(2);
+    dl_prologue<T, PRO, 1, TH, 1, NVT>(a, ra, m, D, KG, snw, codes, 32, 32 * NB, red, s_amax, inv_k ROW_TRACE_ARG);
     __syncthreads();
+    ROW_TRACE(5);
+    ROW_TRACE(6);
     if (tid == 0) {
         int t = 0;
 #pragma unroll
@@ -287,6 +307,7 @@ decode_rows_kernel(const __grid_constant__ mmf_decode_linear_args a, int KG, int
         *rowsum = t;
         *dq = __fdiv_rn(s_amax[0], 127.0f);
     }
+    ROW_TRACE(7);
 }
 
 // Fused: TH threads, MR token rows (M <= MR), NVT 8-value vectors of a row per thread of the row.  Codes from
@@ -311,6 +332,10 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
     __shared__ int s_rs[G][SC];                              // code sum (weights are stored + 1)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, q = lane & 3;
+#ifdef MMF_EXPERIMENTS
+    long long* trace = row_trace_record(p.trace);
+#endif
+    ROW_TRACE(0);
     pdl_trigger();
     const int bid = blockIdx.x, u0 = bid * p.base + min(bid, p.extra), pairs = p.base + (bid < p.extra ? 1 : 0);
     const int nb = (pairs + BP - 1) / BP * G;                // blocks of this CTA; the last one may be partly empty
@@ -383,7 +408,9 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
     if (has_pre && lb) lb_pre = *reinterpret_cast<const uint32_t*>(lb + (u0 + pr_pre) * 2);
     cp_async_wait_all();
     __syncthreads();
+    ROW_TRACE(1);
     pdl_wait();
+    ROW_TRACE(2);
 
     // gates: the state this thread will advance (and whether its token is padding), on the way during the contraction
     float2 h_pre = make_float2(0.0f, 0.0f);
@@ -395,7 +422,7 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
     if constexpr (FUSED) {
         const int m = tid / RT;
         if (MR == 1 || m < M)
-            dl_prologue<T, PRO, G, TH, MR, NVT>(a, ra, m, D, KG, snw, scodes + m * 64, TL, TL, red[m], s_amax[m], p.inv_k);
+            dl_prologue<T, PRO, G, TH, MR, NVT>(a, ra, m, D, KG, snw, scodes + m * 64, TL, TL, red[m], s_amax[m], p.inv_k ROW_TRACE_ARG);
         __syncthreads();                                     // codes complete
         if (has_const) {
             int t = 0;
@@ -410,6 +437,8 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
             s_rs[cg][cm] = *rowsum;
         }
     }
+
+    ROW_TRACE(5);
 
     // the 2-bit fields stay where they are: field f of a byte counts 4^f, one accumulator per field, shifted back at the end
     if (CONST8 ? kq < KG : bq < bw) {
@@ -464,6 +493,7 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
         }
     }
     __syncthreads();
+    ROW_TRACE(6);
 
     // ---- epilogue: a thread finishes two adjacent rows (channels) of a token
     for (int i = tid; i < pairs * M; i += nthr) {
@@ -524,6 +554,7 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
             *reinterpret_cast<uint32_t*>(g_out + (int64_t)m * D + ch) = value(unit * 3 + 2, r, 2);
         }
     }
+    ROW_TRACE(7);
 }
 
 constexpr int DL_SMEM_MAX = 220 * 1024;
@@ -537,7 +568,7 @@ template <auto kernel> int dl_go(const DlParams& p, int threads, int smem, cudaS
 
 template <typename T, int PRO, int TH, int NVT> int dl_rows_go(const mmf_decode_linear_args& a, int G, int KG, int NB, cudaStream_t st) {
     MMF_CUDA(mmf_launch_pdl(decode_rows_kernel<T, PRO, TH, NVT>, dim3((unsigned)a.M, (unsigned)G), dim3(TH),
-                            (size_t)(PRO == MMF_PRO_QUANT ? 1 : 2) * a.K * 4, st, a, KG, NB, 1.0 / (double)a.K));
+                            (size_t)(PRO == MMF_PRO_QUANT ? 1 : 2) * a.K * 4, st, a, KG, NB, 1.0 / (double)a.K ROW_TRACE_BUFFER));
     MMF_LAUNCH_CHECK("decode_rows_kernel");
     return MMF_OK;
 }
@@ -558,6 +589,9 @@ template <typename T, int PRO> int dl_rows(const mmf_decode_linear_args& a, int 
 template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, cudaStream_t st) {
     DlParams p;
     p.a = a;
+#ifdef MMF_EXPERIMENTS
+    p.trace = g_row_trace;
+#endif
     p.KC = (int)(a.K / MMF_TILE_K);
     p.KG = (p.KC + 3) / 4;
     p.inv_k = 1.0 / (double)a.K;
@@ -593,6 +627,10 @@ template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, 
             const int cost = ((p.KG + kw - 1) / kw) * ((nb + bw - 1) / bw) * 64 + kw;
             if (cost < best) { best = cost; p.kw = kw; p.bw = bw; }
         }
+        // Eight warps (rows of 1025 - 2048 and 4097 - 6144 values) all split K, whatever that rule says: constants in the kernel instead
+        // of loops and divisions.  1024 < K <= 6144 to 2048 outputs 3 - 6 % faster (K = 1088 2.24 us a call against 2.31, 2048 2.43 / 2.50,
+        // 6144 3.52 / 3.59), steps of 24 blocks 371 / 375 us (1280 wide), 388 / 388 (1536), 431 / 438 (2048).  It loses where the groups of
+        // K do not divide among eight warps and the outputs are many: 11264 outputs at K = 1088 3.53 / 3.27, at 4160 8.63 / 8.33.
         if (threads == 256) { p.kw = 8; p.bw = 1; }
     } else {
         int best = 1 << 30;

@@ -237,17 +237,6 @@ __device__ __forceinline__ void bitlinear_prologue(float (&v)[P], int D, double 
     }
 }
 
-#ifdef MMF_EXPERIMENTS
-__device__ __forceinline__ long long row_now() {
-    long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-#define ROW_TRACE(slot) do { if (trace) trace[slot] = row_now(); } while (0)
-#else
-#define ROW_TRACE(slot) do { } while (0)
-#endif
-
 template <typename T, int P, int LAT, int RT = FT>
 __global__ void __launch_bounds__(FT, LAT)
 prenorm_quant_kernel(PrenormArgs a) {
@@ -259,11 +248,7 @@ prenorm_quant_kernel(PrenormArgs a) {
     constexpr int V = 16 / sizeof(T);
     const int D = a.D;
 #ifdef MMF_EXPERIMENTS
-    long long* trace = nullptr;
-    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && a.trace) {
-        const int idx = atomicAdd(reinterpret_cast<int*>(a.trace), 1);
-        if (idx < 1000) trace = a.trace + 8 + 8 * idx;
-    }
+    long long* trace = row_trace_record(a.trace);
 #endif
     ROW_TRACE(0);
     pdl_trigger();
@@ -656,7 +641,9 @@ static inline unsigned row_grid(Kern kernel, size_t smem, int64_t M, int rows_pe
 // values, two rows with 128 threads each up to 4096 values.  A thread then holds up to 32 values of its row instead of
 // 8 - 16, so the reductions of a row (two fp64 sums, the absmax, the code sum: a fifth of all instructions at 8 values
 // per thread) cost a quarter (half) per value, and a row's threads meet at a barrier of 64 (128) instead of 256.
-// Measured at 32768 rows of 2048 values: 220 -> 160 us (three projections), 150 -> 89 us (one), 150 -> 104 us (gate norm).
+// Measured at 32768 rows, one row per CTA -> side by side.  fp32, 2048 values: three projections 202 -> 151 us, gate norm 141 -> 103,
+// quantisation alone 75 -> 54, one projection with residual 145 -> 160; 2560 values: 263 -> 239, 179 -> 160, 93 -> 72, 178 -> 199.
+// swiglu: bf16 104 -> 72 (2048), 205 -> 198 (5632), 252 -> 226 (6912); fp32 104 -> 100, 269 -> 251, 341 -> 396.
 constexpr int ROW_QUARTER = 64, ROW_HALF = 128;
 // run `...` with RT bound to the threads per row of a prompt-sized call on rows of D values (D <= ROW_HALF * MAX_PER)
 #define FUSED_DISPATCH_RT(D, RT, ...)                                              \
@@ -713,7 +700,7 @@ int act_quant_regs_launch(const void* x, int dtype, int64_t ld, const float* nw,
 }
 
 #ifdef MMF_EXPERIMENTS
-static long long* g_row_trace = nullptr;
+long long* g_row_trace = nullptr;
 // experiments build only: device buffer ([0] = launch counter, records of 8 stamps from word 8 on) or NULL to switch off
 extern "C" int mmf_row_trace(long long* buffer_dev) { g_row_trace = buffer_dev; return MMF_OK; }
 #endif

@@ -2,6 +2,33 @@
 #pragma once
 #include "common.cuh"
 
+// Timeline of the row kernels and of the decode step's BitLinear (experiments build, see mmf_row_trace): thread 0 of CTA 0 takes a
+// record of eight stamps per launch.
+#ifdef MMF_EXPERIMENTS
+extern long long* g_row_trace;
+__device__ __forceinline__ long long* row_trace_record(long long* buffer) {
+    if (!buffer || threadIdx.x || blockIdx.x || blockIdx.y) return nullptr;
+    const int idx = atomicAdd(reinterpret_cast<int*>(buffer), 1);
+    return idx < 1000 ? buffer + 8 + 8 * idx : nullptr;
+}
+__device__ __forceinline__ long long row_now() {
+    long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+#define ROW_TRACE(slot) do { if (trace) trace[slot] = row_now(); } while (0)
+#define ROW_TRACE_AFTER(slot, value) do { asm volatile("" ::"d"(value)); ROW_TRACE(slot); } while (0)   // once `value` is formed
+#define ROW_TRACE_PARAM , long long* trace
+#define ROW_TRACE_ARG , trace
+#define ROW_TRACE_BUFFER , g_row_trace
+#else
+#define ROW_TRACE(slot) do { } while (0)
+#define ROW_TRACE_AFTER(slot, value) do { } while (0)
+#define ROW_TRACE_PARAM
+#define ROW_TRACE_ARG
+#define ROW_TRACE_BUFFER
+#endif
+
 struct PrenormArgs {
     const void* x; int64_t ld_x;
     const void* res; int64_t ld_res;      // may be null
