@@ -46,13 +46,16 @@ const Api* g_api = nullptr;
 
 int64_t g_launches = 0;    // guarded by the GIL
 
-// Rows of a decode step that take the fused kernels, and from how many on the row work is a kernel of its own.  One row is
-// faster with the row work repeated in every CTA (1.3B step: 435 us against 510 with row kernels, 2.7B 688 against ~800); two
-// rows only up to 2048 columns (1.3B 498 against 519, 2.7B 952 against 806).  Above 16 rows the contraction on tcgen05 with
-// row kernels around it is faster (1.3B, 32 rows: 828 us against 1000).
+// Rows of a decode step that take the fused kernels, and from how many on the row work is a kernel of its own.  Step times, row
+// work repeated in every CTA / in row kernels: one row, width 256 (12 blocks) 156 / 198 us, 1024 (24) 338 / 397, 2048 (24) 434 / 513,
+// 2560 (32) 687 / 797, 3072 (16) 472 / 493, 4096 (16) 574 / 590; two rows, 256 181 / 194, 1024 376 / 404, 2048 498 / 526, but 2304 (24)
+// 588 / 564, 2560 934 / 805, 3072 558 / 500, 4096 689 / 618.  Above 16 rows the contraction on tcgen05 with row kernels around it is
+// faster (2048 wide, 24 blocks, 32 rows: 828 us against 1000).
 constexpr int64_t DECODE_ROWS = MMF_DECODE_LINEAR_MAX_M;
 bool rows_in_contraction(int64_t M, int64_t h) { return M == 1 || (M <= MMF_DECODE_LINEAR_FUSED_MAX_M && h <= 2048); }
-constexpr int64_t HEAD_ROWS = 8;              // lm_head alone: tcgen05 above
+// lm_head (32000 outputs) alone: tcgen05 above.  Whole steps, this kernel / tcgen05: two rows of 2560 788 / 801 us, four to eight rows
+// within 0.5 % either way (256, 2048 and 2560 wide), 12 rows 1166 / 1149 (2560) and 639 / 637 (2048), 16 rows 1181 / 1154 and 651 / 647.
+constexpr int64_t HEAD_ROWS = 8;
 bool on16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 constexpr int64_t FUSED_MAX_N = 262144;       // partial sums of more output rows would not fit in shared memory
 

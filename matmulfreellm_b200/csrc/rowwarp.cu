@@ -12,7 +12,7 @@
 // values, before -> after: three-projection prenorm 162 -> 140 us (4.3 TB/s), one-projection prenorm 92 -> 84 us (5.6 TB/s), gate
 // norm 94 -> 79 us (4.2 TB/s); quantisation of 5632-value rows 386 -> 118 us (4.7 TB/s; it was the one-CTA-per-row kernel of
 // rowwise.cu), 14 instructions per value instead of 22.  What is left: shared-memory wavefronts (the norm weights are read in
-// every pass: pipe 61 - 80 % busy) and issue (2.5 per clock).
+// every pass: pipe 87 / 79 / 67 / 80 % busy in those four) and issue (2.6 / 2.7 / 2.9 / 2.5 instructions per clock of 4).
 #include "common.cuh"
 #include "packed.cuh"
 #include "rowquant.cuh"
@@ -25,7 +25,9 @@ constexpr int WR_MAX_WARPS = 16;
 constexpr int V = 8;                          // values per 16-byte vector
 
 // Between two passes over a packed row: the compiler would keep the widened values of the first pass for the second, twice
-// as many registers as the packed row (at 22 vectors per lane it spilled 560 bytes), instead of widening again.
+// as many registers as the packed row (at 22 vectors per lane it spilled 560 bytes, now none), instead of widening again.
+// Longer rows still spill a little: the quantisation 64 - 72 bytes at 26 and 28 vectors (rows above 6144 values), the prenorm 4 - 40
+// bytes at 12 - 16 (rows above 2560 values).
 template <int NV> __device__ __forceinline__ void forget_widened(uint32_t (&u)[NV][4]) {
 #pragma unroll
     for (int it = 0; it < NV; ++it)

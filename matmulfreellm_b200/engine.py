@@ -34,8 +34,8 @@ class GreedyDecoder:
         self.kernels_per_step = 0
         self.last_logits: Optional[torch.Tensor] = None
         self._use_graph = use_graph
-        # prompt passes of a repeated length are replayed from a graph as well: an eager pass is about 200 launches
-        # through Python (about 19 us of host time each), which is more than the GPU needs for a short prompt
+        # prompt passes of a repeated length are replayed from a graph as well: an eager pass is about 200 launches of
+        # about 2 us of host time each, and a step of few sequences needs little more on the GPU
         self._prompt_seen: dict = {}       # prompt length -> times seen
         self._prompt_graphs: dict = {}     # prompt length -> (graph, static ids and logits buffers, what it reads), at most PROMPT_GRAPHS entries
         self._host_graphs: dict = {}       # (ids_host ptr, out_host ptr) -> (graph with the two copies, its logits buffer, what it reads, the host buffers)
