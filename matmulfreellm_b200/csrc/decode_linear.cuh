@@ -598,12 +598,6 @@ template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, 
     const bool fused = a.codes == nullptr;
     const int G = a.epilogue == MMF_EPI_GATES ? 3 : 1, D = (int)a.K;
     const int NB = fused || a.M <= 8 ? 1 : 2, MR = !fused ? 8 * NB : a.M <= 1 ? 1 : 2;
-    if (!fused) {
-        const int rc = a.prologue == MMF_PRO_QUANT     ? dl_rows<T, MMF_PRO_QUANT>(a, G, p.KG, NB, st)
-                       : a.prologue == MMF_PRO_PRENORM ? dl_rows<T, MMF_PRO_PRENORM>(a, G, p.KG, NB, st)
-                                                       : dl_rows<T, MMF_PRO_GATENORM>(a, G, p.KG, NB, st);
-        if (rc != MMF_OK) return rc;
-    }
     // One CTA on every SM, however the rows divide: two kernels of the chain share an SM (the next one waits with its weights),
     // and an SM that this grid left empty would later take two CTAs of the next one, which then finishes late.
     const int units = a.epilogue == MMF_EPI_GATES ? (int)(a.K / 2) : a.epilogue == MMF_EPI_SWIGLU ? (int)(a.N / 4) : (int)((a.N + 1) / 2);
@@ -659,6 +653,13 @@ template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, 
                 (long long)a.K);
     p.pf = want < room ? want : room;
     const int smem = off + p.pf * per_item;
+    // (after every check: a refused call has launched nothing)
+    if (!fused) {
+        const int rc = a.prologue == MMF_PRO_QUANT     ? dl_rows<T, MMF_PRO_QUANT>(a, G, p.KG, NB, st)
+                       : a.prologue == MMF_PRO_PRENORM ? dl_rows<T, MMF_PRO_PRENORM>(a, G, p.KG, NB, st)
+                                                       : dl_rows<T, MMF_PRO_GATENORM>(a, G, p.KG, NB, st);
+        if (rc != MMF_OK) return rc;
+    }
 
 #define DL_K(PRO, EPI, TH, MR, NVT) return dl_go<decode_linear_kernel<T, PRO, EPI, TH, MR, NVT>>(p, threads, smem, st)
 #define DL_CODES_K(EPI)                                            \

@@ -98,7 +98,8 @@ def test_decode_linear_refuses_bad_arguments(lib):
                   dict(ws, codes=p + 8), dict(gates, state=None), dict(gates, g_out=None), dict(gates, state=p + 4),
                   dict(gates, g_out=p + 2), dict(gates, lower_bound=p + 2), dict(ld_out=63), dict(row_ids=p, x_rows=0),
                   dict(row_ids=p, x_rows=5, residual=p, ld_residual=128), dict(row_ids=p, x_rows=5, prologue=L.PRO_QUANT)],
-        BAD_SHAPE: [dict(M=-1), dict(M=3), dict(ws, M=17), dict(N=0), dict(N=1 << 24), dict(K=0), dict(K=96), dict(K=4160, ld_x=4160),
+        BAD_SHAPE: [dict(ws, M=16, N=(1 << 24) - 128, ld_out=1 << 24),       # partial sums do not fit; the row kernel has not run either
+                    dict(M=-1), dict(M=3), dict(ws, M=17), dict(N=0), dict(N=1 << 24), dict(K=0), dict(K=96), dict(K=4160, ld_x=4160),
                     dict(K=8256, ld_x=8256, prologue=L.PRO_QUANT), dict(gatenorm, K=4160, ld_x=4160, ld_residual=4160),
                     dict(gates, N=256), dict(gates, K=192, N=576, ld_x=192), dict(epilogue=L.EPI_SWIGLU, N=66, ld_out=34),
                     dict(epilogue=L.EPI_SWIGLU, ld_out=33), dict(epilogue=L.EPI_SWIGLU, ld_out=30), dict(ld_x=120), dict(ld_x=0),
