@@ -317,26 +317,28 @@ struct Held {
 struct Slot {
     PyObject *dict, *name;        // owned references
     Held held;                    // what the slot held when the watch was made
-    c10::weak_intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl> impl{c10::intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl>()};
-    c10::weak_intrusive_ptr<c10::StorageImpl> storage{c10::intrusive_ptr<c10::StorageImpl>()};
 };
 struct Watch {
     std::vector<Slot> slots;
+    std::vector<c10::weak_intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl>> impls;
+    std::vector<c10::weak_intrusive_ptr<c10::StorageImpl>> storages;
     ~Watch() {
         for (Slot& s : slots) { Py_DECREF(s.dict); Py_DECREF(s.name); }
     }
 };
 const at::Tensor* in_slot(PyObject* dict, PyObject* name) {
-    PyObject* v = PyDict_GetItem(dict, name);     // borrowed
+    PyObject* v = PyDict_GetItemWithError(dict, name);     // borrowed; a str key raises nothing
     return v && THPVariable_Check(v) ? &THPVariable_Unpack(v) : nullptr;
 }
 Held look(const at::Tensor* t) {
     Held h;
     if (t) {
-        h.impl = t->unsafeGetTensorImpl();
-        if (t->has_storage()) {
-            h.storage = t->storage().unsafeGetStorageImpl();
-            h.data = t->const_data_ptr();
+        c10::TensorImpl* impl = t->unsafeGetTensorImpl();
+        h.impl = impl;
+        if (impl->has_storage()) {
+            const c10::StorageImpl* storage = impl->unsafe_storage().unsafeGetStorageImpl();
+            h.storage = storage;
+            h.data = static_cast<const uint8_t*>(storage->data()) + impl->storage_offset() * impl->itemsize();
         }
         h.version = t->is_inference() ? 0 : (int64_t)t->_version();
         h.dtype = t->scalar_type();
@@ -350,7 +352,8 @@ PyObject* watch(PyObject*, PyObject* slots) {
         if (!seq) return nullptr;
         for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq); ++i) {
             PyObject* item = PySequence_Fast_GET_ITEM(seq, i);
-            if (!PyTuple_Check(item) || PyTuple_GET_SIZE(item) != 2 || !PyDict_Check(PyTuple_GET_ITEM(item, 0))) {
+            if (!PyTuple_Check(item) || PyTuple_GET_SIZE(item) != 2 || !PyDict_Check(PyTuple_GET_ITEM(item, 0)) ||
+                !PyUnicode_Check(PyTuple_GET_ITEM(item, 1))) {
                 Py_DECREF(seq);
                 throw std::domain_error("slots must be a sequence of (dict, name)");
             }
@@ -360,8 +363,8 @@ PyObject* watch(PyObject*, PyObject* slots) {
             s.name = Py_NewRef(PyTuple_GET_ITEM(item, 1));
             if (const at::Tensor* t = in_slot(s.dict, s.name)) {
                 s.held = look(t);
-                s.impl = decltype(s.impl)(t->getIntrusivePtr());
-                if (t->has_storage()) s.storage = t->storage().getWeakStorageImpl();
+                w->impls.emplace_back(t->getIntrusivePtr());
+                if (t->has_storage()) w->storages.push_back(t->storage().getWeakStorageImpl());
             }
         }
         Py_DECREF(seq);
