@@ -670,6 +670,42 @@ def test_native_calls_check_the_device(mm):
         fn()
 
 
+def test_forwards_from_several_threads(mm):
+    """A forward releases the GIL while it launches: four threads on streams of their own, sharing one model, get what one thread gets."""
+    import threading
+    cfg = tiny_cfg()
+    model = build_gpu_model(O.random_weights(cfg, seed=9), cfg, torch.bfloat16)
+    layer = model.model.layers[0].mlp.down_proj
+    g = torch.Generator().manual_seed(2)
+    work = [torch.randint(0, cfg.vocab_size, shape, generator=g).cuda() for shape in ((1, 1), (2, 1), (5, 1), (12, 1), (33, 1), (3, 40), (1, 300), (8, 150))]
+    rows = [torch.randn(m, cfg.intermediate_size, generator=g).bfloat16().cuda() for m in (1, 2, 7, 200)]
+
+    def one_pass():
+        with torch.no_grad():
+            return [model(input_ids=ids).logits for ids in work] + [layer(x) for x in rows]
+
+    want = one_pass()
+    torch.cuda.synchronize()
+    wrong = []
+
+    def thread(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(8):
+                    got = one_pass()
+                    torch.cuda.current_stream().synchronize()
+                    wrong.extend((k, i) for i, (a, b) in enumerate(zip(got, want)) if not torch.equal(a, b))
+        except Exception as e:                       # noqa: BLE001 - reported by the assertion below
+            wrong.append((k, repr(e)))
+
+    threads = [threading.Thread(target=thread, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+
+
 def test_launch_count_is_the_number_of_kernels(mm):
     """`_lib.launch_count`, which the benchmark reports, advances by the kernels that a call really launches: the kernel nodes
     of a graph captured from it (time-split scans make two passes; a forward of one, four or 32 rows takes different chains)."""
