@@ -341,6 +341,55 @@ typedef struct {
 int mmf_decode_linear(const mmf_decode_linear_args* args, void* stream);
 
 /* ------------------------------------------------------------------------------------
+ * All blocks of a decode step (one new token per sequence, few sequences, 16-bit activations) in one resident kernel.
+ * Replaces, for T = 1: the loop over HGRNBitBlock.forward, mmfreelm/models/hgrn_bit/modeling_hgrn_bit.py:86-112, up to the
+ * final norm; results are bit-identical to the chain of mmf_decode_linear calls.
+ * ------------------------------------------------------------------------------------ */
+#define MMF_DECODE_STEP_MAX_M 16
+
+/* What a block's step reads besides the activations: packed weights as mmf_decode_linear takes them (i | f | g stacked [3 h, h], [h, h],
+ * gate | up [2 inner, h], [h, inner]), their scales, fp32 norm weights (NULL: ones). */
+typedef struct {
+    const float *attn_norm_w, *ifg_norm_w[3], *gate_norm_w, *o_norm_w, *mlp_norm_w, *gate_proj_norm_w, *down_norm_w;
+    const void *ifg, *o, *gate, *down;
+    const float *ifg_scale, *o_scale, *gate_scale, *down_scale;
+} mmf_decode_step_weights;
+
+/* The same laid out for the step, once: each SM's share of every link's weights contiguous, norm weights and scales behind them.
+ * mmf_decode_step_layer_bytes() bytes at `out` (16-byte aligned), for the current device (its SM count); 0: sizes not taken. */
+int64_t mmf_decode_step_layer_bytes(int64_t hidden, int64_t inner);
+int mmf_decode_step_pack(const mmf_decode_step_weights* weights, int64_t hidden, int64_t inner, void* out, void* stream);
+
+typedef struct {
+    const void* weights;                    /* from mmf_decode_step_pack */
+    const void* lower_bound;                /* [h] in dtype, or NULL */
+    float* state;                           /* fp32 [M, h], advanced in place */
+    float eps_gate, eps_bl;
+} mmf_decode_step_layer;
+
+typedef struct {
+    int dtype;                              /* MMF_BF16 or MMF_F16 */
+    int64_t M, hidden, inner, layers;
+    const mmf_decode_step_layer* layer;     /* HOST array of `layers` entries, read before the call returns */
+    const void* x;                          /* the tokens' rows [M, ld_x], or the embedding table with row_ids */
+    int64_t ld_x;
+    const int64_t* row_ids;                 /* row m is x[row_ids[m]] (ids are clamped to x_rows), or NULL */
+    int64_t x_rows;
+    const uint8_t* mask;                    /* [M], 0 = padding, or NULL */
+    float eps_norm;                         /* attn_norm and mlp_norm */
+    void* out;                              /* [M, hidden]: the last block's MLP output ... */
+    void* residual_out;                     /* ... and the residual stream it is to be added to */
+    void* workspace;                        /* mmf_decode_step_workspace_bytes() bytes, 256-byte aligned; any contents */
+    int64_t workspace_bytes;
+    int* status;                            /* device word, set to 1 if a bounded wait gave up (outputs are then undefined) */
+} mmf_decode_step_args;
+
+/* 0: the sizes are not taken on the current device. */
+int64_t mmf_decode_step_workspace_bytes(int64_t M, int64_t hidden, int64_t inner, int64_t layers);
+/* A memory fill and a cooperative launch of one CTA per SM. */
+int mmf_decode_step(const mmf_decode_step_args* args, void* stream);
+
+/* ------------------------------------------------------------------------------------
  * Row-wise norms and activations.
  * ------------------------------------------------------------------------------------ */
 

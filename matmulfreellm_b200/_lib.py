@@ -35,6 +35,19 @@ class DecodeLinearArgs(ctypes.Structure):
                 ("ld_out", c_int64), ("g_out", c_void_p), ("lower_bound", c_void_p), ("mask", c_void_p), ("state", c_void_p)]
 
 
+class DecodeStepLayer(ctypes.Structure):
+    """mmf_decode_step_layer of the header."""
+    _fields_ = [("weights", c_void_p), ("lower_bound", c_void_p), ("state", c_void_p), ("eps_gate", c_float), ("eps_bl", c_float)]
+
+
+class DecodeStepArgs(ctypes.Structure):
+    """mmf_decode_step_args of the header, field by field."""
+    _fields_ = [("dtype", c_int), ("M", c_int64), ("hidden", c_int64), ("inner", c_int64), ("layers", c_int64),
+                ("layer", ctypes.POINTER(DecodeStepLayer)), ("x", c_void_p), ("ld_x", c_int64), ("row_ids", c_void_p), ("x_rows", c_int64),
+                ("mask", c_void_p), ("eps_norm", c_float), ("out", c_void_p), ("residual_out", c_void_p), ("workspace", c_void_p),
+                ("workspace_bytes", c_int64), ("status", c_void_p)]
+
+
 PRO_QUANT, PRO_PRENORM, PRO_GATENORM = 1, 2, 3
 EPI_STORE, EPI_GATES, EPI_SWIGLU = 0, 1, 2
 
@@ -76,6 +89,10 @@ PROTOTYPES = {
     "mmf_swiglu_quant": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_void_p, c_float, c_void_p, c_void_p, c_void_p,
                                  c_int64, c_int64, c_void_p]),
     "mmf_decode_linear": (c_int, [c_void_p, c_void_p]),
+    "mmf_decode_step_layer_bytes": (c_int64, [c_int64, c_int64]),
+    "mmf_decode_step_pack": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p]),
+    "mmf_decode_step_workspace_bytes": (c_int64, [c_int64, c_int64, c_int64, c_int64]),
+    "mmf_decode_step": (c_int, [c_void_p, c_void_p]),
     "mmf_rmsnorm": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int64,
                             c_int64, c_void_p]),
     "mmf_rmsnorm_swishgate": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_float, c_void_p, c_int64, c_int64,

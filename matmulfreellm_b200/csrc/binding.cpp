@@ -37,7 +37,7 @@ struct Api {
 #define MMF_FNS(F)                                                                                                      \
     F(mmf_last_error) F(mmf_act_quant) F(mmf_bitlinear) F(mmf_hgrn_workspace_bytes) F(mmf_hgrn_scan) F(mmf_hgrn_gated_masked) \
     F(mmf_prenorm_quant) F(mmf_gatenorm_quant) F(mmf_decode_mix_masked) F(mmf_swiglu_quant) F(mmf_embedding) \
-    F(mmf_decode_linear)
+    F(mmf_decode_linear) F(mmf_decode_step_layer_bytes) F(mmf_decode_step_pack) F(mmf_decode_step_workspace_bytes) F(mmf_decode_step)
     MMF_FNS(MMF_FN)
 #undef MMF_FN
 };
@@ -395,6 +395,7 @@ struct Layer {
     const float *attn_norm_w, *ifg_nw[3], *gnorm_w, *o_nw, *mlp_norm_w, *gate_nw, *down_nw;
     Linear ifg, o, gate, down;
     const void* lb;
+    const void* step = nullptr;        // weights, norm weights and scales as the resident decode step reads them
     float gnorm_eps, eps_bl;
 };
 struct Chain {
@@ -404,6 +405,7 @@ struct Chain {
     const float *final_norm_w, *head_nw;
     Linear head;
     int64_t h = 0, inner = 0;
+    bool step_ok = false;              // the blocks' weights are laid out for the resident decode step as well
     float eps = 0, head_eps = 0;
     int dtype = 0;
 };
@@ -438,6 +440,25 @@ struct Fields {      // positional reader of a Python tuple
         return l;
     }
 };
+// The blocks' weights once more, in the layout of the resident decode step, if it takes the model (16-bit, on the current device, all
+// MLPs as wide): as many bytes again as the blocks' packed weights.
+void lay_out_step(Chain& c) {
+    if (c.dtype == MMF_F32 || c.layers.empty() || !c.table.is_cuda() || c.table.get_device() != c10::cuda::current_device()) return;
+    for (const Layer& L : c.layers)
+        if (L.down.K != c.inner) return;
+    const int64_t bytes = g_api->mmf_decode_step_layer_bytes(c.h, c.inner);
+    if (!bytes || !g_api->mmf_decode_step_workspace_bytes(1, c.h, c.inner, (int64_t)c.layers.size())) return;
+    void* st = c10::cuda::getCurrentCUDAStream(c.table.get_device()).stream();
+    for (Layer& L : c.layers) {
+        const at::Tensor mem = at::empty({bytes}, c.table.options().dtype(at::kByte));
+        const mmf_decode_step_weights w = {L.attn_norm_w, {L.ifg_nw[0], L.ifg_nw[1], L.ifg_nw[2]}, L.gnorm_w, L.o_nw, L.mlp_norm_w, L.gate_nw, L.down_nw,
+                                           L.ifg.packed, L.o.packed, L.gate.packed, L.down.packed, L.ifg.scale, L.o.scale, L.gate.scale, L.down.scale};
+        MMF_CALL(mmf_decode_step_pack, &w, c.h, c.inner, mem.data_ptr(), st);
+        L.step = mem.data_ptr();
+        c.keep.push_back(mem);
+    }
+    c.step_ok = true;
+}
 // chain(table, layers, final_norm_w, head(5 fields), head_nw, eps, head_eps): layers is a list of tuples in the order read below
 PyObject* chain(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
@@ -469,6 +490,7 @@ PyObject* chain(PyObject*, PyObject* const* args, Py_ssize_t n) {
             c->inner = std::max(c->inner, L.down.K);
             c->layers.push_back(L);
         }
+        lay_out_step(*c);
         Fields f{args[2], *c};
         c->final_norm_w = f.f32();
         c->head = f.linear();
@@ -587,6 +609,13 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
             // codes: decode-step contractions want rows of whole 256-column groups, up to 16 of them
             const int64_t Mc = M <= 8 ? 8 : M <= 16 ? 16 : M;
             const int64_t q = s.take(Mc * std::max(3 * ((h + 255) & ~255ll), (c.inner + 255) & ~255ll)), dq = s.take(3 * M * 4), rs = s.take(3 * M * 4);
+            // one token per sequence and few sequences: contractions with the element-wise work around them in one kernel
+            bool decode = T == 1 && M > 0 && M <= DECODE_ROWS && c.dtype != MMF_F32 && h % MMF_TILE_ROWS == 0 && h <= 4096 && c.inner <= 8192 &&
+                          (ids.defined() || on16(emb.data_ptr()));
+            for (const float* s : states) decode = decode && on16(s);
+            // ... and all blocks in one where they fit on the chip's shared memory
+            const int64_t step_bytes = decode && c.step_ok ? g_api->mmf_decode_step_workspace_bytes(M, h, c.inner, (int64_t)c.layers.size()) : 0;
+            const int64_t step = s.take(step_bytes);
             const int64_t hg_bytes = T > 1 ? g_api->mmf_hgrn_workspace_bytes(B, T, h) : 0, hg = s.take(hg_bytes);
             const at::Tensor mem = at::empty({s.used}, opt.dtype(at::kByte));
             uint8_t* b = mem.data_ptr<uint8_t>();
@@ -599,10 +628,6 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                          MMF_KERNEL_AUTO, st);
                 ++launches;
             };
-            // one token per sequence and few sequences: contractions with the element-wise work around them in one kernel
-            bool decode = T == 1 && M > 0 && M <= DECODE_ROWS && c.dtype != MMF_F32 && h % MMF_TILE_ROWS == 0 && h <= 4096 && c.inner <= 8192 &&
-                          (ids.defined() || on16(emb.data_ptr()));
-            for (const float* s : states) decode = decode && on16(s);
             const int64_t* gather = decode && ids.defined() && !c.layers.empty() ? ids.data_ptr<int64_t>() : nullptr;
             const uint8_t* x = b + x0;            // residual stream
             if (gather) {                         // the first block reads the embedding rows itself
@@ -640,7 +665,24 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 MMF_CALL(mmf_decode_linear, &a, st);
                 launches += a.codes ? 2 : 1;
             };
-            if (decode) decode_blocks(c, args_of, run, gather, b + z, b + ifg, b + o, b + gu, mk, states, x, next, advance);
+            if (step_bytes) {
+                std::vector<mmf_decode_step_layer> layers;
+                for (size_t i = 0; i < c.layers.size(); ++i) layers.push_back({c.layers[i].step, c.layers[i].lb, states[i], c.layers[i].gnorm_eps, c.layers[i].eps_bl});
+                mmf_decode_step_args a = {};
+                a.dtype = c.dtype;
+                a.M = M; a.hidden = h; a.inner = c.inner; a.layers = (int64_t)layers.size();
+                a.layer = layers.data();
+                a.x = x; a.ld_x = h;
+                a.row_ids = gather; a.x_rows = c.table.size(0);
+                a.mask = mk;
+                a.eps_norm = c.eps;
+                a.out = b + z; a.residual_out = next;
+                a.workspace = b + step; a.workspace_bytes = step_bytes;
+                a.status = static_cast<int*>(ws.p);
+                MMF_CALL(mmf_decode_step, &a, st);
+                ++launches;
+                advance();
+            } else if (decode) decode_blocks(c, args_of, run, gather, b + z, b + ifg, b + o, b + gu, mk, states, x, next, advance);
             for (size_t i = 0; i < c.layers.size() && !decode; ++i) {
                 const Layer& L = c.layers[i];
                 if (first) {

@@ -114,6 +114,30 @@ def test_decode_linear_refuses_bad_arguments(lib):
         assert rc(**change, M=0) == 0           # an empty problem is accepted without a launch
 
 
+def test_decode_step_refuses_bad_arguments(lib):
+    """What mmf_decode_step refuses on the host, before any CUDA call."""
+    from matmulfreellm_b200 import _lib as L
+    BAD_ARG, BAD_SHAPE, ALIGN = -1, -2, -3
+    p = 4096
+
+    def rc(layer=None, **change):
+        args = dict(dtype=L.BF16, M=2, hidden=256, inner=512, layers=1, x=p, ld_x=256, out=p, residual_out=p, workspace=p, workspace_bytes=1 << 30, status=p)
+        args.update(change)
+        y = L.DecodeStepLayer(**{**dict(weights=p, state=p), **(layer or {})})
+        return lib.mmf_decode_step(ctypes.byref(L.DecodeStepArgs(layer=ctypes.pointer(y), **args)), None)
+
+    assert lib.mmf_decode_step(None, None) == BAD_ARG and lib.mmf_decode_step_pack(None, 256, 512, p, None) == BAD_ARG
+    for want, cases in {
+        BAD_ARG: [dict(dtype=L.F32), dict(x=None), dict(out=None), dict(residual_out=None), dict(workspace=None), dict(status=None),
+                  dict(layer=dict(weights=None)), dict(layer=dict(state=None)), dict(row_ids=p)],
+        BAD_SHAPE: [dict(M=0), dict(layers=0), dict(layers=97), dict(ld_x=248), dict(M=1, row_ids=p, x_rows=5, ld_x=128)],
+        ALIGN: [dict(x=p + 8), dict(ld_x=260), dict(out=p + 8), dict(residual_out=p + 8), dict(workspace=p + 128), dict(layer=dict(weights=p + 8)),
+                dict(layer=dict(state=p + 4)), dict(layer=dict(lower_bound=p + 2))],
+    }.items():
+        for change in cases:
+            assert rc(**change) == want, (change, lib.mmf_last_error())
+
+
 def test_cpu_tensors_are_refused():
     import torch
     from matmulfreellm_b200 import kernels

@@ -837,6 +837,39 @@ def test_decode_step_rows_do_not_depend_on_the_batch(mm, dtype, hidden, intermed
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("hidden,intermediate", [(128, 64), (640, 6144), (2048, 6208), (2560, 6912)])
+def test_resident_decode_step_at_the_ends_of_its_range(mm, dtype, hidden, intermediate):
+    """All blocks of a step in one kernel (up to 16 sequences) against the chain of kernels that 33 sequences take, bit for bit: fewer channel
+    pairs than SMs, the longest inner row of eight warps and one beyond it, the widest rows; one row, one tile of eight, a row more."""
+    from matmulfreellm_b200 import _lib
+    from mmfreelm.models import HGRNBitConfig, HGRNBitForCausalLM
+    torch.manual_seed(hidden)
+    model = HGRNBitForCausalLM(HGRNBitConfig(vocab_size=300, hidden_size=hidden, num_hidden_layers=3, intermediate_size=intermediate)).eval().cuda()
+    with torch.no_grad():
+        for n, p in model.named_parameters():
+            if "lower_bounds" in n or p.dim() == 1: p.add_(0.3 * torch.randn_like(p))
+    model.pack_weights()
+    model = model.to(dtype)
+    g = torch.Generator().manual_seed(7)
+    ids, step = torch.randint(0, 300, (33, 3), generator=g).cuda(), torch.randint(0, 300, (2, 33, 1), generator=g).cuda()
+
+    def run(B):
+        past = model(ids[:B], use_cache=True).past_key_values
+        for s in step:
+            out = model(input_ids=s[:B], past_key_values=past, use_cache=True)
+        return out.logits, [s[0].view(B, -1) for s in out.past_key_values]
+
+    ref, ref_states = run(33)
+    for B in (1, 2, 8, 9, 16):
+        taken = _lib.load().mmf_decode_step_workspace_bytes(B, hidden, intermediate, 3) > 0
+        assert taken == (B <= 8 or hidden < 2560), B
+        logits, states = run(B)
+        assert torch.equal(logits, ref[:B]), B
+        assert all(torch.equal(a, b[:B]) for a, b in zip(states, ref_states)), B
+    mm.kernels.check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("K,N", [(64, 1), (704, 130), (2112, 37), (5632, 2048), (8192, 515)])
 def test_bitlinear_of_one_and_two_rows_equals_more_rows(mm, dtype, K, N):
     from matmulfreellm_b200.ops.fusedbitnet import FusedBitLinear
