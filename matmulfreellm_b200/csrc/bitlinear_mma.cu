@@ -568,11 +568,11 @@ namespace {
 //    what is left after the dependency wait is the activation load, the MMAs and the epilogue;
 //  * "split" (more tokens / few weight tiles): 4 A stages, K split over a cluster when that fills the GPU.
 // The estimate below is a latency model in microseconds fitted to measured phase times of this kernel.
-bool choose_config(const BitLinearArgs& a, MmaParams& best, size_t& best_smem) {
+bool choose_config(const BitLinearArgs& a, MmaParams& best, size_t& best_smem, double& best_cost) {
     const int KC = a.K / MMF_TILE_K;
     const int n_tiles = (a.N + MMF_TILE_ROWS - 1) / MMF_TILE_ROWS;
     const int total_stages = (KC + 1) / 2;
-    double best_cost = 1e30;
+    best_cost = 1e30;
     bool found = false;
     int nts[3], n_nt = 0;
     if (a.M <= 128) nts[n_nt++] = ((a.M + 15) / 16) * 16;
@@ -662,21 +662,26 @@ bool choose_config(const BitLinearArgs& a, MmaParams& best, size_t& best_smem) {
 }  // namespace
 
 int bitlinear_mma_launch(const BitLinearArgs& a, cudaStream_t st) {
+    MmaParams p;
+    size_t smem = 0;
     {
-        // many token rows: the persistent kernel (one CTA per SM) once it has a full wave of work;
-        // knob values >= 10 select experimental variant (value - 10) and force it for every M > 128
+        // Many token rows: the persistent kernel (one CTA per SM) once it has a full wave of work, and below that from 129 rows on (a decode
+        // batch has at most one token tile here) where it is the faster one by both kernels' estimates, this one's a little low for long K.
+        // This kernel / persistent, us: K 2048, N 11264: 130 rows 10.9 / 9.4, 300 18.4 / 13.2, 400 21.7 / 14.3; three projections of 2048: 400
+        // rows 12.3 / 10.2; N 2048: 1500 rows 12.5 / 10.1; K 5632: 300 rows 13.9 / 14.6, 600 16.9 / 15.0, 1000 17.5 / 16.1, 1500 20.8 / 16.7.
+        // Knob values >= 10 select experimental variant (value - 10) and force it for every M > 128.
         const int variant = g_force_persistent >= 10 ? g_force_persistent - 10 : 0;
         const int nt = bitlinear_mma_prefill_tile(a, variant);
         const int64_t n_work = (int64_t)((a.N + MMF_TILE_ROWS - 1) / MMF_TILE_ROWS) * ((a.M + nt - 1) / nt);
         const bool tuned = g_force_ksplit || g_force_nt || g_force_deep || g_force_wt || g_force_sb || g_force_sa || g_force_sw;
-        if ((g_force_persistent == 1 || g_force_persistent >= 10) ? a.M > 128
-                                                                   : (g_force_persistent == 0 && !tuned && a.M >= 512 && n_work >= 148))
+        const bool choice = g_force_persistent == 0 && !tuned;
+        if ((g_force_persistent == 1 || g_force_persistent >= 10) ? a.M > 128 : (choice && a.M >= 512 && n_work >= 148))
             return bitlinear_mma_prefill_launch(a, st, variant);
+        double us = 0.0;
+        const bool fits = choose_config(a, p, smem, us);
+        if (choice && a.M > 128 && bitlinear_mma_prefill_us(a) <= 1.05 * us) return bitlinear_mma_prefill_launch(a, st, variant);
+        MMF_REQUIRE(fits, MMF_ERR_BAD_SHAPE, "mmf_bitlinear(mma): no kernel configuration fits M=%d N=%d K=%d", a.M, a.N, a.K);
     }
-    MmaParams p;
-    size_t smem = 0;
-    MMF_REQUIRE(choose_config(a, p, smem), MMF_ERR_BAD_SHAPE, "mmf_bitlinear(mma): no kernel configuration fits M=%d N=%d K=%d", a.M,
-                a.N, a.K);
     const int m_tiles = (a.M + p.NT - 1) / p.NT;
     p.async_red = g_force_async_red == 1 ? 1 : g_force_async_red == 2 ? 0 : MMF_ASYNC_REDUCE_DEFAULT;
     // instruction descriptor: D=S32, A=S8 (TMEM), B=S8 (smem, K-major), M=128, N=NT
