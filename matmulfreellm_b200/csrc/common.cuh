@@ -198,11 +198,19 @@ __device__ __forceinline__ void store16(T* p, const float (&in)[16 / sizeof(T)])
 // block reductions (blockDim.x a multiple of 32, <= 1024); result broadcast to all threads
 // `red` is shared scratch of >= 33 elements of T.
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+// Sum of a value over a warp, known to every lane: two fp64 MMAs with a matrix of ones (sums of four lanes, then of the eight sums).
+// A butterfly of shuffles takes 187 clocks, this 78 (eight warps at once: 95); over a block of eight warps, 353 and 217.
+__device__ __forceinline__ double mma_sum4(double b) {       // lane (k = lane % 4, j = lane / 4): sums over k for j = 2k, 2k + 1, added
+    double d0, d1;
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %4};" : "=d"(d0), "=d"(d1) : "d"(1.0), "d"(b), "d"(0.0));
+    return d0 + d1;
 }
+__device__ __forceinline__ double mma_sum(double b) {        // over k = lane % 4 alone; every j holds the same values
+    double d0;
+    asm volatile("{\n\t.reg .f64 d1;\n\tmma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, d1}, {%1}, {%2}, {%3, %3};\n\t}" : "=d"(d0) : "d"(1.0), "d"(b), "d"(0.0));
+    return d0;
+}
+__device__ __forceinline__ double warp_sum(double v) { return mma_sum(mma_sum4(v)); }
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -261,15 +269,54 @@ __device__ __forceinline__ int block_sum(int v, int* red) {
 // the exact arithmetic of the quantisation path (mirrored by the CPU oracle): every step is
 // a single IEEE round-to-nearest fp32 operation, never contracted into an fma.
 // ---------------------------------------------------------------------------------------
+__device__ __forceinline__ float rcp_fast(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// The three roundings of the row arithmetic without the general division's range checks and calls, which were a sixth of a row's
+// latency: approximations corrected by exact remainders (Markstein 1990).  Each returns what the IEEE operations beside it return, for
+// every argument they are called with (compared for all floats in their ranges).
+__device__ __forceinline__ float rcp_sqrt(float x) {            // __fdiv_rn(1, __fsqrt_rn(x)), x >= 0
+    const float up = x < 0x1p-96f ? 0x1p32f : x > 0x1p96f ? 0x1p-32f : 1.0f;       // powers of four move out of the root exactly
+    const float v = x * up * up;
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
+    float g = __fmul_rn(v, y), h = __fmul_rn(0.5f, y);
+    const float r = __fmaf_rn(-h, g, 0.5f);
+    g = __fmaf_rn(g, r, g);
+    h = __fmaf_rn(h, r, h);
+    g = __fmaf_rn(__fmaf_rn(-g, g, v), h, g);                  // sqrt(v)
+    float z = __fadd_rn(h, h);
+    z = __fmaf_rn(z, __fmaf_rn(-g, z, 1.0f), z);
+    z = __fmaf_rn(z, __fmaf_rn(-g, z, 1.0f), z);
+    if ((__float_as_uint(g) & 0x7fffffu) == 0x7fffffu) z = __uint_as_float(__float_as_uint(z) + 1);      // the one mantissa the step leaves an ulp low
+    return v > 0.0f && v < __int_as_float(0x7f800000) ? z * up : y;      // 0, infinity and NaN: the approximation is exact
+}
+__device__ __forceinline__ float q127_over(float t) {         // __fdiv_rn(127, t), t >= 1e-5
+    const float down = t > 0x1p64f ? 0x1p-64f : 1.0f, v = t * down;
+    float y = rcp_fast(v);
+    y = __fmaf_rn(y, __fmaf_rn(-v, y, 1.0f), y);
+    float q = __fmul_rn(127.0f, y);
+    q = __fmaf_rn(__fmaf_rn(-q, v, 127.0f), y, q);
+    return v == __int_as_float(0x7f800000) ? 0.0f : q * down;
+}
+__device__ __forceinline__ float over_127(float t) {         // __fdiv_rn(t, 127), t >= 1e-5
+    constexpr float c = 1.0f / 127.0f;
+    const float q = __fmul_rn(t, c);
+    return t == __int_as_float(0x7f800000) ? t : __fmaf_rn(__fmaf_rn(-q, 127.0f, t), c, q);
+}
 // inv_k = 1.0 / K, which a kernel forms before it waits for its input.  The quotient is the product with it plus one correction
 // by the exact remainder (Markstein's division step): the fp64 division itself, about 100 instructions for a K that is not a
 // power of two, would sit on the critical path of every row.  An infinite sum (a row with an infinite entry) has no remainder
 // (inf - inf) and is its own quotient: rstd 0, as the division gives.  The test is on the high word, beside the fp64 chain.
-__device__ __forceinline__ float rstd_from_sumsq(double sumsq, int K, double inv_k, float eps) {
+// LEAN = false: the general division and root (see rowwarp.cu).
+template <bool LEAN = true> __device__ __forceinline__ float rstd_from_sumsq(double sumsq, int K, double inv_k, float eps) {
     const double q0 = sumsq * inv_k;
     const double q = __double2hiint(sumsq) == 0x7ff00000 ? q0 : fma(fma(-q0, (double)K, sumsq), inv_k, q0);
     const float mean = (float)q;
-    return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
+    const float v = __fadd_rn(mean, eps);
+    return LEAN ? rcp_sqrt(v) : __fdiv_rn(1.0f, __fsqrt_rn(v));
 }
 // e^-x and the reciprocal through the special-function unit (ex2.approx, rcp.approx: relative error about 2^-22 each).
 // The results feed values that are rounded to the activation dtype right away, or compared at 1e-4, so the two extra
@@ -278,11 +325,6 @@ __device__ __forceinline__ float exp_neg(float x) {
     float p;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p) : "f"(__fmul_rn(x, -1.4426950408889634f)));
     return p;
-}
-__device__ __forceinline__ float rcp_fast(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
 }
 __device__ __forceinline__ float silu_mul(float x, float y) {
     // float(x) * float(y) / (1.0f + exp(-float(x)))

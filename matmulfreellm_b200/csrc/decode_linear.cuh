@@ -234,7 +234,7 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
         float t = 1e-5f;
 #pragma unroll
         for (int w = 0; w < RT / 32; ++w) t = fmaxf(t, red.f[g][w]);
-        s[g] = __fdiv_rn(127.0f, t);
+        s[g] = q127_over(t);
         sum[g] = 0;
         if (rt == 0) s_amax[g] = t;
     }
@@ -305,7 +305,7 @@ decode_rows_kernel(const __grid_constant__ mmf_decode_linear_args a, int KG, int
 #pragma unroll
         for (int w = 0; w < TH / 32; ++w) t += red.i[0][w];
         *rowsum = t;
-        *dq = __fdiv_rn(s_amax[0], 127.0f);
+        *dq = over_127(s_amax[0]);
     }
     ROW_TRACE(7);
 }
@@ -429,7 +429,7 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
 #pragma unroll
             for (int w = 0; w < RT / 32; ++w) t += red[cm < MR ? cm : 0].i[cg][w];
             s_rs[cg][cm] = t;
-            s_scale[cg][cm] = __fmul_rn(__fdiv_rn(s_amax[cm][cg], 127.0f), ws);
+            s_scale[cg][cm] = __fmul_rn(over_127(s_amax[cm][cg]), ws);
         }
     } else {
         if (has_const) {

@@ -84,29 +84,17 @@ __device__ __forceinline__ void ds_copy(uint32_t dst, const void* src, uint32_t 
                      ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 
-// Sum of a value over a warp, known to every lane: two fp64 MMAs with a matrix of ones (sums of four lanes, then of the eight sums).
-// A butterfly of shuffles takes 187 clocks, this 78 (eight warps at once: 95); over a block of eight warps, 353 and 217.
-__device__ __forceinline__ double ds_mma_sum4(double b) {       // lane (k = lane % 4, j = lane / 4): sums over k for j = 2k, 2k + 1, added
-    double d0, d1;
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %4};" : "=d"(d0), "=d"(d1) : "d"(1.0), "d"(b), "d"(0.0));
-    return d0 + d1;
-}
-__device__ __forceinline__ double ds_mma_sum(double b) {        // over k = lane % 4 alone; every j holds the same values
-    double d0;
-    asm volatile("{\n\t.reg .f64 d1;\n\tmma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, d1}, {%1}, {%2}, {%3, %3};\n\t}" : "=d"(d0) : "d"(1.0), "d"(b), "d"(0.0));
-    return d0;
-}
 // over the CTA
 template <int NW> __device__ __forceinline__ double ds_sum(double s, double* slot) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    s = ds_mma_sum(ds_mma_sum4(s));
+    s = warp_sum(s);
     if (lane == 0) slot[warp] = s;
     __syncthreads();
     double t = slot[lane & 3];
 #pragma unroll
     for (int o = 4; o < NW; o += 4)
         if (o + 4 <= NW || (lane & 3) < NW - o) t += slot[o + (lane & 3)];
-    return ds_mma_sum(t);
+    return mma_sum(t);
 }
 // fold the warps' entries of a 16-byte aligned array
 template <int NW> __device__ __forceinline__ float ds_fold_max(const float* v) {
@@ -126,44 +114,6 @@ template <int NW> __device__ __forceinline__ int ds_fold_sum(const int* v) {
         t += a.x + a.y;
     }
     return t;
-}
-
-// The three roundings of the row arithmetic without the general division's range checks and calls, which were a sixth of a row's
-// latency: approximations corrected by exact remainders (Markstein 1990).  Each returns what the IEEE operations beside it return, for
-// every argument they are called with (compared for all floats in their ranges).
-__device__ __forceinline__ float ds_rsqrt(float x) {            // __fdiv_rn(1, __fsqrt_rn(x)), x >= 0
-    const float up = x < 0x1p-96f ? 0x1p32f : x > 0x1p96f ? 0x1p-32f : 1.0f;       // powers of four move out of the root exactly
-    const float v = x * up * up;
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
-    float g = __fmul_rn(v, y), h = __fmul_rn(0.5f, y);
-    const float r = __fmaf_rn(-h, g, 0.5f);
-    g = __fmaf_rn(g, r, g);
-    h = __fmaf_rn(h, r, h);
-    g = __fmaf_rn(__fmaf_rn(-g, g, v), h, g);                  // sqrt(v)
-    float z = __fadd_rn(h, h);
-    z = __fmaf_rn(z, __fmaf_rn(-g, z, 1.0f), z);
-    z = __fmaf_rn(z, __fmaf_rn(-g, z, 1.0f), z);
-    if ((__float_as_uint(g) & 0x7fffffu) == 0x7fffffu) z = __uint_as_float(__float_as_uint(z) + 1);      // the one mantissa the step leaves an ulp low
-    return v == 0.0f || v == __int_as_float(0x7f800000) ? y : z * up;
-}
-__device__ __forceinline__ float ds_127_over(float t) {         // __fdiv_rn(127, t), t >= 1e-5
-    const float down = t > 0x1p64f ? 0x1p-64f : 1.0f, v = t * down;
-    float y = rcp_fast(v);
-    y = __fmaf_rn(y, __fmaf_rn(-v, y, 1.0f), y);
-    float q = __fmul_rn(127.0f, y);
-    q = __fmaf_rn(__fmaf_rn(-q, v, 127.0f), y, q);
-    return v == __int_as_float(0x7f800000) ? 0.0f : q * down;
-}
-__device__ __forceinline__ float ds_over_127(float t) {         // __fdiv_rn(t, 127), t >= 1e-5
-    constexpr float c = 1.0f / 127.0f;
-    const float q = __fmul_rn(t, c);
-    return t == __int_as_float(0x7f800000) ? t : __fmaf_rn(__fmaf_rn(-q, 127.0f, t), c, q);
-}
-__device__ __forceinline__ float ds_rstd(double sumsq, int K, double inv_k, float eps) {       // rstd_from_sumsq
-    const double q0 = sumsq * inv_k;
-    const double q = __double2hiint(sumsq) == 0x7ff00000 ? q0 : fma(fma(-q0, (double)K, sumsq), inv_k, q0);
-    return ds_rsqrt(__fadd_rn((float)q, eps));
 }
 
 __device__ __forceinline__ void ds_mma(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, int c0, int c1, int c2, int c3) {
@@ -400,7 +350,7 @@ decode_step_kernel(const __grid_constant__ DsParams p) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) sumsq_pair<T>(c[i], s0, s1);
                 }
-                if (me) rstd = ds_rstd(ds_sum<NW>(s0 + s1, s_sum[1]), D, z.inv_d, p.layer[l].eps_bl);
+                if (me) rstd = rstd_from_sumsq(ds_sum<NW>(s0 + s1, s_sum[1]), D, z.inv_d, p.layer[l].eps_bl);
             } else {
                 const uint32_t a[4] = {v[0].x, v[0].y, v[0].z, v[0].w}, b[4] = {v[1].x, v[1].y, v[1].z, v[1].w};
                 uint32_t c[4];
@@ -433,7 +383,7 @@ decode_step_kernel(const __grid_constant__ DsParams p) {
                     }
 #pragma unroll 1
                     for (int pass = 0;; ++pass) {
-                        rstd = ds_rstd(ds_sum<NW>(s0 + s1, s_sum[pass]), D, z.inv_d, pass ? p.layer[l].eps_bl : type == DS_O ? p.layer[l].eps_gate : p.eps_norm);
+                        rstd = rstd_from_sumsq(ds_sum<NW>(s0 + s1, s_sum[pass]), D, z.inv_d, pass ? p.layer[l].eps_bl : type == DS_O ? p.layer[l].eps_gate : p.eps_norm);
                         if (pass) break;
                         DS_TRACE_AFTER(3, (double)rstd);
                         s0 = s1 = 0.0;
@@ -482,7 +432,7 @@ decode_step_kernel(const __grid_constant__ DsParams p) {
                 float sc[NVI];
                 auto scale = [&](int j) {
                     const float top = ds_fold_max<NW>(s_max[j]);
-                    sc[j] = ds_127_over(top);
+                    sc[j] = q127_over(top);
                     if (tid == 0) s_top[j] = top;
                 };
                 uint8_t* dst = xcodes + ((FUSED || type != DS_IFG ? 0 : row_g) * KG + warp) * STEP + code_at;
@@ -519,7 +469,7 @@ decode_step_kernel(const __grid_constant__ DsParams p) {
                 int sum = 0;
 #pragma unroll 1
                 for (int k = 0; k < KG; ++k) sum += s_codes[k];
-                const uint64_t x = (uint64_t)(uint32_t)sum << 32 | __float_as_uint(ds_over_127(s_top[0]));
+                const uint64_t x = (uint64_t)(uint32_t)sum << 32 | __float_as_uint(over_127(s_top[0]));
                 asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(xscale + ((type == DS_IFG ? row_g : 0) * MR + row_m) * 8), "l"(x) : "memory");
             }
         }
@@ -632,7 +582,7 @@ decode_step_kernel(const __grid_constant__ DsParams p) {
             }
             const int rs = FUSED || !on ? 0 : s_rs[g][m];
             float sc;
-            if constexpr (FUSED) sc = __fmul_rn(ds_over_127(s_top[g]), ws);
+            if constexpr (FUSED) sc = __fmul_rn(over_127(s_top[g]), ws);
             else sc = on ? s_scale[g][m] : 0.0f;
             uint32_t val = narrow<T>(make_float2(dl_out(sum.x, rs, sc), dl_out(sum.y, rs, sc)));
             const uint32_t v1 = __shfl_sync(0xffffffffu, val, (lane + per) & 31), v2 = __shfl_sync(0xffffffffu, val, (lane + 2 * per) & 31);

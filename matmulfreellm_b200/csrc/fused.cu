@@ -199,7 +199,7 @@ __device__ __forceinline__ void bitlinear_prologue(float (&v)[P], int D, double 
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         const float a = fmaxf(amax[g], 1e-5f);
-        const float s = __fdiv_rn(127.0f, a);
+        const float s = q127_over(a);
         int8_t* qr = q + ((int64_t)g * M + m) * D;
         lsum[g] = 0;
         ROW_FOREACH(V, D, it, c) {
@@ -228,7 +228,7 @@ __device__ __forceinline__ void bitlinear_prologue(float (&v)[P], int D, double 
             if constexpr (V == 8) *reinterpret_cast<uint2*>(qr + c) = make_uint2(words[0], words[1]);
             else *reinterpret_cast<uint32_t*>(qr + c) = words[0];
         }
-        if (threadIdx.x % RT == 0) dq[(int64_t)g * M + m] = __fdiv_rn(a, 127.0f);
+        if (threadIdx.x % RT == 0) dq[(int64_t)g * M + m] = over_127(a);
     }
     block_sum_i_t0<G, RT>(lsum, red.i0);
     if (threadIdx.x % RT == 0) {

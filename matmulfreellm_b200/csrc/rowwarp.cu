@@ -23,6 +23,10 @@ namespace {
 // rows.  24 warps at 80 registers were 8 % slower than 16 at 128 (2048-value rows) and leave a nearly empty last wave earlier.
 constexpr int WR_MAX_WARPS = 16;
 constexpr int V = 8;                          // values per 16-byte vector
+// Rows of at most 2048 values take the short forms of division and root (32768 rows: gate norm 78 -> 71 us, quantisation 43 -> 35).  The
+// general ones branch, and without those branches between the passes the compiler reads a longer row's weights, and the prenorm's, ahead
+// and spills (5632 values: 117 us -> 217; one-projection prenorm 83 -> 87).
+__host__ __device__ constexpr bool lean(int NV) { return NV <= 8; }
 
 // Between two passes over a packed row: the compiler would keep the widened values of the first pass for the second, twice
 // as many registers as the packed row (at 22 vectors per lane it spilled 560 bytes, now none), instead of widening again.
@@ -49,7 +53,7 @@ __device__ __forceinline__ void stage(float* dst, const float* src, int n) {
 }
 
 // BitLinear prologue of the packed row u: y = (v * rstd) * w, absmax -> scale -> int8 codes, dq, code sum
-template <typename T, int NV>
+template <typename T, int NV, bool LEAN>
 __device__ __forceinline__ void warp_quant(uint32_t (&u)[NV][4], int D, float rstd, const float* sw, int8_t* qr, float* dq,
                                            int32_t* rowsum, int lane) {
     float am0 = 0.0f, am1 = 0.0f;
@@ -66,7 +70,7 @@ __device__ __forceinline__ void warp_quant(uint32_t (&u)[NV][4], int D, float rs
     }
     // non-negative floats order like their bit patterns
     const float a = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(am0, am1)))), 1e-5f);
-    const float s = __fdiv_rn(127.0f, a);
+    const float s = LEAN ? q127_over(a) : __fdiv_rn(127.0f, a);
     int lsum = 0;
     forget_widened<NV>(u);
     WR_FOREACH(it, c) {
@@ -83,7 +87,7 @@ __device__ __forceinline__ void warp_quant(uint32_t (&u)[NV][4], int D, float rs
     }
     lsum = __reduce_add_sync(0xffffffffu, lsum);
     if (lane == 0) {
-        *dq = __fdiv_rn(a, 127.0f);
+        *dq = LEAN ? over_127(a) : __fdiv_rn(a, 127.0f);
         *rowsum = lsum;
     }
 }
@@ -119,8 +123,8 @@ warp_act_quant_kernel(const T* __restrict__ x, int64_t ld, const float* __restri
             for (int i = 0; i < 4; ++i) sumsq_pair<T>(u[it][i], s0, s1);
         }
         if (m + step < M) fetch(m + step);          // this lane's slots have just been read
-        const float rstd = use_norm ? rstd_from_sumsq(warp_sum(s0 + s1), D, inv_d, eps) : 1.0f;   // v * 1 * 1 is v itself
-        warp_quant<T, NV>(u, D, rstd, sw, q + m * (int64_t)D, dq + m, rowsum + m, lane);
+        const float rstd = use_norm ? rstd_from_sumsq<lean(NV)>(warp_sum(s0 + s1), D, inv_d, eps) : 1.0f;   // v * 1 * 1 is v itself
+        warp_quant<T, NV, lean(NV)>(u, D, rstd, sw, q + m * (int64_t)D, dq + m, rowsum + m, lane);
     }
 }
 
@@ -187,7 +191,7 @@ warp_prenorm_quant_kernel(PrenormArgs a) {
                 if (ro) *reinterpret_cast<uint4*>(ro + c) = make_uint4(o[0], o[1], o[2], o[3]);
             }
         }
-        const float rstd1 = rstd_from_sumsq(warp_sum(s0 + s1), D, inv_d, a.eps_norm);
+        const float rstd1 = rstd_from_sumsq<false>(warp_sum(s0 + s1), D, inv_d, a.eps_norm);
         s0 = s1 = 0.0;
         forget_widened<NV>(u);
         if (!res || a.round_sum_first) {
@@ -219,10 +223,10 @@ warp_prenorm_quant_kernel(PrenormArgs a) {
             WR_FOREACH(it, c) *reinterpret_cast<uint4*>(yo + c) = make_uint4(u[it][0], u[it][1], u[it][2], u[it][3]);
         }
         if (a.G == 0) continue;
-        const float rstd2 = rstd_from_sumsq(warp_sum(s0 + s1), D, inv_d, a.eps_bl);
+        const float rstd2 = rstd_from_sumsq<false>(warp_sum(s0 + s1), D, inv_d, a.eps_bl);
         for (int g = 0; g < a.G; ++g) {
             const int64_t gm = (int64_t)g * a.M + m;
-            warp_quant<T, NV>(u, D, rstd2, sw + (1 + g) * D, a.q + gm * D, a.dq + gm, a.rowsum + gm, lane);
+            warp_quant<T, NV, false>(u, D, rstd2, sw + (1 + g) * D, a.q + gm * D, a.dq + gm, a.rowsum + gm, lane);
         }
     }
 }
@@ -263,7 +267,7 @@ warp_gatenorm_quant_kernel(const T* __restrict__ gx, int64_t ld_g, const T* __re
 #pragma unroll
             for (int i = 0; i < 4; ++i) sumsq_pair<T>(u[it][i], s0, s1);
         }
-        const float rstd1 = rstd_from_sumsq(warp_sum(s0 + s1), D, inv_d, eps_g);
+        const float rstd1 = rstd_from_sumsq<lean(NV)>(warp_sum(s0 + s1), D, inv_d, eps_g);
         s0 = s1 = 0.0;
         forget_widened<NV>(u);
         WR_FOREACH(it, c) {
@@ -280,8 +284,8 @@ warp_gatenorm_quant_kernel(const T* __restrict__ gx, int64_t ld_g, const T* __re
             }
         }
         if (m + step < M) fetch(m + step);            // this lane's slots have been read for the last time
-        const float rstd2 = rstd_from_sumsq(warp_sum(s0 + s1), D, inv_d, eps_bl);
-        warp_quant<T, NV>(u, D, rstd2, sw + D, q + m * (int64_t)D, dq + m, rowsum + m, lane);
+        const float rstd2 = rstd_from_sumsq<lean(NV)>(warp_sum(s0 + s1), D, inv_d, eps_bl);
+        warp_quant<T, NV, lean(NV)>(u, D, rstd2, sw + D, q + m * (int64_t)D, dq + m, rowsum + m, lane);
     }
 }
 

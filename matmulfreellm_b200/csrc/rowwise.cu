@@ -75,7 +75,7 @@ act_quant_kernel(const T* __restrict__ x, int64_t ld_x, const float* __restrict_
     }
     amax = block_max(amax, redf);
     const float a = fmaxf(amax, 1e-5f);
-    const float s = __fdiv_rn(127.0f, a);
+    const float s = q127_over(a);
 
     int lsum = 0;
     int8_t* qr = q + m * (int64_t)K;
@@ -95,7 +95,7 @@ act_quant_kernel(const T* __restrict__ x, int64_t ld_x, const float* __restrict_
     }
     lsum = block_sum(lsum, redi);
     if (threadIdx.x == 0) {
-        dq[m] = __fdiv_rn(a, 127.0f);
+        dq[m] = over_127(a);
         rowsum[m] = lsum;
     }
 }

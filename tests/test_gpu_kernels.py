@@ -93,6 +93,22 @@ def test_act_quant_rows_side_by_side(K, dtype, M, Kdim, use_norm):
     assert np.array_equal(dq.cpu().numpy()[rows], dq_ref) and np.array_equal(rs.cpu().numpy()[rows], rs_ref)
 
 
+@pytest.mark.parametrize("M,Kdim,dtype", [(241, 256, torch.float32), (241, 704, torch.bfloat16), (3133, 2048, torch.bfloat16)])
+def test_act_quant_rows_of_every_magnitude(K, M, Kdim, dtype):
+    """Rows from 2^-120 to 2^120, both sides of where the divisions and the root change their scaling and of where the mean square
+    overflows: the roundings of the IEEE operations, bit for bit."""
+    g = torch.Generator().manual_seed(M)
+    e = torch.arange(M) % 241 - 120
+    x = torch.ldexp(torch.randn(M, Kdim, generator=g).clamp(-4, 4), e[:, None]).to(dtype)
+    for eps, use_norm in [(1e-6, True), (1e-37, True), (1e-6, False)]:
+        q, dq, rs = K.act_quant(dev(x), None, eps, use_norm=use_norm)
+        rows = torch.arange(0, M, 1 if M < 300 else 13)
+        with np.errstate(over="ignore"):
+            q_ref, dq_ref, rs_ref = O.act_codes(x[rows], None, eps, use_norm=use_norm)
+        assert np.array_equal(dq.cpu().numpy()[rows], dq_ref) and np.array_equal(q.cpu().numpy()[rows], q_ref)
+        assert np.array_equal(rs.cpu().numpy()[rows], rs_ref)
+
+
 def test_act_quant_edge_rows(K):
     """Zero row (absmax clamps to 1e-5), a row with one huge outlier, no-norm mode, strided input, M = 0."""
     x = torch.randn(4, 256)
