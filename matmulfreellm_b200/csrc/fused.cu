@@ -726,8 +726,9 @@ extern "C" int mmf_prenorm_quant(const void* x, int64_t ld_x, const void* residu
     a.q = q; a.dq = dq; a.rowsum = rowsum; a.M = M; a.D = (int)D; a.G = groups; a.round_sum_first = round_sum_first;
     // decode-sized call with three projections: one CTA per (row, projection).  The shared statistics are recomputed
     // by each of the three CTAs (same loads, same operations, same results), the three quantisation passes run side by
-    // side: measured 1.5 us -> 0.8 us of prologue after the grid dependency resolves
-    a.gsplit = groups == 3 && M <= 128 ? 1 : 0;
+    // side: measured 1.5 us -> 0.8 us of prologue after the grid dependency resolves.  Up to 64 rows (us whole -> split: 48 rows 2.95 ->
+    // 2.75, 64 equal, 96 3.03 -> 3.21, 128 3.4 -> 5.4: more CTAs than fit beside the next launch's)
+    a.gsplit = groups == 3 && M <= 64 ? 1 : 0;
 #ifdef MMF_EXPERIMENTS
     a.trace = g_row_trace;
 #endif

@@ -46,9 +46,10 @@ struct PrenormArgs {
 #endif
 };
 
-// From this many rows on, rows of 16-bit activations are worked on by one warp each (rowwarp.cu).  Fewer rows leave warps
-// idle: at 1000 rows of 2048 values both forms take the same time (gate norm 6.9 / 6.5 us, three-projection prenorm 10.9 /
-// 11.1), at 2000 rows the warps win (7.7 / 10.3, 11.7 / 17.6), at 300 one CTA per row does (4.1 / 3.2).
+// From this many rows on, rows of 16-bit activations are worked on by one warp each (rowwarp.cu), from 593 on by four where a quarter of
+// the row is long enough (see there, with the times of whole prompt passes).  Fewer rows leave warps idle.  Launched back to back, where a
+// kernel's start hides behind the one before, the warps win earlier (999 rows of 2048 values, us, CTA per row -> one warp: gate norm 7.1 ->
+// 4.6, three-projection prenorm 10.4 -> 7.3), but not between contractions.
 #ifndef MMF_ROW_WARP_MIN_M
 #define MMF_ROW_WARP_MIN_M 1024
 #endif

@@ -626,6 +626,37 @@ def test_fused_row_kernels_many_rows(K, dtype, D):
     check(lambda sl: K.swiglu_quant(gu[sl], bl[2], 1e-6), 1)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [16, 512, 528, 2048, 2064, 4096, 4112])
+def test_row_kernels_of_one_and_four_warps_per_row(K, dtype, D):
+    """593 - 1184 rows of 513 - 4096 values take four warps each, more rows one: the first count, one beside a multiple of the SMs, the last
+    of four and the first of one, against the same rows in calls of at most 200, bit for bit.  Strided rows, with and without a residual,
+    a weight, outputs and projections."""
+    g = torch.Generator().manual_seed(D)
+    wide = [dev((torch.randn(1185, D + 64, generator=g) * 2).to(dtype)) for _ in range(2)]
+    x, res = wide[0][:, :D], wide[1][:, 64:]
+    w = [dev(1.0 + 0.1 * torch.randn(D, generator=g)) for _ in range(4)]
+
+    def check(fn, M, groups=1):
+        whole, parts = fn(slice(0, M)), [fn(slice(i, min(i + 200, M))) for i in range(0, M, 200)]
+        for k, t in enumerate(whole):
+            if t is not None:
+                n = t.shape[0] // M
+                assert torch.equal(t.view(n, M, -1), torch.cat([p[k].view(n, -1, t[0].numel()) for p in parts], 1)), (k, M)
+
+    for M in (593, 741, 1184, 1185):
+        for norm in (True, False):
+            check(lambda sl: K.act_quant(x[sl], w[0] if norm else None, 1e-6, use_norm=norm), M)
+        if D > 4096:
+            continue
+        check(lambda sl: K.gatenorm_quant(x[sl], res[sl], w[0], 1e-6, None, 1e-6), M)
+        for r in (None, res):
+            for first in (False, True):
+                for bl in ([], w[1:2], w[1:]):
+                    check(lambda sl: K.prenorm_quant(x[sl], None if r is None else r[sl], w[0], 1e-6, bl, 1e-6, first, want_residual_out=r is not None,
+                                                     want_y=not bl or first), M)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("D", [512, 704, 2048, 2560])
 def test_fused_row_kernels_four_rows_per_cta(K, dtype, D):
