@@ -667,6 +667,7 @@ int bitlinear_mma_launch(const BitLinearArgs& a, cudaStream_t st) {
     {
         // Many token rows: the persistent kernel (one CTA per SM) once it has a full wave of work, and below that from 129 rows on (a decode
         // batch has at most one token tile here) where it is the faster one by both kernels' estimates, this one's a little low for long K.
+        // The estimates hold from K = 2048 on (a two-block model 256 wide, 600 - 2000 tokens: 5 % slower by them).
         // This kernel / persistent, us: K 2048, N 11264: 130 rows 10.9 / 9.4, 300 18.4 / 13.2, 400 21.7 / 14.3; three projections of 2048: 400
         // rows 12.3 / 10.2; N 2048: 1500 rows 12.5 / 10.1; K 5632: 300 rows 13.9 / 14.6, 600 16.9 / 15.0, 1000 17.5 / 16.1, 1500 20.8 / 16.7.
         // Knob values >= 10 select experimental variant (value - 10) and force it for every M > 128.
@@ -679,7 +680,7 @@ int bitlinear_mma_launch(const BitLinearArgs& a, cudaStream_t st) {
             return bitlinear_mma_prefill_launch(a, st, variant);
         double us = 0.0;
         const bool fits = choose_config(a, p, smem, us);
-        if (choice && a.M > 128 && bitlinear_mma_prefill_us(a) <= 1.05 * us) return bitlinear_mma_prefill_launch(a, st, variant);
+        if (choice && a.M > 128 && a.K >= 2048 && bitlinear_mma_prefill_us(a) <= 1.05 * us) return bitlinear_mma_prefill_launch(a, st, variant);
         MMF_REQUIRE(fits, MMF_ERR_BAD_SHAPE, "mmf_bitlinear(mma): no kernel configuration fits M=%d N=%d K=%d", a.M, a.N, a.K);
     }
     const int m_tiles = (a.M + p.NT - 1) / p.NT;

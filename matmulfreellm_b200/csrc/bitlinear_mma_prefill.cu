@@ -673,7 +673,7 @@ int pf_pick(const BitLinearArgs& a, int variant) {
     // Paired shapes with the stmatrix + TMA-store epilogue: the token tile that takes less time by the estimate above.  (K = 5632, 192 /
     // 256 columns: 1000 rows 16.1 / 17.9 us, 2000 25.9 / 19.4, 3000 27.2 / 31.9, 4096 36.9 / 33.3; K = 6912, 4096 rows 44.5 / 54.1; K = 2048, N =
     // 11264: 200 rows 12.8 / 10.7, 300 13.2 / 15.4.)
-    if (a.K >= 4096 || pf_rounds(a, 192) <= 6) return pf_us(a, 256) < pf_us(a, 192) ? 12 : 10;
+    if (a.K >= 4096 || (a.K >= 2048 && pf_rounds(a, 192) <= 6)) return pf_us(a, 256) < pf_us(a, 192) ? 12 : 10;
     // shorter K and many rounds: 256 columns when their work items fill the 74 CTA pairs' last round clearly better (e.g. N = 2048,
     // M = 16384: 512 items = 6.9 rounds against 688 items = 9.3 rounds)
     auto fill = [&](int nt) {
