@@ -58,6 +58,10 @@ inline DsPlan ds_plan(DsParams& p, int64_t M, int64_t h, int64_t inner, int64_t 
     d.fused = M == 1;
     const int mr = d.fused ? 1 : M <= 8 ? 8 : 16;
     if (!d.fused && 3 * M > sms) return d;
+    // The second exchange and the fill of the codes are not won back by a single block (256 - 1024 wide, 4 rows: 24.7 us as kernels, 26.8
+    // here), nor by two rows of at most 1024 (kernels of their own then repeat the row work: 8 blocks of 1024 126 / 131 us, 24 of 256 340 / 342;
+    // 4 blocks of 2048 86 / 78).
+    if (!d.fused && (layers < 2 || (M == 2 && h <= 1024))) return d;
     d.grid = sms;
     // A thread holds eight columns of a hidden row and three times eight of an inner one.  Eight warps where they suffice: twice or three
     // times as many make no link shorter (they share the issue slots) and leave fewer registers (24 warps: 558 us a step against 329).

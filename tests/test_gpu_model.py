@@ -862,7 +862,7 @@ def test_resident_decode_step_at_the_ends_of_its_range(mm, dtype, hidden, interm
     ref, ref_states = run(33)
     for B in (1, 2, 8, 9, 16):
         taken = _lib.load().mmf_decode_step_workspace_bytes(B, hidden, intermediate, 3) > 0
-        assert taken == (B <= 8 or hidden < 2560), B
+        assert taken == ((B <= 8 or hidden < 2560) and (B != 2 or hidden > 1024)), B
         logits, states = run(B)
         assert torch.equal(logits, ref[:B]), B
         assert all(torch.equal(a, b[:B]) for a, b in zip(states, ref_states)), B
