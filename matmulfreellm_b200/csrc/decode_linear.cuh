@@ -1,5 +1,6 @@
 // BitLinear of a decode step in one kernel: row work before the contraction (prologue), the contraction, and what the next
-// kernel would do first (epilogue).
+// kernel would do first (epilogue).  Steps whose sizes the resident kernel of all blocks takes (decode_step.cuh: 1 row 305 us, 4 rows 443) run
+// there; here run the others, and BitLinear calls of one and two rows.
 //
 // A decode step is a chain of dependent kernels, so its time is the number of links times what a link cannot go below: a
 // kernel boundary (0.9 us with programmatic dependent launch) and a read of the previous kernel's rows across the L2 (0.7 us).
@@ -9,8 +10,8 @@
 //   * for one token row, and for two of at most 2048 values, every CTA repeats the row work that precedes the contraction - norms,
 //     statistics, int8 codes - instead of waiting for a kernel that did it: the row work is latency, and the SMs would idle meanwhile.
 // That leaves four links per block; up to 16 rows, where repeating the row work costs more than a link, it is a kernel of its
-// own that stores the codes in the contraction's operand order (eight links).  Step of a 24-block, 2048-wide model, before and
-// now: 1 row 595 -> 435 us, 2 rows 635 -> 500, 4 rows 735 -> 534, 8 rows 737 -> 530, 16 rows 769 -> 663; 32 blocks of 2560: 1 row
+// own that stores the codes in the contraction's operand order (eight links).  Step of a 24-block, 2048-wide model, eight
+// links of row kernels and tcgen05 contractions -> here: 1 row 595 -> 435 us, 2 rows 635 -> 500, 4 rows 735 -> 534, 8 rows 737 -> 530, 16 rows 769 -> 663; 32 blocks of 2560: 1 row
 // 980 -> 688, 8 rows 1127 -> 831.  What remains is latency.  One row, 2048 wide, a link of 4.3 us on average: 0.85 us from the end
 // of the link before it to its release, 0.8 until the row is there, 0.8 - 1.1 until the last norm's statistic is known (down_proj,
 // which has one norm: 0.35), 0.45 - 0.95 codes, 0.35 - 1.5 products, 0.2 - 0.4 epilogue.  Four rows: row kernel 1.8 us, of which 0.55 is the row's load;

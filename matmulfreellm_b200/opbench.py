@@ -179,7 +179,7 @@ def chain(a):
 def timeline(a):
     """Experiments build: global-timer stamps of CTA 0 of every prenorm_quant launch of one decode step (replayed from
     a CUDA graph): how long after the grid dependency resolves the row is loaded, reduced, normalised and quantised, and
-    how far apart consecutive launches of the chain are.  Up to 16 sequences: the same of every decode_linear launch."""
+    how far apart consecutive launches of the chain are.  Up to 16 sequences: clock stamps of every link of the resident kernel."""
     from . import _lib
     from .engine import GreedyDecoder
     with _lib.experiments_library() as lib:
@@ -245,25 +245,17 @@ def timeline(a):
 
 
 def _decode_links(a, buf):
-    """Medians over the blocks of a step, per link: nanoseconds after the link's grid dependency resolved, and from the release of
-    the link before it to its own."""
-    n = int(buf.view(torch.int32)[0].item())
-    rec = buf[8:8 + 8 * n].view(n, 8).cpu().tolist()
-    names = ["i/f/g", "o_proj", "gate_proj", "down_proj"]
-    per_block = 8 if n >= 8 * a.layers else 4
-    if per_block == 8:
-        names = [f"{x} {part}" for x in names for part in ("rows", "contraction")]
-    stamps = ("row_loaded_ns", "last_statistic_ns", "codes_complete_ns", "products_done_ns", "end_ns")
+    """Medians over the blocks of a step, per link of the resident kernel: SM clocks of CTA 0 from the link's start, and from the link before
+    it to its own start.  (With two and more rows CTA 0 works on row 0's first projection: other links have no row stamps.)"""
+    rec = buf[8:8 + 8 * 4 * a.layers].view(4 * a.layers, 8).cpu().tolist()
+    stamps = ("weights_there", "row_loaded", "first_statistic", "absmax", "codes_complete", "products_done", "end")
     med = lambda v: sorted(v)[len(v) // 2]                                                    # noqa: E731
     links = {}
-    for k, name in enumerate(names):
-        own = list(range(per_block + k, per_block * a.layers, per_block))      # (without the first block)
-        row = {s: med([rec[i][3 + j] - rec[i][2] for i in own]) for j, s in enumerate(stamps) if rec[own[0]][3 + j]}
-        row["start_before_release_ns"] = med([rec[i][2] - rec[i][0] for i in own])
-        row["since_previous_release_ns"] = med([rec[i][2] - rec[i - 1][2] for i in own])
-        row["since_previous_end_ns"] = med([rec[i][2] - rec[i - 1][7] for i in own])
-        links[name] = row
-    print(json.dumps({"op": "timeline", "batch": a.batch, "layers": a.layers, "launches": n, "links": links}))
+    for k, name in enumerate(("i/f/g", "o_proj", "gate_proj", "down_proj")):
+        own = list(range(4 + k, 4 * a.layers, 4))                              # (without the first block)
+        links[name] = {s: med([rec[i][1 + j] - rec[i][0] for i in own]) for j, s in enumerate(stamps) if rec[own[0]][1 + j]}
+        links[name]["since_previous_start"] = med([rec[i][0] - rec[i - 1][0] for i in own])
+    print(json.dumps({"op": "timeline", "batch": a.batch, "layers": a.layers, "unit": "clocks", "links": links}))
 
 
 def int8peak(a):
