@@ -680,7 +680,7 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 a.workspace = b + step; a.workspace_bytes = step_bytes;
                 a.status = static_cast<int*>(ws.p);
                 MMF_CALL(mmf_decode_step, &a, st);
-                ++launches;
+                launches += 2;                    // fill, blocks
                 advance();
             } else if (decode) decode_blocks(c, args_of, run, gather, b + z, b + ifg, b + o, b + gu, mk, states, x, next, advance);
             for (size_t i = 0; i < c.layers.size() && !decode; ++i) {
