@@ -349,8 +349,11 @@ int wr_launch(size_t weight_bytes, size_t row_bytes, int64_t M, cudaStream_t st,
     int64_t rows = fit < wr_max_warps(W) / W ? fit : wr_max_warps(W) / W;
     if (share < rows) rows = share;
     MMF_REQUIRE(rows >= 1, MMF_ERR_CUDA, "%s: a row of this length does not fit in shared memory", name);
-    MMF_CUDA(mmf_launch_pdl(kernel, dim3((unsigned)(M < 148 ? M : 148)), dim3((unsigned)rows * 32 * W), weight_bytes + (size_t)rows * row_bytes,
-                            st, args...));
+    size_t smem = weight_bytes + (size_t)rows * row_bytes;
+    // Short rows leave registers and shared memory for two CTAs, and an SM that the kernel before leaves early would be given two while
+    // others get none (12000 rows of 256 values to 1408 outputs 27.4 us, 24.9 with one): more than half of the shared memory each.
+    if (share > rows && smem < WR_SMEM_MAX / 2 + 4096) smem = WR_SMEM_MAX / 2 + 4096;
+    MMF_CUDA(mmf_launch_pdl(kernel, dim3((unsigned)(M < 148 ? M : 148)), dim3((unsigned)rows * 32 * W), smem, st, args...));
     MMF_LAUNCH_CHECK(name);
     return MMF_OK;
 }
