@@ -6,6 +6,10 @@
 int decode_step_bf16(const DsParams& p, const DsPlan& d, cudaStream_t st);
 int decode_step_fp16(const DsParams& p, const DsPlan& d, cudaStream_t st);
 
+#ifdef MMF_EXPERIMENTS
+int g_step_wait_limit = 0;     // mmf_tuning(MMF_TUNE_STEP_WAIT_LIMIT, polls)
+#endif
+
 namespace {
 
 struct PackParams {
@@ -131,6 +135,7 @@ extern "C" int mmf_decode_step(const mmf_decode_step_args* args, void* stream) {
     p.eps_norm = a.eps_norm;
 #ifdef MMF_EXPERIMENTS
     p.trace = g_row_trace;
+    p.wait_limit = g_step_wait_limit ? g_step_wait_limit : DS_WAIT_LIMIT;
 #endif
     const cudaStream_t st = (cudaStream_t)stream;
     const int64_t fill_rows = a.layers * p.rows_layer / 16, fill = fill_rows + a.layers * p.codes_layer / 16;

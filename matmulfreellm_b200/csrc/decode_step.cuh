@@ -49,16 +49,19 @@ __device__ __forceinline__ void ds_st(void* p, uint2 v) {
 __device__ __forceinline__ bool ds_there(uint4 v, uint32_t none) { return v.x != none && v.y != none && v.z != none && v.w != none; }
 __device__ __forceinline__ uint32_t ds_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// A thread's side of the bounded waits.  One that runs out sets the status word; the others see it and stop waiting too.
+// A thread's side of the bounded waits.  One that runs out sets the status word; the others see it and stop waiting for rows and codes
+// too.  For its own bulk copies (`barrier`) a CTA waits all the same, whatever other CTAs do: none is under way when it ends, and a
+// region is not read or filled again before its copy is complete.
 struct DsWait {
     int* status;
+    int limit;                                         // polls (DS_WAIT_LIMIT; the experiments build can set less)
     bool dead = false;
     __device__ __forceinline__ bool again(int& n) {    // another poll?
         if (dead) return false;
-        if ((++n & 4095) == 0) {
+        if ((++n & 4095) == 0 || n >= limit) {
             int s;
             asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(s) : "l"(status) : "memory");
-            if (s || n >= DS_WAIT_LIMIT) {
+            if (s || n >= limit) {
                 *status = 1;
                 dead = true;
                 return false;
@@ -72,7 +75,11 @@ struct DsWait {
         do {
             asm volatile("{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\tselp.b32 %0, 1, 0, P1;\n\t}"
                          : "=r"(done) : "r"(bar), "r"((uint32_t)parity) : "memory");
-        } while (!done && again(n));
+        } while (!done && ++n < DS_WAIT_LIMIT);
+        if (!done) {
+            *status = 1;
+            dead = true;
+        }
     }
 };
 __device__ __forceinline__ void ds_expect(uint32_t bar, uint32_t bytes) {
@@ -201,7 +208,11 @@ decode_step_kernel(const __grid_constant__ DsParams p) {
     // not FUSED: the CTAs of a row take turns with the links of one projection
     auto mine = [&](int type) { return FUSED || (has_row && (type == DS_IFG || row_g == (type == DS_O ? 1 : type == DS_GATE ? 0 : 2))); };
     const uint32_t bars = ds_smem(s_bar);
-    DsWait wait{p.status};
+#ifdef MMF_EXPERIMENTS
+    DsWait wait{p.status, p.wait_limit};
+#else
+    DsWait wait{p.status, DS_WAIT_LIMIT};
+#endif
 
     // one thread: weights of link idx into its region, norm weights into the region of even / odd links
     auto fetch = [&](int idx) {

@@ -39,6 +39,7 @@ struct DsParams {
     float eps_norm;
 #ifdef MMF_EXPERIMENTS
     long long* trace;
+    int wait_limit;
 #endif
 };
 

@@ -882,3 +882,36 @@ def test_bitlinear_of_one_and_two_rows_equals_more_rows(mm, dtype, K, N):
     for rows in (x[:1], x[:2], x[::7][:2]):
         pick = ref[:rows.shape[0]] if rows.stride(0) == K or rows.shape[0] == 1 else ref[::7][:2]
         assert torch.equal(layer(rows), pick)
+
+
+def test_resident_decode_step_whose_waits_give_up(mm):
+    """A step whose waits run out ends by itself, sets the status word and leaves the GPU usable: with a limit of one poll every wait that does
+    not find its words at once gives up (with several rows most CTAs look for codes long before they are made)."""
+    from matmulfreellm_b200 import _lib
+    cfg = tiny_cfg()
+    model = build_gpu_model(O.random_weights(cfg, seed=4), cfg, torch.bfloat16)
+    for B in (1, 5, 16):
+        prompt, ids = torch.randint(0, 32000, (B, 7), device="cuda"), torch.randint(0, 32000, (B, 1), device="cuda")
+
+        def step():
+            past = model(prompt, use_cache=True).past_key_values
+            torch.cuda.synchronize()
+            with _lib.experiments_library() as lib:
+                lib.mmf_tuning(13, limit)
+                out = model(input_ids=ids, past_key_values=past, use_cache=True)
+                torch.cuda.synchronize()
+            return out.logits
+
+        limit = 0
+        want = step()
+        mm.kernels.check_status()
+        limit = 1
+        step()
+        if B > 1:
+            with pytest.raises(_lib.MMFreeError, match="MMF_ERR_TIMEOUT"):
+                mm.kernels.check_status()
+        else:                                   # (one sequence's words may all be there at the first look)
+            mm.kernels._rezero_workspaces()
+        limit = 0
+        assert torch.equal(step(), want)
+        mm.kernels.check_status()
