@@ -29,7 +29,7 @@
 extern "C" {
 #endif
 
-#define MMF_ABI_VERSION 2
+#define MMF_ABI_VERSION 3
 
 /* element types of activation tensors */
 #define MMF_F32 0
@@ -381,7 +381,9 @@ typedef struct {
     void* residual_out;                     /* ... and the residual stream it is to be added to */
     void* workspace;                        /* mmf_decode_step_workspace_bytes() bytes, 256-byte aligned; any contents */
     int64_t workspace_bytes;
-    int* status;                            /* device word, set to 1 if a bounded wait gave up (outputs are then undefined) */
+    int* status;                            /* device word, set to 1 if a bounded wait gave up (outputs and states are then undefined) */
+    int* gave_up_host;                      /* HOST word in mapped pinned memory, set to 1 then as well, so that a host can tell without
+                                             * synchronising; or NULL */
 } mmf_decode_step_args;
 
 /* 0: the sizes are not taken on the current device. */

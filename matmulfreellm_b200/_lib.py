@@ -17,9 +17,9 @@ KERNEL_STREAM = 3   # Python-level selector: the mma.sync decode experiment (mmf
 STREAM_MAX_M = 64
 TILE_ROWS, TILE_K = 128, 64
 ABSMEAN_PARTIALS = 1024
-ABI_VERSION = 2
+ABI_VERSION = 3
 
-ERR_CUDA = -4
+ERR_CUDA, ERR_TIMEOUT = -4, -7
 _ERR_NAMES = {
     -1: "MMF_ERR_BAD_ARG", -2: "MMF_ERR_BAD_SHAPE", -3: "MMF_ERR_ALIGN", -4: "MMF_ERR_CUDA",
     -5: "MMF_ERR_ARCH", -6: "MMF_ERR_WORKSPACE", -7: "MMF_ERR_TIMEOUT",
@@ -45,7 +45,7 @@ class DecodeStepArgs(ctypes.Structure):
     _fields_ = [("dtype", c_int), ("M", c_int64), ("hidden", c_int64), ("inner", c_int64), ("layers", c_int64),
                 ("layer", ctypes.POINTER(DecodeStepLayer)), ("x", c_void_p), ("ld_x", c_int64), ("row_ids", c_void_p), ("x_rows", c_int64),
                 ("mask", c_void_p), ("eps_norm", c_float), ("out", c_void_p), ("residual_out", c_void_p), ("workspace", c_void_p),
-                ("workspace_bytes", c_int64), ("status", c_void_p)]
+                ("workspace_bytes", c_int64), ("status", c_void_p), ("gave_up_host", c_void_p)]
 
 
 PRO_QUANT, PRO_PRENORM, PRO_GATENORM = 1, 2, 3

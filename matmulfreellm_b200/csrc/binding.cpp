@@ -12,12 +12,14 @@
 //   take_launches()                      kernels launched since the last call of it
 //   bitlinear(x, norm_w, packed, scale, N, eps)       RMSNorm + int8 quantisation + contraction, [..., K] -> [..., N]
 //   hgrn_scan(x, g, h0 | None, want_state, gate_is_log, state_dtype)      -> (o, final state | None)
+//   check_gave_up(device_index), take_gave_up()       raise if a decode step gave up waiting; forget that any did
 //   watch(slots), unchanged(watch)       cheap "has any parameter been replaced, cast or modified" over (dict, name) slots
 //   chain(...), chain_forward(...)       the fused forward of a model (engine.FusedRunner)
 #include <Python.h>
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -156,6 +158,28 @@ Ws workspace(int dev, void* stream) {
     Py_DECREF(o);
     g_ws.push_back(Ws{dev, stream, t.data_ptr(), t.numel()});
     return g_ws.back();
+}
+
+// One word of pinned host memory per device, which a decode step sets when it gives up waiting (mmf_decode_step_args.gave_up_host).  Never
+// released: a captured graph may point at it.
+int* g_gave_up[64];       // made under the GIL
+void make_gave_up_word(int dev) {
+    if (dev >= 64 || g_gave_up[dev]) return;
+    const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);      // (allocating is no part of a capture under way)
+    static std::vector<at::Tensor> keep;
+    keep.push_back(at::zeros({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true)));
+    g_gave_up[dev] = keep.back().data_ptr<int>();
+}
+bool take_gave_up_word(int dev) {
+    volatile int* w = dev >= 0 && dev < 64 ? g_gave_up[dev] : nullptr;
+    const bool set = w && *w;
+    if (set) *w = 0;
+    return set;
+}
+void require_not_given_up(int dev) {
+    if (take_gave_up_word(dev))
+        throw MmfStatus{"mmf_decode_step", MMF_ERR_TIMEOUT, "an earlier decode step on cuda:" + std::to_string(dev) +
+                        " gave up waiting: its outputs and the recurrent states are undefined"};
 }
 
 // carve 256-byte aligned pieces out of one allocation
@@ -457,6 +481,7 @@ void lay_out_step(Chain& c) {
         L.step = mem.data_ptr();
         c.keep.push_back(mem);
     }
+    make_gave_up_word(c.table.get_device());
     c.step_ok = true;
 }
 // chain(table, layers, final_norm_w, head(5 fields), head_nw, eps, head_eps): layers is a list of tuples in the order read below
@@ -569,6 +594,7 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
         const at::Tensor& src = ids.defined() ? ids : emb;
         if (!src.defined() || src.dim() != (ids.defined() ? 2 : 3)) throw std::invalid_argument("input_ids [B, T] or inputs_embeds [B, T, h] expected");
         const int dev = need_cuda({&c.table, &src, &mask});
+        require_not_given_up(dev);
         const int64_t B = src.size(0), T = src.size(1), M = B * T, h = c.h;
         const int64_t es = c.dtype == MMF_F32 ? 4 : 2;
         if (ids.defined()) ids = ids.to(at::kLong).contiguous();
@@ -679,6 +705,7 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 a.out = b + z; a.residual_out = next;
                 a.workspace = b + step; a.workspace_bytes = step_bytes;
                 a.status = static_cast<int*>(ws.p);
+                a.gave_up_host = dev < 64 ? g_gave_up[dev] : nullptr;
                 MMF_CALL(mmf_decode_step, &a, st);
                 launches += 2;                    // fill, blocks
                 advance();
@@ -747,7 +774,23 @@ PyObject* take_launches(PyObject*, PyObject*) {
     return PyLong_FromLongLong(n);
 }
 
+// check_gave_up(device index): raises if a decode step there gave up waiting since the last look; take_gave_up(): forget all of them
+PyObject* check_gave_up(PyObject*, PyObject* index) {
+    return guarded([&]() -> PyObject* {
+        const long dev = PyLong_AsLong(index);
+        if (dev == -1 && PyErr_Occurred()) return nullptr;
+        require_not_given_up((int)dev);
+        Py_RETURN_NONE;
+    });
+}
+PyObject* take_gave_up(PyObject*, PyObject*) {
+    for (int dev = 0; dev < 64; ++dev) take_gave_up_word(dev);
+    Py_RETURN_NONE;
+}
+
 PyMethodDef methods[] = {
+    {"check_gave_up", check_gave_up, METH_O, nullptr},
+    {"take_gave_up", take_gave_up, METH_NOARGS, nullptr},
     {"take_launches", take_launches, METH_NOARGS, nullptr},
     {"use_library", use_library, METH_O, nullptr},
     {"set_hooks", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(set_hooks)), METH_FASTCALL, nullptr},

@@ -130,6 +130,7 @@ extern "C" int mmf_decode_step(const mmf_decode_step_args* args, void* stream) {
     p.mask = a.mask;
     p.out = a.out; p.residual_out = a.residual_out;
     p.status = a.status;
+    p.gave_up = a.gave_up_host;
     p.rows = (uint8_t*)a.workspace;
     p.codes = p.rows + a.layers * p.rows_layer;
     p.eps_norm = a.eps_norm;

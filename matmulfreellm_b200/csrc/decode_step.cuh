@@ -53,17 +53,25 @@ __device__ __forceinline__ uint32_t ds_smem(const void* p) { return (uint32_t)__
 // too.  For its own bulk copies (`barrier`) a CTA waits all the same, whatever other CTAs do: none is under way when it ends, and a
 // region is not read or filled again before its copy is complete.
 struct DsWait {
-    int* status;
-    int limit;                                         // polls (DS_WAIT_LIMIT; the experiments build can set less)
+    const DsParams& p;
     bool dead = false;
+#ifdef MMF_EXPERIMENTS
+    __device__ __forceinline__ int limit() const { return p.wait_limit; }
+#else
+    __device__ __forceinline__ int limit() const { return DS_WAIT_LIMIT; }
+#endif
+    __device__ __forceinline__ void give_up() {        // the host's word too: it is read without synchronising
+        *p.status = 1;
+        if (p.gave_up) asm volatile("st.relaxed.sys.global.b32 [%0], %1;" ::"l"(p.gave_up), "r"(1) : "memory");
+        dead = true;
+    }
     __device__ __forceinline__ bool again(int& n) {    // another poll?
         if (dead) return false;
-        if ((++n & 4095) == 0 || n >= limit) {
+        if ((++n & 4095) == 0 || n >= limit()) {
             int s;
-            asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(s) : "l"(status) : "memory");
-            if (s || n >= limit) {
-                *status = 1;
-                dead = true;
+            asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(s) : "l"(p.status) : "memory");
+            if (s || n >= limit()) {
+                give_up();
                 return false;
             }
         }
@@ -76,10 +84,7 @@ struct DsWait {
             asm volatile("{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\tselp.b32 %0, 1, 0, P1;\n\t}"
                          : "=r"(done) : "r"(bar), "r"((uint32_t)parity) : "memory");
         } while (!done && ++n < DS_WAIT_LIMIT);
-        if (!done) {
-            *status = 1;
-            dead = true;
-        }
+        if (!done) give_up();
     }
 };
 __device__ __forceinline__ void ds_expect(uint32_t bar, uint32_t bytes) {
@@ -208,11 +213,7 @@ decode_step_kernel(const __grid_constant__ DsParams p) {
     // not FUSED: the CTAs of a row take turns with the links of one projection
     auto mine = [&](int type) { return FUSED || (has_row && (type == DS_IFG || row_g == (type == DS_O ? 1 : type == DS_GATE ? 0 : 2))); };
     const uint32_t bars = ds_smem(s_bar);
-#ifdef MMF_EXPERIMENTS
-    DsWait wait{p.status, p.wait_limit};
-#else
-    DsWait wait{p.status, DS_WAIT_LIMIT};
-#endif
+    DsWait wait{p};
 
     // one thread: weights of link idx into its region, norm weights into the region of even / odd links
     auto fetch = [&](int idx) {

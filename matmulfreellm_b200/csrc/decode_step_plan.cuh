@@ -29,7 +29,7 @@ struct DsParams {
     const void* x; int64_t ld_x; const int64_t* row_ids; int64_t x_rows;
     const uint8_t* mask;
     void *out, *residual_out;
-    int* status;
+    int *status, *gave_up;
     uint8_t* rows;                               // exchanged rows, [layer]: o, g, attention output, MLP output [M][h], act [M][inner]
     uint8_t* codes;                              // exchanged codes and their scales, [layer]
     int64_t rows_layer, codes_layer;             // bytes per layer

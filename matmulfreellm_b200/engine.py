@@ -155,6 +155,7 @@ class GreedyDecoder:
             self.last_logits = self._step_eager()
             self.kernels_per_step = _lib.launch_count - before
         else:
+            kernels.raise_if_gave_up(self.device)
             if self.graph is None:
                 self.graph, self._graph_logits, self._graph_reads = self._capture()
             self.graph.replay()
@@ -177,6 +178,7 @@ class GreedyDecoder:
             self.step()
             out_host.copy_(self.next, non_blocking=True)
             return
+        kernels.raise_if_gave_up(self.device)
         key = (ids_host.data_ptr(), out_host.data_ptr())
         entry = self._host_graphs.get(key)
         if entry is None:

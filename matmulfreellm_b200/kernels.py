@@ -205,12 +205,22 @@ def _rezero_workspaces() -> None:
 
 def _after_failure(e: _lib.MMFreeError) -> None:
     """After a native call failed: clear the workspaces unless its arguments were refused, when nothing was launched."""
-    if e.code == _lib.ERR_CUDA:
+    if e.code in (_lib.ERR_CUDA, _lib.ERR_TIMEOUT):
         _rezero_workspaces()
 
 
+def raise_if_gave_up(device: torch.device) -> None:
+    """Raise if a decode step that ran on `device` gave up waiting (its outputs and the recurrent states are then undefined).  Reads a word
+    that such a step sets in host memory: no synchronisation, and a step still under way is not waited for.  Forwards check it themselves."""
+    try:
+        _lib.native().check_gave_up(device.index)
+    except _lib.MMFreeError as e:
+        _after_failure(e)
+        raise
+
+
 def check_status() -> None:
-    """Synchronise and raise if any BitLinear kernel reported a device-side wait that gave up (status word
+    """Synchronise and raise if any BitLinear kernel or decode step reported a device-side wait that gave up (status word
     at the start of the split-K workspace).  Costs a device sync; meant for tests and debugging."""
     failed = ctypes.c_int(0)
     _lib.call("mmf_hgrn_status", ctypes.addressof(failed))
@@ -221,6 +231,7 @@ def check_status() -> None:
         status = int(ws[:4].view(torch.int32).item())
         if status != 0:
             _rezero_workspaces()
+            _lib.native().take_gave_up()
             raise _lib.MMFreeError("mmf_bitlinear", -7, f"device-side wait timed out (status word {status})")
 
 

@@ -313,6 +313,7 @@ class HGRNBitForCausalLM(HGRNBitPreTrainedModel):
             if bool(hit.any(dim=1).all()):                  # the step loop stops once the last sequence emits eos
                 first = torch.where(hit, torch.arange(n, device=toks.device).expand_as(hit), n).min(dim=1).values
                 toks = toks[:, : int(first.max().item()) + 1]
+        kernels.raise_if_gave_up(input_ids.device)          # (what has arrived: this call need not have synchronised)
         return torch.cat([input_ids, toks], dim=1)
 
     # -- fused execution -------------------------------------------------------------------------------------

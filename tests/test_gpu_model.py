@@ -912,6 +912,35 @@ def test_resident_decode_step_whose_waits_give_up(mm):
                 mm.kernels.check_status()
         else:                                   # (one sequence's words may all be there at the first look)
             mm.kernels._rezero_workspaces()
+            _lib.native().take_gave_up()
         limit = 0
         assert torch.equal(step(), want)
+        mm.kernels.check_status()
+
+
+def test_step_that_gave_up_is_reported_by_the_next_call(mm):
+    """Without anyone asking for the status word: a forward, a decoder's step (eager and replayed) and `generate` raise once a step of that
+    device has given up, and work again afterwards."""
+    from matmulfreellm_b200 import _lib
+    from matmulfreellm_b200.engine import GreedyDecoder
+    cfg = tiny_cfg()
+    model = build_gpu_model(O.random_weights(cfg, seed=4), cfg, torch.bfloat16)
+    prompt = torch.randint(0, 32000, (5, 7), device="cuda")
+    host = torch.zeros(5, 1, dtype=torch.int64).pin_memory(), torch.zeros(5, dtype=torch.int64).pin_memory()
+    eager, graph = GreedyDecoder(model, 5, use_graph=False), GreedyDecoder(model, 5)
+    calls = {"forward": lambda: model(prompt[:1, :1]), "prompt": lambda: model(prompt), "decoder": eager.step, "graph": graph.step,
+             "host buffers": lambda: graph.step_host(*host), "generate": lambda: model.generate(prompt, max_new_tokens=4)}
+    for call in calls.values():
+        call()
+    for name, call in calls.items():
+        past = model(prompt, use_cache=True).past_key_values
+        with _lib.experiments_library() as lib:
+            lib.mmf_tuning(13, 1)
+            model(input_ids=prompt[:, :1], past_key_values=past, use_cache=True)
+            torch.cuda.synchronize()
+        with pytest.raises(_lib.MMFreeError, match="mmf_decode_step failed with MMF_ERR_TIMEOUT"):
+            call()
+        assert all(not ws[:4].any() for ws in mm.kernels._ws_cache.values()), name
+        call()
+        torch.cuda.synchronize()
         mm.kernels.check_status()

@@ -86,3 +86,30 @@ def test_replaced_norm_weight_is_noticed_where_memory_is_reused():
         lin.norm.weight.add_(1)
     assert torch.equal(lin.norm_weight_f32(), lin.norm.weight.float())
     assert lin.norm_weight_f32() is lin.norm_weight_f32()
+
+
+def test_a_step_that_gave_up_clears_the_workspaces(monkeypatch):
+    """The report that a step gave up waiting clears its status word, wherever it is raised; no step has given up here, so the real look at
+    the words raises nothing."""
+    from matmulfreellm_b200.engine import FusedRunner
+    for index in (0, 63, 64, -1):
+        _lib.native().check_gave_up(index)
+    _lib.native().take_gave_up()
+
+    class GaveUp:
+        def check_gave_up(self, *args):
+            raise _lib.MMFreeError("mmf_decode_step", _lib.ERR_TIMEOUT, "gave up")
+
+        chain_forward = check_gave_up
+
+    cleared = []
+    monkeypatch.setattr(kernels, "_rezero_workspaces", lambda: cleared.append(1))
+    monkeypatch.setattr(_lib, "native", GaveUp)
+    with pytest.raises(_lib.MMFreeError, match="MMF_ERR_TIMEOUT"):
+        kernels.raise_if_gave_up(torch.device("cuda", 0))
+    assert len(cleared) == 1
+    runner = object.__new__(FusedRunner)
+    runner._native, runner.chain, runner.device = GaveUp(), None, torch.device("cpu")
+    with pytest.raises(_lib.MMFreeError, match="MMF_ERR_TIMEOUT"):
+        runner.forward(None, None, [], False)
+    assert len(cleared) == 2
