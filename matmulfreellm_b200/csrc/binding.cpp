@@ -14,7 +14,7 @@
 //   hgrn_scan(x, g, h0 | None, want_state, gate_is_log, state_dtype)      -> (o, final state | None)
 //   check_gave_up(device_index), take_gave_up()       raise if a decode step gave up waiting; forget that any did
 //   watch(slots), unchanged(watch)       cheap "has any parameter been replaced, cast or modified" over (dict, name) slots
-//   chain(...), chain_forward(...)       the fused forward of a model (engine.FusedRunner)
+//   chain(...), chain_forward(...), prepare_step(...)     the fused forward of a model (engine.FusedRunner)
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -25,7 +25,9 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Dtype.h>
 
+#include <atomic>
 #include <map>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -162,16 +164,18 @@ Ws workspace(int dev, void* stream) {
 
 // One word of pinned host memory per device, which a decode step sets when it gives up waiting (mmf_decode_step_args.gave_up_host).  Never
 // released: a captured graph may point at it.
-int* g_gave_up[64];       // made under the GIL
+std::atomic<int*> g_gave_up[64];
 void make_gave_up_word(int dev) {
-    if (dev >= 64 || g_gave_up[dev]) return;
+    static std::mutex lock;
+    const std::lock_guard<std::mutex> hold(lock);
+    if (dev >= 64 || g_gave_up[dev].load()) return;
     const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);      // (allocating is no part of a capture under way)
     static std::vector<at::Tensor> keep;
     keep.push_back(at::zeros({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true)));
     g_gave_up[dev] = keep.back().data_ptr<int>();
 }
 bool take_gave_up_word(int dev) {
-    volatile int* w = dev >= 0 && dev < 64 ? g_gave_up[dev] : nullptr;
+    volatile int* w = dev >= 0 && dev < 64 ? g_gave_up[dev].load() : nullptr;
     const bool set = w && *w;
     if (set) *w = 0;
     return set;
@@ -419,9 +423,10 @@ struct Layer {
     const float *attn_norm_w, *ifg_nw[3], *gnorm_w, *o_nw, *mlp_norm_w, *gate_nw, *down_nw;
     Linear ifg, o, gate, down;
     const void* lb;
-    const void* step = nullptr;        // weights, norm weights and scales as the resident decode step reads them
+    const void* step = nullptr;        // weights, norm weights and scales as the resident decode step reads them (see step_ready)
     float gnorm_eps, eps_bl;
 };
+enum { STEP_OPEN, STEP_READY, STEP_NEVER };
 struct Chain {
     std::vector<Layer> layers;
     std::vector<at::Tensor> keep;      // everything the raw pointers above point into
@@ -429,7 +434,8 @@ struct Chain {
     const float *final_norm_w, *head_nw;
     Linear head;
     int64_t h = 0, inner = 0;
-    bool step_ok = false;              // the blocks' weights are laid out for the resident decode step as well
+    std::atomic<int> step{STEP_OPEN};  // are the blocks' weights laid out for the resident decode step as well?
+    std::mutex step_lock;              // held by the thread that does it
     float eps = 0, head_eps = 0;
     int dtype = 0;
 };
@@ -464,30 +470,49 @@ struct Fields {      // positional reader of a Python tuple
         return l;
     }
 };
-// The blocks' weights once more, in the layout of the resident decode step, if it takes the model (16-bit, on the current device, all
-// MLPs as wide): as many bytes again as the blocks' packed weights.
-void lay_out_step(Chain& c) {
-    if (c.dtype == MMF_F32 || c.layers.empty() || !c.table.is_cuda() || c.table.get_device() != c10::cuda::current_device()) return;
-    for (const Layer& L : c.layers)
-        if (L.down.K != c.inner) return;
-    const int64_t bytes = g_api->mmf_decode_step_layer_bytes(c.h, c.inner);
-    if (!bytes || !g_api->mmf_decode_step_workspace_bytes(1, c.h, c.inner, (int64_t)c.layers.size())) return;
-    void* st = c10::cuda::getCurrentCUDAStream(c.table.get_device()).stream();
+// The blocks' weights once more, in the layout of the resident decode step: as many bytes again as the blocks' packed weights, so only once
+// a step wants them (a model that never decodes up to 16 sequences holds none), in one allocation.  True: they are there.  Called without the
+// GIL, by several threads at once.  Made on the caller's stream and complete before any other stream can use them; not while that stream is
+// captured (the memory would be the graph's and the packing a part of it), and not again once memory was refused: the chain of kernels needs
+// none of it.
+bool step_ready(Chain& c, int dev) {
+    int s = c.step.load(std::memory_order_acquire);
+    if (s != STEP_OPEN) return s == STEP_READY;
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return false;
+    const std::lock_guard<std::mutex> lock(c.step_lock);
+    if ((s = c.step.load(std::memory_order_acquire)) != STEP_OPEN) return s == STEP_READY;
+    const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(dev);
+    const int64_t bytes = (g_api->mmf_decode_step_layer_bytes(c.h, c.inner) + 255) / 256 * 256;
+    at::Tensor mem;
+    try {
+        mem = at::empty({bytes * (int64_t)c.layers.size()}, c.table.options().dtype(at::kByte));
+    } catch (const c10::OutOfMemoryError&) {
+        c.step.store(STEP_NEVER, std::memory_order_release);
+        return false;
+    }
+    make_gave_up_word(dev);
+    uint8_t* at = mem.data_ptr<uint8_t>();
     for (Layer& L : c.layers) {
-        const at::Tensor mem = at::empty({bytes}, c.table.options().dtype(at::kByte));
         const mmf_decode_step_weights w = {L.attn_norm_w, {L.ifg_nw[0], L.ifg_nw[1], L.ifg_nw[2]}, L.gnorm_w, L.o_nw, L.mlp_norm_w, L.gate_nw, L.down_nw,
                                            L.ifg.packed, L.o.packed, L.gate.packed, L.down.packed, L.ifg.scale, L.o.scale, L.gate.scale, L.down.scale};
-        MMF_CALL(mmf_decode_step_pack, &w, c.h, c.inner, mem.data_ptr(), st);
-        L.step = mem.data_ptr();
-        c.keep.push_back(mem);
+        MMF_CALL(mmf_decode_step_pack, &w, c.h, c.inner, at, stream.stream());
+        L.step = at;
+        at += bytes;
     }
-    make_gave_up_word(c.table.get_device());
-    c.step_ok = true;
+    stream.synchronize();
+    c.keep.push_back(mem);
+    c.step.store(STEP_READY, std::memory_order_release);
+    return true;
 }
-// chain(table, layers, final_norm_w, head(5 fields), head_nw, eps, head_eps): layers is a list of tuples in the order read below
+// scratch of the resident decode step for M rows, 0: this chain or these sizes do not take it
+int64_t step_workspace(const Chain& c, int64_t M) {
+    return c.step.load(std::memory_order_relaxed) == STEP_NEVER ? 0 : g_api->mmf_decode_step_workspace_bytes(M, c.h, c.inner, (int64_t)c.layers.size());
+}
+// chain(table, layers, (final_norm_w, head (5 fields), head_nw, eps, head_eps), resident): layers is a list of tuples in the order read
+// below; resident: decode steps may use the resident kernel, which takes a second copy of the blocks' weights
 PyObject* chain(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
-        if (n != 3 || !PyList_Check(args[1]) || !PyTuple_Check(args[2])) throw std::domain_error("chain(table, layers, tail)");
+        if (n != 4 || !PyList_Check(args[1]) || !PyTuple_Check(args[2])) throw std::domain_error("chain(table, layers, tail, resident)");
         auto c = std::make_unique<Chain>();
         c->table = tensor(args[0], "table").detach().contiguous();
         c->h = c->table.size(1);
@@ -515,7 +540,9 @@ PyObject* chain(PyObject*, PyObject* const* args, Py_ssize_t n) {
             c->inner = std::max(c->inner, L.down.K);
             c->layers.push_back(L);
         }
-        lay_out_step(*c);
+        bool resident = PyObject_IsTrue(args[3]) && c->dtype != MMF_F32 && !c->layers.empty();
+        for (const Layer& L : c->layers) resident = resident && L.down.K == c->inner;       // (its MLPs are all as wide)
+        if (!resident) c->step = STEP_NEVER;
         Fields f{args[2], *c};
         c->final_norm_w = f.f32();
         c->head = f.linear();
@@ -587,7 +614,7 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (n != 8) throw std::domain_error("chain_forward takes 8 arguments");
         auto* cp = static_cast<Chain*>(PyCapsule_GetPointer(args[0], "mmf.chain"));
         if (!cp) return nullptr;
-        const Chain& c = *cp;
+        Chain& c = *cp;
         at::Tensor ids = maybe_tensor(args[1], "input_ids"), emb = maybe_tensor(args[2], "inputs_embeds");
         at::Tensor mask = maybe_tensor(args[4], "attention_mask");
         const bool last_only = PyObject_IsTrue(args[5]), want_logits = PyObject_IsTrue(args[6]), want_hidden = PyObject_IsTrue(args[7]);
@@ -640,7 +667,8 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                           (ids.defined() || on16(emb.data_ptr()));
             for (const float* s : states) decode = decode && on16(s);
             // ... and all blocks in one where they fit on the chip's shared memory
-            const int64_t step_bytes = decode && c.step_ok ? g_api->mmf_decode_step_workspace_bytes(M, h, c.inner, (int64_t)c.layers.size()) : 0;
+            int64_t step_bytes = decode ? step_workspace(c, M) : 0;
+            if (step_bytes && !step_ready(c, dev)) step_bytes = 0;
             const int64_t step = s.take(step_bytes);
             const int64_t hg_bytes = T > 1 ? g_api->mmf_hgrn_workspace_bytes(B, T, h) : 0, hg = s.take(hg_bytes);
             const at::Tensor mem = at::empty({s.used}, opt.dtype(at::kByte));
@@ -705,7 +733,7 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 a.out = b + z; a.residual_out = next;
                 a.workspace = b + step; a.workspace_bytes = step_bytes;
                 a.status = static_cast<int*>(ws.p);
-                a.gave_up_host = dev < 64 ? g_gave_up[dev] : nullptr;
+                a.gave_up_host = dev < 64 ? g_gave_up[dev].load() : nullptr;
                 MMF_CALL(mmf_decode_step, &a, st);
                 launches += 2;                    // fill, blocks
                 advance();
@@ -768,6 +796,25 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     });
 }
 
+// prepare_step(chain, M): what the first decode step of M sequences would do once for all (step_ready), on the current stream; for a caller that
+// takes its steps on another one.  True if those steps take the resident kernel.
+PyObject* prepare_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        if (n != 2) throw std::domain_error("prepare_step takes 2 arguments");
+        auto* c = static_cast<Chain*>(PyCapsule_GetPointer(args[0], "mmf.chain"));
+        if (!c) return nullptr;
+        const int64_t M = PyLong_AsLongLong(args[1]);
+        if (PyErr_Occurred()) return nullptr;
+        const int dev = need_cuda({&c->table});
+        bool ready;
+        {
+            NoGil nogil;
+            ready = step_workspace(*c, M) && step_ready(*c, dev);
+        }
+        return PyBool_FromLong(ready);
+    });
+}
+
 PyObject* take_launches(PyObject*, PyObject*) {
     const int64_t n = g_launches;
     g_launches = 0;
@@ -799,6 +846,7 @@ PyMethodDef methods[] = {
     {"watch", watch, METH_O, nullptr},
     {"unchanged", unchanged, METH_O, nullptr},
     {"chain", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(chain)), METH_FASTCALL, nullptr},
+    {"prepare_step", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(prepare_step)), METH_FASTCALL, nullptr},
     {"chain_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(chain_forward)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "native host path of matmulfreellm_b200", -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -65,6 +65,7 @@ class GreedyDecoder:
         to the device and of the new tokens back are nodes of the same graph."""
         saved = [tuple(s.clone() for s in layer) for layer in self.cache.states]
         saved_ids = self.ids.clone()
+        self.model.prepare_step(self.ids)          # here and not in the warm-up: the copy belongs to the stream that replays the step
         side = torch.cuda.Stream(device=self.device)
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
@@ -101,6 +102,8 @@ class GreedyDecoder:
 
     def _capture_prompt(self, T: int):
         ids = torch.zeros(self.B, T, dtype=torch.int64, device=self.device)
+        if T == 1:                                 # (such a prompt is a step)
+            self.model.prepare_step(ids)
         side = torch.cuda.Stream(device=self.device)
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
@@ -240,7 +243,8 @@ class FusedRunner:
         tail = (self._w32(model.norm.weight), *self._linear(head), lm.lm_head.norm_weight_f32(), float(cfg.rms_norm_eps),
                 float(lm.lm_head.NORM_EPS))
         self._native = _lib.native()
-        self.chain = self._native.chain(model.embeddings.weight, layers, tail)
+        self.resident = bool(lm.resident_step)
+        self.chain = self._native.chain(model.embeddings.weight, layers, tail, self.resident)
         self.watch = self._native.watch(self._slots(lm))
 
     @staticmethod
@@ -261,6 +265,11 @@ class FusedRunner:
             slots = [(m._parameters, n) for m in lm.modules() for n in m._parameters]
             object.__setattr__(lm, "_fused_param_slots", slots)
         return slots
+
+    def prepare_step(self, batch: int) -> bool:
+        """Do now, on the current stream, what the first decode step of `batch` sequences would do once for all: lay the weights out for
+        the resident kernel.  True if those steps take it."""
+        return self._native.prepare_step(self.chain, batch)
 
     def current(self) -> bool:
         """False once a parameter was replaced, cast or modified in place."""
@@ -286,9 +295,9 @@ class FusedRunner:
 
 
 def fused_runner(lm) -> FusedRunner:
-    """The model's cached FusedRunner, rebuilt if any parameter changed since it was made."""
+    """The model's cached FusedRunner, rebuilt if any parameter (or `resident_step`) changed since it was made."""
     r = getattr(lm, "_fused_runner", None)
-    if r is None or not r.current():
+    if r is None or r.resident != lm.resident_step or not r.current():
         r = FusedRunner(lm)
         object.__setattr__(lm, "_fused_runner", r)
     return r

@@ -319,6 +319,16 @@ class HGRNBitForCausalLM(HGRNBitPreTrainedModel):
     # -- fused execution -------------------------------------------------------------------------------------
     fuse = True   # set False to run module by module (same kernels, unfused; used to cross-check the fused chain)
 
+    # Decode steps of up to 16 sequences run all blocks in one kernel where the sizes allow it, which reads a second copy of the blocks' packed
+    # weights (made by the first such step; without memory for it, or with False here, the steps take several kernels per block instead: the
+    # same results)
+    resident_step = True
+
+    def prepare_step(self, input_ids) -> bool:
+        """Make that copy now, on the current stream, if steps with ids like these [B, 1] would.  True if they take the one kernel."""
+        from ...engine import fused_runner
+        return self._can_fuse(input_ids, None, None, None) and fused_runner(self).prepare_step(input_ids.shape[0])
+
     def _can_fuse(self, input_ids, inputs_embeds, attention_mask, output_hidden_states) -> bool:
         if not self.fuse or (input_ids is None) == (inputs_embeds is None):
             return False

@@ -944,3 +944,133 @@ def test_step_that_gave_up_is_reported_by_the_next_call(mm):
         call()
         torch.cuda.synchronize()
         mm.kernels.check_status()
+
+
+def _resident_model(resident=True):
+    """Ten blocks whose packed weights (33 MB) are larger than what the allocator keeps for the scratch of a few tokens."""
+    from mmfreelm.models import HGRNBitConfig, HGRNBitForCausalLM
+    torch.manual_seed(5)
+    with torch.device("cuda"):
+        model = HGRNBitForCausalLM(HGRNBitConfig(vocab_size=1003, hidden_size=1024, num_hidden_layers=10, intermediate_size=2816)).eval()
+    model.pack_weights()
+    model.resident_step = resident
+    return model.bfloat16()
+
+
+def _one_step(model, ids):
+    """(logits, states, kernels launched) of a cached step after a fixed prompt."""
+    from matmulfreellm_b200 import _lib
+    past = model(torch.arange(ids.shape[0] * 3, device="cuda").view(-1, 3), use_cache=True).past_key_values
+    torch.cuda.synchronize()
+    before = _lib.launch_count
+    out = model(input_ids=ids, past_key_values=past, use_cache=True)
+    return out.logits, [s[0].clone() for s in out.past_key_values], _lib.launch_count - before
+
+
+def _same_step(a, b):
+    return torch.equal(a[0], b[0]) and all(torch.equal(x, y) for x, y in zip(a[1], b[1]))
+
+
+def test_second_copy_of_the_weights_is_made_by_the_first_step_that_reads_it(mm):
+    """Prompts, larger batches, two rows of 1024 (which the resident kernel does not take) and a model that was told not to hold no copy."""
+    from matmulfreellm_b200.engine import GreedyDecoder
+    ids = torch.arange(33, device="cuda").view(33, 1)
+    for resident in (False, True):
+        model = _resident_model(resident)
+        copy = sum(m._packed.packed.numel() for n, m in model.named_modules() if hasattr(m, "_packed") and "lm_head" not in n)
+
+        def held(*batches):
+            before = torch.cuda.memory_allocated()
+            for b in batches:
+                _one_step(model, ids[:b])
+            torch.cuda.synchronize()
+            return torch.cuda.memory_allocated() - before >= copy
+
+        model(ids[:2])                                       # the runner
+        assert copy > 30 << 20 and not held(33, 2, 17)
+        assert model.prepare_step(ids[:2]) is False and not held(2)
+        assert held(16) == resident and not held(1, 16, 4)
+        assert model.prepare_step(ids[:1]) is resident
+        steps = [_one_step(model, ids[:b])[2] for b in (1, 16)]
+        assert (max(steps) < 10) == resident and (min(steps) > 40) != resident
+        if resident:                                         # told not to: the copy goes with the runner
+            model.resident_step = False
+            dec = GreedyDecoder(model, 4)
+            dec.prefill(ids[:4])
+            dec.step()
+            assert dec.kernels_per_step > 40
+        del model
+
+
+def test_step_without_memory_for_the_second_copy(mm):
+    """A step that fitted without the copy of the weights still runs where the copy cannot be allocated, with the same results; a model that is
+    told to try again (a new runner) takes the resident kernel."""
+    ids = torch.arange(5, device="cuda").view(5, 1)
+    want = _one_step(_resident_model(False), ids)
+    model = _resident_model()
+    _one_step(model, ids.repeat(5, 1))
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.mem_get_info()[1]
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (24 << 20)) / total)       # the copy takes 33 MB
+    try:
+        got = _one_step(model, ids)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert _same_step(got, want) and got[2] == want[2]
+    again = _one_step(model, ids)                            # (not tried on every step)
+    assert _same_step(again, want) and again[2] == want[2]
+    model.resident_step = False
+    _one_step(model, ids)
+    model.resident_step = True
+    again = _one_step(model, ids)
+    assert _same_step(again, want) and again[2] < want[2]
+
+
+def test_first_step_under_capture(mm):
+    """A step that a user's own graph captures before any other has run: no allocation and no packing become part of the graph."""
+    ids = torch.arange(5, device="cuda").view(5, 1)
+    want = _one_step(_resident_model(False), ids)
+    model = _resident_model()
+    past = model(torch.arange(15, device="cuda").view(5, 3), use_cache=True).past_key_values
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        model(torch.arange(40, device="cuda").view(8, 5))    # this stream's workspace
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        out = model(input_ids=ids, past_key_values=past, use_cache=True)
+    graph.replay()
+    assert torch.equal(out.logits, want[0]) and all(torch.equal(s[0], w) for s, w in zip(out.past_key_values, want[1]))
+    assert _one_step(model, ids)[2] < 10
+
+
+def test_first_steps_of_several_threads(mm):
+    """Threads on streams of their own that all meet a model without the copy: one makes it, and none reads it before it is complete."""
+    import threading
+    ids = torch.arange(16, device="cuda").view(16, 1)
+    want = {B: _one_step(_resident_model(False), ids[:B]) for B in (1, 3, 8, 16)}
+    for _ in range(3):
+        model = _resident_model()
+        model(ids[:3])
+        del model._fused_runner
+        model(ids.repeat(3, 1))                              # a new runner
+        torch.cuda.synchronize()
+        start, wrong = threading.Barrier(4), []
+
+        def thread(B):
+            try:
+                with torch.no_grad(), torch.cuda.stream(torch.cuda.Stream()):
+                    past = model(torch.arange(B * 3, device="cuda").view(-1, 3), use_cache=True).past_key_values
+                    torch.cuda.current_stream().synchronize()
+                    start.wait()
+                    out = model(input_ids=ids[:B], past_key_values=past, use_cache=True)
+                    torch.cuda.current_stream().synchronize()
+                    if not torch.equal(out.logits, want[B][0]): wrong.append(B)
+            except Exception as e:                           # noqa: BLE001 - reported by the assertion below
+                wrong.append((B, repr(e)))
+
+        threads = [threading.Thread(target=thread, args=(B,)) for B in want]
+        for t in threads: t.start()
+        for t in threads: t.join()
+        assert not wrong
