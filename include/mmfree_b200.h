@@ -45,6 +45,7 @@ extern "C" {
 #define MMF_ERR_ARCH (-5)        /* device is not compute capability 10.x                  */
 #define MMF_ERR_WORKSPACE (-6)   /* workspace smaller than mmf_*_workspace_bytes() says    */
 #define MMF_ERR_TIMEOUT (-7)     /* a bounded device-side wait gave up (see status word)   */
+#define MMF_ERR_NOT_RESIDENT (-8) /* a cooperative launch was refused: take another path    */
 
 /* layout constants of the packed ternary weight format (see mmf_pack_ternary) */
 #define MMF_TILE_ROWS 128 /* output rows per weight tile                               */
@@ -388,7 +389,8 @@ typedef struct {
 
 /* 0: the sizes are not taken on the current device. */
 int64_t mmf_decode_step_workspace_bytes(int64_t M, int64_t hidden, int64_t inner, int64_t layers);
-/* A memory fill and a cooperative launch of one CTA per SM. */
+/* A kernel that fills the workspace and a cooperative launch of one CTA per SM.  MMF_ERR_NOT_RESIDENT: the context cannot hold them all at once
+ * (it has fewer SMs than the device); only the workspace has been written then, and the chain of mmf_decode_linear calls does the same. */
 int mmf_decode_step(const mmf_decode_step_args* args, void* stream);
 
 /* ------------------------------------------------------------------------------------

@@ -31,6 +31,7 @@ extern "C" {
 #define MMF_TUNE_PREFILL_SKIP 12 /* persistent large-M kernel, timing only (results are wrong): bit 0 = no activation loads, bit 1 = no weight expansion, bit 2 = no output stores */
 #define MMF_TUNE_ASYNC_REDUCE 10 /* split-K partial sums by st.async + the owner's mbarrier: 1 = on, 2 = off, 0 = library default */
 #define MMF_TUNE_STEP_WAIT_LIMIT 13 /* mmf_decode_step: polls after which a wait for another CTA's words gives up (1: every one that does not find them at once) */
+#define MMF_TUNE_STEP_REFUSE 14 /* mmf_decode_step: 1 = answers as if its cooperative launch had been refused (nothing is launched) */
 int mmf_tuning(int knob, int value);
 
 /* Timeline trace: buffer_dev is a device buffer of at least 8 + 8 * 1000 int64 ([0] = launch counter, then one record of 8

@@ -23,6 +23,7 @@ ERR_CUDA, ERR_TIMEOUT = -4, -7
 _ERR_NAMES = {
     -1: "MMF_ERR_BAD_ARG", -2: "MMF_ERR_BAD_SHAPE", -3: "MMF_ERR_ALIGN", -4: "MMF_ERR_CUDA",
     -5: "MMF_ERR_ARCH", -6: "MMF_ERR_WORKSPACE", -7: "MMF_ERR_TIMEOUT",
+    -8: "MMF_ERR_NOT_RESIDENT",
 }
 
 class DecodeLinearArgs(ctypes.Structure):
@@ -153,7 +154,7 @@ class experiments_library:
     goes to libmmfree_b200_experiments.so (the same sources built with -DMMF_EXPERIMENTS), which also exports
     mmf_tuning; on exit all overrides are reset and the product library is current again."""
 
-    KNOBS = 14
+    KNOBS = 15
     _handle = None
 
     def __enter__(self):

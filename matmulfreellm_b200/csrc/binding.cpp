@@ -734,10 +734,19 @@ PyObject* chain_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 a.workspace = b + step; a.workspace_bytes = step_bytes;
                 a.status = static_cast<int*>(ws.p);
                 a.gave_up_host = dev < 64 ? g_gave_up[dev].load() : nullptr;
-                MMF_CALL(mmf_decode_step, &a, st);
-                launches += 2;                    // fill, blocks
-                advance();
-            } else if (decode) decode_blocks(c, args_of, run, gather, b + z, b + ifg, b + o, b + gu, mk, states, x, next, advance);
+                const int rc = g_api->mmf_decode_step(&a, st);
+                ++launches;                       // fill
+                if (rc == MMF_ERR_NOT_RESIDENT) {       // this context cannot hold it: the chain of kernels, now and from now on
+                    c.step.store(STEP_NEVER, std::memory_order_release);
+                    step_bytes = 0;
+                } else if (rc != MMF_OK) {
+                    throw MmfStatus{"mmf_decode_step", rc, g_api->mmf_last_error()};
+                } else {
+                    ++launches;                   // blocks
+                    advance();
+                }
+            }
+            if (decode && !step_bytes) decode_blocks(c, args_of, run, gather, b + z, b + ifg, b + o, b + gu, mk, states, x, next, advance);
             for (size_t i = 0; i < c.layers.size() && !decode; ++i) {
                 const Layer& L = c.layers[i];
                 if (first) {

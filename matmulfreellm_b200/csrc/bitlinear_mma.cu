@@ -536,7 +536,7 @@ static int g_force_ksplit = 0, g_force_nt = 0, g_force_deep = 0, g_force_wt = 0,
 extern int g_probe_commits;
 extern int g_probe_issuers;
 extern int g_pf_skip;
-extern int g_step_wait_limit;
+extern int g_step_wait_limit, g_step_refuse;
 
 extern "C" int mmf_tuning(int knob, int value) {
     switch (knob) {
@@ -554,6 +554,7 @@ extern "C" int mmf_tuning(int knob, int value) {
         case MMF_TUNE_ACCUMULATORS: g_force_nacc = value; return MMF_OK;
         case MMF_TUNE_ASYNC_REDUCE: g_force_async_red = value; return MMF_OK;
         case MMF_TUNE_STEP_WAIT_LIMIT: g_step_wait_limit = value; return MMF_OK;
+        case MMF_TUNE_STEP_REFUSE: g_step_refuse = value; return MMF_OK;
         default: return mmf_set_error(MMF_ERR_BAD_ARG, "mmf_tuning: unknown knob %d", knob);
     }
 }

@@ -8,6 +8,7 @@ int decode_step_fp16(const DsParams& p, const DsPlan& d, cudaStream_t st);
 
 #ifdef MMF_EXPERIMENTS
 int g_step_wait_limit = 0;     // mmf_tuning(MMF_TUNE_STEP_WAIT_LIMIT, polls)
+int g_step_refuse = 0;         // mmf_tuning(MMF_TUNE_STEP_REFUSE, 1)
 #endif
 
 namespace {

@@ -632,6 +632,11 @@ decode_step_kernel(const __grid_constant__ DsParams p) {
     }
 }
 
+#ifdef MMF_EXPERIMENTS
+}  // namespace
+extern int g_step_refuse;      // mmf_tuning(MMF_TUNE_STEP_REFUSE, 1)
+namespace {
+#endif
 template <auto kernel> int ds_go(const DsParams& p, const DsPlan& d, cudaStream_t st) {
     MMF_CUDA(mmf_allow_smem<kernel>(DS_SMEM_MAX));
     cudaLaunchConfig_t cfg = {};
@@ -644,8 +649,18 @@ template <auto kernel> int ds_go(const DsParams& p, const DsPlan& d, cudaStream_
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    MMF_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
-    MMF_LAUNCH_CHECK("decode_step_kernel");
+#ifdef MMF_EXPERIMENTS
+    const cudaError_t e = g_step_refuse ? cudaErrorCooperativeLaunchTooLarge : cudaLaunchKernelEx(&cfg, kernel, p);
+#else
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
+#endif
+    // A context of fewer SMs than the device has (the attribute counts the device's), or one without cooperative launches: the caller's call
+    // is not lost, the chain of kernels needs no co-residency.
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported) {
+        (void)cudaGetLastError();
+        return mmf_set_error(MMF_ERR_NOT_RESIDENT, "mmf_decode_step: %d CTAs are not resident at once here: %s", d.grid, cudaGetErrorString(e));
+    }
+    MMF_CUDA(e);
     return MMF_OK;
 }
 

@@ -1074,3 +1074,26 @@ def test_first_steps_of_several_threads(mm):
         for t in threads: t.start()
         for t in threads: t.join()
         assert not wrong
+
+
+def test_step_whose_cooperative_launch_is_refused(mm):
+    """Where the context cannot hold all CTAs of the resident kernel (the refusal is answered by the experiments build; nothing is launched) the
+    call runs as the chain of kernels, and so do the later ones of the model, eager and captured."""
+    from matmulfreellm_b200 import _lib
+    from matmulfreellm_b200.engine import GreedyDecoder
+    ids = torch.arange(16, device="cuda").view(16, 1)
+    plain = _resident_model(False)
+    for B in (1, 16):
+        want = _one_step(plain, ids[:B])
+        model = _resident_model()
+        with _lib.experiments_library() as lib:
+            lib.mmf_tuning(14, 1)
+            got = _one_step(model, ids[:B])
+            dec = GreedyDecoder(model, B)
+            dec.prefill(ids[:B])
+            dec.step()
+        assert _same_step(got, want) and got[2] == want[2] + 1           # the fill in front of the refused launch
+        got = _one_step(model, ids[:B])
+        assert _same_step(got, want) and got[2] == want[2]
+        assert dec.kernels_per_step > 40 and model.prepare_step(ids[:B]) is False
+    mm.kernels.check_status()
