@@ -1097,3 +1097,48 @@ def test_step_whose_cooperative_launch_is_refused(mm):
         assert _same_step(got, want) and got[2] == want[2]
         assert dec.kernels_per_step > 40 and model.prepare_step(ids[:B]) is False
     mm.kernels.check_status()
+
+
+@pytest.mark.parametrize("bad_weights", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_resident_decode_step_with_infinities_and_nan(mm, dtype, bad_weights):
+    """The words that CTAs hand to one another say by their value that they have arrived, so no value that a step can form may look like an
+    absent one, which would be waited for in vain.  Embeddings, states and norm weights that are infinite, NaN, as large as the type holds,
+    subnormal or zero: every wait ends, and outputs and states are those of the chain of kernels, NaN for NaN."""
+    from mmfreelm.models import HGRNBitConfig, HGRNBitForCausalLM
+    torch.manual_seed(3)
+    D, inf, nan, top = 640, float("inf"), float("nan"), torch.finfo(dtype).max
+    model = HGRNBitForCausalLM(HGRNBitConfig(vocab_size=40, hidden_size=D, num_hidden_layers=3, intermediate_size=1984)).eval().cuda()
+    model.pack_weights()
+    model = model.to(dtype)
+    special = [inf, -inf, nan, -nan, top, -top, torch.finfo(dtype).smallest_normal / 4, 0.0, -0.0]
+    g = torch.Generator().manual_seed(1)
+    with torch.no_grad():
+        emb = model.model.embeddings.weight
+        for k, v in enumerate(special):
+            emb[k, torch.randperm(D, generator=g)[:3].cuda()] = v        # a few entries of a row, a whole row, a row with all of them
+            emb[10 + k] = v
+        emb[20, :len(special)] = torch.tensor(special, device="cuda").to(dtype)
+        if bad_weights:
+            for k, (n, p) in enumerate((n, p) for n, p in model.named_parameters() if n.endswith("norm.weight")):
+                p[torch.randperm(p.numel(), generator=g)[:2].cuda()] = special[k % len(special)]
+
+    def run(ids, states, resident):
+        model.resident_step = resident
+        past = model.model.init_cache(len(ids))
+        for (s,), v in zip(past.states, states):
+            s.copy_(v.view_as(s))
+        for _ in range(2):
+            out = model(input_ids=ids, past_key_values=past, use_cache=True)
+        mm.kernels.check_status()
+        return [out.logits, *(s[0] for s in past.states)]
+
+    batches = [[k] for k in range(21)] + [[k, k + 10, 30, 20, 31] for k in range(9)] + [list(range(16)), list(range(5, 21))]
+    for rows in batches:
+        ids = torch.tensor(rows, device="cuda").view(-1, 1)
+        states = [torch.randn(len(rows), D, generator=g).cuda() for _ in range(3)]
+        for k, s in enumerate(states):
+            s.view(-1)[k::97] = special[(rows[0] + k) % len(special)]
+        got, want = (run(ids, states, r) for r in (True, False))
+        for a, b in zip(got, want):
+            assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.nan_to_num(7.0), b.nan_to_num(7.0)), rows
