@@ -42,6 +42,10 @@ int mmf_tuning(int knob, int value);
  * (these two stay 0 in a contraction with ready codes), codes complete, products done (row kernel: as before), end. */
 int mmf_row_trace(long long* buffer_dev);
 
+/* Compares the row arithmetic's 1 / sqrt(x) (x >= 0), 127 / x and x / 127 (x >= 1e-5), which are made without the general division and root, with
+ * the IEEE operations over all floats of those ranges: differ_dev[0..2] += the arguments whose results differ (NaN equals NaN). */
+int mmf_rounding_check(unsigned long long* differ_dev, void* stream);
+
 /* Slab-major copy of a packed weight for mmf_bitlinear_decode (experiment; no counterpart in the reference).  The tile-major layout of mmf_pack_ternary keeps a 16-row slab as K/64 pieces of 256 bytes that lie
  * 2 KB apart; the decode kernel fetches whole slabs with one bulk copy each, so it reads a second copy in which slab
  * s (16 rows) of tile t occupies the (K/64)*256 contiguous bytes at ((t*8 + s) * (K/64)) * 256: chunk c at + c*256,

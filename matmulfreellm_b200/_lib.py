@@ -118,6 +118,7 @@ _lib = None
 EXPERIMENTS_LIB_PATH = LIB_PATH.with_name("libmmfree_b200_experiments.so")
 _EXPERIMENT_PROTOTYPES = {
     "mmf_tuning": (c_int, [c_int, c_int]), "mmf_row_trace": (c_int, [c_void_p]),
+    "mmf_rounding_check": (c_int, [c_void_p, c_void_p]),
     "mmf_repack_slabs": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p]),
     "mmf_bitlinear_decode_fits": (c_int, [c_int64, c_int64]),
     "mmf_bitlinear_decode": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int64,

@@ -429,3 +429,29 @@ extern "C" int mmf_sync_probe(int iters, unsigned* scratch_dev, double* barrier_
     rc = chain_us(200, sms, 256, false, scratch_dev + 64, scratch_dev + 128, chain_plain_us_host);
     return rc;
 }
+
+#ifdef MMF_EXPERIMENTS
+// The short forms of the row arithmetic (common.cuh) against the IEEE operations that they stand for, over every float they can be given.
+namespace {
+__global__ void rounding_check_kernel(unsigned long long* differ) {
+    unsigned long long n[3] = {0, 0, 0};
+    auto other = [](float a, float b) { return __float_as_uint(a) != __float_as_uint(b) && !(isnan(a) && isnan(b)); };
+    for (unsigned long long i = blockIdx.x * blockDim.x + threadIdx.x; i <= 0x7fffffffull; i += gridDim.x * blockDim.x) {
+        const float x = __uint_as_float((uint32_t)i);      // not negative; infinity and NaN are among them
+        n[0] += other(rcp_sqrt(x), __fdiv_rn(1.0f, __fsqrt_rn(x)));
+        if (x >= 1e-5f) {
+            n[1] += other(q127_over(x), __fdiv_rn(127.0f, x));
+            n[2] += other(over_127(x), __fdiv_rn(x, 127.0f));
+        }
+    }
+    for (int k = 0; k < 3; ++k)
+        if (n[k]) atomicAdd(differ + k, n[k]);
+}
+}  // namespace
+extern "C" int mmf_rounding_check(unsigned long long* differ_dev, void* stream) {
+    MMF_REQUIRE(differ_dev, MMF_ERR_BAD_ARG, "mmf_rounding_check: null pointer");
+    rounding_check_kernel<<<148 * 8, 256, 0, (cudaStream_t)stream>>>(differ_dev);
+    MMF_LAUNCH_CHECK("rounding_check_kernel");
+    return MMF_OK;
+}
+#endif

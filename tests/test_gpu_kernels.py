@@ -990,3 +990,13 @@ def test_decode_linear_equals_the_separate_kernels(K, dtype, M, D, N, inner):
                 assert all(torch.equal(a, b) for a, b in zip(got, codes_ref))
         torch.cuda.synchronize()
         assert guard.untouched()
+
+
+def test_short_divisions_and_root_are_the_ieee_operations(K):
+    """rcp_sqrt, q127_over and over_127, on which the bit-exact codes and scales of every row kernel rest, for every float of their ranges."""
+    from matmulfreellm_b200 import _lib
+    differ = torch.zeros(3, dtype=torch.int64, device="cuda")
+    with _lib.experiments_library() as lib:
+        assert lib.mmf_rounding_check(differ.data_ptr(), None) == 0
+        torch.cuda.synchronize()
+    assert differ.tolist() == [0, 0, 0]
