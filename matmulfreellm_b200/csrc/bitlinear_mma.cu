@@ -571,7 +571,7 @@ namespace {
 //    what is left after the dependency wait is the activation load, the MMAs and the epilogue;
 //  * "split" (more tokens / few weight tiles): 4 A stages, K split over a cluster when that fills the GPU.
 // The estimate below is a latency model in microseconds fitted to measured phase times of this kernel.
-bool choose_config(const BitLinearArgs& a, MmaParams& best, size_t& best_smem, double& best_cost) {
+bool choose_config(const BitLinearArgs& a, int sms, MmaParams& best, size_t& best_smem, double& best_cost) {
     const int KC = a.K / MMF_TILE_K;
     const int n_tiles = (a.N + MMF_TILE_ROWS - 1) / MMF_TILE_ROWS;
     const int total_stages = (KC + 1) / 2;
@@ -650,7 +650,7 @@ bool choose_config(const BitLinearArgs& a, MmaParams& best, size_t& best_smem, d
                 // (0.30 at 256 token columns), and for a K split the cluster barriers and the push reduction.  More
                 // split than a stand-alone launch would want wins there (measured on the whole step).  Clusters of
                 // 8 with more than 32 token columns no longer fit side by side (measured +6 us).
-                const int64_t waves = (ctas + 148 * occ - 1) / (148 * occ);
+                const int64_t waves = (ctas + sms * occ - 1) / (sms * occ);
                 const double t_stage = mode == 2 ? 0.90 : NT > 128 ? 0.30 : 0.24;   // (two tiles per CTA measured slower: kept for experiments)
                 double t = 2.5 + stages * t_stage + 0.5 + p.wt * NT * 0.012;
                 if (ks > 1) t += 0.75 + 0.22 * ks + NT * 0.012 + (ks == 8 && NT > 32 ? 6.0 : 0.0);   // measured: 1.2 / 1.6 / 2.5 us at 2 / 4 / 8
@@ -675,15 +675,15 @@ int bitlinear_mma_launch(const BitLinearArgs& a, cudaStream_t st) {
         // rows 12.3 / 10.2; N 2048: 1500 rows 12.5 / 10.1; K 5632: 300 rows 13.9 / 14.6, 600 16.9 / 15.0, 1000 17.5 / 16.1, 1500 20.8 / 16.7.
         // Knob values >= 10 select experimental variant (value - 10) and force it for every M > 128.
         const int variant = g_force_persistent >= 10 ? g_force_persistent - 10 : 0;
-        const int nt = bitlinear_mma_prefill_tile(a, variant);
+        const int sms = mmf_sms(), nt = bitlinear_mma_prefill_tile(a, variant, sms);
         const int64_t n_work = (int64_t)((a.N + MMF_TILE_ROWS - 1) / MMF_TILE_ROWS) * ((a.M + nt - 1) / nt);
         const bool tuned = g_force_ksplit || g_force_nt || g_force_deep || g_force_wt || g_force_sb || g_force_sa || g_force_sw;
         const bool choice = g_force_persistent == 0 && !tuned;
-        if ((g_force_persistent == 1 || g_force_persistent >= 10) ? a.M > 128 : (choice && a.M >= 512 && n_work >= 148))
+        if ((g_force_persistent == 1 || g_force_persistent >= 10) ? a.M > 128 : (choice && a.M >= 512 && n_work >= sms))
             return bitlinear_mma_prefill_launch(a, st, variant);
         double us = 0.0;
-        const bool fits = choose_config(a, p, smem, us);
-        if (choice && a.M > 128 && a.K >= 2048 && bitlinear_mma_prefill_us(a) <= 1.05 * us) return bitlinear_mma_prefill_launch(a, st, variant);
+        const bool fits = choose_config(a, sms, p, smem, us);
+        if (choice && a.M > 128 && a.K >= 2048 && bitlinear_mma_prefill_us(a, sms) <= 1.05 * us) return bitlinear_mma_prefill_launch(a, st, variant);
         MMF_REQUIRE(fits, MMF_ERR_BAD_SHAPE, "mmf_bitlinear(mma): no kernel configuration fits M=%d N=%d K=%d", a.M, a.N, a.K);
     }
     const int m_tiles = (a.M + p.NT - 1) / p.NT;

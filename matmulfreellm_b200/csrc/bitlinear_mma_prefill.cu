@@ -654,30 +654,31 @@ bool pf_pairs(const BitLinearArgs& a) {      // every projection is a whole, eve
     const int n_tiles = (a.N + MMF_TILE_ROWS - 1) / MMF_TILE_ROWS;
     return a.N % MMF_TILE_ROWS == 0 && n_tiles % a.groups == 0 && (n_tiles / a.groups) % 2 == 0;
 }
-int pf_rounds(const BitLinearArgs& a, int nt) {
+int pf_rounds(const BitLinearArgs& a, int nt, int sms) {
     const int64_t n_tiles = (a.N + MMF_TILE_ROWS - 1) / MMF_TILE_ROWS, m_tiles = (a.M + nt - 1) / nt;
-    return (int)(pf_pairs(a) ? (n_tiles / 2 * m_tiles + 73) / 74 : (n_tiles * m_tiles + 147) / 148);
+    const int64_t items = pf_pairs(a) ? n_tiles / 2 * m_tiles : n_tiles * m_tiles, units = !pf_pairs(a) ? sms : sms > 1 ? sms / 2 : 1;
+    return (int)((items + units - 1) / units);
 }
 // Time of a few rounds in microseconds: start and first tiles, 128-K stages, and what of the epilogue no other item hides.  Fitted to
 // launches of 129 - 4096 token rows, K = 2048 (16 stages; 192 columns 8.2 / 13.2 / 17.5 / 22.7 us for 1 - 4 rounds, 256 columns 9.4 / 15.7 /
 // 22.3 for 1 - 3) and K = 5632 (44 stages; 14.5 - 16.7 / 27.2 / 36.9 and 17.4 - 19.4 / 32 - 33); within 10 % at 2560 and 6912.
-double pf_us(const BitLinearArgs& a, int nt) {
+double pf_us(const BitLinearArgs& a, int nt, int sms) {
     const double stages = (double)((a.K / MMF_TILE_K + 1) / 2);
-    return 3.6 + pf_rounds(a, nt) * (nt == 192 ? stages * 0.255 + 0.45 : stages * 0.28 + 1.5);
+    return 3.6 + pf_rounds(a, nt, sms) * (nt == 192 ? stages * 0.255 + 0.45 : stages * 0.28 + 1.5);
 }
 
 // Default: the paired shapes where they apply, else the single-CTA shapes.
-int pf_pick(const BitLinearArgs& a, int variant) {
+int pf_pick(const BitLinearArgs& a, int variant, int sms) {
     if (variant) return variant;
     if (!pf_pairs(a)) return a.K >= 4096 ? 1 : 2;
     // Paired shapes with the stmatrix + TMA-store epilogue: the token tile that takes less time by the estimate above.  (K = 5632, 192 /
     // 256 columns: 1000 rows 16.1 / 17.9 us, 2000 25.9 / 19.4, 3000 27.2 / 31.9, 4096 36.9 / 33.3; K = 6912, 4096 rows 44.5 / 54.1; K = 2048, N =
     // 11264: 200 rows 12.8 / 10.7, 300 13.2 / 15.4.)
-    if (a.K >= 4096 || (a.K >= 2048 && pf_rounds(a, 192) <= 6)) return pf_us(a, 256) < pf_us(a, 192) ? 12 : 10;
-    // shorter K and many rounds: 256 columns when their work items fill the 74 CTA pairs' last round clearly better (e.g. N = 2048,
+    if (a.K >= 4096 || (a.K >= 2048 && pf_rounds(a, 192, sms) <= 6)) return pf_us(a, 256, sms) < pf_us(a, 192, sms) ? 12 : 10;
+    // shorter K and many rounds: 256 columns when their work items fill the CTA pairs' last round clearly better (e.g. N = 2048,
     // M = 16384: 512 items = 6.9 rounds against 688 items = 9.3 rounds)
     auto fill = [&](int nt) {
-        const double items = (double)(a.N / MMF_TILE_ROWS / 2) * (double)((a.M + nt - 1) / nt), units = 74.0;
+        const double items = (double)(a.N / MMF_TILE_ROWS / 2) * (double)((a.M + nt - 1) / nt), units = sms / 2;
         const double rounds = (double)(long long)((items + units - 1) / units);
         return items / (rounds * units);
     };
@@ -686,17 +687,17 @@ int pf_pick(const BitLinearArgs& a, int variant) {
 
 }  // namespace
 
-int bitlinear_mma_prefill_tile(const BitLinearArgs& a, int variant) {
-    const int v = pf_pick(a, variant);
+int bitlinear_mma_prefill_tile(const BitLinearArgs& a, int variant, int sms) {
+    const int v = pf_pick(a, variant, sms);
     return v == 2 || v == 3 || v == 6 || v == 7 || v == 8 || v == 10 ? 192 : 256;
 }
 
-double bitlinear_mma_prefill_us(const BitLinearArgs& a) { return pf_us(a, bitlinear_mma_prefill_tile(a, 0)); }
+double bitlinear_mma_prefill_us(const BitLinearArgs& a, int sms) { return pf_us(a, bitlinear_mma_prefill_tile(a, 0, sms), sms); }
 
 // Launch the persistent kernel (large M).  Same argument contract as bitlinear_mma_launch; `variant` selects one
 // of the compiled shapes (0 = by problem shape).
 int bitlinear_mma_prefill_launch(const BitLinearArgs& a, cudaStream_t st, int variant) {
-    switch (pf_pick(a, variant)) {
+    switch (pf_pick(a, variant, mmf_sms())) {
         case 1: return pf_launch<PfLongK>(a, st);
         case 3: return pf_launch<PfOverlapTma>(a, st);
         case 4: return pf_launch<PfSeparate>(a, st);

@@ -98,6 +98,12 @@ inline cudaError_t mmf_sm_count(int* sms) {
     return e;
 }
 
+// The same for grids and estimates: where the runtime does not say (the launch that follows then reports why), a whole B200.
+inline int mmf_sms() {
+    int n = 0;
+    return mmf_sm_count(&n) == cudaSuccess ? n : 148;
+}
+
 // ---------------------------------------------------------------------------------------
 // element conversion (round-to-nearest-even on store, exact on load)
 // ---------------------------------------------------------------------------------------

@@ -345,7 +345,7 @@ warp_gatenorm_quant_kernel(const T* __restrict__ gx, int64_t ld_g, const T* __re
 template <auto kernel, int W, typename... Args>
 int wr_launch(size_t weight_bytes, size_t row_bytes, int64_t M, cudaStream_t st, const char* name, Args... args) {
     MMF_CUDA(mmf_allow_smem<kernel>((int)WR_SMEM_MAX));
-    const int64_t fit = (int64_t)((WR_SMEM_MAX - weight_bytes) / row_bytes), share = (M + 147) / 148;
+    const int64_t fit = (int64_t)((WR_SMEM_MAX - weight_bytes) / row_bytes), sms = mmf_sms(), share = (M + sms - 1) / sms;
     int64_t rows = fit < wr_max_warps(W) / W ? fit : wr_max_warps(W) / W;
     if (share < rows) rows = share;
     MMF_REQUIRE(rows >= 1, MMF_ERR_CUDA, "%s: a row of this length does not fit in shared memory", name);
@@ -353,7 +353,7 @@ int wr_launch(size_t weight_bytes, size_t row_bytes, int64_t M, cudaStream_t st,
     // Short rows leave registers and shared memory for two CTAs, and an SM that the kernel before leaves early would be given two while
     // others get none (12000 rows of 256 values to 1408 outputs 27.4 us, 24.9 with one): more than half of the shared memory each.
     if (share > rows && smem < WR_SMEM_MAX / 2 + 4096) smem = WR_SMEM_MAX / 2 + 4096;
-    MMF_CUDA(mmf_launch_pdl(kernel, dim3((unsigned)(M < 148 ? M : 148)), dim3((unsigned)rows * 32 * W), smem, st, args...));
+    MMF_CUDA(mmf_launch_pdl(kernel, dim3((unsigned)(M < sms ? M : sms)), dim3((unsigned)rows * 32 * W), smem, st, args...));
     MMF_LAUNCH_CHECK(name);
     return MMF_OK;
 }
@@ -363,7 +363,10 @@ constexpr int wr_vectors(int64_t D, int W) { return (int)((D + 512 * W - 1) / (5
 // counts, which is what a pass over 64 values per lane takes.  Prompt passes of 24 blocks, 2048 wide, us with a CTA / one warp / two /
 // four per row: 592 tokens 2475 / 2630 / - / 2528, 700 2581 / 2780 / 2748 / 2565, 999 2957 / 3059 / 3065 / 2901, 1184 - / 3171 / 3208 /
 // 3010; more rows than fit at once, 1600 - / 3573 / 3542 / 3609, 2368 - / 4499 / 4554 / 4557.
-inline bool wr_four(int64_t M, int64_t D) { return D > 512 && D <= 4096 && M > 4 * 148 && M <= 8 * 148; }
+inline bool wr_four(int64_t M, int64_t D) {
+    const int64_t sms = mmf_sms();
+    return D > 512 && D <= 4096 && M > 4 * sms && M <= 8 * sms;
+}
 // run `...` with W bound to the warps per row and NV to the even number of 256 W-value vectors per lane that holds a row of D values
 #define WR_CASE(N, ...) case N: { constexpr int NV = N; __VA_ARGS__; break; }
 #define WR_LAST(N, ...) default: { constexpr int NV = N; __VA_ARGS__; }
