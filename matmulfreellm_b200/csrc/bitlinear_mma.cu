@@ -674,6 +674,8 @@ int bitlinear_mma_launch(const BitLinearArgs& a, cudaStream_t st) {
         // This kernel / persistent, us: K 2048, N 11264: 130 rows 10.9 / 9.4, 300 18.4 / 13.2, 400 21.7 / 14.3; three projections of 2048: 400
         // rows 12.3 / 10.2; N 2048: 1500 rows 12.5 / 10.1; K 5632: 300 rows 13.9 / 14.6, 600 16.9 / 15.0, 1000 17.5 / 16.1, 1500 20.8 / 16.7.
         // Knob values >= 10 select experimental variant (value - 10) and force it for every M > 128.
+        // fp32 outputs, N 2048: 400 rows 8.2 / 9.1; K 5632, 700 rows 16.6 / 15.5; K 6912, 511 rows 19.6 / 17.8.  (There this kernel's estimate for
+        // long K, which is up to a tenth low, would keep it too often.)
         const int variant = g_force_persistent >= 10 ? g_force_persistent - 10 : 0;
         const int sms = mmf_sms(), nt = bitlinear_mma_prefill_tile(a, variant, sms);
         const int64_t n_work = (int64_t)((a.N + MMF_TILE_ROWS - 1) / MMF_TILE_ROWS) * ((a.M + nt - 1) / nt);
@@ -683,7 +685,7 @@ int bitlinear_mma_launch(const BitLinearArgs& a, cudaStream_t st) {
             return bitlinear_mma_prefill_launch(a, st, variant);
         double us = 0.0;
         const bool fits = choose_config(a, sms, p, smem, us);
-        if (choice && a.M > 128 && a.K >= 2048 && bitlinear_mma_prefill_us(a, sms) <= 1.05 * us) return bitlinear_mma_prefill_launch(a, st, variant);
+        if (choice && a.M > 128 && a.K >= 2048 && bitlinear_mma_prefill_us(a, sms) <= (a.out_dtype == MMF_F32 && a.K >= 4096 ? 1.1 : 1.05) * us) return bitlinear_mma_prefill_launch(a, st, variant);
         MMF_REQUIRE(fits, MMF_ERR_BAD_SHAPE, "mmf_bitlinear(mma): no kernel configuration fits M=%d N=%d K=%d", a.M, a.N, a.K);
     }
     const int m_tiles = (a.M + p.NT - 1) / p.NT;

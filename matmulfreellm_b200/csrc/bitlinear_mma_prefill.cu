@@ -556,6 +556,9 @@ static constexpr int g_pf_skip = 0;
 #endif
 namespace {
 
+bool pf_stages_out(const BitLinearArgs& a) {      // 16-bit outputs go through shared memory and leave by TMA (with the accumulators they do not)
+    return a.out_dtype != MMF_F32 && !a.acc_out && mmf_aligned(a.out, 16) && (a.ld_out * 2) % 16 == 0;
+}
 template <typename C>
 int pf_launch(const BitLinearArgs& a, cudaStream_t st) {
     PfParams p;
@@ -588,8 +591,7 @@ int pf_launch(const BitLinearArgs& a, cudaStream_t st) {
     // output map for the staged epilogue: [M][N] rows of ld_out elements, box = one [NT tokens x 128 rows] tile
     CUtensorMap out_map = q_map;
     p.tma_out = 0;
-    // (calls that also want the int32 accumulators take the direct-store epilogue)
-    if (C::STAGE_OUT && a.out_dtype != MMF_F32 && !a.acc_out && mmf_aligned(a.out, 16) && (a.ld_out * 2) % 16 == 0) {
+    if (C::STAGE_OUT && pf_stages_out(a)) {
         const cuuint64_t odim[2] = {(cuuint64_t)a.N, (cuuint64_t)a.M};
         const cuuint64_t ostride[1] = {(cuuint64_t)a.ld_out * 2};
         const cuuint32_t obox[2] = {64u, (cuuint32_t)C::NT};     // one half tile: [NT tokens][64 rows], 128-byte swizzle
@@ -662,9 +664,14 @@ int pf_rounds(const BitLinearArgs& a, int nt, int sms) {
 // Time of a few rounds in microseconds: start and first tiles, 128-K stages, and what of the epilogue no other item hides.  Fitted to
 // launches of 129 - 4096 token rows, K = 2048 (16 stages; 192 columns 8.2 / 13.2 / 17.5 / 22.7 us for 1 - 4 rounds, 256 columns 9.4 / 15.7 /
 // 22.3 for 1 - 3) and K = 5632 (44 stages; 14.5 - 16.7 / 27.2 / 36.9 and 17.4 - 19.4 / 32 - 33); within 10 % at 2560 and 6912.
+// Projections that are not pairs of tiles run the single-CTA shapes, whose times the same line gives: N = 2176, 130 - 1500 rows 8.3 - 9.3, N =
+// 11136 9.0 - 26.8, K = 5632, N = 1920 18.0 - 19.2.  An epilogue that stores from registers (fp32 outputs) costs pairs, which otherwise stage
+// their tiles, a little more with two accumulators and much more with one: N = 2048, 400 rows 8.2 -> 9.0 and 9.5 -> 11.1; N = 11264, 1000 rows
+// 21.8 -> 22.6 and 21.8 -> 28.1, 4096 65.5 -> 73.1 and 65.1 -> 90.4.
 double pf_us(const BitLinearArgs& a, int nt, int sms) {
-    const double stages = (double)((a.K / MMF_TILE_K + 1) / 2);
-    return 3.6 + pf_rounds(a, nt, sms) * (nt == 192 ? stages * 0.255 + 0.45 : stages * 0.28 + 1.5);
+    const double stages = (double)((a.K / MMF_TILE_K + 1) / 2), rounds = pf_rounds(a, nt, sms);
+    const double t = 3.6 + rounds * (nt == 192 ? stages * 0.255 + 0.45 : stages * 0.28 + 1.5);
+    return !pf_pairs(a) || pf_stages_out(a) ? t : t + (nt == 192 ? 0.45 * (rounds + 1) : 2.6 * rounds);
 }
 
 // Default: the paired shapes where they apply, else the single-CTA shapes.
@@ -674,7 +681,10 @@ int pf_pick(const BitLinearArgs& a, int variant, int sms) {
     // Paired shapes with the stmatrix + TMA-store epilogue: the token tile that takes less time by the estimate above.  (K = 5632, 192 /
     // 256 columns: 1000 rows 16.1 / 17.9 us, 2000 25.9 / 19.4, 3000 27.2 / 31.9, 4096 36.9 / 33.3; K = 6912, 4096 rows 44.5 / 54.1; K = 2048, N =
     // 11264: 200 rows 12.8 / 10.7, 300 13.2 / 15.4.)
-    if (a.K >= 4096 || (a.K >= 2048 && pf_rounds(a, 192, sms) <= 6)) return pf_us(a, 256, sms) < pf_us(a, 192, sms) ? 12 : 10;
+    // Stores from registers: at any number of rounds, from K = 1024 on (K = 1088, N = 2048, 4096 rows 15.6 / 14.2 by the next rule / the estimate;
+    // K = 704, N = 256, 16384 rows 10.1 / 10.6).
+    if (a.K >= 4096 || (a.K >= 1024 && !pf_stages_out(a)) || (a.K >= 2048 && pf_rounds(a, 192, sms) <= 6))
+        return pf_us(a, 256, sms) < pf_us(a, 192, sms) ? 12 : 10;
     // shorter K and many rounds: 256 columns when their work items fill the CTA pairs' last round clearly better (e.g. N = 2048,
     // M = 16384: 512 items = 6.9 rounds against 688 items = 9.3 rounds)
     auto fill = [&](int nt) {

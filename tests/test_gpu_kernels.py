@@ -1000,3 +1000,24 @@ def test_short_divisions_and_root_are_the_ieee_operations(K):
         assert lib.mmf_rounding_check(differ.data_ptr(), None) == 0
         torch.cuda.synchronize()
     assert differ.tolist() == [0, 0, 0]
+
+
+@pytest.mark.parametrize("Kd,N,groups", [(1088, 640, 1), (2048, 2048, 1), (2048, 2048, 3), (2048, 384, 1), (2112, 1003, 1), (2560, 13824, 1), (5632, 2048, 1),
+                                         (5632, 1920, 1)])
+def test_bitlinear_of_a_short_prompt_by_the_librarys_own_choice(K, Kd, N, groups):
+    """129 - 1100 rows: which tensor-core kernel and token tile run is decided by estimates, which count rounds of work, the epilogue of the
+    output type and whether projections are pairs of tiles.  Whatever is chosen gives the integers of the CUDA-core kernel."""
+    pw = [K.pack_weight(dev(O.bitlinear_case(1, Kd, N, seed=s)[1])) for s in range(groups)]
+    pw = pw[0] if groups == 1 else K.stack_packed(pw)
+    for M in (129, 192, 193, 256, 257, 384, 385, 511, 512, 1100):
+        x, _, _ = O.bitlinear_case(M, Kd, 1, seed=M)
+        q, dq, rs = K.act_quant(dev(x), None, 1e-6)
+        if groups > 1: q, dq, rs = q.repeat(groups, 1), dq.repeat(groups), rs.repeat(groups)
+        ref, acc_ref = K.bitlinear(q, dq, rs, pw, torch.float32, kernel=K.KERNEL_GEMV, return_acc=True)
+        out, acc = K.bitlinear(q, dq, rs, pw, torch.float32, return_acc=True)
+        assert torch.equal(acc, acc_ref) and torch.equal(out, ref), M
+        for dt in (torch.float32, torch.bfloat16, torch.float16):
+            assert torch.equal(K.bitlinear(q, dq, rs, pw, dt), ref.to(dt)), (M, dt)
+            wide = torch.empty(M, pw.N + 3, dtype=dt, device="cuda")[:, :pw.N]         # rows that TMA cannot store
+            assert torch.equal(K.bitlinear(q, dq, rs, pw, dt, out=wide), ref.to(dt)), (M, dt)
+    K.check_status()
