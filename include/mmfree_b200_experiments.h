@@ -34,12 +34,12 @@ extern "C" {
 #define MMF_TUNE_STEP_REFUSE 14 /* mmf_decode_step: 1 = answers as if its cooperative launch had been refused (nothing is launched) */
 int mmf_tuning(int knob, int value);
 
-/* Timeline trace: buffer_dev is a device buffer of at least 8 + 8 * 1000 int64 ([0] = launch counter, then one record of 8
- * global-timer stamps per launch, taken by thread 0 of CTA 0); NULL switches it off.
- * mmf_prenorm_quant: start, weights staged, grid dependency resolved, row loaded, first row sum done, second norm done, codes
- * written, end.
- * mmf_decode_linear (row kernel and contraction): start, set up, grid dependency resolved, row loaded, last norm's statistic known
- * (these two stay 0 in a contraction with ready codes), codes complete, products done (row kernel: as before), end. */
+/* Timeline trace: buffer_dev is a device buffer of at least 8 + 8 * 1000 int64 ([0] = launch counter, then records of 8 stamps taken by
+ * thread 0 of CTA 0); NULL switches it off.
+ * mmf_prenorm_quant, a record per launch, nanoseconds: start, weights staged, grid dependency resolved, row loaded, first row sum done,
+ * second norm done, codes written, end.
+ * mmf_decode_step, record k is link k of the step, SM clocks: start, weights there, row loaded, first statistic, absmax, codes complete,
+ * products done, end (what CTA 0 does not do in a link stays as it was). */
 int mmf_row_trace(long long* buffer_dev);
 
 /* Compares the row arithmetic's 1 / sqrt(x) (x >= 0), 127 / x and x / 127 (x >= 1e-5), which are made without the general division and root, with

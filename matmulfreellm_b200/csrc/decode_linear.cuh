@@ -53,9 +53,6 @@ struct DlParams {
     int kgw;                            // column groups per warp
     int pf;                             // weight items per warp fetched ahead into shared memory
     int smem_codes, smem_acc, smem_w;   // byte offsets in dynamic shared memory
-#ifdef MMF_EXPERIMENTS
-    long long* trace;
-#endif
 };
 
 // weights unsigned (2-bit fields in place, up to 2 << 6), codes signed
@@ -127,7 +124,7 @@ template <typename T> __device__ __forceinline__ DlVec dl_load(const T* p) {
 // `codes`; a group is 4 * step pieces, a projection KG groups.
 template <typename T, int PRO, int G, int TH, int MR, int NVT>
 __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, const DlRowArgs<T>& ra, int m, int D, int KG, const float* snw, uint8_t* codes,
-                                            int word, int step, DlScratch<TH / MR>& red, float (&s_amax)[G], double inv_d ROW_TRACE_PARAM) {
+                                            int word, int step, DlScratch<TH / MR>& red, float (&s_amax)[G], double inv_d) {
     constexpr int RT = TH / MR;
     const int rt = threadIdx.x % RT, lane = threadIdx.x & 31, rw = rt >> 5;
     const T* x = ra.x;
@@ -162,7 +159,6 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
             }
             if (ro) *reinterpret_cast<uint4*>(ro + c) = make_uint4(o[0], o[1], o[2], o[3]);
         }
-        ROW_TRACE_AFTER(3, s0 + s1);
         const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d0), D, inv_d, ra.eps_norm);
         s0 = s1 = 0.0;
         DL_FOREACH(it, c) {
@@ -182,7 +178,6 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
 #pragma unroll
             for (int i = 0; i < 4; ++i) sumsq_pair<T>(u[it].v[i], s0, s1);
         }
-        ROW_TRACE_AFTER(3, s0 + s1);
         const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d0), D, inv_d, ra.eps_norm);
         s0 = s1 = 0.0;
         DL_FOREACH(it, c) {
@@ -202,11 +197,9 @@ __device__ __forceinline__ void dl_prologue(const mmf_decode_linear_args& a, con
 #pragma unroll
             for (int i = 0; i < 4; ++i) sumsq_pair<T>(u[it].v[i], s0, s1);
         }
-        ROW_TRACE_AFTER(3, s0 + s1);
     }
     // BitLinear prologue: y = (v * rstd) * w, absmax -> scale -> int8 codes
     const float rstd = rstd_from_sumsq(dl_row_sum<TH, RT>(s0 + s1, red.d1), D, inv_d, ra.eps_bl);
-    ROW_TRACE_AFTER(4, (double)rstd);
     float am[G];
 #pragma unroll
     for (int g = 0; g < G; ++g) am[g] = 0.0f;
@@ -269,16 +262,12 @@ __device__ __forceinline__ float dl_out(int acc, int rs, float scale) { return _
 // contraction that follows, 8 * NB tokens side by side.
 template <typename T, int PRO, int TH, int NVT>
 __global__ void __launch_bounds__(TH)
-decode_rows_kernel(const __grid_constant__ mmf_decode_linear_args a, int KG, int NB, double inv_k ROW_TRACE_PARAM) {
+decode_rows_kernel(const __grid_constant__ mmf_decode_linear_args a, int KG, int NB, double inv_k) {
     extern __shared__ __align__(16) uint8_t smem[];
     float* snw = reinterpret_cast<float*>(smem);
     __shared__ DlScratch<TH> red;
     __shared__ float s_amax[1];
     const int m = blockIdx.x, g = blockIdx.y, D = (int)a.K, tid = threadIdx.x;
-#ifdef MMF_EXPERIMENTS
-    trace = row_trace_record(trace);
-#endif
-    ROW_TRACE(0);
     pdl_trigger();
     auto stage = [&](float* dst, const float* src) {
         if (src) for (int i = tid * 4; i < D; i += TH * 4) cp_async16(dst + i, src + i);
@@ -294,13 +283,9 @@ decode_rows_kernel(const __grid_constant__ mmf_decode_linear_args a, int KG, int
     pin(codes); pin(dq); pin(rowsum);
     cp_async_wait_all();
     __syncthreads();
-    ROW_TRACE(1);
     pdl_wait();
-    ROW_TRACE(2);
-    dl_prologue<T, PRO, 1, TH, 1, NVT>(a, ra, m, D, KG, snw, codes, 32, 32 * NB, red, s_amax, inv_k ROW_TRACE_ARG);
+    dl_prologue<T, PRO, 1, TH, 1, NVT>(a, ra, m, D, KG, snw, codes, 32, 32 * NB, red, s_amax, inv_k);
     __syncthreads();
-    ROW_TRACE(5);
-    ROW_TRACE(6);
     if (tid == 0) {
         int t = 0;
 #pragma unroll
@@ -308,7 +293,6 @@ decode_rows_kernel(const __grid_constant__ mmf_decode_linear_args a, int KG, int
         *rowsum = t;
         *dq = over_127(s_amax[0]);
     }
-    ROW_TRACE(7);
 }
 
 // Fused: TH threads, MR token rows (M <= MR), NVT 8-value vectors of a row per thread of the row.  Codes from
@@ -333,10 +317,6 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
     __shared__ int s_rs[G][SC];                              // code sum (weights are stored + 1)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, q = lane & 3;
-#ifdef MMF_EXPERIMENTS
-    long long* trace = row_trace_record(p.trace);
-#endif
-    ROW_TRACE(0);
     pdl_trigger();
     const int bid = blockIdx.x, u0 = bid * p.base + min(bid, p.extra), pairs = p.base + (bid < p.extra ? 1 : 0);
     const int nb = (pairs + BP - 1) / BP * G;                // blocks of this CTA; the last one may be partly empty
@@ -409,9 +389,7 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
     if (has_pre && lb) lb_pre = *reinterpret_cast<const uint32_t*>(lb + (u0 + pr_pre) * 2);
     cp_async_wait_all();
     __syncthreads();
-    ROW_TRACE(1);
     pdl_wait();
-    ROW_TRACE(2);
 
     // gates: the state this thread will advance (and whether its token is padding), on the way during the contraction
     float2 h_pre = make_float2(0.0f, 0.0f);
@@ -423,7 +401,7 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
     if constexpr (FUSED) {
         const int m = tid / RT;
         if (MR == 1 || m < M)
-            dl_prologue<T, PRO, G, TH, MR, NVT>(a, ra, m, D, KG, snw, scodes + m * 64, TL, TL, red[m], s_amax[m], p.inv_k ROW_TRACE_ARG);
+            dl_prologue<T, PRO, G, TH, MR, NVT>(a, ra, m, D, KG, snw, scodes + m * 64, TL, TL, red[m], s_amax[m], p.inv_k);
         __syncthreads();                                     // codes complete
         if (has_const) {
             int t = 0;
@@ -439,7 +417,6 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
         }
     }
 
-    ROW_TRACE(5);
 
     // the 2-bit fields stay where they are: field f of a byte counts 4^f, one accumulator per field, shifted back at the end
     if (CONST8 ? kq < KG : bq < bw) {
@@ -494,7 +471,6 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
         }
     }
     __syncthreads();
-    ROW_TRACE(6);
 
     // ---- epilogue: a thread finishes two adjacent rows (channels) of a token
     for (int i = tid; i < pairs * M; i += nthr) {
@@ -555,7 +531,6 @@ decode_linear_kernel(const __grid_constant__ DlParams p) {
             *reinterpret_cast<uint32_t*>(g_out + (int64_t)m * D + ch) = value(unit * 3 + 2, r, 2);
         }
     }
-    ROW_TRACE(7);
 }
 
 constexpr int DL_SMEM_MAX = 220 * 1024;
@@ -569,7 +544,7 @@ template <auto kernel> int dl_go(const DlParams& p, int threads, int smem, cudaS
 
 template <typename T, int PRO, int TH, int NVT> int dl_rows_go(const mmf_decode_linear_args& a, int G, int KG, int NB, cudaStream_t st) {
     MMF_CUDA(mmf_launch_pdl(decode_rows_kernel<T, PRO, TH, NVT>, dim3((unsigned)a.M, (unsigned)G), dim3(TH),
-                            (size_t)(PRO == MMF_PRO_QUANT ? 1 : 2) * a.K * 4, st, a, KG, NB, 1.0 / (double)a.K ROW_TRACE_BUFFER));
+                            (size_t)(PRO == MMF_PRO_QUANT ? 1 : 2) * a.K * 4, st, a, KG, NB, 1.0 / (double)a.K));
     MMF_LAUNCH_CHECK("decode_rows_kernel");
     return MMF_OK;
 }
@@ -590,9 +565,6 @@ template <typename T, int PRO> int dl_rows(const mmf_decode_linear_args& a, int 
 template <typename T> int decode_linear_launch(const mmf_decode_linear_args& a, cudaStream_t st) {
     DlParams p;
     p.a = a;
-#ifdef MMF_EXPERIMENTS
-    p.trace = g_row_trace;
-#endif
     p.KC = (int)(a.K / MMF_TILE_K);
     p.KG = (p.KC + 3) / 4;
     p.inv_k = 1.0 / (double)a.K;

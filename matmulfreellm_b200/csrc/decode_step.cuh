@@ -43,9 +43,6 @@ __device__ __forceinline__ uint4 ds_ld(const void* p) {
     return v;
 }
 __device__ __forceinline__ void ds_st(void* p, uint32_t v) { asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
-__device__ __forceinline__ void ds_st(void* p, uint2 v) {
-    asm volatile("st.relaxed.gpu.global.v2.b32 [%0], {%1, %2};" ::"l"(p), "r"(v.x), "r"(v.y) : "memory");
-}
 __device__ __forceinline__ bool ds_there(uint4 v, uint32_t none) { return v.x != none && v.y != none && v.z != none && v.w != none; }
 __device__ __forceinline__ uint32_t ds_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

@@ -2,8 +2,7 @@
 #pragma once
 #include "common.cuh"
 
-// Timeline of the row kernels and of the decode step's BitLinear (experiments build, see mmf_row_trace): thread 0 of CTA 0 takes a
-// record of eight stamps per launch.
+// Timeline of prenorm_quant (experiments build, see mmf_row_trace): thread 0 of CTA 0 takes a record of eight stamps per launch.
 #ifdef MMF_EXPERIMENTS
 extern long long* g_row_trace;
 __device__ __forceinline__ long long* row_trace_record(long long* buffer) {
@@ -17,16 +16,8 @@ __device__ __forceinline__ long long row_now() {
     return t;
 }
 #define ROW_TRACE(slot) do { if (trace) trace[slot] = row_now(); } while (0)
-#define ROW_TRACE_AFTER(slot, value) do { asm volatile("" ::"d"(value)); ROW_TRACE(slot); } while (0)   // once `value` is formed
-#define ROW_TRACE_PARAM , long long* trace
-#define ROW_TRACE_ARG , trace
-#define ROW_TRACE_BUFFER , g_row_trace
 #else
 #define ROW_TRACE(slot) do { } while (0)
-#define ROW_TRACE_AFTER(slot, value) do { } while (0)
-#define ROW_TRACE_PARAM
-#define ROW_TRACE_ARG
-#define ROW_TRACE_BUFFER
 #endif
 
 struct PrenormArgs {
