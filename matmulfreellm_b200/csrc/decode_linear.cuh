@@ -1,5 +1,5 @@
 // BitLinear of a decode step in one kernel: row work before the contraction (prologue), the contraction, and what the next
-// kernel would do first (epilogue).  Steps whose sizes the resident kernel of all blocks takes (decode_step.cuh: 1 row 305 us, 4 rows 443) run
+// kernel would do first (epilogue).  Steps whose sizes the resident kernel of all blocks takes (decode_step.cuh: 1 row 304 us, 4 rows 454) run
 // there; here run the others, and BitLinear calls of one and two rows.
 //
 // A decode step is a chain of dependent kernels, so its time is the number of links times what a link cannot go below: a

@@ -5,7 +5,7 @@
 // (decode_linear.cuh) a link of one row takes 4.3 us, of which 1.6 are the hand-over: the boundary and the first read across the L2.
 // Here an epilogue stores its outputs as they are and the next link's readers poll them: a 32-bit word of a row cannot be two 0xffff (no
 // rounding produces that NaN), of codes not four times -128 (codes are -127 .. 127), so a word that differs from the fill has arrived and
-// needs no flag, fence or counter.  Every word is written once per step; a memory fill before the kernel makes them all absent.
+// needs no flag, fence or counter.  Every word is written once per step; a kernel in front makes them all absent.
 //
 // The exchange alone (148 CTAs, each stores 28 bytes and reads 4 KB): 0.7 us if the first look comes 400 - 600 clocks after the stores,
 // 2.0 us if at once, because polls of all SMs for the same lines queue in front of the stores.  What a link prepares (weights unpacked
@@ -20,8 +20,8 @@
 // shorter with more warps.  So: one copy of the code for all four links (unrolled per link it was 120 KB, beyond every instruction cache,
 // and a step took 674 us; code that leaves the 32 KB cache by branches costs up to twice the time), fp64 sums by the tensor core, the three
 // IEEE roundings of the row arithmetic without the general division, operand pairs of the codes stored side by side.
-// Step of a 24-block, 2048-wide model, kernels / this: 1 row 434 -> 304 us, 2 rows 500 -> 429, 4 rows 534 -> 443, 8 rows 530 -> 467, 16 rows
-// 663 -> 561; 32 blocks of 2560: 1 row 688 -> 577, 4 rows 831 -> 701, 8 rows 831 -> 738.
+// Step of a 24-block, 2048-wide model, kernels / this, in turn in one process: 1 row 413 / 304 us, 2 rows 478 / 440, 4 rows 516 / 454, 8 rows
+// 516 / 465, 9 rows 622 / 518, 16 rows 655 / 559; 32 blocks of 2560: 1 row 666 / 560, 2 rows 804 / 689, 4 rows 814 / 711, 8 rows 816 / 736.
 #pragma once
 #include "decode_linear.cuh"
 #include "decode_step_plan.cuh"
@@ -187,7 +187,7 @@ template <typename T> __device__ __forceinline__ uint32_t ds_add16(uint32_t a, u
 // hands the codes round; the contraction is split the same way.  A thread holds 8 columns of a hidden row (NW * 256 >= hidden), up to
 // three times 8 of an inner row.  FUSED: the weights of a warp's first PRE (block, column group) items are unpacked into registers while
 // the row is on its way (unpacking is two thirds of a product's time: 2.2 k clocks of a block; in the other form the code grew out of the
-// instruction cache: 494 us against 452 at eight rows).
+// instruction cache: a tenth slower at eight rows).
 template <typename T, int MR, bool FUSED, int NW, int PRE>
 __global__ void __launch_bounds__(NW * 32, 1)
 decode_step_kernel(const __grid_constant__ DsParams p) {

@@ -55,7 +55,7 @@ inline DsPlan ds_plan(DsParams& p, int64_t M, int64_t h, int64_t inner, int64_t 
         inner < MMF_TILE_K || inner % MMF_TILE_K || inner > 8192)
         return d;
     // One row: every CTA repeats its row work.  More: a CTA per row and projection does it and hands the codes round, which costs a second
-    // exchange per link (two rows of 2048: 429 us a step, 457 with the row work repeated; four: 443 and 1170).
+    // exchange per link (two rows of 2048: 429 us a step and 457 with the row work repeated, in turn; four: 443 and 1170).
     d.fused = M == 1;
     const int mr = d.fused ? 1 : M <= 8 ? 8 : 16;
     if (!d.fused && 3 * M > sms) return d;
