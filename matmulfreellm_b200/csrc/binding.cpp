@@ -170,9 +170,7 @@ void make_gave_up_word(int dev) {
     const std::lock_guard<std::mutex> hold(lock);
     if (dev >= 64 || g_gave_up[dev].load()) return;
     const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);      // (allocating is no part of a capture under way)
-    static std::vector<at::Tensor> keep;
-    keep.push_back(at::zeros({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true)));
-    g_gave_up[dev] = keep.back().data_ptr<int>();
+    g_gave_up[dev] = (new at::Tensor(at::zeros({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true))))->data_ptr<int>();
 }
 bool take_gave_up_word(int dev) {
     volatile int* w = dev >= 0 && dev < 64 ? g_gave_up[dev].load() : nullptr;

@@ -60,12 +60,16 @@ class GreedyDecoder:
         latent = {id(m.weight) for m in layers}
         return [(m._packed, m._norm_w32, m._norm_seen) for m in layers] + [p.detach() for p in model.parameters() if id(p) not in latent]
 
+    def _prepare_step(self) -> None:
+        if hasattr(self.model, "prepare_step"):    # (a model of the caller's own need not have it)
+            self.model.prepare_step(self.ids)
+
     def _capture(self, ids_host: Optional[torch.Tensor] = None, out_host: Optional[torch.Tensor] = None):
         """Capture one decode step; returns (graph, its logits buffer, what it reads).  With pinned host buffers the copy of the input ids
         to the device and of the new tokens back are nodes of the same graph."""
         saved = [tuple(s.clone() for s in layer) for layer in self.cache.states]
         saved_ids = self.ids.clone()
-        self.model.prepare_step(self.ids)          # here and not in the warm-up: the copy belongs to the stream that replays the step
+        self._prepare_step()                       # here and not in the warm-up: the copy belongs to the stream that replays the step
         side = torch.cuda.Stream(device=self.device)
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
@@ -103,7 +107,7 @@ class GreedyDecoder:
     def _capture_prompt(self, T: int):
         ids = torch.zeros(self.B, T, dtype=torch.int64, device=self.device)
         if T == 1:                                 # (such a prompt is a step)
-            self.model.prepare_step(ids)
+            self._prepare_step()
         side = torch.cuda.Stream(device=self.device)
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):

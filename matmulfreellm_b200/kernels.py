@@ -205,6 +205,11 @@ def _rezero_workspaces() -> None:
 
 def _after_failure(e: _lib.MMFreeError) -> None:
     """After a native call failed: clear the workspaces unless its arguments were refused, when nothing was launched."""
+    if e.code == _lib.ERR_TIMEOUT:       # a step gave up: it may still be ending, and would report itself once more
+        for device in {ws.device for ws in list(_ws_cache.values()) + _ws_retired}:
+            if not torch.cuda.is_current_stream_capturing():
+                torch.cuda.synchronize(device)
+        _lib.native().take_gave_up()
     if e.code in (_lib.ERR_CUDA, _lib.ERR_TIMEOUT):
         _rezero_workspaces()
 

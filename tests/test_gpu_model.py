@@ -1011,12 +1011,17 @@ def test_step_without_memory_for_the_second_copy(mm):
     _one_step(model, ids.repeat(5, 1))
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
-    total = torch.cuda.mem_get_info()[1]
-    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (24 << 20)) / total)       # the copy takes 33 MB
+    total, held = torch.cuda.mem_get_info()[1], []
     try:
+        torch.cuda.set_per_process_memory_fraction(torch.cuda.memory_reserved() / total)
+        with pytest.raises(torch.OutOfMemoryError):          # no hole that earlier tests left is as large as the copy (33 MB)
+            while True:
+                held.append(torch.empty(16 << 20, dtype=torch.uint8, device="cuda"))
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (24 << 20)) / total)
         got = _one_step(model, ids)
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
+        del held
     assert _same_step(got, want) and got[2] == want[2]
     again = _one_step(model, ids)                            # (not tried on every step)
     assert _same_step(again, want) and again[2] == want[2]

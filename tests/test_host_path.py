@@ -102,6 +102,9 @@ def test_a_step_that_gave_up_clears_the_workspaces(monkeypatch):
 
         chain_forward = check_gave_up
 
+        def take_gave_up(self):
+            pass
+
     cleared = []
     monkeypatch.setattr(kernels, "_rezero_workspaces", lambda: cleared.append(1))
     monkeypatch.setattr(_lib, "native", GaveUp)
